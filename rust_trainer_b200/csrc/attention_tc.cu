@@ -106,7 +106,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* pv_done = bars + 14;
   uint32_t* tmem_slot = (uint32_t*)(bars + 16);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // the last query tiles of a sequence see the most keys: start them first
   const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * BM, h = blockIdx.y, g = h / (nh / nkv);
   const int kbeg = seq_start[m0];
@@ -143,7 +143,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
 
   if (warp == 4) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(q_full, L::Q_BYTES);
       for (int p = 0; p < L::PAN; ++p) tma_load_2d(sm + L::OFF_Q + p * L::Q_PANEL, &tm_q, h * HD + p * 64, m0, q_full);
       for (int n = 0; n < ntiles; ++n) {
@@ -162,7 +162,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------ MMA issue (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(0, 0, 0, 0, BM, BN);   // S: A, B K-major, N = 64 keys
       const uint32_t idesc_o = umma_idesc(0, 0, 0, 1, BM, HD);   // O: A K-major (P), B MN-major (V), N = hd
       const uint32_t sQ = smem_u32(sm + L::OFF_Q), sK = smem_u32(sm + L::OFF_K), sV = smem_u32(sm + L::OFF_V), sP = smem_u32(sm + L::OFF_P);
@@ -438,7 +438,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   uint32_t* tmem_slot = (uint32_t*)(bars + 14);
   constexpr int NS = L::NS;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * 128, g = blockIdx.y, group = nh / nkv;
   // queries that can see these keys: [n0, end of the sequence holding the tile's last key)
   const int last_key = min(n0 + 128, M) - 1;
@@ -483,7 +483,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 
   if (warp == BWD_TMA_WARP) {
     // ------------------------------------------------------------ producer: TMA + the per-query vectors
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * L::KV_BYTES);
       for (int p = 0; p < L::PAN; ++p) {
         tma_load_2d(sm + L::OFF_K + p * L::KV_PANEL, &tm_k, g * HD + p * 64, n0, kv_full);
@@ -497,7 +497,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       if (lane == 0) ok = mbar_wait(&q_free[b], (((uint32_t)(it / NS)) & 1) ^ 1, status, SITE_B_QFREE);
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_expect_tx(&q_full[b], 2 * L::Q_BYTES);
         for (int p = 0; p < L::PAN; ++p) {
           tma_load_2d(sm + L::OFF_Q + b * L::Q_BYTES + p * L::Q_PANEL, &tm_q, h * HD + p * 64, m0, &q_full[b]);
@@ -524,7 +524,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     }
   } else if (warp == BWD_MMA_WARP) {
     // ------------------------------------------------------------ MMA issue (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(0, 0, 0, 0, 128, BQ);
       const uint32_t idesc_g = umma_idesc(0, 0, 0, 1, 128, HD);
       const uint32_t sK = smem_u32(sm + L::OFF_K), sV = smem_u32(sm + L::OFF_V), sQ = smem_u32(sm + L::OFF_Q);
@@ -752,7 +752,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint64_t* dq_done = bars + 18;
   uint32_t* tmem_slot = (uint32_t*)(bars + 20);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // the last query tiles of a sequence see the most keys: start them first
   const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * BM, h = blockIdx.y, g = h / (nh / nkv);
   const int kbeg = seq_start[m0];
@@ -792,7 +792,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   AT_STAMP_Q(511);
 
   if (warp == BWD_TMA_WARP) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(qdo_full, 2 * L::Q_BYTES);
       for (int p = 0; p < L::PAN; ++p) {
         tma_load_2d(sm + L::OFF_Q + p * L::Q_PANEL, &tm_q, h * HD + p * 64, m0, qdo_full);
@@ -813,7 +813,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
     }
   } else if (warp == BWD_MMA_WARP) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(0, 0, 0, 0, BM, BN);
       const uint32_t idesc_g = umma_idesc(0, 0, 0, 1, BM, HD);
       const uint32_t sQ = smem_u32(sm + L::OFF_Q), sDO = smem_u32(sm + L::OFF_DO), sK = smem_u32(sm + L::OFF_K);

@@ -59,7 +59,7 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
   uint32_t* tmem_slot = (uint32_t*)(bars + 3 * LG_NS + 2);
   __shared__ float s_red[4];
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const bool isB = (int)blockIdx.x < g.nbB;
   const CUtensorMap* tm_p = isB ? &tm_pb : &tm_pa;
   const CUtensorMap* tm_q = isB ? &tm_qb : &tm_qa;
@@ -91,7 +91,7 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
 
   if (warp == 4 || warp >= 6) {
     // three producer threads, one TMA instruction per stage each (an instruction costs its thread about 0.1 us)
-    if (lane == 0) {
+    if (elect_one()) {
       const int which = warp == 4 ? 0 : warp - 5;  // 0, 1: the two 64-column panels of Big; 2: the Small tile
       for (int ch = 0; ch < nchunks; ++ch) {
         const int s = ch % LG_NS;
@@ -103,7 +103,7 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc(0, 0, 1, 1, 128, 64);
       const uint32_t s0 = smem_u32(sm);
       bool ok = true;

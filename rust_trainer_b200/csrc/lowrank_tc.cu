@@ -57,7 +57,7 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * LR_NS + 2);
   pdl_launch_dependents();
   if (threadIdx.x == 0) LR_STAMP(0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * LR_TN;
   const int nk = (K + 63) / 64;
 
@@ -84,7 +84,7 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 
   if (warp == 4 || warp == 3) {
     // two producer threads (one TMA instruction costs its thread about 0.1 us): X tiles and factor tiles
-    if (lane == 0) {
+    if (elect_one()) {
       const bool xs = warp == 4;
       for (int kc = 0; kc < nk; ++kc) {
         const int s = kc % LR_NS;
@@ -101,7 +101,7 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       if (xs) LR_STAMP(3);
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = umma_idesc(0, 0, 0, 0, 128, LR_TN);
       const uint32_t s0 = smem_u32(sm);
       bool ok = true;

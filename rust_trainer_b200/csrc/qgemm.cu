@@ -304,7 +304,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   uint32_t* tmem_slot = (uint32_t*)(bars + C::N_BARS);
   pdl_launch_dependents();
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 #ifdef RT_B200_QPROF
 #define QG_STAMP(i) do { if (p.prof && blockIdx.x == 0) p.prof[512 * 24 + (i)] = (long long)globaltimer_ns(); } while (0)
 #else
@@ -514,7 +514,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
 
   if (role == R_PROD) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       QG_PROF_BEGIN();
@@ -569,7 +569,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     tail_helper(warp >> 2, warp - 4);
   } else if (role == R_MMA) {
     // ------------------------------------------------------------ MMA issue (the leader's thread only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       uint32_t tcount = 0, itg = 0;
       bool it_first = true;
       int st = 0;        // stage ring position and its phase, advanced without divisions
@@ -725,7 +725,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     // ------------------------------------------------------------ packed-brick producer
     // Runs ahead of the stage ring: a brick pair is fetched as soon as its slot in the raw ring
     // is free, so its latency is not added to the time a weight stage is held.
-    if (lane == 0 && !is16 && !QDBG(p, 16)) {
+    if (!is16 && !QDBG(p, 16) && elect_one()) {
       uint32_t rit = 0;
       bool ok = true;
       QG_PROF_BEGIN();
