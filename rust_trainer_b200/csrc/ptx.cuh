@@ -53,18 +53,6 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity
       : "memory");
   return ok;
 }
-// the same with acquire at cluster scope: for a barrier that threads of the peer CTA arrive on
-__device__ __forceinline__ uint32_t mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok;
-}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -74,21 +62,25 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // seconds).  The bound counts this SM's own cycle counter, which nothing outside the kernel can
 // step or re-synchronise.
 constexpr long long MBAR_WAIT_LIMIT_CYCLES = 4000000000ll;
-template <bool CLUSTER = false>
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
-                                          long long limit_cycles = MBAR_WAIT_LIMIT_CYCLES) {
-  if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+// The spin is a function of its own: inlined at every wait it made the loops of the single-thread
+// roles long and branchy (the instruction fetches and branch resolutions of one iteration, not the
+// work in it, set the pace of the matmul's pipeline).
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, int* status, int code, long long limit_cycles) {
   const long long t0 = clock64();
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 256; ++i)
-      if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+      if (mbar_try_wait(bar, parity)) return true;
     if (clock64() - t0 > limit_cycles) {
       atomicCAS(status, 0, code);
       return false;
     }
     if (*(volatile int*)status != 0) return false;  // another role already gave up
   }
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
+                                          long long limit_cycles = MBAR_WAIT_LIMIT_CYCLES) {
+  return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, status, code, limit_cycles);
 }
 
 // ---------------------------------------------------------------- CTA pairs (cluster of 2)

@@ -15,7 +15,7 @@
 // pair (2p, 2p+1) in the two halves of a 32-bit register.
 //
 //   Q4_0 : [128 x 16 B codes][128 x f16 d]                                   2304 B
-//   Q8_0 : [128 x 32 B codes+128][128 x f16 d]                               4352 B
+//   Q8_0 : [128 x 16 B codes+128, first half][128 x 16 B, second half][128 x f16 d]  4352 B
 //   Q4_K : [128 x 16 B codes][64 x (f16 d, f16 dmin)][128 x (u8 sc, u8 m)]   2560 B
 //   Q6_K : [128 x 16 B low4][128 x 8 B high2][128 x 2 x i8 sc][64 x f16 d]   3456 B
 //
@@ -48,7 +48,7 @@ __host__ __device__ inline int fmt_block_bytes(int fmt) {
     default: return 0;
   }
 }
-__host__ __device__ inline int fmt_brick_bytes(int fmt) {
+__host__ __device__ constexpr int fmt_brick_bytes(int fmt) {
   switch (fmt) {
     case GGML_Q4_0: return 2304;
     case GGML_Q8_0: return 4352;
@@ -56,6 +56,14 @@ __host__ __device__ inline int fmt_brick_bytes(int fmt) {
     case GGML_Q6_K: return 3456;
     default: return 0;
   }
+}
+
+// Where the two high bits of a 6-bit code stand in the 32-bit word that holds them for 16 codes (code
+// words `word` even and odd, pair p, half hi): the word rotated right by 0 or 8 (even, pairs 0-1 or
+// 2-3), 2 or 10 (odd) shows them at bits 4-5 of an even pair's halves and 8-9 of an odd pair's, right
+// above the low nibble that the unpacker extracts in place.
+__host__ __device__ inline int q6k_hi_pos(int word, int p, int hi) {
+  return (((p & 1) ? 8 : 4) + 16 * hi + ((word & 1) ? 2 : 0) + (p < 2 ? 0 : 8)) & 31;
 }
 
 struct QWeight {
@@ -93,7 +101,7 @@ __device__ inline float brick_value(const QWeight& w, int r, int k) {
       return __fmul_rn((float)(q - 8), d);
     }
     case GGML_Q8_0: {
-      int q = (int)b[t * 32 + e] - 128;
+      int q = (int)b[(e >> 4) * 2048 + t * 16 + (e & 15)] - 128;
       float d = __half2float(((const __half*)(b + 4096))[t]);
       return __fmul_rn((float)q, d);
     }
@@ -108,8 +116,7 @@ __device__ inline float brick_value(const QWeight& w, int r, int k) {
     case GGML_Q6_K: {
       uint32_t lo = ((const uint32_t*)(b + t * 16))[word];
       uint32_t hw = ((const uint32_t*)(b + 2048 + t * 8))[word >> 1];
-      if (word & 1) hw = __funnelshift_r(hw, hw, 8);
-      int q = ((lo >> (4 * field)) & 15) | (((hw >> (2 * p + 16 * hi)) & 0x30));
+      int q = ((lo >> (4 * field)) & 15) | (((hw >> q6k_hi_pos(word, p, hi)) & 3) << 4);
       float d = __half2float(((const __half*)(b + 3328))[rr]);
       float sc = (float)((const int8_t*)(b + 3072))[t * 2 + (e >> 4)];
       return __fmul_rn(__fmul_rn(d, sc), (float)(q - 32));

@@ -43,13 +43,13 @@ __global__ void repack_kernel(const uint8_t* __restrict__ raw, QWeight w) {
     ((uint16_t*)(b + 2048))[t] = d;
   } else if (w.fmt == GGML_Q8_0) {
     uint16_t d = 0;
-    uint8_t* dst = b + t * 32;
+    uint8_t* dst = b + t * 16;  // codes 16.. of the unit go to the second plane, 2048 bytes on
     if (inside) {
       const uint8_t* blk = raw + ((size_t)r * (w.cols / 32) + ku) * 34;
       d = blk[0] | (blk[1] << 8);
-      for (int i = 0; i < 32; ++i) dst[i] = blk[2 + i] ^ 0x80;  // int8 -> offset-128 unsigned
+      for (int i = 0; i < 32; ++i) dst[(i >> 4) * 2048 + (i & 15)] = blk[2 + i] ^ 0x80;  // int8 -> offset-128 unsigned
     } else {
-      for (int i = 0; i < 32; ++i) dst[i] = 0x80;
+      for (int i = 0; i < 32; ++i) dst[(i >> 4) * 2048 + (i & 15)] = 0x80;
     }
     ((uint16_t*)(b + 4096))[t] = d;
   } else if (w.fmt == GGML_Q4_K) {
@@ -113,9 +113,7 @@ __global__ void repack_kernel(const uint8_t* __restrict__ raw, QWeight w) {
         for (int hi = 0; hi < 2; ++hi) {
           int c = code[wd * 8 + 2 * p + hi];
           u |= (uint32_t)(c & 15) << (4 * p + 16 * hi);
-          int pos = 4 + 2 * p + 16 * hi;
-          if (wd & 1) pos = (pos + 8) & 31;
-          H[wd >> 1] |= (uint32_t)(c >> 4) << pos;
+          H[wd >> 1] |= (uint32_t)(c >> 4) << q6k_hi_pos(wd, p, hi);
         }
       }
       dlo[wd] = u;
