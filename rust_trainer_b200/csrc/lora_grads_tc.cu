@@ -14,8 +14,11 @@
 // dY arrives row-normalised with one factor per token.  The factors go onto the Small rows
 // relative to the split's largest factor (rounded up to a power of two, so what a row rounds to
 // does not depend on its split mates), and the largest factor multiplies the split's sums.
-// Partial sums of the splits are added in order by the reduce kernels of lora_kernels.cu:
-// deterministic, no atomics.
+// Up to eight splits (every batch of up to 8192 tokens) are one cluster: each CTA leaves its split's sums in
+// shared memory, and the CTAs add them in split order straight into the gradient buffers, each its
+// share of the tile.  (A second launch used to do that from partial sums in memory: 2.6 us per linear
+// and 6.1 per group, 0.5 ms of a 1024-token step.)  More splits go through memory and the reduce
+// kernels of lora_kernels.cu.  Deterministic either way, no atomics.
 #include "ctx.h"
 #include "ops.h"
 #include "pdl.cuh"
@@ -41,7 +44,18 @@ struct LoraGradTcArgs {
   int M, N, K, r, nbB, tps;
   float* partB;  // [splits][r x N]
   float* partA;  // [splits][r x K]
+  int direct;       // the splits are one cluster: add into the members' gradients
+  LoraGroupTable t; // of one linear (offsets 0) or of a stacked group
 };
+// sums of a split, [rank index][128 columns + 1] f32, over the operand stages once those are used up
+constexpr int LG_PITCH = 129;
+static_assert(64 * LG_PITCH * 4 <= (int)(LG_NS * LG_STAGE), "the sums fit over the stages");
+
+__device__ __forceinline__ float ld_cluster_f1(uint32_t cluster_addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
 
 __global__ void __launch_bounds__(256, 2)
 lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_constant__ CUtensorMap tm_qb,
@@ -177,7 +191,12 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
       if (g.r > 32) tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + 32, v + 32);
       tmem_ld_wait();
       const int j = j0 + warp * 32 + lane;
-      if (j < C) {
+      if (g.direct) {
+        float* mine = (float*)sm + warp * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i < g.r) mine[i * LG_PITCH] = __uint_as_float(v[i]) * out_mul;
+      } else if (j < C) {
         float* dst = (isB ? g.partB : g.partA) + (size_t)blockIdx.y * g.r * C + j;
 #pragma unroll
         for (int i = 0; i < 64; ++i)
@@ -189,7 +208,36 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
     for (int k = 0; k < 1000; ++k) __nanosleep(1000);
   }
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if (g.direct && gridDim.y > 1) cluster_sync_all();  // every split's sums are in its CTA's shared memory
+  else __syncthreads();
+  if (g.direct && *(volatile int*)status == 0) {
+    const int n_cta = (int)gridDim.y, ncol = min(128, C - j0);
+    auto add_splits = [&](int i, int col, float* dst) {
+      const uint32_t a = smem_u32(sm) + (uint32_t)(i * LG_PITCH + col) * 4u;
+      float x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k < n_cta) x[k] = n_cta > 1 ? ld_cluster_f1(mapa_u32(a, (uint32_t)k)) : ((const float*)sm)[i * LG_PITCH + col];
+      float sum = x[0];
+#pragma unroll
+      for (int k = 1; k < 8; ++k)
+        if (k < n_cta) sum += x[k];
+      *dst += sum;  // nobody else adds to it
+    };
+    for (int q = 0; q < g.t.n; ++q) {
+      const LoraGroupMember& mb = g.t.m[q];
+      // a member owns whole column tiles of dB (its rows start on a multiple of 128) and r rows of dA
+      if (isB && (j0 < mb.row_off || j0 >= mb.row_off + mb.rows)) continue;
+      const int items = ncol * mb.r, per = (items + n_cta - 1) / n_cta, end = min(items, ((int)blockIdx.y + 1) * per);
+      for (int e = (int)blockIdx.y * per + threadIdx.x; e < end; e += 256) {
+        if (isB) add_splits(mb.rank_off + e % mb.r, e / mb.r, mb.gb + (size_t)(j0 - mb.row_off) * mb.r + e);
+        else add_splits(mb.rank_off + e / ncol, e % ncol, mb.ga + (size_t)(e / ncol) * g.K + j0 + e % ncol);
+      }
+    }
+  }
+  __syncwarp();
+  if (g.direct && gridDim.y > 1) cluster_sync_all();  // nobody leaves while its shared memory may still be read
   if (warp == 5) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 64);
@@ -199,12 +247,19 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
 }  // namespace
 
 // Tokens per split of the tcgen05 contraction: fixed by the token count's range only.
-int lora_grads_tc_tokens_per_split(int M) { return M >= 4096 ? 1024 : M >= 1024 ? 256 : M >= 512 ? 128 : 64; }
+int lora_grads_tc_tokens_per_split(int M) { return M >= 4096 ? 1024 : M >= 2048 ? 512 : M >= 1024 ? 256 : M >= 512 ? 128 : 64; }
+// whether the splits fit one cluster (of the portable size), which then adds them itself
+bool lora_grads_tc_direct(int M) {
+  const int tps = lora_grads_tc_tokens_per_split(M);
+  return (M + tps - 1) / tps <= 8;
+}
 
-// Launches the product kernel only (the caller adds the splits).  partB / partA: [splits][r x N] / [splits][r x K]
-// with splits = ceil(M / lora_grads_tc_tokens_per_split(M)).  0: launched; 1: shape not covered; 3: launch failure.
+// Up to eight splits: adds dB and dA into the gradients of the table's members, which is all there is to
+// do.  More: launches the product kernel only and leaves partial sums, partB / partA: [splits][r x N] /
+// [splits][r x K] with splits = ceil(M / lora_grads_tc_tokens_per_split(M)), for the caller to add.
+// 0: launched; 1: shape not covered; 3: launch failure.
 int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy, const __half* gs, const __half* x16,
-                         const float* dscale, int M, int N, int K, int r, float* partB, float* partA) {
+                         const float* dscale, int M, int N, int K, int r, const LoraGroupTable& t, float* partB, float* partA) {
   if (M <= 0) return 0;
   if (r <= 0 || r > 64 || N % 8 != 0 || K % 8 != 0 || ld_dy % 8 != 0) return 1;
   if (((uintptr_t)hs | (uintptr_t)dy16 | (uintptr_t)gs | (uintptr_t)x16) & 15) return 1;
@@ -226,8 +281,23 @@ int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld
   g.partB = partB;
   g.partA = partA;
   const int splits = (M + g.tps - 1) / g.tps;
-  dim3 grid(g.nbB + (K + 127) / 128, splits);
-  pdl(lora_grads_tc_kernel, grid, 256, LG_TOTAL, c->stream)(tpb, tqb, tpa, tqa, g, c->status_dev);
+  g.direct = lora_grads_tc_direct(M) ? 1 : 0;
+  g.t = t;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1;
+  at[1].val.clusterDim.y = (unsigned)splits;
+  at[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(g.nbB + (K + 127) / 128), (unsigned)splits);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = LG_TOTAL;
+  cfg.stream = c->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = g.direct && splits > 1 ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, lora_grads_tc_kernel, tpb, tqb, tpa, tqa, g, c->status_dev) != cudaSuccess) return 3;
   RT_COUNT_LAUNCH(1);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }

@@ -156,8 +156,6 @@ __global__ void tok_reduce_kernel(const float* __restrict__ part, int splits, in
 // C = K); grid.y is the token split.  The per-token factors of dY are applied to the rows of the
 // skinny operand relative to the LARGEST FACTOR OF THE SPLIT (found by the block itself), and
 // that maximum multiplies the split's partial sums, so no pass over all factors comes first.
-struct LoraGroupMember { float *gb, *ga; int row_off, rows, rank_off, r; };
-struct LoraGroupTable { int n; LoraGroupMember m[3]; };
 struct LoraGradArgs {
   const __half *Pb, *Qb, *Pa, *Qa;  // Hs, dY, Gs, X
   const float* pscale;              // per-token factors of dY, or null
@@ -376,8 +374,12 @@ int launch_lora_grads(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy
     const int tps_tc = lora_grads_tc_tokens_per_split(M), splits_tc = (M + tps_tc - 1) / tps_tc;
     float* pB = workspace;
     float* pA = workspace + (size_t)splits_tc * r * N;
-    const int rc = launch_lora_grads_tc(c, hs, dy16, ld_dy, gs, x16, dscale, M, N, K, r, pB, pA);
+    LoraGroupTable t;
+    t.n = 1;
+    t.m[0] = LoraGroupMember{gb, ga, 0, N, 0, r};
+    const int rc = launch_lora_grads_tc(c, hs, dy16, ld_dy, gs, x16, dscale, M, N, K, r, t, pB, pA);
     if (rc == 3) return 3;
+    if (rc == 0 && lora_grads_tc_direct(M)) return 0;
     if (rc == 0) {
       const size_t n = (size_t)r * ((size_t)N + (size_t)K);
       pdl(lora_grads_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, st)(pB, pA, splits_tc, N, K, r, gb, ga);
@@ -421,21 +423,22 @@ int launch_lora_grads_group(rt_ctx* c, const __half* hs, const __half* dy16, con
                             cudaStream_t st) {
   if (M <= 0 || n <= 0) return 0;
   if (n > 3 || R <= 0 || R > 64 || NT % 8 != 0 || K % 8 != 0) return 1;
+  LoraGroupTable t;
+  t.n = n;
+  size_t total = 0;  // gradient elements
+  for (int j = 0; j < n; ++j) {
+    t.m[j] = LoraGroupMember{gb[j], ga[j], row_off[j], rows[j], rank_off[j], rank[j]};
+    total += (size_t)rank[j] * ((size_t)rows[j] + (size_t)K);
+  }
   int tps, splits;
   {
     const int tps_tc = lora_grads_tc_tokens_per_split(M), splits_tc = (M + tps_tc - 1) / tps_tc;
     float* pB = workspace;
     float* pA = workspace + (size_t)splits_tc * R * NT;
-    const int rc = launch_lora_grads_tc(c, hs, dy16, NT, gs, x16, dscale, M, NT, K, R, pB, pA);
+    const int rc = launch_lora_grads_tc(c, hs, dy16, NT, gs, x16, dscale, M, NT, K, R, t, pB, pA);
     if (rc == 3) return 3;
+    if (rc == 0 && lora_grads_tc_direct(M)) return 0;
     if (rc == 0) {
-      LoraGroupTable t;
-      t.n = n;
-      size_t total = 0;
-      for (int j = 0; j < n; ++j) {
-        t.m[j] = LoraGroupMember{gb[j], ga[j], row_off[j], rows[j], rank_off[j], rank[j]};
-        total += (size_t)rank[j] * ((size_t)rows[j] + (size_t)K);
-      }
       pdl(lora_grads_group_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, st)(pB, pA, splits_tc, NT, K, R, t);
       RT_COUNT_LAUNCH(1);
       return cudaGetLastError() == cudaSuccess ? 0 : 3;
@@ -463,13 +466,6 @@ int launch_lora_grads_group(rt_ctx* c, const __half* hs, const __half* dy16, con
   if (R <= 16) lora_grads_kernel<1><<<grid, 128, TOK_SMEM, st>>>(g);
   else if (R <= 32) lora_grads_kernel<2><<<grid, 128, TOK_SMEM, st>>>(g);
   else lora_grads_kernel<4><<<grid, 128, TOK_SMEM, st>>>(g);
-  LoraGroupTable t;
-  t.n = n;
-  size_t total = 0;
-  for (int j = 0; j < n; ++j) {
-    t.m[j] = LoraGroupMember{gb[j], ga[j], row_off[j], rows[j], rank_off[j], rank[j]};
-    total += (size_t)rank[j] * ((size_t)rows[j] + (size_t)K);
-  }
   pdl(lora_grads_group_reduce_kernel, (unsigned)((total + 255) / 256), 256, 0, st)(g.partB, g.partA, splits, NT, K, R, t);
   RT_COUNT_LAUNCH(2);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;

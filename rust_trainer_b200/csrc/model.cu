@@ -112,7 +112,7 @@ rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out) 
 }
 
 rt_status linear_forward_dev(rt_linear* l, LinearScratch& sc, const __half* x16, int M, void* y, int y_dtype,
-                             int accumulate, __half* hs_keep, bool hs_ready) {
+                             int accumulate, __half* hs_keep, bool hs_ready, const float* residual) {
   rt_ctx* c = l->ctx;
   if (M <= 0) return RT_OK;
   QGemmArgs a;
@@ -123,6 +123,7 @@ rt_status linear_forward_dev(rt_linear* l, LinearScratch& sc, const __half* x16,
   a.out = y;
   a.out_dtype = y_dtype;
   a.accumulate = accumulate;
+  a.residual = residual;
   a.bias = l->bias;
   if (l->lora_active()) {
     lora_refresh(l);
@@ -1164,8 +1165,8 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   if (attn_forward(c, A.q16, A.k16, A.v16, m->seq_start.as<int>(), m->staged_gap ? m->gap.as<int>() : nullptr, M, g.n_heads,
                    g.n_kv_heads, g.head_dim, A.o16, A.lse))
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
-  if (h != x_in) RT_CUDA(c, cudaMemcpyAsync(h, x_in, (size_t)M * d * 4, cudaMemcpyDeviceToDevice, st));
-  RT_TRY(linear_forward_dev(b.lin[3], m->lsc, A.o16, M, h, RT_DT_F32, 1, keep ? A.hs[3] : nullptr, hs_ready));
+  // the residual comes in where the product goes out: in place, or from the buffer that keeps it
+  RT_TRY(linear_forward_dev(b.lin[3], m->lsc, A.o16, M, h, RT_DT_F32, h == x_in, keep ? A.hs[3] : nullptr, hs_ready, h == x_in ? nullptr : x_in));
   launch_rmsnorm_fwd(h, b.post_norm, M, d, g.rms_eps, A.n2, st);
   if (A.gu_group) {
     RT_TRY(group_forward_dev(b.gu, m->lsc, A.n2, M, A.g16, RT_DT_F16, keep ? A.hs[4] : nullptr, hs_ready));
@@ -1175,8 +1176,7 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   }
   launch_swiglu_fwd(A.g16, A.u16, A.gu_pitch, M, g.ff, A.hm16, c->status_dev, st);
   if (x_out) {
-    if (x_out != h) RT_CUDA(c, cudaMemcpyAsync(x_out, h, (size_t)M * d * 4, cudaMemcpyDeviceToDevice, st));
-    RT_TRY(linear_forward_dev(b.lin[6], m->lsc, A.hm16, M, x_out, RT_DT_F32, 1, keep ? A.hs[6] : nullptr, hs_ready));
+    RT_TRY(linear_forward_dev(b.lin[6], m->lsc, A.hm16, M, x_out, RT_DT_F32, x_out == h, keep ? A.hs[6] : nullptr, hs_ready, x_out == h ? nullptr : h));
   } else if (keep && !hs_ready && b.lin[6]->lora_active()) {
     RT_TRY(linear_lora_h(b.lin[6], A.hm16, M, A.hs[6]));  // the backward needs it
   }
@@ -1355,13 +1355,16 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
   const rt_model_config& g = m->cfg;
   const size_t xd = (size_t)M * g.hidden;
   float* x = m->x.as<float>();
-  launch_gather_rows(m->embed->w, m->tokens.as<int>(), M, x, c->status_dev, st);
+  // A training pass writes every block's input where the backward will look for it; a forward-only
+  // pass keeps one residual stream in place.
+  float* ckpt = m->ckpt.as<float>();
+  launch_gather_rows(m->embed->w, m->tokens.as<int>(), M, backward ? ckpt : x, c->status_dev, st);
   const bool store = backward && m->store_acts;
   for (int li = 0; li < g.n_layers; ++li) {
-    if (backward) RT_CUDA(c, cudaMemcpyAsync(m->ckpt.as<float>() + (size_t)li * xd, x, xd * 4, cudaMemcpyDeviceToDevice, st));
     const BlockActs A = block_acts(m, li, M, store);
-    if (store) RT_TRY(block_forward(m, li, M, m->ckpt.as<float>() + (size_t)li * xd, A.h, x, A, 1));  // keeps h and every Hs
-    else RT_TRY(block_forward(m, li, M, x, x, x, A, backward ? 1 : 0));  // a training pass keeps every Hs for the second forward
+    // a training pass keeps every Hs, for the backward and for the second forward of a recomputed block
+    if (backward) RT_TRY(block_forward(m, li, M, ckpt + (size_t)li * xd, A.h, li + 1 < g.n_layers ? ckpt + (size_t)(li + 1) * xd : x, A, 1));
+    else RT_TRY(block_forward(m, li, M, x, x, x, A, 0));
   }
   if (backward) RT_CUDA(c, cudaMemsetAsync(m->dx.p, 0, xd * 4, st));
   if (n_targets > 0) RT_TRY(model_head(m, M, n_targets, backward, logits_out_host));

@@ -77,10 +77,21 @@ void launch_global_normalize(const float* x, size_t n, float* amax_dev, __half* 
 int launch_lowrank_tc(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64);
 size_t tok_contract_workspace_floats(int M, int C, int r);
 size_t lora_grads_workspace_floats(int M, int N, int K, int r);
-// lora_grads_tc.cu: the product kernel on tcgen05 (partial sums per split of lora_grads_tc_tokens_per_split(M) tokens)
+// A linear's (or a stacked group's) adapters as the token contractions see them: member j owns rows
+// rank_off..+r of the rank axis and columns row_off..+rows of dY.
+struct LoraGroupMember {
+  float *gb, *ga;
+  int row_off, rows, rank_off, r;
+};
+struct LoraGroupTable {
+  LoraGroupMember m[3];
+  int n;
+};
+// lora_grads_tc.cu: the product kernel on tcgen05 (splits of lora_grads_tc_tokens_per_split(M) tokens)
 int lora_grads_tc_tokens_per_split(int M);
+bool lora_grads_tc_direct(int M);
 int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy, const __half* gs, const __half* x16,
-                         const float* dscale, int M, int N, int K, int r, float* partB, float* partA);
+                         const float* dscale, int M, int N, int K, int r, const LoraGroupTable& t, float* partB, float* partA);
 int launch_lora_grads_group(rt_ctx* c, const __half* hs, const __half* dy16, const __half* gs, const __half* x16, const float* dscale,
                             int M, int NT, int K, int R, int n, float* const* gb, float* const* ga, const int* row_off,
                             const int* rows, const int* rank_off, const int* rank, float* workspace, cudaStream_t st);

@@ -92,6 +92,7 @@ struct KParams {
   void* out;
   int out_dtype, accumulate, ld_out;
   const float* row_scale;  // optional per-token factor applied to the result
+  const float* residual;   // optional f32 matrix laid out as `out` that the result is added to
   const float* bias;
   uint32_t idesc;
   int* status;
@@ -388,7 +389,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   // bytes per token.  (f32 blocks used to go through two 4 KB staging buffers and TMA: the store of
   // the block before last had to be read out first, and the 4096x1024 product at 8192 tokens
   // waited for its epilogue, 73 us; its stores knocked out it ran in 61.)
+  // The epilogue warps share their schedulers with the unpack warps, so what counts is the number of
+  // instructions per value: whole blocks take straight-line code without a test per value (with one,
+  // the same product took 135 us).
   auto direct_chunk = [&](int acc, int wq, int c, int r0, int m0, int split) {
+    if (m0 + c * 32 >= p.M) return;
     uint32_t v[32];
     tmem_ld32(tmem_base + acc * 256 + ((uint32_t)(wq * 32) << 16) + c * 32, v);
     const int tok0 = m0 + c * 32, row = r0 + wq * 32 + lane;
@@ -404,29 +409,51 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * __shfl_sync(0xffffffffu, rs_lane, j));
     }
     if (!row_ok) return;
-    if (fin_out && p.out_dtype != OUT_F32) {
-      const size_t base = (size_t)tok0 * p.ld_out + row;
+    const size_t ld = fin_out ? (size_t)p.ld_out : (size_t)p.out_rows;
+    const size_t base = fin_out ? (size_t)tok0 * ld + row : ((size_t)split * p.M + tok0) * ld + row;
+    float* o = (fin_out ? (float*)p.out : p.part) + base;
+    if (nvalid == 32 && (!fin_out || p.out_dtype == OUT_F32)) {
+      if (fin_out && p.residual) {
+        const float* res = p.residual + base;
+#pragma unroll
+        for (int q = 0; q < 32; q += 8) {  // eight loads in flight: what the registers have room for
+          float old[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j, res += ld) old[j] = *res;
+#pragma unroll
+          for (int j = 0; j < 8; ++j, o += ld) *o = __uint_as_float(v[q + j]) + bias_v + old[j];
+        }
+      } else if (fin_out && p.accumulate) {  // each element receives exactly one addition per launch
+#pragma unroll
+        for (int j = 0; j < 32; ++j, o += ld) atomicAdd(o, __uint_as_float(v[j]) + bias_v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j, o += ld) *o = __uint_as_float(v[j]) + bias_v;
+      }
+      return;
+    }
+    if (!fin_out || p.out_dtype == OUT_F32) {  // the ragged last block of a batch
+      const bool add = fin_out && p.accumulate;
+      const float* res = fin_out && p.residual ? p.residual + base : nullptr;
 #pragma unroll
       for (int j = 0; j < 32; ++j)
         if (j < nvalid) {
-          const float val = __uint_as_float(v[j]) + bias_v;
-          const size_t idx = base + (size_t)j * p.ld_out;
-          if (p.out_dtype == OUT_BF16) ((__nv_bfloat16*)p.out)[idx] = __float2bfloat16_rn(val);
-          else ((__half*)p.out)[idx] = __float2half_rn(val);
+          float val = __uint_as_float(v[j]) + bias_v;
+          if (res) val += res[(size_t)j * ld];
+          if (add) atomicAdd(o + (size_t)j * ld, val);
+          else o[(size_t)j * ld] = val;
         }
       return;
     }
-    const size_t ld = fin_out ? (size_t)p.ld_out : (size_t)p.out_rows;
-    float* o = fin_out ? (float*)p.out + (size_t)tok0 * ld + row : p.part + ((size_t)split * p.M + tok0) * ld + row;
-    if (fin_out && p.accumulate) {  // each element receives exactly one addition per launch
+    // 16-bit outputs TMA cannot address
+    __half* o16 = (__half*)p.out + base;
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < nvalid) atomicAdd(o + (size_t)j * ld, __uint_as_float(v[j]) + bias_v);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < nvalid) o[(size_t)j * ld] = __uint_as_float(v[j]) + bias_v;
-    }
+    for (int j = 0; j < 32; ++j)
+      if (j < nvalid) {
+        const float val = __uint_as_float(v[j]) + bias_v;
+        if (p.out_dtype == OUT_BF16) ((__nv_bfloat16*)o16)[(size_t)j * ld] = __float2bfloat16_rn(val);
+        else o16[(size_t)j * ld] = __float2half_rn(val);
+      }
   };
   // The epilogue of a CTA's LAST tile has nothing to hide behind, so the warps whose own work
   // is over by then help: every warp with residue q (mod 4) may read TMEM lane quarter q.
@@ -728,7 +755,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int M, int R, float* __restrict__ out,
                                      size_t s_tok, size_t s_row, const float* __restrict__ row_scale,
                                      const float* __restrict__ alpha_dev, const float* __restrict__ bias,
-                                     int accumulate) {
+                                     int accumulate, const float* __restrict__ residual) {
   pdl_entry();
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = (size_t)M * R;
@@ -741,6 +768,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
   if (bias) v += bias[row];
   float* o = out + tok * s_tok + row * s_row;
   if (accumulate) v += *o;
+  if (residual) v += residual[tok * s_tok + row * s_row];
   *o = v;
 }
 
@@ -954,7 +982,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   const int out_rows = a.dir == QG_FWD ? w.rows : w.cols;
   if ((!a.tok_mode && contract % 8 != 0) || (is16 && w.cols % 8 != 0)) return RT_ERR_BAD_SHAPE;
   if (a.tok_mode && (!is16 || a.dir != QG_BWD || a.M > 64 || a.lora.rank > 0 || a.out_dtype != OUT_F32)) return RT_ERR_BAD_ARG;
-  if (a.accumulate && a.out_dtype != OUT_F32) return RT_ERR_BAD_ARG;
+  if ((a.accumulate || a.residual) && a.out_dtype != OUT_F32) return RT_ERR_BAD_ARG;
   if (a.lora.rank > 64 || (a.lora.rank > 0 && (!a.lora.act || !a.lora.w))) return RT_ERR_BAD_ARG;
 
   KParams p;
@@ -965,6 +993,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   p.conv16 = (w.fmt == GGML_F16 && !a.act_f16) ? 1 : (w.fmt == GGML_BF16 && a.act_f16) ? 2 : 0;
   const int kfmt = !is16 ? w.fmt : p.conv16 ? QF_16CONV : QF_16;
   p.row_scale = a.row_scale;
+  p.residual = a.residual;
   p.dir = a.dir;
   p.out_rows = out_rows;
   p.M = a.M;
@@ -1086,7 +1115,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     const size_t n = (size_t)a.M * out_rows;
     const size_t s_tok = a.tok_mode ? a.out_s_tok : (size_t)p.ld_out, s_row = a.tok_mode ? a.out_s_row : 1;
     pdl(splitk_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, st)(p.part, p.n_splits, a.M, out_rows, (float*)a.out, s_tok,
-                                                                    s_row, a.row_scale, a.alpha_dev, p.bias, a.accumulate);
+                                                                    s_row, a.row_scale, a.alpha_dev, p.bias, a.accumulate, a.residual);
     RT_COUNT_LAUNCH(1);
   }
   if (e1) {
@@ -1094,7 +1123,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     const double out_bytes = a.out_dtype == OUT_F32 ? 4.0 : 2.0;
     ctx->prof_flops += 2.0 * (double)a.M * (double)w.rows * (double)w.cols;
     ctx->prof_recs.push_back({a.tok_mode ? 3 : (a.aux ? 2 : a.dir), a.M, out_rows, contract});
-    ctx->prof_bytes += (double)w.dev_nbytes + 2.0 * (double)a.M * contract + out_bytes * (double)a.M * out_rows * (a.accumulate ? 2.0 : 1.0);
+    ctx->prof_bytes += (double)w.dev_nbytes + 2.0 * (double)a.M * contract + out_bytes * (double)a.M * out_rows * (a.accumulate || a.residual ? 2.0 : 1.0);
   }
   return cudaGetLastError() == cudaSuccess ? RT_OK : RT_ERR_CUDA;
 }

@@ -50,6 +50,7 @@ struct QGemmArgs {
   void* out = nullptr;                 // forward: Y [M x N]; backward: dX [M x K]
   int out_dtype = OUT_F32;
   int accumulate = 0;                  // out += result (f32 only)
+  const float* residual = nullptr;     // out = residual + result (f32 only; laid out as out, and not out itself)
   int ld_out = 0;                      // row pitch of out in elements (0: the output width)
   const float* bias = nullptr;         // forward only, per output feature
   const float* row_scale = nullptr;    // optional per-token factor on the result (before bias)
