@@ -95,7 +95,7 @@ rt_status rt_ctx_create(int device, rt_ctx** out) {
   if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->status_dev, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the clear ran on the legacy stream; own_stream does not wait for it
-  if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, sizeof(int));
+  if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, 2 * sizeof(int));
   if (e != cudaSuccess || rt::qgemm_init() != RT_OK) {
     fprintf(stderr, "rt_b200: context creation failed: %s\n", cudaGetErrorString(e));
     delete c;

@@ -13,7 +13,7 @@ struct rt_ctx {
   cudaStream_t stream = nullptr;       // the stream in use (own_stream unless the host set one)
   cudaStream_t own_stream = nullptr;
   int* status_dev = nullptr;   // device word the kernels report bounded-wait failures into
-  int* status_host = nullptr;  // pinned mirror
+  int* status_host = nullptr;  // pinned: the mirror of that word, then one word for a scalar result
   std::string err;
   uint64_t launches = 0;       // kernels launched through this ctx
   bool profiling = false;

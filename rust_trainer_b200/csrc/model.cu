@@ -29,6 +29,21 @@ void DevBuf::release() {
   bytes = 0;
 }
 
+bool PinnedBuf::reserve(size_t want) {
+  if (want <= bytes) return true;
+  if (p) cudaFreeHost(p);
+  p = nullptr;
+  bytes = 0;
+  if (cudaMallocHost(&p, want + want / 4) != cudaSuccess) return false;
+  bytes = want + want / 4;
+  return true;
+}
+void PinnedBuf::release() {
+  if (p) cudaFreeHost(p);
+  p = nullptr;
+  bytes = 0;
+}
+
 #define RT_TRY(expr)          \
   do {                        \
     rt_status s__ = (expr);   \
@@ -671,16 +686,18 @@ void rt_model_destroy(rt_model* m) {
   if (m->embed) rt_frozen_destroy(m->embed);
   for (void* p : m->owned) cudaFree(p);
   DevBuf* bufs[] = {&m->P, &m->G, &m->Mo, &m->Vo, &m->opt_scalars, &m->inv_freq, &m->rope_cos, &m->rope_sin,
-                    &m->lsc.hs, &m->lsc.gs, &m->lsc.hs2, &m->lsc.gs2, &m->lsc.smax, &m->lsc.grad_ws, &m->tokens, &m->pos, &m->seq_start, &m->x, &m->ckpt, &m->h,
+                    &m->lsc.hs, &m->lsc.gs, &m->lsc.hs2, &m->lsc.gs2, &m->lsc.smax, &m->lsc.grad_ws, &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
                     &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw, &m->q16, &m->k16, &m->v16, &m->o16, &m->lse,
                     &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16, &m->sc_y, &m->dhm, &m->dg16, &m->du16,
                     &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->amax, &m->dq, &m->dk, &m->dv, &m->dq16, &m->dk16,
-                    &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->tpos, &m->ttok, &m->tw, &m->logp, &m->hits, &m->xs,
+                    &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs,
                     &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) b->release();
   for (int i = 0; i < 7; ++i) m->hs_keep[i].release();
-  m->gap.release();
   m->argmax.release();
+  m->h_batch.release();
+  m->h_results.release();
+  if (m->batch_sent) cudaEventDestroy(m->batch_sent);
   for (auto& ge : m->graphs) cudaGraphExecDestroy(ge.exec);
   delete m;
 }
@@ -1032,7 +1049,6 @@ static bool ensure_tokens(rt_model* m, int M) {
   }
   const size_t L = m->store_acts ? (size_t)g.n_layers : 1;
   bool ok = true;
-  ok &= m->tokens.reserve(T * 4) && m->pos.reserve(T * 4) && m->seq_start.reserve(T * 4);
   ok &= m->x.reserve(T * d * 4) && m->ckpt.reserve(T * d * 4 * g.n_layers) && m->h.reserve(T * d * 4 * L);
   ok &= m->n1.reserve(T * d * 2 * L) && m->n2.reserve(T * d * 2 * L);
   ok &= m->q_raw.reserve(T * (qd + 2 * kvd) * 4 * L);  // q | k | v before RoPE
@@ -1096,8 +1112,7 @@ static bool ensure_targets(rt_model* m, int n, bool backward) {
   const rt_model_config& g = m->cfg;
   bool ok = true;
   if (n > m->cap_targets) {
-    ok &= m->tpos.reserve((size_t)n * 4) && m->ttok.reserve((size_t)n * 4) && m->tw.reserve((size_t)n * 4) &&
-          m->logp.reserve((size_t)n * 4) && m->hits.reserve(16);
+    ok &= m->results.reserve(16 + (size_t)n * 4) && m->h_results.reserve(16 + (size_t)n * 4);
     if (ok) m->cap_targets = n;
   }
   const int R = n < g.head_rows ? n : g.head_rows;
@@ -1160,9 +1175,9 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
     RT_TRY(linear_forward_dev(b.lin[2], m->lsc, A.n1, M, A.v_raw, RT_DT_F32, 0, keep ? A.hs[2] : nullptr, hs_ready));
   }
   launch_qk_rope_fwd(A.q_raw, A.k_raw, A.v_raw, A.qkv_pitch, g.qk_norm ? b.q_norm : nullptr,
-                     g.qk_norm ? b.k_norm : nullptr, m->pos.as<int>(), m->rope_cos.as<float>(), m->rope_sin.as<float>(), M,
+                     g.qk_norm ? b.k_norm : nullptr, m->pos, m->rope_cos.as<float>(), m->rope_sin.as<float>(), M,
                      g.n_heads, g.n_kv_heads, g.head_dim, g.rot_dim, g.rope_neox, g.rms_eps, A.q16, A.k16, A.v16, st);
-  if (attn_forward(c, A.q16, A.k16, A.v16, m->seq_start.as<int>(), m->staged_gap ? m->gap.as<int>() : nullptr, M, g.n_heads,
+  if (attn_forward(c, A.q16, A.k16, A.v16, m->seq_start, m->gap, M, g.n_heads,
                    g.n_kv_heads, g.head_dim, A.o16, A.lse))
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   // the residual comes in where the product goes out: in place, or from the buffer that keeps it
@@ -1216,9 +1231,9 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   // takes the factors per query row (in amax, for every token, the largest one of its own sequence:
   // nothing a sequence's backward sees may depend on its batch mates)
   RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16, sc_y, M, m->dO16.p, 0, HS(3), true));
-  launch_rowscale_seqmax(sc_y, m->seq_start.as<int>(), M, m->amax.as<float>(), st);
+  launch_rowscale_seqmax(sc_y, m->seq_start, M, m->amax.as<float>(), st);
   if (attn_backward(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(),
-                    m->amax.as<float>(), sc_y, A.lse, m->seq_start.as<int>(), m->staged_gap ? m->gap.as<int>() : nullptr, M,
+                    m->amax.as<float>(), sc_y, A.lse, m->seq_start, m->gap, M,
                     g.n_heads, g.n_kv_heads, g.head_dim,
                     m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
@@ -1227,7 +1242,7 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   __half* dk16 = A.qkv_group ? dq16 + qd : dq16 + T * qd;
   __half* dv16 = A.qkv_group ? dq16 + qd + kvd : dq16 + T * (qd + kvd);
   launch_qk_rope_bwd(m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>(), A.q_raw, A.k_raw, A.qkv_pitch,
-                     g.qk_norm ? b.q_norm : nullptr, g.qk_norm ? b.k_norm : nullptr, m->pos.as<int>(), m->rope_cos.as<float>(),
+                     g.qk_norm ? b.q_norm : nullptr, g.qk_norm ? b.k_norm : nullptr, m->pos, m->rope_cos.as<float>(),
                      m->rope_sin.as<float>(), M, g.n_heads, g.n_kv_heads, g.head_dim, g.rot_dim, g.rope_neox, g.rms_eps,
                      dq16, dk16, dv16, A.qkv_pitch, m->sc_q.as<float>(), m->sc_k.as<float>(), m->sc_v.as<float>(), st);
   if (A.qkv_group) {
@@ -1250,20 +1265,20 @@ static rt_status model_head(rt_model* m, int M, int n_targets, bool backward, fl
   cudaStream_t st = c->stream;
   const int d = g.hidden, V = g.vocab;
   (void)M;
-  RT_CUDA(c, cudaMemsetAsync(m->hits.p, 0, 4, st));
+  RT_CUDA(c, cudaMemsetAsync(m->hits(), 0, 4, st));
   rt_linear head;  // a bias-free, adapter-free Linear over the lm_head weight
   head.ctx = c;
   head.w = m->lm_head;
   for (int c0 = 0; c0 < n_targets; c0 += g.head_rows) {
     const int R = n_targets - c0 < g.head_rows ? n_targets - c0 : g.head_rows;
-    const int* tpos = m->tpos.as<int>() + c0;
+    const int* tpos = m->tpos + c0;
     launch_gather_f32_rows(m->x.as<float>(), tpos, R, d, m->xs.as<float>(), st);
     launch_rmsnorm_fwd(m->xs.as<float>(), m->final_norm, R, d, g.rms_eps, m->ns16.as<__half>(), st);
     RT_TRY(linear_forward_dev(&head, m->lsc, m->ns16.as<__half>(), R, m->logits.p, RT_DT_F32, 0));
     if (logits_out_host)
       RT_CUDA(c, cudaMemcpyAsync(logits_out_host + (size_t)c0 * V, m->logits.p, (size_t)R * V * 4, cudaMemcpyDeviceToHost, st));
-    launch_ce_rows(m->logits.as<float>(), R, V, m->ttok.as<int>() + c0, m->tw.as<float>() + c0, m->logp.as<float>() + c0,
-                   m->hits.as<int>(), backward ? m->dl16.as<__half>() : nullptr, backward ? m->sc_l.as<float>() : nullptr,
+    launch_ce_rows(m->logits.as<float>(), R, V, m->ttok + c0, m->tw + c0, m->logp() + c0,
+                   m->hits(), backward ? m->dl16.as<__half>() : nullptr, backward ? m->sc_l.as<float>() : nullptr,
                    m->want_argmax ? m->argmax.as<int>() + c0 : nullptr, c->status_dev, st);
     if (backward) {
       RT_TRY(linear_backward_dev(&head, m->lsc, m->ns16.as<__half>(), m->dl16.as<__half>(), m->sc_l.as<float>(), R, m->dns.as<float>(), 0));
@@ -1288,14 +1303,24 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
   const long long M = seq_offsets[n_seq];
   if (M <= 0 || M > (1 << 24)) return c->fail(RT_ERR_BAD_SHAPE, "token count out of range");
   if ((positions == nullptr) != (segments == nullptr)) return c->fail(RT_ERR_BAD_ARG, "positions and segments go together");
-  m->h_pos.resize(M);
-  m->h_seq_start.resize(M);
-  if (positions) m->h_gap.assign((size_t)M * 2, 0);
+  RT_CUDA(c, cudaSetDevice(c->device));
+  // the block: every array on a 256-byte boundary
+  const size_t n_tiles = ((size_t)M + 127) / 128;
+  size_t at = 0;
+  auto place = [&](size_t words) { const size_t o = at; at += (words * 4 + 255) / 256 * 256; return o; };
+  const size_t o_tok = place(M), o_pos = place(M), o_seq = place(M), o_gap = positions ? place(2 * M) : 0, o_oq = place(n_tiles),
+               o_ok = place(n_tiles), o_tp = place(n_targets), o_tt = place(n_targets), o_tw = place(n_targets);
+  if (!m->batch_sent) RT_CUDA(c, cudaEventCreateWithFlags(&m->batch_sent, cudaEventDisableTiming));
+  RT_CUDA(c, cudaEventSynchronize(m->batch_sent));  // the block before this one has left pinned memory
+  if (!m->h_batch.reserve(at)) return c->fail(RT_ERR_CUDA, "out of page-locked memory (batch)");
+  uint8_t* hb = (uint8_t*)m->h_batch.p;
+  int *h_pos = (int*)(hb + o_pos), *h_seq_start = (int*)(hb + o_seq), *h_gap = (int*)(hb + o_gap);
+  if (positions) memset(h_gap, 0, (size_t)M * 8);
   int max_len = 0;
   for (int s = 0; s < n_seq; ++s) {
     const int a = seq_offsets[s], e = seq_offsets[s + 1];
-    if (e <= a) return c->fail(RT_ERR_BAD_SHAPE, "empty or unordered sequence");
-    for (int i = a; i < e; ++i) { m->h_pos[i] = i - a; m->h_seq_start[i] = a; }
+    if (e <= a || e > M) return c->fail(RT_ERR_BAD_SHAPE, "empty or unordered sequence");
+    for (int i = a; i < e; ++i) { h_pos[i] = i - a; h_seq_start[i] = a; }
     if (e - a > max_len) max_len = e - a;
     if (positions) {
       // segments: zeros (the shared prompt), then runs of 1, 2, ...; a token of run k may not see the
@@ -1310,10 +1335,10 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
           if (sg <= 0 || sg < prev || sg > prev + 1) return c->fail(RT_ERR_BAD_ARG, "segments must be 0.., then 1, 2, ... in runs");
           if (sg != prev) run_start = i;
           prev = sg;
-          m->h_gap[2 * (size_t)i] = a + shared;
-          m->h_gap[2 * (size_t)i + 1] = run_start;
+          h_gap[2 * (size_t)i] = a + shared;
+          h_gap[2 * (size_t)i + 1] = run_start;
         }
-        m->h_pos[i] = ps;
+        h_pos[i] = ps;
         if (ps + 1 > max_len) max_len = ps + 1;
       }
     }
@@ -1324,24 +1349,45 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
     if (tpos[i] < 0 || tpos[i] >= M) return c->fail(RT_ERR_BAD_INDEX, "target position out of range");  // model.rs:573 asserts
     if (ttok[i] < 0 || ttok[i] >= m->cfg.vocab) return c->fail(RT_ERR_BAD_INDEX, "target token out of vocabulary");
   }
-  RT_CUDA(c, cudaSetDevice(c->device));
-  if (!ensure_tokens(m, (int)M) || !ensure_targets(m, n_targets > 0 ? n_targets : 1, backward))
+  if (!ensure_tokens(m, (int)M) || !ensure_targets(m, n_targets > 0 ? n_targets : 1, backward) || !m->batch.reserve(at))
     return c->fail(RT_ERR_CUDA, "out of device memory (activations)");
   RT_TRY(ensure_rope(m, max_len));
+  // The attention kernels take the tiles with the longest loops first: a query tile walks the keys from
+  // its first row's sequence start, a key tile the queries up to the end of its last row's sequence.
+  {
+    std::vector<std::pair<int, int>> wq(n_tiles), wk(n_tiles);
+    for (int t = (int)n_tiles - 1, s = n_seq; t >= 0; --t) {
+      const int t0 = t * 128, t1 = (int)std::min<long long>(M, t0 + 128);
+      while (seq_offsets[s - 1] > t1 - 1) --s;  // the sequence holding the tile's last row
+      wq[t] = {h_seq_start[t0] - t1, -t};
+      wk[t] = {t0 - seq_offsets[s], t};
+    }
+    std::sort(wq.begin(), wq.end());
+    std::sort(wk.begin(), wk.end());
+    for (size_t t = 0; t < n_tiles; ++t) {
+      ((int*)(hb + o_oq))[t] = -wq[t].second;
+      ((int*)(hb + o_ok))[t] = wk[t].second;
+    }
+  }
   cudaStream_t st = c->stream;
-  RT_CUDA(c, cudaMemcpyAsync(m->tokens.p, tokens, M * 4, cudaMemcpyHostToDevice, st));
-  RT_CUDA(c, cudaMemcpyAsync(m->pos.p, m->h_pos.data(), M * 4, cudaMemcpyHostToDevice, st));
-  RT_CUDA(c, cudaMemcpyAsync(m->seq_start.p, m->h_seq_start.data(), M * 4, cudaMemcpyHostToDevice, st));
-  m->staged_gap = positions != nullptr;
-  if (positions) {
-    if (!m->gap.reserve((size_t)M * 8)) return c->fail(RT_ERR_CUDA, "out of device memory (activations)");
-    RT_CUDA(c, cudaMemcpyAsync(m->gap.p, m->h_gap.data(), (size_t)M * 8, cudaMemcpyHostToDevice, st));
-  }
+  memcpy(hb + o_tok, tokens, (size_t)M * 4);
   if (n_targets > 0) {
-    RT_CUDA(c, cudaMemcpyAsync(m->tpos.p, tpos, (size_t)n_targets * 4, cudaMemcpyHostToDevice, st));
-    RT_CUDA(c, cudaMemcpyAsync(m->ttok.p, ttok, (size_t)n_targets * 4, cudaMemcpyHostToDevice, st));
-    if (tw) RT_CUDA(c, cudaMemcpyAsync(m->tw.p, tw, (size_t)n_targets * 4, cudaMemcpyHostToDevice, st));
+    memcpy(hb + o_tp, tpos, (size_t)n_targets * 4);
+    memcpy(hb + o_tt, ttok, (size_t)n_targets * 4);
+    if (tw) memcpy(hb + o_tw, tw, (size_t)n_targets * 4);
   }
+  RT_CUDA(c, cudaMemcpyAsync(m->batch.p, hb, at, cudaMemcpyHostToDevice, st));
+  RT_CUDA(c, cudaEventRecord(m->batch_sent, st));
+  uint8_t* db = (uint8_t*)m->batch.p;
+  m->tokens = (int*)(db + o_tok);
+  m->pos = (int*)(db + o_pos);
+  m->seq_start = (int*)(db + o_seq);
+  m->gap = positions ? (int*)(db + o_gap) : nullptr;
+  m->order_q = (int*)(db + o_oq);
+  m->order_k = (int*)(db + o_ok);
+  m->tpos = (int*)(db + o_tp);
+  m->ttok = (int*)(db + o_tt);
+  m->tw = (float*)(db + o_tw);
   *M_out = (int)M;
   return RT_OK;
 }
@@ -1358,7 +1404,7 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
   // A training pass writes every block's input where the backward will look for it; a forward-only
   // pass keeps one residual stream in place.
   float* ckpt = m->ckpt.as<float>();
-  launch_gather_rows(m->embed->w, m->tokens.as<int>(), M, backward ? ckpt : x, c->status_dev, st);
+  launch_gather_rows(m->embed->w, m->tokens, M, backward ? ckpt : x, c->status_dev, st);
   const bool store = backward && m->store_acts;
   for (int li = 0; li < g.n_layers; ++li) {
     const BlockActs A = block_acts(m, li, M, store);
@@ -1368,7 +1414,7 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
   }
   if (backward) RT_CUDA(c, cudaMemsetAsync(m->dx.p, 0, xd * 4, st));
   if (n_targets > 0) RT_TRY(model_head(m, M, n_targets, backward, logits_out_host));
-  else RT_CUDA(c, cudaMemsetAsync(m->hits.p, 0, 4, st));
+  else RT_CUDA(c, cudaMemsetAsync(m->hits(), 0, 4, st));
   if (!backward) return RT_OK;
   launch_normalize_rows(m->dx.as<float>(), M, g.hidden, m->dy16.as<__half>(), m->sc_y.as<float>(), st);
   for (int li = g.n_layers - 1; li >= 0; --li) {
@@ -1385,17 +1431,16 @@ static uint64_t buffer_signature(rt_model* m) {
   uint64_t h = 1469598103934665603ull;
   auto mix = [&](const void* p) { h = (h ^ (uint64_t)(uintptr_t)p) * 1099511628211ull; };
   DevBuf* bufs[] = {&m->P, &m->G, &m->rope_cos, &m->rope_sin, &m->lsc.hs, &m->lsc.gs, &m->lsc.hs2, &m->lsc.gs2, &m->lsc.smax, &m->lsc.grad_ws,
-                    &m->tokens, &m->pos, &m->seq_start, &m->x, &m->ckpt, &m->h, &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw,
+                    &m->batch, &m->results, &m->x, &m->ckpt, &m->h, &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw,
                     &m->q16, &m->k16, &m->v16, &m->o16, &m->lse, &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16,
                     &m->sc_y, &m->dhm, &m->dg16, &m->du16, &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->amax, &m->dq,
-                    &m->dk, &m->dv, &m->dq16, &m->dk16, &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->tpos, &m->ttok, &m->tw,
-                    &m->logp, &m->hits, &m->xs, &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
+                    &m->dk, &m->dv, &m->dq16, &m->dk16, &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs, &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) mix(b->p);
   for (int i = 0; i < 7; ++i) mix(m->hs_keep[i].p);
   for (int i = 0; i < 4; ++i) mix(m->ctx->scratch[i]);
   mix((const void*)(uintptr_t)m->n_params);
   mix((const void*)(uintptr_t)(m->store_acts ? 1 : 0));
-  mix(m->staged_gap ? m->gap.p : nullptr);
+  mix(m->gap);
   for (auto& b : m->blocks)
     for (int i = 0; i < 7; ++i) mix((const void*)(uintptr_t)(b.lin[i]->lora_active() ? b.lin[i]->lora.rank : 0));
   return h;
@@ -1415,15 +1460,15 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
   if (!m->use_graphs || c->profiling || logits_out_host || m->want_argmax || c->stream == nullptr)
     return run_staged_body(m, backward, logits_out_host);
   RT_CUDA(c, cudaSetDevice(c->device));
-  const int M = m->staged_tokens, nt = m->staged_targets, bw = backward ? 1 : 0;
-  const uint64_t sig = buffer_signature(m);
-  for (auto& ge : m->graphs)
-    if (ge.M == M && ge.n_targets == nt && ge.backward == bw && ge.sig == sig) {
-      RT_CUDA(c, cudaGraphLaunch(ge.exec, c->stream));
-      RT_COUNT_LAUNCH(ge.kernels);
+  rt_model::Shape shape{m->staged_tokens, m->staged_targets, backward ? 1 : 0, buffer_signature(m)};
+  for (size_t i = 0; i < m->graphs.size(); ++i)
+    if (m->graphs[i].shape == shape) {
+      std::rotate(m->graphs.begin() + i, m->graphs.begin() + i + 1, m->graphs.end());  // now the most recently used
+      RT_CUDA(c, cudaGraphLaunch(m->graphs.back().exec, c->stream));
+      RT_COUNT_LAUNCH(m->graphs.back().kernels);
       return RT_OK;
     }
-  if (m->eager_M == M && m->eager_targets == nt && m->eager_backward == bw && m->eager_sig == sig) {
+  if (std::find(m->seen.begin(), m->seen.end(), shape) != m->seen.end()) {
     const unsigned long long before = g_launch_count.load();
     cudaGraph_t graph = nullptr;
     RT_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -1434,11 +1479,11 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
     cudaGraphExec_t exec = nullptr;
     if (st == RT_OK && e == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
       cudaGraphDestroy(graph);
-      if (m->graphs.size() >= 8) {
+      if (m->graphs.size() >= rt_model::MAX_GRAPHS) {
         cudaGraphExecDestroy(m->graphs.front().exec);
         m->graphs.erase(m->graphs.begin());
       }
-      m->graphs.push_back({M, nt, bw, sig, exec, kernels});
+      m->graphs.push_back({shape, exec, kernels});
       RT_CUDA(c, cudaGraphLaunch(exec, c->stream));
       RT_COUNT_LAUNCH(kernels);
       return RT_OK;
@@ -1449,10 +1494,9 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
     return run_staged_body(m, backward, nullptr);
   }
   rt_status st = run_staged_body(m, backward, nullptr);
-  m->eager_M = M;
-  m->eager_targets = nt;
-  m->eager_backward = bw;
-  m->eager_sig = buffer_signature(m);
+  shape.sig = buffer_signature(m);  // the eager run may have sized buffers
+  if (m->seen.size() >= rt_model::MAX_SEEN) m->seen.erase(m->seen.begin());
+  m->seen.push_back(shape);
   return st;
 }
 
@@ -1481,11 +1525,11 @@ rt_status rt_model_read_results(rt_model* m, float* logp_out, int32_t n_targets,
   if (n_targets > m->staged_targets) return c->fail(RT_ERR_BAD_ARG, "more results requested than targets staged");
   RT_CUDA(c, cudaSetDevice(c->device));
   cudaStream_t st = c->stream;
-  if (n_targets > 0 && logp_out) RT_CUDA(c, cudaMemcpyAsync(logp_out, m->logp.p, (size_t)n_targets * 4, cudaMemcpyDeviceToHost, st));
-  int hits = 0;
-  RT_CUDA(c, cudaMemcpyAsync(&hits, m->hits.p, 4, cudaMemcpyDeviceToHost, st));
+  const size_t nb = 16 + (n_targets > 0 && logp_out ? (size_t)n_targets * 4 : 0);
+  RT_CUDA(c, cudaMemcpyAsync(m->h_results.p, m->results.p, nb, cudaMemcpyDeviceToHost, st));
   rt_status s = c->check_device_status("rt_model_read_results");
-  if (hits_out) *hits_out = hits;
+  if (hits_out) *hits_out = *(const int*)m->h_results.p;
+  if (nb > 16) memcpy(logp_out, (const uint8_t*)m->h_results.p + 16, nb - 16);
   return s;
 }
 
@@ -1591,10 +1635,9 @@ rt_status rt_optim_step(rt_model* m, float lr, float max_norm, float beta1, floa
   launch_adamw(m->P.as<float>(), m->G.as<float>(), m->Mo.as<float>(), m->Vo.as<float>(), m->n_params, sum, max_norm, lr,
                beta1, beta2, eps, wd, bc1, bc2, normd, st);
   for (rt_linear* l : m->lora_order) { l->lora.stale = true; ++l->lora.version; }
-  float nrm = 0.f;
-  RT_CUDA(c, cudaMemcpyAsync(&nrm, normd, 4, cudaMemcpyDeviceToHost, st));
+  RT_CUDA(c, cudaMemcpyAsync(c->status_host + 1, normd, 4, cudaMemcpyDeviceToHost, st));
   rt_status s = c->check_device_status("rt_optim_step");
-  if (norm_out) *norm_out = nrm;
+  if (norm_out) memcpy(norm_out, c->status_host + 1, 4);
   return s;
 }
 

@@ -18,6 +18,14 @@ struct DevBuf {
   template <class T> T* as() const { return (T*)p; }
 };
 
+// Page-locked host memory, grow-only.
+struct PinnedBuf {
+  void* p = nullptr;
+  size_t bytes = 0;
+  bool reserve(size_t want);
+  void release();
+};
+
 struct LoraDev {
   int rank = 0;
   float alpha = 0.f;
@@ -131,22 +139,38 @@ struct rt_model {
   int cap_tokens = 0, cap_targets = 0, cap_head_rows = 0;
   // q_raw holds q|k|v before RoPE (three regions, or one matrix with q, k, v as column slices when the
   // block runs them as a group); g16 holds gate|up the same way; dq16, dg16 likewise for the gradients
-  DevBuf tokens, pos, seq_start, x, ckpt, h, n1, n2, q_raw, k_raw, v_raw, q16, k16, v16, o16, lse, delta, g16, u16, hm16;
+  DevBuf x, ckpt, h, n1, n2, q_raw, k_raw, v_raw, q16, k16, v16, o16, lse, delta, g16, u16, hm16;
   DevBuf dx, dy16, sc_y, dhm, dg16, du16, sc_g, sc_u, dn, d_o, dO16, amax, dq, dk, dv, dq16, dk16, dv16, sc_q, sc_k, sc_v;
-  DevBuf tpos, ttok, tw, logp, hits, xs, ns16, logits, dl16, sc_l, dns, dxs;
+  DevBuf xs, ns16, logits, dl16, sc_l, dns, dxs;
   DevBuf argmax;            // per target, the greedy token of the last pass that asked for it
   bool want_argmax = false;
-  std::vector<int> h_pos, h_seq_start, h_gap;
   DevBuf refresh_tab;       // device copy of refresh_sent
   std::vector<rt::LoraRefreshJob> refresh_jobs, refresh_sent;
-  DevBuf gap;               // per token (first, end) of the key range hidden from it: packed shared-prompt groups
+  // A batch travels as one block: laid out in pinned memory, one copy to `batch`, the pointers below into it
+  // (they depend on the block's base, the token and target counts and staged_gap only).  Results come back as
+  // one block too: hit count, then log-probabilities.
+  DevBuf batch, results;
+  PinnedBuf h_batch, h_results;
+  cudaEvent_t batch_sent = nullptr;
+  int *tokens = nullptr, *pos = nullptr, *seq_start = nullptr, *tpos = nullptr, *ttok = nullptr;
+  int *order_q = nullptr, *order_k = nullptr;  // the batch's 128-token tiles, heaviest first, as queries and as keys
+  int* gap = nullptr;       // per token (first, end) of the key range hidden from it: packed shared-prompt groups, or null
+  float* tw = nullptr;
   bool staged_gap = false;  // the staged batch has such ranges
+  int* hits() const { return results.as<int>(); }
+  float* logp() const { return results.as<float>() + 4; }
   int staged_tokens = 0, staged_targets = 0;
   bool staged_has_weights = false;
-  // CUDA graphs of the staged step, one per (tokens, targets, backward) once it has run eagerly
-  struct GraphEntry { int M, n_targets, backward; uint64_t sig; cudaGraphExec_t exec; unsigned long long kernels; };
+  // CUDA graphs of the staged step, one per shape of batch once it has run eagerly; least recently used first.
+  // A trainer meets several shapes in turn (accumulated batches, a preference update's three passes).
+  struct Shape {
+    int M, n_targets, backward;
+    uint64_t sig;
+    bool operator==(const Shape& o) const { return M == o.M && n_targets == o.n_targets && backward == o.backward && sig == o.sig; }
+  };
+  struct GraphEntry { Shape shape; cudaGraphExec_t exec; unsigned long long kernels; };
+  static constexpr size_t MAX_GRAPHS = 32, MAX_SEEN = 256;
   std::vector<GraphEntry> graphs;
-  int eager_M = -1, eager_targets = -1, eager_backward = -1;
-  uint64_t eager_sig = 0;
+  std::vector<Shape> seen;  // shapes that have run eagerly, oldest first
   int use_graphs = -1;  // -1: decide from the environment on first use
 };
