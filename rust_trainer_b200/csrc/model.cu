@@ -3,6 +3,7 @@
 // sequencing the reference does in src/linear.rs, src/attention.rs, src/model.rs and
 // src/optim.rs, plus buffer management.
 #include "model.h"
+#include "pdl.cuh"
 #include <math.h>
 #include <algorithm>
 #include <stdio.h>
@@ -78,16 +79,6 @@ static __half* lowrank_buf(rt_ctx* c, DevBuf& b, int& cur_rank, int M, int rank)
   if (clear) cudaMemsetAsync(b.p, 0, want, c->stream);
   cur_rank = rank;
   return b.as<__half>();
-}
-
-int attn_forward(rt_ctx* c, const __half* q, const __half* k, const __half* v, const int* seq_start, const int* gap, int M, int nh,
-                 int nkv, int hd, __half* o, float* lse) {
-  return launch_attn_fwd_tc(c, q, k, v, seq_start, gap, M, nh, nkv, hd, o, lse);
-}
-int attn_backward(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,
-                  const float* do_scale, const float* row_scale, const float* lse, const int* seq_start, const int* gap, int M,
-                  int nh, int nkv, int hd, float* delta, float* dq, float* dk, float* dv) {
-  return launch_attn_bwd_tc(c, q, k, v, o, dO16, do_scale, row_scale, lse, seq_start, gap, M, nh, nkv, hd, delta, dq, dk, dv);
 }
 
 // out[M x 64] = X[M x K] . Wt[r x K]^T: the tcgen05 stream kernel, or (return 1) a shape it does not take
@@ -551,6 +542,7 @@ rt_status rt_linear_forward_dev(rt_linear* l, const void* x, size_t t, void* y, 
   if (y_dtype < 0 || y_dtype > 2) return c->fail(RT_ERR_BAD_ARG, "bad output dtype");
   if (accumulate && y_dtype != RT_DT_F32) return c->fail(RT_ERR_BAD_ARG, "accumulate needs an f32 output");
   RT_CUDA(c, cudaSetDevice(c->device));
+  const PdlScope pdl_scope(t);
   return linear_forward_dev(l, ctx_scratch(c), (const __half*)x, (int)t, y, y_dtype, accumulate);
 }
 
@@ -560,6 +552,7 @@ rt_status rt_linear_backward_dev(rt_linear* l, const void* x, const void* dy, co
   rt_ctx* c = l->ctx;
   if (t > (1u << 24)) return c->fail(RT_ERR_BAD_SHAPE, "too many rows");
   RT_CUDA(c, cudaSetDevice(c->device));
+  const PdlScope pdl_scope(t);
   return linear_backward_dev(l, ctx_scratch(c), (const __half*)x, (const __half*)dy, dscale, (int)t, dx, accumulate);
 }
 
@@ -1177,8 +1170,7 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   launch_qk_rope_fwd(A.q_raw, A.k_raw, A.v_raw, A.qkv_pitch, g.qk_norm ? b.q_norm : nullptr,
                      g.qk_norm ? b.k_norm : nullptr, m->pos, m->rope_cos.as<float>(), m->rope_sin.as<float>(), M,
                      g.n_heads, g.n_kv_heads, g.head_dim, g.rot_dim, g.rope_neox, g.rms_eps, A.q16, A.k16, A.v16, st);
-  if (attn_forward(c, A.q16, A.k16, A.v16, m->seq_start, m->gap, M, g.n_heads,
-                   g.n_kv_heads, g.head_dim, A.o16, A.lse))
+  if (launch_attn_fwd_tc(c, A.q16, A.k16, A.v16, m->attn_batch(M), g.n_heads, g.n_kv_heads, g.head_dim, A.o16, A.lse))
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   // the residual comes in where the product goes out: in place, or from the buffer that keeps it
   RT_TRY(linear_forward_dev(b.lin[3], m->lsc, A.o16, M, h, RT_DT_F32, h == x_in, keep ? A.hs[3] : nullptr, hs_ready, h == x_in ? nullptr : x_in));
@@ -1232,10 +1224,8 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   // nothing a sequence's backward sees may depend on its batch mates)
   RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16, sc_y, M, m->dO16.p, 0, HS(3), true));
   launch_rowscale_seqmax(sc_y, m->seq_start, M, m->amax.as<float>(), st);
-  if (attn_backward(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(),
-                    m->amax.as<float>(), sc_y, A.lse, m->seq_start, m->gap, M,
-                    g.n_heads, g.n_kv_heads, g.head_dim,
-                    m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
+  if (launch_attn_bwd_tc(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(), m->amax.as<float>(), sc_y, A.lse, m->attn_batch(M),
+                         g.n_heads, g.n_kv_heads, g.head_dim, m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
   const size_t qd = (size_t)g.n_heads * g.head_dim, kvd = (size_t)g.n_kv_heads * g.head_dim;
   __half* dq16 = m->dq16.as<__half>();
@@ -1309,7 +1299,7 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
   size_t at = 0;
   auto place = [&](size_t words) { const size_t o = at; at += (words * 4 + 255) / 256 * 256; return o; };
   const size_t o_tok = place(M), o_pos = place(M), o_seq = place(M), o_gap = positions ? place(2 * M) : 0, o_oq = place(n_tiles),
-               o_ok = place(n_tiles), o_tp = place(n_targets), o_tt = place(n_targets), o_tw = place(n_targets);
+               o_ok = place(2 * n_tiles), o_tp = place(n_targets), o_tt = place(n_targets), o_tw = place(n_targets);
   if (!m->batch_sent) RT_CUDA(c, cudaEventCreateWithFlags(&m->batch_sent, cudaEventDisableTiming));
   RT_CUDA(c, cudaEventSynchronize(m->batch_sent));  // the block before this one has left pinned memory
   if (!m->h_batch.reserve(at)) return c->fail(RT_ERR_CUDA, "out of page-locked memory (batch)");
@@ -1352,23 +1342,7 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
   if (!ensure_tokens(m, (int)M) || !ensure_targets(m, n_targets > 0 ? n_targets : 1, backward) || !m->batch.reserve(at))
     return c->fail(RT_ERR_CUDA, "out of device memory (activations)");
   RT_TRY(ensure_rope(m, max_len));
-  // The attention kernels take the tiles with the longest loops first: a query tile walks the keys from
-  // its first row's sequence start, a key tile the queries up to the end of its last row's sequence.
-  {
-    std::vector<std::pair<int, int>> wq(n_tiles), wk(n_tiles);
-    for (int t = (int)n_tiles - 1, s = n_seq; t >= 0; --t) {
-      const int t0 = t * 128, t1 = (int)std::min<long long>(M, t0 + 128);
-      while (seq_offsets[s - 1] > t1 - 1) --s;  // the sequence holding the tile's last row
-      wq[t] = {h_seq_start[t0] - t1, -t};
-      wk[t] = {t0 - seq_offsets[s], t};
-    }
-    std::sort(wq.begin(), wq.end());
-    std::sort(wk.begin(), wk.end());
-    for (size_t t = 0; t < n_tiles; ++t) {
-      ((int*)(hb + o_oq))[t] = -wq[t].second;
-      ((int*)(hb + o_ok))[t] = wk[t].second;
-    }
-  }
+  attn_plan_tiles(h_seq_start, (int)M, (int*)(hb + o_oq), (int*)(hb + o_ok));
   cudaStream_t st = c->stream;
   memcpy(hb + o_tok, tokens, (size_t)M * 4);
   if (n_targets > 0) {
@@ -1383,8 +1357,8 @@ static rt_status upload_batch(rt_model* m, const int32_t* tokens, const int32_t*
   m->pos = (int*)(db + o_pos);
   m->seq_start = (int*)(db + o_seq);
   m->gap = positions ? (int*)(db + o_gap) : nullptr;
-  m->order_q = (int*)(db + o_oq);
-  m->order_k = (int*)(db + o_ok);
+  m->tiles_q = (int*)(db + o_oq);
+  m->tiles_k = (int*)(db + o_ok);
   m->tpos = (int*)(db + o_tp);
   m->ttok = (int*)(db + o_tt);
   m->tw = (float*)(db + o_tw);
@@ -1397,6 +1371,7 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
   const int M = m->staged_tokens, n_targets = m->staged_targets;
   if (M <= 0) return c->fail(RT_ERR_BAD_ARG, "no batch staged");
   RT_CUDA(c, cudaSetDevice(c->device));
+  const PdlScope pdl_scope((size_t)M);
   cudaStream_t st = c->stream;
   const rt_model_config& g = m->cfg;
   const size_t xd = (size_t)M * g.hidden;

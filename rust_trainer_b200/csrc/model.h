@@ -72,11 +72,6 @@ rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16
                               const float* dscale, int M, void* dx, int accumulate,
                               const __half* hs_saved = nullptr, bool unscaled_f16_out = false);
 rt_status lora_refresh(rt_linear* l);
-int attn_backward(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,
-                  const float* do_scale, const float* row_scale, const float* lse, const int* seq_start, const int* gap, int M,
-                  int nh, int nkv, int hd, float* delta, float* dq, float* dk, float* dv);
-int attn_forward(rt_ctx* c, const __half* q, const __half* k, const __half* v, const int* seq_start, const int* gap, int M, int nh,
-                 int nkv, int hd, __half* o, float* lse);
 }  // namespace rt
 
 // Linears that read the same input (q|k|v, gate|up) as ONE matmul: their packed weights lie
@@ -153,7 +148,8 @@ struct rt_model {
   PinnedBuf h_batch, h_results;
   cudaEvent_t batch_sent = nullptr;
   int *tokens = nullptr, *pos = nullptr, *seq_start = nullptr, *tpos = nullptr, *ttok = nullptr;
-  int *order_q = nullptr, *order_k = nullptr;  // the batch's 128-token tiles, heaviest first, as queries and as keys
+  int *tiles_q = nullptr, *tiles_k = nullptr;  // see AttnBatch
+  rt::AttnBatch attn_batch(int M) const { return {seq_start, gap, tiles_q, tiles_k, M}; }
   int* gap = nullptr;       // per token (first, end) of the key range hidden from it: packed shared-prompt groups, or null
   float* tw = nullptr;
   bool staged_gap = false;  // the staged batch has such ranges

@@ -108,10 +108,18 @@ int launch_tok_contract(const __half* P, const __half* Q, const float* pscale, i
 // Backward: dO row i stands for do_scale[0] * dO16[i], or, with row_scale, for row_scale[i] *
 // dO16[i] (then do_scale is the array [2 M] of launch_rowscale_seqmax: for each token a power of two >=
 // the largest row_scale of its own sequence, then each row's weight against it); outputs are true-scale f32.
+// What the kernels need to know of a batch, all on the device.  tiles_q: its 128-token tiles as query tiles,
+// longest loops first; tiles_k: as key tiles, pairs (tile, end of the sequence holding its last key).
+struct AttnBatch {
+  const int *seq_start, *gap, *tiles_q, *tiles_k;
+  int M;
+};
+// fills the two tile lists (host memory, n and 2 n ints for n = ceil(M / 128) tiles) from seq_start (host memory)
+void attn_plan_tiles(const int* seq_start, int M, int* tiles_q, int* tiles_k);
 int launch_attn_bwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,
-                       const float* do_scale, const float* row_scale, const float* lse, const int* seq_start, const int* gap,
-                       int M, int nh, int nkv, int hd, float* delta, float* dq, float* dk, float* dv);
-int launch_attn_fwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const int* seq_start, const int* gap, int M,
-                       int nh, int nkv, int hd, __half* o, float* lse);
+                       const float* do_scale, const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, int hd,
+                       float* delta, float* dq, float* dk, float* dv);
+int launch_attn_fwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const AttnBatch& b, int nh, int nkv, int hd,
+                       __half* o, float* lse);
 
 }  // namespace rt

@@ -188,13 +188,18 @@ rt_status rt_op_attention(rt_ctx* c, const float* q, const float* k, const float
   const size_t nq = M * nh * hd, nk = M * nkv * hd;
   float *qd = t.up(q, nq, c->stream), *kd = t.up(k, nk, c->stream), *vd = t.up(v, nk, c->stream);
   int* ss = t.up((const int*)seq_start, M, c->stream);
+  const size_t nt = (M + 127) / 128;
+  std::vector<int> tq(nt), tk(2 * nt);
+  attn_plan_tiles(seq_start, (int)M, tq.data(), tk.data());
+  int *tqd = t.up(tq.data(), nt, c->stream), *tkd = t.up(tk.data(), 2 * nt, c->stream);
   __half *q16 = t.get<__half>(nq), *k16 = t.get<__half>(nk), *v16 = t.get<__half>(nk), *o16 = t.get<__half>(nq);
   float* lsed = t.get<float>(M * nh);
-  if (!qd || !kd || !vd || !ss || !q16 || !k16 || !v16 || !o16 || !lsed) return c->fail(RT_ERR_CUDA, "out of device memory");
+  if (!qd || !kd || !vd || !ss || !tqd || !tkd || !q16 || !k16 || !v16 || !o16 || !lsed) return c->fail(RT_ERR_CUDA, "out of device memory");
   launch_f32_to_16(qd, q16, nq, true, c->stream);
   launch_f32_to_16(kd, k16, nk, true, c->stream);
   launch_f32_to_16(vd, v16, nk, true, c->stream);
-  if (attn_forward(c, q16, k16, v16, ss, nullptr, (int)M, nh, nkv, hd, o16, lsed))
+  const AttnBatch ab{ss, nullptr, tqd, tkd, (int)M};
+  if (launch_attn_fwd_tc(c, q16, k16, v16, ab, nh, nkv, hd, o16, lsed))
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   rt_status s = down_f16(c, o16, nullptr, 1, nq, o, t);
   if (s) return s;
@@ -216,20 +221,25 @@ rt_status rt_op_attention_backward(rt_ctx* c, const float* q, const float* k, co
   const size_t nq = M * nh * hd, nk = M * nkv * hd;
   float *qd = t.up(q, nq, c->stream), *kd = t.up(k, nk, c->stream), *vd = t.up(v, nk, c->stream), *dod = t.up(d_o, nq, c->stream);
   int* ss = t.up((const int*)seq_start, M, c->stream);
+  const size_t nt = (M + 127) / 128;
+  std::vector<int> tq(nt), tk(2 * nt);
+  attn_plan_tiles(seq_start, (int)M, tq.data(), tk.data());
+  int *tqd = t.up(tq.data(), nt, c->stream), *tkd = t.up(tk.data(), 2 * nt, c->stream);
   __half *q16 = t.get<__half>(nq), *k16 = t.get<__half>(nk), *v16 = t.get<__half>(nk), *o16 = t.get<__half>(nq), *do16 = t.get<__half>(nq);
   float *lsed = t.get<float>(M * nh), *delta = t.get<float>(M * nh), *sc = t.get<float>(M), *amax = t.get<float>(2 * M + 4);
   float *dqd = t.get<float>(nq), *dkd = t.get<float>(nk), *dvd = t.get<float>(nk);
-  if (!qd || !kd || !vd || !dod || !ss || !q16 || !k16 || !v16 || !o16 || !do16 || !lsed || !delta || !sc || !amax || !dqd || !dkd || !dvd)
+  if (!qd || !kd || !vd || !dod || !ss || !tqd || !tkd || !q16 || !k16 || !v16 || !o16 || !do16 || !lsed || !delta || !sc || !amax || !dqd || !dkd || !dvd)
     return c->fail(RT_ERR_CUDA, "out of device memory");
   launch_f32_to_16(qd, q16, nq, true, c->stream);
   launch_f32_to_16(kd, k16, nk, true, c->stream);
   launch_f32_to_16(vd, v16, nk, true, c->stream);
-  if (attn_forward(c, q16, k16, v16, ss, nullptr, (int)M, nh, nkv, hd, o16, lsed))
+  const AttnBatch ab{ss, nullptr, tqd, tkd, (int)M};
+  if (launch_attn_fwd_tc(c, q16, k16, v16, ab, nh, nkv, hd, o16, lsed))
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   // dO as the model passes it: f16 rows divided by their largest magnitude, factors beside them
   launch_normalize_rows(dod, (int)M, nh * hd, do16, sc, c->stream);
   launch_rowscale_seqmax(sc, ss, (int)M, amax, c->stream);
-  if (attn_backward(c, q16, k16, v16, o16, do16, amax, sc, lsed, ss, nullptr, (int)M, nh, nkv, hd, delta, dqd, dkd, dvd))
+  if (launch_attn_bwd_tc(c, q16, k16, v16, o16, do16, amax, sc, lsed, ab, nh, nkv, hd, delta, dqd, dkd, dvd))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
   RT_CUDA(c, cudaMemcpyAsync(dq, dqd, nq * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   RT_CUDA(c, cudaMemcpyAsync(dk, dkd, nk * sizeof(float), cudaMemcpyDeviceToHost, c->stream));

@@ -8,11 +8,11 @@
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
 //     every CTA of this one has started.
 // Inside stream capture these launches become programmatic edges of the graph.
-// OFF by default: measured on the headline step (one graph replay of 1290 launches) it gained
-// nothing (52.2 / 52.0 ms with, 51.8 / 51.7 ms without, alternating runs on one GPU): the heavy
-// kernels fill every SM, so a successor's CTAs only start when a predecessor's CTA exits, and the
-// graph's own kernel-to-kernel gaps are already short.  RT_B200_PDL=1 in the environment turns
-// it on (the kernels carry the wait either way; without the launch attribute it returns at once).
+// Used for passes of up to PDL_MAX_TOKENS tokens, whose kernels leave SMs free for the next one's CTAs to
+// start on: the 28-layer 0.6B step 10.67 -> 10.14 ms at 1024 tokens, scoring 157 tokens 3.01 -> 2.84 ms.  At
+// 8192 tokens the kernels fill every SM and a waiting successor only takes room from them: 46.2 -> 46.9
+// ms, and the 3B step 153.7 -> 155.5.  RT_B200_PDL=0 or 1 in the environment decides for every size.
+// (The kernels carry the wait either way; without the launch attribute it returns at once.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -28,13 +28,19 @@ __device__ __forceinline__ void pdl_entry() {
   pdl_wait();
 }
 
+constexpr int PDL_MAX_TOKENS = 4096;
+inline thread_local int g_pdl_tokens = 0;  // tokens of the pass this thread is launching, see PdlScope
+struct PdlScope {
+  int before;
+  explicit PdlScope(size_t tokens) : before(g_pdl_tokens) { g_pdl_tokens = tokens > (1u << 30) ? 1 << 30 : (int)tokens; }
+  ~PdlScope() { g_pdl_tokens = before; }
+};
 inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
+  static const int forced = [] {
     const char* e = getenv("RT_B200_PDL");
-    on = (e && atoi(e)) ? 1 : 0;
-  }
-  return on != 0;
+    return e ? (atoi(e) ? 1 : 0) : -1;
+  }();
+  return forced >= 0 ? forced != 0 : g_pdl_tokens > 0 && g_pdl_tokens <= PDL_MAX_TOKENS;
 }
 
 template <typename... KArgs>

@@ -49,25 +49,29 @@ struct QCfg {
   // 406 us against 363.)  Without unpacking eight warps stay, to help with the last tile's epilogue.
   static constexpr int NUW = PACKED ? 16 : 8;
   static constexpr int THREADS = 32 * (7 + NUW);  // + activation / brick producers, MMA, 4 epilogue warps
-  // Activation / unpacked-weight stages and packed brick-pair stages: as many as fit beside the
-  // epilogue staging.  NS <= NR + 1 is part of the phase rule below.
-  static constexpr bool DEEP = KIND == QK_NARROW && FMT != GGML_Q8_0;
-  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : PACKED ? (DEEP ? 6 : 5) : 8;
-  static constexpr int NR = !PACKED ? 0 : DEEP ? 8 : 4;
-  static constexpr int RAW_STAGE = PACKED ? 2 * fmt_brick_bytes(FMT) : 0;
-  // The unpack warps work as UG groups on alternate contraction steps.  Waits are by phase parity,
+  // 64-element contraction steps per stage.  Two for narrow tiles: their MMAs are short, and one hand-off
+  // between the roles costs about 500 cycles whatever it hands over.
+  static constexpr int KS = KIND == QK_NARROW ? 2 : 1;
+  // Activation / unpacked-weight stages and packed-brick stages: as many as fit beside the epilogue
+  // staging.  NS <= NR + 1 is part of the phase rule below.
+  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : PACKED ? 3 : 4;
+  static constexpr int NR = !PACKED ? 0 : PAIR ? 4 : 3;
+  static constexpr int RAW_STAGE = PACKED ? KS * 2 * fmt_brick_bytes(FMT) : 0;
+  // The unpack warps work as UG groups on alternate stages.  Waits are by phase parity,
   // which is only sound while a waiter cannot run two phases ahead of its barrier: UG <= NS keeps a
   // group from reaching a stage before the use two back has been released, and NS <= NR + 1 keeps a
-  // group from reaching a brick slot's next use (NR steps later, NR + 1 across a low-rank step,
+  // group from reaching a brick slot's next use (NR stages later, NR + 1 across a low-rank step,
   // which takes a stage but no bricks) before the MMAs of its previous use are done, so that a copy
   // that lands late cannot be taken for the one after it.
-  static constexpr int UG = KIND == QK_WIDE ? 2 : 4;       // a power of two
+  static constexpr int UG = PAIR ? 4 : 2;                  // a power of two
   static constexpr int UTG = NUW * 32 / UG;                // threads per group
   static_assert(UG <= NS && (!PACKED || NS <= NR + 1), "unpack groups would alias barrier phases");
-  static_assert(!PACKED || UTG == 128, "a thread of a group owns one unit of each brick");
-  static constexpr int ACT_STAGE = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
+  static_assert(!PACKED || UTG == KS * 128, "a thread of a group owns one unit of each half of a weight tile");
+  static constexpr int W_BYTES = KS * W_STAGE;             // unpacked weights of a stage
+  static constexpr int ACT_SUB = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
+  static constexpr int ACT_STAGE = KS * ACT_SUB;
   static constexpr int OFF_W = NS * ACT_STAGE;
-  static constexpr int OFF_RAW = OFF_W + NS * W_STAGE;
+  static constexpr int OFF_RAW = OFF_W + NS * W_BYTES;
   static constexpr int OFF_OUT = OFF_RAW + NR * RAW_STAGE;
   // Epilogue staging of 16-bit outputs per warp: three blocks of [32 tokens x 32 features], 2 KB each.
   static constexpr int OUT_BUFS = 3, OUT_WARP = OUT_BUFS * 2048;
@@ -231,7 +235,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
              const __grid_constant__ CUtensorMap tm_out, const KParams p) {
   using C = QCfg<KIND, FMT>;
   constexpr bool PAIR = C::PAIR, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
-  constexpr int NS = C::NS, NR = C::NR, UG = C::UG, UTG = C::UTG;
+  constexpr int NS = C::NS, NR = C::NR, UG = C::UG, UTG = C::UTG, KS = C::KS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sAct = smem;
@@ -284,8 +288,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   const int tile = (item) % n_tiles, split = (item) / n_tiles;                                \
   const int s_begin = split * p.steps_per_split;                                              \
   const int s_main = min(p.n_main, s_begin + p.steps_per_split) - s_begin;                    \
-  const int n_steps = s_main + ((p.lora_mmas > 0 && split == p.n_splits - 1) ? 1 : 0);        \
-  (void)split
+  const int n_main_st = (s_main + KS - 1) / KS;  /* stages of the weight's own contraction */  \
+  const int n_steps = n_main_st + ((p.lora_mmas > 0 && split == p.n_splits - 1) ? 1 : 0);     \
+  (void)split; (void)n_main_st
 // first weight row (output feature) of this CTA's half of the tile, first token of the tile
 #define QG_TILE_ORIGIN()                                                                      \
   const int r0 = (tile % p.n_row_tiles) * (128 * n_cta) + (int)rank * 128;                    \
@@ -492,28 +497,35 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         QG_TILE_ORIGIN();
         const int m_cta = m0 + (int)rank * tn_cta;  // this CTA's half of the tokens
         for (int si = 0; si < n_steps; ++si) {
-          const int s = s_begin + si;
           if (!mbar_wait(&stage_empty[st], ph ^ 1, p.status, 101)) { ok = false; break; }
-          const bool lora = si >= s_main;
+          const bool lora = si >= n_main_st;
+          const int subs = KS == 1 || lora ? 1 : min(KS, s_main - si * KS);
           uint8_t* a_dst = sAct + st * C::ACT_STAGE;
-          uint8_t* w_dst = sW + st * W_STAGE;
+          uint8_t* w_dst = sW + st * C::W_BYTES;
           // the leader's barrier counts the bytes both CTAs will bring
-          if (rank == 0) mbar_expect_tx(&full[st], (uint32_t)p.TN * 128u + ((IS16 || lora) ? (uint32_t)(W_STAGE * n_cta) : 0u));
+          if (rank == 0)
+            mbar_expect_tx(&full[st], (uint32_t)subs * ((uint32_t)p.TN * 128u + ((IS16 || lora) ? (uint32_t)(W_STAGE * n_cta) : 0u)));
           const uint32_t fbar = PAIR ? mapa_u32(smem_u32(&full[st]), 0) : 0u;
           auto load2d = [&](void* dst, const CUtensorMap* map, int x, int y) {
             if (PAIR) tma_load_2d_pair(dst, map, x, y, fbar);
             else tma_load_2d(dst, map, x, y, &full[st]);
           };
           if (!lora) {
-            if (p.b_mn) load2d(a_dst, &tm_act, 0, s * 64);  // [64 contraction rows x 64]
-            else load2d(a_dst, &tm_act, s * 64, m_cta);
-            if (IS16) {
-              if (p.dir == QG_FWD) {
-                load2d(w_dst, &tm_w16, s * 64, r0);
-                load2d(w_dst + 8192, &tm_w16, s * 64, r0 + 64);
-              } else {
-                load2d(w_dst, &tm_w16, r0, s * 64);
-                load2d(w_dst + 8192, &tm_w16, r0 + 64, s * 64);
+#pragma unroll
+            for (int u = 0; u < KS; ++u) {
+              if (u >= subs) break;
+              const int s = s_begin + si * KS + u;
+              if (p.b_mn) load2d(a_dst + u * C::ACT_SUB, &tm_act, 0, s * 64);  // [64 contraction rows x 64]
+              else load2d(a_dst + u * C::ACT_SUB, &tm_act, s * 64, m_cta);
+              if (IS16) {
+                uint8_t* w = w_dst + u * W_STAGE;
+                if (p.dir == QG_FWD) {
+                  load2d(w, &tm_w16, s * 64, r0);
+                  load2d(w + 8192, &tm_w16, s * 64, r0 + 64);
+                } else {
+                  load2d(w, &tm_w16, r0, s * 64);
+                  load2d(w + 8192, &tm_w16, r0 + 64, s * 64);
+                }
               }
             }
           } else {
@@ -569,19 +581,24 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
           ph ^= (uint32_t)wrap;
         };
 #pragma unroll 1
-        for (int s = 0; s < s_main; ++s) {
+        for (int s = 0; s < n_main_st; ++s) {
           if (!step_ready()) { ok = false; break; }
-          const uint32_t a_lo = (uint32_t)a_d0 + (uint32_t)st * (W_STAGE >> 4);
+          const uint32_t a_lo = (uint32_t)a_d0 + (uint32_t)st * (C::W_BYTES >> 4);
           const uint32_t b_lo = (uint32_t)b_d0 + (uint32_t)st * (C::ACT_STAGE >> 4);
-          umma_f16_split<PAIR>(d_tmem, a_lo, a_hi, b_lo, b_hi, idesc, (uint32_t)(s != 0));
-          umma_f16_split<PAIR>(d_tmem, a_lo + a_k, a_hi, b_lo + b_k, b_hi, idesc, 1u);
-          umma_f16_split<PAIR>(d_tmem, a_lo + 2 * a_k, a_hi, b_lo + 2 * b_k, b_hi, idesc, 1u);
-          umma_f16_split<PAIR>(d_tmem, a_lo + 3 * a_k, a_hi, b_lo + 3 * b_k, b_hi, idesc, 1u);
+#pragma unroll
+          for (int u = 0; u < KS; ++u) {
+            if (u > 0 && s * KS + u >= s_main) break;
+            const uint32_t au = a_lo + u * (W_STAGE >> 4), bu = b_lo + u * (C::ACT_SUB >> 4);
+            umma_f16_split<PAIR>(d_tmem, au, a_hi, bu, b_hi, idesc, (uint32_t)(u != 0 || s != 0));
+            umma_f16_split<PAIR>(d_tmem, au + a_k, a_hi, bu + b_k, b_hi, idesc, 1u);
+            umma_f16_split<PAIR>(d_tmem, au + 2 * a_k, a_hi, bu + 2 * b_k, b_hi, idesc, 1u);
+            umma_f16_split<PAIR>(d_tmem, au + 3 * a_k, a_hi, bu + 3 * b_k, b_hi, idesc, 1u);
+          }
           step_done();
         }
-        if (ok && n_steps > s_main) {
+        if (ok && n_steps > n_main_st) {
           if (!step_ready()) { ok = false; break; }
-          const uint32_t a_lo = (uint32_t)a_d0 + (uint32_t)st * (W_STAGE >> 4);
+          const uint32_t a_lo = (uint32_t)a_d0 + (uint32_t)st * (C::W_BYTES >> 4);
           const uint32_t b_lo = (uint32_t)b_d0 + (uint32_t)st * (C::ACT_STAGE >> 4);
 #pragma unroll 1
           for (int kk = 0; kk < p.lora_mmas; ++kk)
@@ -605,6 +622,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       const int grp = t / UTG, tg = t % UTG;
       const UnitDst ud(tg & 127);
       const uint32_t w_base = smem_u32(sW);
+      constexpr int BB = PACKED ? C::RAW_STAGE / (2 * KS) : 0;  // bytes of a brick
       int st = 0, rs = 0, turn = 0;  // ring positions of the current step, and the group whose step it is
       uint32_t ph = 0, rph = 0;
       bool ok = true;
@@ -612,16 +630,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         QG_ITEM_DECODE(item);
         (void)tile; (void)s_begin;
         for (int s = 0; s < n_steps; ++s) {
-          const bool main_step = s < s_main;
+          const bool main_step = s < n_main_st;
           if (turn == grp) {
+            const int subs = KS == 1 ? 1 : min(KS, s_main - s * KS);
             if (!mbar_wait(&stage_empty[st], ph ^ 1, p.status, 201)) { ok = false; break; }
             if (CONV && main_step) {
               // the TMA'd 16-bit weight tile has the other 16-bit type: convert it in place
               // (element-wise, so the swizzled placement is untouched)
               if (!mbar_wait(&full[st], ph, p.status, 203)) { ok = false; break; }
-              uint4* tile16 = (uint4*)(sW + st * W_STAGE);
-#pragma unroll
-              for (int i = 0; i < 1024 / UTG; ++i) {
+              uint4* tile16 = (uint4*)(sW + st * C::W_BYTES);
+              for (int i = 0; i < subs * 1024 / UTG; ++i) {
                 uint4 v = tile16[tg + i * UTG];
                 uint32_t* w = (uint32_t*)&v;
 #pragma unroll
@@ -640,15 +658,20 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
             }
             if (PACKED && main_step) {
               if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
-              const uint8_t* raw = sRaw + rs * C::RAW_STAGE;
-              const uint32_t dst = w_base + (uint32_t)st * W_STAGE;
-              // two bricks per tile: brick b fills the 8 KB half b
-              if (p.act_f16) {
+              // two bricks per 64-element tile: brick b fills the 8 KB half b.  A stage of two tiles goes to the
+              // two halves of the group.
+              const int u = tg >> 7;
+              if (u < subs) {
+                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : 2 * u * BB);
+                const int next = p.dir == QG_FWD ? KS * BB : BB;
+                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * W_STAGE;
+                if (p.act_f16) {
 #pragma unroll
-                for (int b = 0; b < 2; ++b) unpack_unit<FMT, false>(raw + b * (C::RAW_STAGE / 2), tg, dst + b * 8192, ud);
-              } else {
+                  for (int b = 0; b < 2; ++b) unpack_unit<FMT, false>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                } else {
 #pragma unroll 1
-                for (int b = 0; b < 2; ++b) unpack_unit<FMT, true>(raw + b * (C::RAW_STAGE / 2), tg, dst + b * 8192, ud);
+                  for (int b = 0; b < 2; ++b) unpack_unit<FMT, true>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                }
               }
               fence_proxy_async_smem();
             }
@@ -677,7 +700,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       int rs = 0;
       uint32_t rph = 0;
       bool ok = true;
-      constexpr uint32_t bb = (uint32_t)C::RAW_STAGE / 2;
+      constexpr uint32_t bb = (uint32_t)C::RAW_STAGE / (2 * KS);
       for (int item = worker; item < n_items && ok; item += n_workers) {
         QG_ITEM_DECODE(item);
         (void)n_steps;
@@ -689,14 +712,17 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         const uint8_t* b0 = p.bricks + (p.dir == QG_FWD ? ((size_t)br * p.nbk + s_begin) * bb : ((size_t)s_begin * p.nbk + br) * bb);
         const size_t b1 = p.dir == QG_FWD ? (size_t)p.nbk * bb : (size_t)bb;    // the tile's second brick
         const size_t step = p.dir == QG_FWD ? (size_t)bb : (size_t)p.nbk * bb;  // the next contraction step
-        for (int si = 0; si < s_main; ++si, b0 += step) {
+        for (int si = 0; si < n_main_st; ++si, b0 += KS * step) {
           if (!mbar_wait(&raw_empty[rs], rph ^ 1, p.status, 102)) { ok = false; break; }
-          mbar_expect_tx(&raw_full[rs], 2 * bb);
-          if (p.dir == QG_FWD) {
-            bulk_load_1d(sRaw + rs * C::RAW_STAGE, b0, bb, &raw_full[rs]);
-            bulk_load_1d(sRaw + rs * C::RAW_STAGE + bb, b0 + b1, bb, &raw_full[rs]);
-          } else {
-            bulk_load_1d(sRaw + rs * C::RAW_STAGE, b0, 2 * bb, &raw_full[rs]);  // column neighbours are adjacent
+          const uint32_t subs = KS == 1 ? 1u : (uint32_t)min(KS, s_main - si * KS);
+          uint8_t* dst = sRaw + rs * C::RAW_STAGE;
+          mbar_expect_tx(&raw_full[rs], subs * 2 * bb);
+          if (p.dir == QG_FWD) {  // a brick row's steps are adjacent
+            bulk_load_1d(dst, b0, subs * bb, &raw_full[rs]);
+            bulk_load_1d(dst + KS * bb, b0 + b1, subs * bb, &raw_full[rs]);
+          } else {  // column neighbours are adjacent
+            bulk_load_1d(dst, b0, 2 * bb, &raw_full[rs]);
+            if (KS > 1 && subs > 1) bulk_load_1d(dst + 2 * bb, b0 + step, 2 * bb, &raw_full[rs]);
           }
           if (++rs == NR) { rs = 0; rph ^= 1; }
         }
@@ -937,10 +963,11 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 // Which kernel and token-tile width a product gets: the one whose persistent grid is estimated to finish
 // first, rounds of tiles x (contraction steps x the step's time + a tile's fixed time).  The step times
 // (us, 64 contraction elements) are fitted to sweeps over both kernels and all widths (eight weight shapes
-// of 128..151936 rows, 1..8192 tokens): about 0.33 while the single-thread roles and the unpack passes set the
-// pace, which a pair's tile leaves behind from about 64 tokens of width per CTA on, when the MMAs do.
+// of 128..151936 rows, 1..8192 tokens): about 0.33 for a pair while the single-thread roles and the unpack
+// passes set the pace, more from about 64 tokens of width per CTA on, when the MMAs do; 0.25 for narrow
+// tiles, which hand over two steps at a time.
 // Narrow tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
-// backward at 1024 tokens 36 us (44 on pairs of 128 tokens before), 1024x1024 at 157 tokens 10 us (15).
+// backward at 1024 tokens 31 us (44 on pairs of 128 tokens before), 1024x1024 at 157 tokens 10 us (15).
 // The choice changes no result: an output element's contraction is one chain in any tile.
 struct QPlan {
   int kind, TN;
@@ -956,8 +983,8 @@ static QPlan qgemm_plan(int kfmt, bool tok_mode, int M, int out_rows, int n_spli
     const double cost = (double)((tiles + workers - 1) / workers) * (steps * step_us + 0.5);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {kind, tn}; }
   };
-  if (M > 32) consider(QK_NARROW, 64, 0.325);
-  consider(QK_NARROW, 32, 0.325);
+  if (M > 32) consider(QK_NARROW, 64, 0.25);
+  consider(QK_NARROW, 32, 0.25);
   if (kfmt == QF_16CONV) {
     for (int tn = 256; tn >= 128; tn -= 32) consider(QK_WIDE, tn, 0.25 + 0.0012 * tn);
   } else if (g_pair_workers > 0 && M > 64) {
