@@ -342,9 +342,9 @@ int fwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
 // factor / top (top = a power of two >= the largest factor, so the weights change no mantissa),
 // and dQ rows get their own factor back.
 //
-// Both kernels: sixteen compute warps in two groups that take alternate work items, so one group's
-// exponentials run under the other's products and four warps per scheduler cover each other's
-// latencies; in a group, warps w and w + 4 share TMEM lane quarter w and take 32 of an item's 64
+// Both kernels keep sixteen compute warps on an SM in two groups, so one group's exponentials run
+// under the other's products and four warps per scheduler cover each other's latencies: in one CTA that
+// takes alternate work items (dK/dV), or as two CTAs (dQ).  In a group, warps w and w + 4 share TMEM lane quarter w and take 32 of an item's 64
 // columns each.  P and dS go back into the TMEM columns that S and dP came in, as the A operands of
 // the next products: no shared-memory round trip, no proxy fence, and no wait for a buffer, because
 // an item's scores are issued after the products that read the P of the item two before, and the
@@ -355,10 +355,11 @@ int fwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
 // Thread = key row = TMEM lane.  K and V stay in shared memory; the query tiles of 64 rows that can see
 // these keys stream through a ring.  Per item: S^T = K.Q^T and dP^T = V.dO^T into TMEM, the threads
 // turn them into P^T and dS^T, then dV += P^T.dO and dK += dS^T.Q with Q and dO read MN-major from the
-// same tiles.  The query heads that share a KV head go to the CTAs of one cluster (up to eight), whose
+// same tiles.  More than three query heads to a KV head go to the CTAs of one cluster (up to eight), whose
 // sums meet in shared memory at the end and are added in head order: with two KV heads, one CTA per
 // key tile left the GPU waiting for the first tiles of each sequence (8 x 1024 tokens, 14 heads over
-// 2: 172 us).  TMEM: 2 x 64 + 2 x 64 + hd + hd columns (512 for hd = 128).
+// 2: 172 us); for two or three heads the exchange costs more than it gives (16 heads over 8, 16 x 512:
+// 137 us against 112).  The line depends on the model only, so a sequence's sums do not depend on its batch.  TMEM: 2 x 64 + 2 x 64 + hd + hd columns (512 for hd = 128).
 // P (<= 1, times a row weight <= 1) and dS are handed to the tensor cores in f16, whose normal
 // range ends at 6e-5: attention probabilities of long rows and the gradients of lightly weighted
 // rows live below that.  They are therefore stored times a power of two (exact), which the f32
@@ -370,6 +371,13 @@ constexpr int BWD_THREADS = 576, BWD_TMA_WARP = 16, BWD_MMA_WARP = 17;  // warps
 constexpr int MAX_HEAD_CTAS = 8;  // portable cluster size
 enum { SITE_B_KV = 451, SITE_B_QFREE, SITE_B_QFULL, SITE_B_PFULL, SITE_B_SFULL, SITE_B_PDDONE, SITE_B_END };
 
+// What dK/dV needs per (head, query row), prepared by the delta kernel as [nh][query_pitch(M)] f32 (whole
+// tiles, so that a tile's 64 values are one aligned bulk copy): the exponent offset
+// log2(weight * 2^14) - lse * log2(e), so that P.w.2^14 = 2^(s.scale.log2(e) + offset), -inf for rows past the
+// batch and rows of weight 0; and -delta * scale * 2^10 / 2^14.  (Gathered per item by the producer warp, their
+// latency, not the products, set the pace: 3400 cycles per item.)
+__host__ __device__ inline size_t query_pitch(int M) { return ((size_t)M + 63) / 64 * 64; }
+
 template <int HD>
 struct DkvLayout {
   static constexpr int PAN = HD / 64;
@@ -378,7 +386,7 @@ struct DkvLayout {
   static constexpr int NS = 4;  // ring of items: Q, dO and the per-query vectors; a slot is released by the item's last product
   static constexpr uint32_t OFF_K = 0, OFF_V = KV_BYTES, OFF_Q = 2 * KV_BYTES, OFF_DO = OFF_Q + NS * Q_BYTES;
   static constexpr uint32_t OFF_AUX = OFF_DO + NS * Q_BYTES;
-  static constexpr uint32_t AUX_BYTES = 5 * BQ * 4;  // exponent offset, -delta * scale, seq_start, gap.x, gap.y per query row
+  static constexpr uint32_t AUX_BYTES = 2 * BQ * 4;  // exponent offset and scaled -delta per query row
   static constexpr uint32_t OFF_BAR = OFF_AUX + NS * AUX_BYTES;
   static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 1024;
   static constexpr uint32_t COL_ST = 0, COL_DPT = 2 * BQ, COL_DV = 4 * BQ, COL_DK = 4 * BQ + HD;
@@ -399,7 +407,7 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                         const float* __restrict__ do_scale, const float* __restrict__ row_scale,
-                        const float* __restrict__ lse, const float* __restrict__ delta, const int* __restrict__ seq_start,
+                        const float* __restrict__ query_vecs, const int* __restrict__ seq_start,
                         const int2* __restrict__ gap, const int2* __restrict__ tiles, int M, int nh, int nkv, int heads_per_cta,
                         int n_ctas, float scale, float* __restrict__ dk, float* __restrict__ dv, int* status) {
   using L = DkvLayout<HD>;
@@ -429,7 +437,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
     for (int i = 0; i < NS; ++i) {
-      mbar_init(&q_full[i], 2);  // the expect-tx arrival + the producer warp's arrival after the vectors
+      mbar_init(&q_full[i], 1);
       mbar_init(&q_free[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -455,47 +463,31 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 
   bool ok = true;
   if (warp == BWD_TMA_WARP) {
-    // ------------------------------------------------------------ producer: TMA + the per-query vectors
+    // ------------------------------------------------------------ producer
     if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * L::KV_BYTES);
       for (int p = 0; p < L::PAN; ++p) {
         tma_load_2d(sm + L::OFF_K + p * L::KV_PANEL, &tm_k, g * HD + p * 64, n0, kv_full);
         tma_load_2d(sm + L::OFF_V + p * L::KV_PANEL, &tm_v, g * HD + p * 64, n0, kv_full);
       }
-    }
-    int rb = 0, qt = 0, h = h0;
-    uint32_t ph = 0;
-    for (int it = 0; it < n_items; ++it) {
-      const int m0 = n0 + qt * BQ;
-      if (!mbar_wait(&q_free[rb], ph ^ 1, status, SITE_B_QFREE)) break;
-      __syncwarp();
-      if (elect_one()) {
-        mbar_expect_tx(&q_full[rb], 2 * L::Q_BYTES);
+      const size_t pitch = query_pitch(M);
+      int rb = 0, qt = 0, h = h0;
+      uint32_t ph = 0;
+      for (int it = 0; it < n_items; ++it) {
+        const int m0 = n0 + qt * BQ;
+        if (!mbar_wait(&q_free[rb], ph ^ 1, status, SITE_B_QFREE)) break;
+        mbar_expect_tx(&q_full[rb], 2 * L::Q_BYTES + L::AUX_BYTES);
         for (int p = 0; p < L::PAN; ++p) {
           tma_load_2d(sm + L::OFF_Q + rb * L::Q_BYTES + p * L::Q_PANEL, &tm_q, h * HD + p * 64, m0, &q_full[rb]);
           tma_load_2d(sm + L::OFF_DO + rb * L::Q_BYTES + p * L::Q_PANEL, &tm_do, h * HD + p * 64, m0, &q_full[rb]);
         }
+        const float* vec = query_vecs + (size_t)h * pitch + m0;
+        uint8_t* aux = sm + L::OFF_AUX + rb * L::AUX_BYTES;
+        bulk_load_1d(aux, vec, BQ * 4, &q_full[rb]);
+        bulk_load_1d(aux + BQ * 4, vec + (size_t)nh * pitch, BQ * 4, &q_full[rb]);
+        if (++rb == NS) { rb = 0; ph ^= 1; }
+        if (++qt == nqt) { qt = 0; ++h; }
       }
-      float* aux = (float*)(sm + L::OFF_AUX + rb * L::AUX_BYTES);
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int il = lane + 32 * k, m = m0 + il;
-        const bool in = m < M;
-        // With per-row factors do_scale[m] is the largest factor (a power of two) of m's own sequence and
-        // do_scale[M + m] the row's weight against it.  The weight and the boost go into the exponent:
-        // P.w.2^14 = 2^(s.scale.log2(e) + this); rows past the batch and rows of weight 0 get -inf.
-        const float w = in ? (row_scale ? do_scale[M + m] : 1.0f) : 0.f;
-        aux[il] = w > 0.f ? log2f(w) + P_BOOST_LOG2 - lse[(size_t)h * M + m] * LOG2E : -INFINITY;
-        aux[BQ + il] = in ? -delta[(size_t)h * M + m] * (scale * (DS_BOOST / P_BOOST)) : 0.f;
-        ((int*)aux)[2 * BQ + il] = in ? seq_start[m] : 0x7fffffff;
-        const int2 gp = (gap && in) ? gap[m] : make_int2(0, 0);
-        ((int*)aux)[3 * BQ + il] = gp.x;
-        ((int*)aux)[4 * BQ + il] = gp.y;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&q_full[rb]);  // (release: the warp's vectors are visible to whoever passes the barrier)
-      if (++rb == NS) { rb = 0; ph ^= 1; }
-      if (++qt == nqt) { qt = 0; ++h; }
     }
   } else if (warp == BWD_MMA_WARP) {
     // ------------------------------------------------------------ MMA issue (one thread)
@@ -558,6 +550,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     const uint64_t sl2v = f32x2(sl2, sl2), dscv = f32x2(dsc, dsc);
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const uint32_t st_col = lane_addr + L::COL_ST + grp * BQ + hf * 32, dp_col = lane_addr + L::COL_DPT + grp * BQ + hf * 32;
+    const int ss_last = seq_start[min(n0 + 128, M) - 1];  // where the sequence of the tile's last key starts
     int qt = grp < nqt ? grp : grp % nqt;  // query tile of the item, advanced by two
     for (int it = grp; it < n_items; it += 2) {
       const int rb = it % NS;
@@ -565,13 +558,13 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       qt += 2;
       while (qt >= nqt) qt -= nqt;
       if (!mbar_wait(&s_full[grp], ((uint32_t)it >> 1) & 1, status, SITE_B_SFULL)) { ok = false; break; }
-      // (completed long ago; passing it orders the producer lanes' per-query vectors before the reads below)
+      // (completed long ago; passing it makes the copied per-query vectors visible here)
       if (!mbar_wait(&q_full[rb], (uint32_t)(it / NS) & 1, status, SITE_B_QFULL)) { ok = false; break; }
       tc_fence_after();
       const float* aux = (const float*)(sm + L::OFF_AUX + rb * L::AUX_BYTES);
-      const int* auxi = (const int*)aux;
-      // a tile whose queries all lie past these keys, inside one sequence, without hidden ranges, needs no mask
-      const bool need_mask = (m0 < n0 + 127) || auxi[2 * BQ + BQ - 1] > n0;  // (rows past the batch carry INT_MAX)
+      // A tile whose queries all lie past these keys, inside the sequence of all of them, without hidden
+      // ranges, needs no mask.  (Past the last key every query up to tile.y is of that key's sequence.)
+      const bool need_mask = m0 < n0 + 127 || ss_last > n0 || m0 + BQ > tile.y;
 #pragma unroll
       for (int h2 = 0; h2 < 2; ++h2) {  // 16 of this thread's 32 query columns at a time: what the registers have room for
         uint32_t st[16], dp[16], ph[8], dh[8];
@@ -588,16 +581,18 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
           const float2 x1 = unpack_f32x2(fma_f32x2(f32x2(__uint_as_float(st[c4 * 4 + 2]), __uint_as_float(st[c4 * 4 + 3])), sl2v, f32x2(ea.z, ea.w)));
           float pv[4] = {ex2_approx(x0.x), ex2_approx(x0.y), ex2_approx(x1.x), ex2_approx(x1.y)};
           if (need_mask) {
-            const int4 sq = *(const int4*)(auxi + 2 * BQ + il0);
-            const int sqv[4] = {sq.x, sq.y, sq.z, sq.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) pv[e] = (j <= m0 + il0 + e && j >= sqv[e]) ? pv[e] : 0.f;
+            for (int e = 0; e < 4; ++e) {
+              const int m = m0 + il0 + e;
+              pv[e] = (j <= m && j >= seq_start[min(m, M - 1)]) ? pv[e] : 0.f;  // (rows past the batch: p is 0 already)
+            }
           }
           if (gap != nullptr) {
-            const int4 ga = *(const int4*)(auxi + 3 * BQ + il0), gb = *(const int4*)(auxi + 4 * BQ + il0);
-            const int gav[4] = {ga.x, ga.y, ga.z, ga.w}, gbv[4] = {gb.x, gb.y, gb.z, gb.w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e) pv[e] = (j < gav[e] || j >= gbv[e]) ? pv[e] : 0.f;
+            for (int e = 0; e < 4; ++e) {
+              const int2 gm = gap[min(m0 + il0 + e, M - 1)];
+              pv[e] = (j < gm.x || j >= gm.y) ? pv[e] : 0.f;
+            }
           }
           const uint64_t d0 = fma_f32x2(f32x2(__uint_as_float(dp[c4 * 4]), __uint_as_float(dp[c4 * 4 + 1])), dscv, f32x2(de.x, de.y));
           const uint64_t d1 = fma_f32x2(f32x2(__uint_as_float(dp[c4 * 4 + 2]), __uint_as_float(dp[c4 * 4 + 3])), dscv, f32x2(de.z, de.w));
@@ -680,8 +675,10 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 // ------------------------------------------------------------------ dQ: one CTA per (128 query rows, head)
 // Thread = query row = TMEM lane.  Q and dO stay in shared memory; per key tile of 64:
 // S = Q.K^T and dP = dO.V^T into TMEM, dS = P*(dP - delta)*scale back into S's columns in f16, then
-// dQ += dS.K with K read MN-major from the tile that just served Q.K^T.  K and V tiles go through
-// a ring of four slots each (a K slot is released by the tile's dQ product).
+// dQ += dS.K with K read MN-major from the tile that just served Q.K^T.  Two CTAs fit an SM (112 KB of
+// shared memory, 256 TMEM columns, eight compute warps each): they are each other's second group, and
+// one's prologue and output run under the other's tiles, which is most of the time at 512 tokens a
+// sequence.
 enum { SITE_Q_QDO = 471, SITE_Q_KFREE, SITE_Q_VFREE, SITE_Q_KFULL, SITE_Q_VFULL, SITE_Q_DSFULL, SITE_Q_SFULL, SITE_Q_DQDONE, SITE_Q_END };
 
 template <int HD>
@@ -689,36 +686,44 @@ struct DqLayout {
   static constexpr int PAN = HD / 64;
   static constexpr uint32_t Q_PANEL = BM * 128, KV_PANEL = BN * 128;
   static constexpr uint32_t Q_BYTES = PAN * Q_PANEL, KV_BYTES = PAN * KV_PANEL;
-  static constexpr int NS = 4;
-  static constexpr uint32_t OFF_Q = 0, OFF_DO = Q_BYTES, OFF_K = 2 * Q_BYTES, OFF_V = OFF_K + NS * KV_BYTES;
-  static constexpr uint32_t OFF_BAR = OFF_V + NS * KV_BYTES;
-  static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 1024;
-  static constexpr uint32_t COL_S = 0, COL_DP = 2 * BN, COL_DQ = 4 * BN, TMEM_COLS = 512;
+  static constexpr int NK = 2;  // K slots (a slot is released by its tile's dQ product; V's one slot by the dP product)
+  static constexpr uint32_t OFF_Q = 0, OFF_DO = Q_BYTES, OFF_K = 2 * Q_BYTES, OFF_V = OFF_K + NK * KV_BYTES;
+  static constexpr uint32_t OFF_BAR = OFF_V + KV_BYTES;
+  static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 768;  // slack as in the forward's layout
+  static constexpr uint32_t COL_S = 0, COL_DP = BN, COL_DQ = 2 * BN, TMEM_COLS = 256;
 };
 
+constexpr int DQ_THREADS = 320, DQ_TMA_WARP = 8, DQ_MMA_WARP = 9;  // warps 0-7 compute
+
 template <int HD>
-__global__ void __launch_bounds__(BWD_THREADS, 1)
+__global__ void __launch_bounds__(DQ_THREADS, 2)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const float* __restrict__ do_scale, const float* __restrict__ row_scale, const float* __restrict__ lse,
-                      const float* __restrict__ delta, const int* __restrict__ seq_start, const int2* __restrict__ gap,
+                      const float* __restrict__ query_vecs, const int* __restrict__ seq_start, const int2* __restrict__ gap,
                       const int* __restrict__ tiles, int M, int nh, int nkv, float scale, float* __restrict__ dq, int* status) {
   using L = DqLayout<HD>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
-  uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+  const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;
   pdl_launch_dependents();
+  if (pad + L::USED > L::TOTAL) {
+    pdl_wait();
+    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_CUDA);
+    return;
+  }
+  uint8_t* sm = smem_raw + pad;
   uint64_t* bars = (uint64_t*)(sm + L::OFF_BAR);
-  constexpr int NS = L::NS;
+  constexpr int NK = L::NK;
   uint64_t* qdo_full = bars + 0;
-  uint64_t* k_full = bars + 1;            // [NS]
-  uint64_t* v_full = bars + 1 + NS;       // [NS]
-  uint64_t* k_free = bars + 1 + 2 * NS;   // [NS]
-  uint64_t* v_free = bars + 1 + 3 * NS;   // [NS]
-  uint64_t* s_full = bars + 1 + 4 * NS;   // [2]
-  uint64_t* ds_full = bars + 3 + 4 * NS;  // [2]
-  uint64_t* dq_done = bars + 5 + 4 * NS;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 6 + 4 * NS);
+  uint64_t* k_full = bars + 1;            // [NK]
+  uint64_t* k_free = bars + 1 + NK;       // [NK]
+  uint64_t* v_full = bars + 1 + 2 * NK;
+  uint64_t* v_free = bars + 2 + 2 * NK;
+  uint64_t* s_full = bars + 3 + 2 * NK;
+  uint64_t* ds_full = bars + 4 + 2 * NK;
+  uint64_t* dq_done = bars + 5 + 2 * NK;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 6 + 2 * NK);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   // the tiles that see the most keys start first, every head of one before the next
@@ -729,16 +734,14 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 
   if (threadIdx.x == 0) {
     mbar_init(qdo_full, 1);
-    for (int i = 0; i < NS; ++i) {
+    for (int i = 0; i < NK; ++i) {
       mbar_init(&k_full[i], 1);
-      mbar_init(&v_full[i], 1);
       mbar_init(&k_free[i], 1);
-      mbar_init(&v_free[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&ds_full[i], 8);
-    }
+    mbar_init(v_full, 1);
+    mbar_init(v_free, 1);
+    mbar_init(s_full, 1);
+    mbar_init(ds_full, 8);
     mbar_init(dq_done, 1);
     mbar_fence_init();
     prefetch_tmap(&tm_q);
@@ -746,7 +749,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     prefetch_tmap(&tm_k);
     prefetch_tmap(&tm_v);
   }
-  if (warp == BWD_MMA_WARP) {
+  if (warp == DQ_MMA_WARP) {
     tmem_alloc(tmem_slot, L::TMEM_COLS);
     tmem_relinquish();
   }
@@ -756,68 +759,66 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   pdl_wait();
 
-  if (warp == BWD_TMA_WARP) {
+  if (warp == DQ_TMA_WARP) {
     if (elect_one()) {
       mbar_expect_tx(qdo_full, 2 * L::Q_BYTES);
       for (int p = 0; p < L::PAN; ++p) {
         tma_load_2d(sm + L::OFF_Q + p * L::Q_PANEL, &tm_q, h * HD + p * 64, m0, qdo_full);
         tma_load_2d(sm + L::OFF_DO + p * L::Q_PANEL, &tm_do, h * HD + p * 64, m0, qdo_full);
       }
-      int rb = 0;
-      uint32_t ph = 0;
       for (int n = 0; n < ntiles; ++n) {
-        const int n0 = kbeg + n * BN;
-        if (!mbar_wait(&v_free[rb], ph ^ 1, status, SITE_Q_VFREE)) break;
-        mbar_expect_tx(&v_full[rb], L::KV_BYTES);
-        for (int p = 0; p < L::PAN; ++p)
-          tma_load_2d(sm + L::OFF_V + rb * L::KV_BYTES + p * L::KV_PANEL, &tm_v, g * HD + p * 64, n0, &v_full[rb]);
-        if (!mbar_wait(&k_free[rb], ph ^ 1, status, SITE_Q_KFREE)) break;
+        const int rb = n % NK, n0 = kbeg + n * BN;
+        if (!mbar_wait(&k_free[rb], ((uint32_t)(n / NK) & 1) ^ 1, status, SITE_Q_KFREE)) break;
         mbar_expect_tx(&k_full[rb], L::KV_BYTES);
         for (int p = 0; p < L::PAN; ++p)
           tma_load_2d(sm + L::OFF_K + rb * L::KV_BYTES + p * L::KV_PANEL, &tm_k, g * HD + p * 64, n0, &k_full[rb]);
-        if (++rb == NS) { rb = 0; ph ^= 1; }
+        if (!mbar_wait(v_free, ((uint32_t)n & 1) ^ 1, status, SITE_Q_VFREE)) break;
+        mbar_expect_tx(v_full, L::KV_BYTES);
+        for (int p = 0; p < L::PAN; ++p) tma_load_2d(sm + L::OFF_V + p * L::KV_PANEL, &tm_v, g * HD + p * 64, n0, v_full);
       }
     }
-  } else if (warp == BWD_MMA_WARP) {
+  } else if (warp == DQ_MMA_WARP) {
     if (elect_one()) {
       const uint32_t idesc_s = umma_idesc(0, 0, 0, 0, BM, BN);
       const uint32_t idesc_g = umma_idesc(0, 0, 0, 1, BM, HD);
       const uint32_t sQ = smem_u32(sm + L::OFF_Q), sDO = smem_u32(sm + L::OFF_DO), sK = smem_u32(sm + L::OFF_K);
       const uint32_t sV = smem_u32(sm + L::OFF_V);
       bool ok = mbar_wait(qdo_full, 0, status, SITE_Q_QDO);
+      // S and dP have one buffer each: a tile's are issued after the product that reads the dS before them
       auto issue_s = [&](int n) -> bool {
-        const int b = n & 1, rb = n % NS;  // TMEM buffer, ring slot
-        const uint32_t rph = (uint32_t)(n / NS) & 1;
-        if (!mbar_wait(&v_full[rb], rph, status, SITE_Q_VFULL) || !mbar_wait(&k_full[rb], rph, status, SITE_Q_KFULL)) return false;
+        const int rb = n % NK;
+        if (!mbar_wait(&k_full[rb], (uint32_t)(n / NK) & 1, status, SITE_Q_KFULL)) return false;
         tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint64_t ad = umma_desc_sw128(sDO + (kk >> 2) * L::Q_PANEL + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_desc_sw128(sV + rb * L::KV_BYTES + (kk >> 2) * L::KV_PANEL + (kk & 3) * 32, 16, 1024);
-          umma_f16(tmem_base + L::COL_DP + b * BN, ad, bd, idesc_s, kk != 0);
-        }
-        umma_commit(&v_free[rb]);  // V served dP only
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint64_t ad = umma_desc_sw128(sQ + (kk >> 2) * L::Q_PANEL + (kk & 3) * 32, 16, 1024);
           const uint64_t bd = umma_desc_sw128(sK + rb * L::KV_BYTES + (kk >> 2) * L::KV_PANEL + (kk & 3) * 32, 16, 1024);
-          umma_f16(tmem_base + L::COL_S + b * BN, ad, bd, idesc_s, kk != 0);
+          umma_f16(tmem_base + L::COL_S, ad, bd, idesc_s, kk != 0);
         }
-        umma_commit(&s_full[b]);
+        if (!mbar_wait(v_full, (uint32_t)n & 1, status, SITE_Q_VFULL)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) {
+          const uint64_t ad = umma_desc_sw128(sDO + (kk >> 2) * L::Q_PANEL + (kk & 3) * 32, 16, 1024);
+          const uint64_t bd = umma_desc_sw128(sV + (kk >> 2) * L::KV_PANEL + (kk & 3) * 32, 16, 1024);
+          umma_f16(tmem_base + L::COL_DP, ad, bd, idesc_s, kk != 0);
+        }
+        umma_commit(s_full);
+        umma_commit(v_free);
         return true;
       };
-      if (ok) ok = issue_s(0) && (ntiles < 2 || issue_s(1));
+      if (ok) ok = issue_s(0);
       for (int n = 0; n < ntiles && ok; ++n) {
-        const int b = n & 1, rb = n % NS;
-        if (!mbar_wait(&ds_full[b], ((uint32_t)n >> 1) & 1, status, SITE_Q_DSFULL)) { ok = false; break; }
+        const int rb = n % NK;
+        if (!mbar_wait(ds_full, (uint32_t)n & 1, status, SITE_Q_DSFULL)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
           const uint64_t bd = umma_desc_sw128(sK + rb * L::KV_BYTES + kk * 2048, L::KV_PANEL, 1024);  // K tile read MN-major: rows are keys
-          umma_f16_ta(tmem_base + L::COL_DQ, tmem_base + L::COL_S + b * BN + (kk >> 1) * 32 + (kk & 1) * 8, bd, idesc_g, (n | kk) != 0);
+          umma_f16_ta(tmem_base + L::COL_DQ, tmem_base + L::COL_S + (kk >> 1) * 32 + (kk & 1) * 8, bd, idesc_g, (n | kk) != 0);
         }
         umma_commit(&k_free[rb]);
-        if (n + 2 < ntiles && !issue_s(n + 2)) { ok = false; break; }
+        if (n + 1 < ntiles && !issue_s(n + 1)) { ok = false; break; }
       }
       if (ok) {
         umma_commit(dq_done);
@@ -826,7 +827,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   } else {
     // ------------------------------------------------------------ compute: query row = TMEM lane
-    const int grp = warp >> 3, quarter = warp & 3, hf = (warp >> 2) & 1;
+    const int quarter = warp & 3, hf = warp >> 2;
     const int r = quarter * 32 + lane;
     const int i = m0 + r;
     const int ss_i = i < M ? seq_start[i] : 0x7fffffff;
@@ -834,14 +835,14 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const int ss_last = seq_start[kend - 1];
     const float sl2 = scale * LOG2E, dsc = scale * DS_BOOST;
     const float l2 = i < M ? -lse[(size_t)h * M + i] * LOG2E : 0.f;
-    const float dl = i < M ? -delta[(size_t)h * M + i] * dsc : 0.f;
+    const float dl = i < M ? query_vecs[(nh + h) * query_pitch(M) + i] * P_BOOST : 0.f;  // -delta * scale * 2^10
     const uint64_t sl2v = f32x2(sl2, sl2), l2v = f32x2(l2, l2), dscv = f32x2(dsc, dsc), dlv = f32x2(dl, dl);
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const uint32_t s_col = lane_addr + L::COL_S + grp * BN + hf * 32, dp_col = lane_addr + L::COL_DP + grp * BN + hf * 32;
+    const uint32_t s_col = lane_addr + L::COL_S + hf * 32, dp_col = lane_addr + L::COL_DP + hf * 32;
     bool ok = true;
-    for (int n = grp; n < ntiles; n += 2) {
+    for (int n = 0; n < ntiles; ++n) {
       const int n0 = kbeg + n * BN;
-      if (!mbar_wait(&s_full[grp], ((uint32_t)n >> 1) & 1, status, SITE_Q_SFULL)) { ok = false; break; }
+      if (!mbar_wait(s_full, (uint32_t)n & 1, status, SITE_Q_SFULL)) { ok = false; break; }
       tc_fence_after();
       const bool need_mask = (n0 + BN - 1 > m0) || (n0 < ss_last);
       const int c_lo = ss_i - n0, c_hi = i - n0, g_lo = gp.x - n0, g_hi = gp.y - n0;
@@ -872,15 +873,15 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&ds_full[grp]);
+      if (lane == 0) mbar_arrive(ds_full);
     }
-    // each group hands out half of the columns, each of a row's two threads half of those
+    // each of a row's two threads hands out half of its columns
     if (ok && mbar_wait(dq_done, 0, status, SITE_Q_DQDONE)) {
       tc_fence_after();
       // a query row's gradient carries only that row's factor
       const float sc = (row_scale ? (i < M ? row_scale[i] : 0.f) : do_scale[0]) * (1.0f / DS_BOOST);
-      constexpr int NC = HD / 4;
-      const int c0 = (grp * 2 + hf) * NC;
+      constexpr int NC = HD / 2;
+      const int c0 = hf * NC;
       float* qrow = dq + ((size_t)i * nh + h) * HD + c0;
 #pragma unroll
       for (int c = 0; c < NC; c += 16) {
@@ -902,23 +903,24 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == BWD_MMA_WARP) {
+  if (warp == DQ_MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem_base, L::TMEM_COLS);
   }
 }
 
-// delta[h, m] = sum_d O * dO (the row sum of P * dP, src/attention.rs:282-287).  A pure stream:
-// HD / 8 lanes share a row with one 16-byte load of each operand per lane, four rows per lane
-// group in flight.
+// delta[h, m] = sum_d O * dO (the row sum of P * dP, src/attention.rs:282-287), handed on as the two
+// per-query vectors of dK/dV (see query_pitch).  A pure stream: HD / 8 lanes share a row with one 16-byte
+// load of each operand per lane, four rows per lane group in flight.
 template <int HD>
-__global__ void attn_delta_tc_kernel(const __half* __restrict__ o, const __half* __restrict__ dO, int M, int nh,
-                                     float* __restrict__ delta) {
+__global__ void attn_delta_tc_kernel(const __half* __restrict__ o, const __half* __restrict__ dO, const float* __restrict__ lse,
+                                     const float* __restrict__ weight, int M, int nh, float scale, float* __restrict__ query_vecs) {
   pdl_entry();
   constexpr int LPR = HD / 8, RPW = 32 / LPR, UN = 4;
   const int lane = threadIdx.x & 31, sub = lane % LPR, grp = lane / LPR;
   const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long total = (long long)M * nh, row0 = wg * (UN * RPW) + grp;
+  const size_t pitch = query_pitch(M);
+  const long long total = (long long)M * nh, padded = (long long)pitch * nh, row0 = wg * (UN * RPW) + grp;
   uint4 av[UN], bv[UN];
 #pragma unroll
   for (int u = 0; u < UN; ++u) {
@@ -943,7 +945,13 @@ __global__ void attn_delta_tc_kernel(const __half* __restrict__ o, const __half*
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     const long long r = row0 + u * RPW;
-    if (sub == 0 && r < total) delta[(size_t)(r % nh) * M + (size_t)(r / nh)] = s;
+    if (sub == 0 && r < padded) {
+      const int h = (int)(r % nh);
+      const size_t m = (size_t)(r / nh), at = (size_t)h * pitch + m;
+      const float w = r < total ? (weight ? weight[m] : 1.0f) : 0.f;
+      query_vecs[at] = w > 0.f ? log2f(w) + P_BOOST_LOG2 - lse[(size_t)h * M + m] * LOG2E : -INFINITY;
+      query_vecs[(size_t)nh * pitch + at] = -s * (scale * (DS_BOOST / P_BOOST));
+    }
   }
 }
 
@@ -973,9 +981,10 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   const float scale = 1.0f / sqrtf((float)HD);
   cudaStream_t st = c->stream;
   // one warp takes 4 passes of 32 / (HD / 8) rows
-  const long long delta_warps = ((long long)M * nh + (4 * 32 / (HD / 8)) - 1) / (4 * 32 / (HD / 8));
-  pdl(attn_delta_tc_kernel<HD>, (unsigned)((delta_warps * 32 + 255) / 256), 256, 0, st)(o, dO, M, nh, delta);
-  const int group = nh / nkv, hpc = (group + MAX_HEAD_CTAS - 1) / MAX_HEAD_CTAS, n_ctas = (group + hpc - 1) / hpc, n_tiles = (M + 127) / 128;
+  const long long delta_warps = ((long long)query_pitch(M) * nh + (4 * 32 / (HD / 8)) - 1) / (4 * 32 / (HD / 8));
+  pdl(attn_delta_tc_kernel<HD>, (unsigned)((delta_warps * 32 + 255) / 256), 256, 0, st)(o, dO, lse, row_scale ? do_scale + M : nullptr, M, nh,
+                                                                                       scale, delta);
+  const int group = nh / nkv, hpc = group > 3 ? (group + MAX_HEAD_CTAS - 1) / MAX_HEAD_CTAS : group, n_ctas = (group + hpc - 1) / hpc, n_tiles = (M + 127) / 128;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -990,16 +999,18 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = n_ctas > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_tc_kernel<HD>, tk128, tv128, tq64, tdo64, do_scale, row_scale, lse, (const float*)delta,
+  if (cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_tc_kernel<HD>, tk128, tv128, tq64, tdo64, do_scale, row_scale, (const float*)delta,
                          b.seq_start, gap, (const int2*)b.tiles_k, M, nh, nkv, hpc, n_ctas, scale, dk, dv, c->status_dev) != cudaSuccess)
     return 3;
-  pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, BWD_THREADS, LQ::TOTAL, st)(tq128, tdo128, tk64, tv64, do_scale, row_scale, lse, delta,
+  pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st)(tq128, tdo128, tk64, tv64, do_scale, row_scale, lse, delta,
                                                                                b.seq_start, gap, b.tiles_q, M, nh, nkv, scale, dq, c->status_dev);
   RT_COUNT_LAUNCH(3);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 
 }  // namespace
+
+size_t attn_delta_floats(int M, int nh) { return 2 * (size_t)nh * query_pitch(M); }
 
 void attn_plan_tiles(const int* seq_start, int M, int* tiles_q, int* tiles_k) {
   const int n = (M + 127) / 128;

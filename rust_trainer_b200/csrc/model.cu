@@ -1046,7 +1046,7 @@ static bool ensure_tokens(rt_model* m, int M) {
   ok &= m->n1.reserve(T * d * 2 * L) && m->n2.reserve(T * d * 2 * L);
   ok &= m->q_raw.reserve(T * (qd + 2 * kvd) * 4 * L);  // q | k | v before RoPE
   ok &= m->q16.reserve(T * qd * 2 * L) && m->k16.reserve(T * kvd * 2 * L) && m->v16.reserve(T * kvd * 2 * L) && m->o16.reserve(T * qd * 2 * L);
-  ok &= m->lse.reserve(T * g.n_heads * 4 * L) && m->delta.reserve(T * g.n_heads * 4);
+  ok &= m->lse.reserve(T * g.n_heads * 4 * L) && m->delta.reserve(attn_delta_floats(M, g.n_heads) * 4);
   ok &= m->g16.reserve(T * ff * 2 * 2 * L) && m->hm16.reserve(T * ff * 2 * L);  // gate | up
   ok &= m->dx.reserve(T * d * 4) && m->dy16.reserve(T * d * 2) && m->sc_y.reserve(T * 4);
   ok &= m->dhm.reserve(T * ff * 2) && m->dg16.reserve(T * ff * 2 * 2);  // d(gate) | d(up)

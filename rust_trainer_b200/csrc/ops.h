@@ -114,6 +114,8 @@ struct AttnBatch {
   const int *seq_start, *gap, *tiles_q, *tiles_k;
   int M;
 };
+// floats of the `delta` workspace of the backward
+size_t attn_delta_floats(int M, int nh);
 // fills the two tile lists (host memory, n and 2 n ints for n = ceil(M / 128) tiles) from seq_start (host memory)
 void attn_plan_tiles(const int* seq_start, int M, int* tiles_q, int* tiles_k);
 int launch_attn_bwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,

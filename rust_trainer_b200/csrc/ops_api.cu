@@ -226,7 +226,7 @@ rt_status rt_op_attention_backward(rt_ctx* c, const float* q, const float* k, co
   attn_plan_tiles(seq_start, (int)M, tq.data(), tk.data());
   int *tqd = t.up(tq.data(), nt, c->stream), *tkd = t.up(tk.data(), 2 * nt, c->stream);
   __half *q16 = t.get<__half>(nq), *k16 = t.get<__half>(nk), *v16 = t.get<__half>(nk), *o16 = t.get<__half>(nq), *do16 = t.get<__half>(nq);
-  float *lsed = t.get<float>(M * nh), *delta = t.get<float>(M * nh), *sc = t.get<float>(M), *amax = t.get<float>(2 * M + 4);
+  float *lsed = t.get<float>(M * nh), *delta = t.get<float>(attn_delta_floats((int)M, nh)), *sc = t.get<float>(M), *amax = t.get<float>(2 * M + 4);
   float *dqd = t.get<float>(nq), *dkd = t.get<float>(nk), *dvd = t.get<float>(nk);
   if (!qd || !kd || !vd || !dod || !ss || !tqd || !tkd || !q16 || !k16 || !v16 || !o16 || !do16 || !lsed || !delta || !sc || !amax || !dqd || !dkd || !dvd)
     return c->fail(RT_ERR_CUDA, "out of device memory");
