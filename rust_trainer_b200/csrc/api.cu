@@ -65,6 +65,7 @@ int frozen_matmul_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   lo.dense16_lo = nullptr;
   QGemmArgs b = a;  // the low term adds into the result; bias and the adapter chunk went in with the high term
   b.accumulate = 1;
+  b.late_wait = 0;
   b.residual = nullptr;
   b.bias = nullptr;
   b.lora = LoraSide();

@@ -355,11 +355,11 @@ int fwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
 // Thread = key row = TMEM lane.  K and V stay in shared memory; the query tiles of 64 rows that can see
 // these keys stream through a ring.  Per item: S^T = K.Q^T and dP^T = V.dO^T into TMEM, the threads
 // turn them into P^T and dS^T, then dV += P^T.dO and dK += dS^T.Q with Q and dO read MN-major from the
-// same tiles.  More than three query heads to a KV head go to the CTAs of one cluster (up to eight), whose
-// sums meet in shared memory at the end and are added in head order: with two KV heads, one CTA per
-// key tile left the GPU waiting for the first tiles of each sequence (8 x 1024 tokens, 14 heads over
-// 2: 172 us); for two or three heads the exchange costs more than it gives (16 heads over 8, 16 x 512:
-// 137 us against 112).  The line depends on the model only, so a sequence's sums do not depend on its batch.  TMEM: 2 x 64 + 2 x 64 + hd + hd columns (512 for hd = 128).
+// same tiles.  A CTA takes four of the query heads that share a KV head; more go to the CTAs of one cluster
+// (up to eight), whose sums meet in shared memory at the end and are added in head order.  (14 heads over
+// two KV heads, 8 x 1024 tokens: one CTA for the seven heads 105 us, four and three 74, clusters of four 95, of
+// seven 142; 24 heads over 8, 4 x 2048: three heads in one CTA 289 us, clusters of two 371.)  The line
+// depends on the model only, so a sequence's sums do not depend on its batch.  TMEM: 2 x 64 + 2 x 64 + hd + hd columns (512 for hd = 128).
 // P (<= 1, times a row weight <= 1) and dS are handed to the tensor cores in f16, whose normal
 // range ends at 6e-5: attention probabilities of long rows and the gradients of lightly weighted
 // rows live below that.  They are therefore stored times a power of two (exact), which the f32
@@ -406,8 +406,7 @@ template <int HD>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                        const float* __restrict__ do_scale, const float* __restrict__ row_scale,
-                        const float* __restrict__ query_vecs, const int* __restrict__ seq_start,
+                        const float* __restrict__ tops, const float* __restrict__ query_vecs, const int* __restrict__ seq_start,
                         const int2* __restrict__ gap, const int2* __restrict__ tiles, int M, int nh, int nkv, int heads_per_cta,
                         int n_ctas, float scale, float* __restrict__ dk, float* __restrict__ dv, int* status) {
   using L = DkvLayout<HD>;
@@ -615,7 +614,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
     if (ok) {
       tc_fence_after();
       // a key row only ever meets queries of its own sequence, so its sums are in units of that sequence's largest factor
-      const float top_j = row_scale ? do_scale[j < M ? j : M - 1] : do_scale[0];
+      const float top_j = tops[min(j, M - 1)];
       const float sc = n_ctas > 1 ? 1.0f : top_j * (grp == 0 ? 1.0f / DS_BOOST : 1.0f / P_BOOST);
       float* row = n_ctas > 1 ? (float*)sm + (grp * 128 + r) * L::PITCH : (grp == 0 ? dk : dv) + ((size_t)j * nkv + g) * HD;
 #pragma unroll
@@ -658,7 +657,7 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
 #pragma unroll
         for (int k = 1; k < MAX_HEAD_CTAS; ++k)
           if (k < n_ctas) { s.x += x[k].x; s.y += x[k].y; s.z += x[k].z; s.w += x[k].w; }
-        const float sc = (row_scale ? do_scale[j] : do_scale[0]) * (which == 0 ? 1.0f / DS_BOOST : 1.0f / P_BOOST);
+        const float sc = tops[j] * (which == 0 ? 1.0f / DS_BOOST : 1.0f / P_BOOST);
         *(float4*)((which == 0 ? dk : dv) + ((size_t)j * nkv + g) * HD + c) = make_float4(s.x * sc, s.y * sc, s.z * sc, s.w * sc);
       }
     __syncwarp();
@@ -699,7 +698,7 @@ template <int HD>
 __global__ void __launch_bounds__(DQ_THREADS, 2)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                      const float* __restrict__ do_scale, const float* __restrict__ row_scale, const float* __restrict__ lse,
+                      const float* __restrict__ row_scale, const float* __restrict__ lse,
                       const float* __restrict__ query_vecs, const int* __restrict__ seq_start, const int2* __restrict__ gap,
                       const int* __restrict__ tiles, int M, int nh, int nkv, float scale, float* __restrict__ dq, int* status) {
   using L = DqLayout<HD>;
@@ -879,7 +878,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (ok && mbar_wait(dq_done, 0, status, SITE_Q_DQDONE)) {
       tc_fence_after();
       // a query row's gradient carries only that row's factor
-      const float sc = (row_scale ? (i < M ? row_scale[i] : 0.f) : do_scale[0]) * (1.0f / DS_BOOST);
+      const float sc = (i < M ? row_scale[i] : 0.f) * (1.0f / DS_BOOST);
       constexpr int NC = HD / 2;
       const int c0 = hf * NC;
       float* qrow = dq + ((size_t)i * nh + h) * HD + c0;
@@ -910,26 +909,45 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 }
 
 // delta[h, m] = sum_d O * dO (the row sum of P * dP, src/attention.rs:282-287), handed on as the two
-// per-query vectors of dK/dV (see query_pitch).  A pure stream: HD / 8 lanes share a row with one 16-byte
-// load of each operand per lane, four rows per lane group in flight.
+// per-query vectors of dK/dV (see query_pitch), and the row weights: tops[m] is a power of two >= the
+// largest factor among the rows of m's own sequence (nothing a sequence's backward sees may depend on its
+// batch mates; 1 for an all-zero sequence), a row's weight its factor / tops[m].  A pure stream over O and
+// dO, one block per (128 tokens, head): HD / 8 lanes share a row with one 16-byte load of each operand per
+// lane, all of the block's loads in flight before the first use; the scan of the sequence's factors (a
+// launch of its own before, one block for the whole batch: 12 us at 8192 tokens) runs under them.
 template <int HD>
-__global__ void attn_delta_tc_kernel(const __half* __restrict__ o, const __half* __restrict__ dO, const float* __restrict__ lse,
-                                     const float* __restrict__ weight, int M, int nh, float scale, float* __restrict__ query_vecs) {
+__global__ void __launch_bounds__(256)
+attn_delta_tc_kernel(const __half* __restrict__ o, const __half* __restrict__ dO, const float* __restrict__ lse,
+                     const float* __restrict__ row_scale, const int* __restrict__ seq_start, const int2* __restrict__ tiles, int M, int nh,
+                     float scale, float* __restrict__ query_vecs, float* __restrict__ tops) {
   pdl_entry();
-  constexpr int LPR = HD / 8, RPW = 32 / LPR, UN = 4;
-  const int lane = threadIdx.x & 31, sub = lane % LPR, grp = lane / LPR;
-  const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const size_t pitch = query_pitch(M);
-  const long long total = (long long)M * nh, padded = (long long)pitch * nh, row0 = wg * (UN * RPW) + grp;
+  constexpr int LPR = HD / 8, RPW = 32 / LPR, UN = 16 / RPW;
+  __shared__ int s_max[129];     // by where the sequence starts: its first token in this tile, 128: before the tile
+  __shared__ float s_delta[128];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LPR, grp = lane / LPR;
+  const int2 tile = tiles[blockIdx.x];
+  const int h = blockIdx.y, t0 = tile.x * 128;
   uint4 av[UN], bv[UN];
 #pragma unroll
   for (int u = 0; u < UN; ++u) {
-    const long long r = row0 + u * RPW;
-    if (r < total) {
-      av[u] = *(const uint4*)(o + r * HD + sub * 8);
-      bv[u] = *(const uint4*)(dO + r * HD + sub * 8);
+    const int m = t0 + warp * 16 + u * RPW + grp;
+    const size_t at = ((size_t)m * nh + h) * HD + sub * 8;
+    av[u] = m < M ? *(const uint4*)(o + at) : make_uint4(0u, 0u, 0u, 0u);
+    bv[u] = m < M ? *(const uint4*)(dO + at) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (threadIdx.x < 129) s_max[threadIdx.x] = 0;
+  __syncthreads();
+  for (int i0 = seq_start[t0]; i0 < tile.y; i0 += 256) {
+    const int i = min(i0 + (int)threadIdx.x, tile.y - 1), ss = seq_start[i];
+    const int slot = ss < t0 ? 128 : ss - t0;
+    const int v = __float_as_int(fmaxf(row_scale[i], 0.f));  // (of values >= 0 the bits order as the values do)
+    int same;
+    __match_all_sync(0xffffffffu, slot, &same);
+    if (same) {
+      const int w = __reduce_max_sync(0xffffffffu, v);
+      if (lane == 0) atomicMax(&s_max[slot], w);
     } else {
-      av[u] = bv[u] = make_uint4(0u, 0u, 0u, 0u);
+      atomicMax(&s_max[slot], v);
     }
   }
 #pragma unroll
@@ -944,21 +962,29 @@ __global__ void attn_delta_tc_kernel(const __half* __restrict__ o, const __half*
     }
 #pragma unroll
     for (int off = LPR / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    const long long r = row0 + u * RPW;
-    if (sub == 0 && r < padded) {
-      const int h = (int)(r % nh);
-      const size_t m = (size_t)(r / nh), at = (size_t)h * pitch + m;
-      const float w = r < total ? (weight ? weight[m] : 1.0f) : 0.f;
-      query_vecs[at] = w > 0.f ? log2f(w) + P_BOOST_LOG2 - lse[(size_t)h * M + m] * LOG2E : -INFINITY;
-      query_vecs[(size_t)nh * pitch + at] = -s * (scale * (DS_BOOST / P_BOOST));
-    }
+    if (sub == 0) s_delta[warp * 16 + u * RPW + grp] = s;
   }
+  __syncthreads();
+  const int m = t0 + threadIdx.x;
+  const size_t pitch = query_pitch(M);
+  if (threadIdx.x >= 128 || (size_t)m >= pitch) return;
+  float off = -INFINITY, delta = 0.f;
+  if (m < M) {
+    const int ss = seq_start[m], mx = s_max[ss < t0 ? 128 : ss - t0];
+    const float top = mx > 0 ? __int_as_float((mx + 0x007FFFFF) & 0x7F800000) : 1.f;
+    const float w = fmaxf(row_scale[m], 0.f) / top;
+    if (h == 0) tops[m] = top;
+    if (w > 0.f) off = log2f(w) + P_BOOST_LOG2 - lse[(size_t)h * M + m] * LOG2E;
+    delta = s_delta[threadIdx.x];
+  }
+  query_vecs[(size_t)h * pitch + m] = off;
+  query_vecs[(size_t)(nh + h) * pitch + m] = -delta * (scale * (DS_BOOST / P_BOOST));
 }
 
 template <int HD>
 int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO,
-                const float* do_scale, const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, float* delta,
-                float* dq, float* dk, float* dv) {
+                const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, float* work, float* dq, float* dk,
+                float* dv) {
   const int M = b.M;
   const int2* gap = (const int2*)b.gap;
   using LK = DkvLayout<HD>;
@@ -980,11 +1006,10 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   if (tensor_map_f16_2d(c, &tv64, v, (uint64_t)M, (uint64_t)nkv * HD, 64, 64)) return 3;
   const float scale = 1.0f / sqrtf((float)HD);
   cudaStream_t st = c->stream;
-  // one warp takes 4 passes of 32 / (HD / 8) rows
-  const long long delta_warps = ((long long)query_pitch(M) * nh + (4 * 32 / (HD / 8)) - 1) / (4 * 32 / (HD / 8));
-  pdl(attn_delta_tc_kernel<HD>, (unsigned)((delta_warps * 32 + 255) / 256), 256, 0, st)(o, dO, lse, row_scale ? do_scale + M : nullptr, M, nh,
-                                                                                       scale, delta);
-  const int group = nh / nkv, hpc = group > 3 ? (group + MAX_HEAD_CTAS - 1) / MAX_HEAD_CTAS : group, n_ctas = (group + hpc - 1) / hpc, n_tiles = (M + 127) / 128;
+  float *query_vecs = work, *tops = work + 2 * (size_t)nh * query_pitch(M);
+  pdl(attn_delta_tc_kernel<HD>, dim3((M + 127) / 128, nh), 256, 0, st)(o, dO, lse, row_scale, b.seq_start, (const int2*)b.tiles_k, M, nh, scale,
+                                                                      query_vecs, tops);
+  const int group = nh / nkv, hpc = std::min(group, std::max(4, (group + MAX_HEAD_CTAS - 1) / MAX_HEAD_CTAS)), n_ctas = (group + hpc - 1) / hpc, n_tiles = (M + 127) / 128;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -999,10 +1024,10 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = n_ctas > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_tc_kernel<HD>, tk128, tv128, tq64, tdo64, do_scale, row_scale, (const float*)delta,
+  if (cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_tc_kernel<HD>, tk128, tv128, tq64, tdo64, (const float*)tops, (const float*)query_vecs,
                          b.seq_start, gap, (const int2*)b.tiles_k, M, nh, nkv, hpc, n_ctas, scale, dk, dv, c->status_dev) != cudaSuccess)
     return 3;
-  pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st)(tq128, tdo128, tk64, tv64, do_scale, row_scale, lse, delta,
+  pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st)(tq128, tdo128, tk64, tv64, row_scale, lse, query_vecs,
                                                                                b.seq_start, gap, b.tiles_q, M, nh, nkv, scale, dq, c->status_dev);
   RT_COUNT_LAUNCH(3);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
@@ -1010,7 +1035,7 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
 
 }  // namespace
 
-size_t attn_delta_floats(int M, int nh) { return 2 * (size_t)nh * query_pitch(M); }
+size_t attn_bwd_work_floats(int M, int nh) { return 2 * (size_t)nh * query_pitch(M) + (size_t)M; }
 
 void attn_plan_tiles(const int* seq_start, int M, int* tiles_q, int* tiles_k) {
   const int n = (M + 127) / 128;
@@ -1044,11 +1069,11 @@ int launch_attn_fwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half
 }
 
 int launch_attn_bwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,
-                       const float* do_scale, const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, int hd,
-                       float* delta, float* dq, float* dk, float* dv) {
+                       const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, int hd, float* work, float* dq,
+                       float* dk, float* dv) {
   if (b.M <= 0) return 0;
-  if (hd == 128) return bwd_tc_impl<128>(c, q, k, v, o, dO16, do_scale, row_scale, lse, b, nh, nkv, delta, dq, dk, dv);
-  if (hd == 64) return bwd_tc_impl<64>(c, q, k, v, o, dO16, do_scale, row_scale, lse, b, nh, nkv, delta, dq, dk, dv);
+  if (hd == 128) return bwd_tc_impl<128>(c, q, k, v, o, dO16, row_scale, lse, b, nh, nkv, work, dq, dk, dv);
+  if (hd == 64) return bwd_tc_impl<64>(c, q, k, v, o, dO16, row_scale, lse, b, nh, nkv, work, dq, dk, dv);
   return 1;
 }
 

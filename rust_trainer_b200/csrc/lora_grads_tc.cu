@@ -10,10 +10,13 @@
 //   A = Big tile   [64 tokens][128 columns]  (two swizzled panels of 64 columns, TMA)
 //   B = Small tile [64 tokens][64]           (TMA, then scaled in place, see below)
 //   D[column (lane), i] in 64 TMEM columns.
-// Warps: 0-3 scale the Small tiles and run the epilogue, 4, 6, 7 are TMA producers, 5 issues the MMAs.
+// Warps: 0-3 the epilogue, 4 the TMA producer, 5 issues the MMAs.
 // dY arrives row-normalised with one factor per token.  The factors go onto the Small rows
 // relative to the split's largest factor (rounded up to a power of two, so what a row rounds to
-// does not depend on its split mates), and the largest factor multiplies the split's sums.
+// does not depend on its split mates), and the largest factor multiplies the split's sums.  A launch of its
+// own does that for all the jobs (scaling each tile in place between its landing and its MMAs, in each
+// of the 40-odd column tiles, was the pipeline's longest link: 100 us for the four jobs of a block at 8192
+// tokens, 320 MB to read).
 // Up to eight splits (every batch of up to 8192 tokens) are one cluster: each CTA leaves its split's sums in
 // shared memory, and the CTAs add them in split order straight into the gradient buffers, each its
 // share of the tile.  (A second launch used to do that from partial sums in memory: 2.6 us per linear
@@ -31,21 +34,27 @@ namespace rt {
 
 namespace {
 
-constexpr int LG_NS = 4;
+constexpr int LG_NS = 4, LG_THREADS = 192;
 constexpr uint32_t LG_Q_BYTES = 2 * 64 * 128, LG_P_BYTES = 64 * 128, LG_STAGE = LG_Q_BYTES + LG_P_BYTES;
-constexpr uint32_t LG_OFF_SCALE = LG_NS * LG_STAGE;         // factors of this split's tokens / largest
-constexpr int LG_MAX_TPS = 1024;
-constexpr uint32_t LG_OFF_BAR = LG_OFF_SCALE + LG_MAX_TPS * 4;
+constexpr uint32_t LG_OFF_BAR = LG_NS * LG_STAGE;
 constexpr uint32_t LG_TOTAL = LG_OFF_BAR + 256 + 1024;
-enum { SITE_LG_FREE = 495, SITE_LG_FULL, SITE_LG_READY, SITE_LG_DONE };
+enum { SITE_LG_FREE = 495, SITE_LG_FULL, SITE_LG_DONE };
 
-struct LoraGradTcArgs {
-  const float* pscale;  // [M] or null
-  int M, N, K, r, nbB, tps;
-  float* partB;  // [splits][r x N]
-  float* partA;  // [splits][r x K]
-  int direct;       // the splits are one cluster: add into the members' gradients
-  LoraGroupTable t; // of one linear (offsets 0) or of a stacked group
+struct LgMaps {
+  CUtensorMap pb, qb, pa, qa;
+};
+struct LgJob {
+  const float* top;     // [splits] largest factor, or null: the rows carry none
+  int N, K, r;
+  int first, nbB;       // the job's first column tile in the grid, and how many of its tiles are dB's
+  float *partB, *partA; // [splits][r x N], [splits][r x K]
+  LoraGroupTable t;     // of one linear (offsets 0) or of a stacked group
+};
+struct LgArgs {
+  LgMaps maps[LORA_GRAD_JOBS];
+  LgJob job[LORA_GRAD_JOBS];
+  int n_jobs, M, tps;
+  int direct;  // the splits are one cluster: add into the members' gradients
 };
 // sums of a split, [rank index][128 columns + 1] f32, over the operand stages once those are used up
 constexpr int LG_PITCH = 129;
@@ -57,35 +66,34 @@ __device__ __forceinline__ float ld_cluster_f1(uint32_t cluster_addr) {
   return v;
 }
 
-__global__ void __launch_bounds__(256, 2)
-lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_constant__ CUtensorMap tm_qb,
-                     const __grid_constant__ CUtensorMap tm_pa, const __grid_constant__ CUtensorMap tm_qa,
-                     const LoraGradTcArgs g, int* status) {
+__global__ void __launch_bounds__(LG_THREADS, 2)
+lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-  float* s_scale = (float*)(sm + LG_OFF_SCALE);
   uint64_t* bars = (uint64_t*)(sm + LG_OFF_BAR);
-  uint64_t* full = bars;               // [NS] TMA landed
-  uint64_t* ready = bars + LG_NS;      // [NS] Small tile scaled
-  uint64_t* empty = bars + 2 * LG_NS;  // [NS] MMAs retired
-  uint64_t* done = bars + 3 * LG_NS;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 3 * LG_NS + 2);
-  __shared__ float s_red[4];
+  uint64_t* full = bars;           // [NS] TMA landed
+  uint64_t* empty = bars + LG_NS;  // [NS] MMAs retired
+  uint64_t* done = bars + 2 * LG_NS;
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * LG_NS + 2);
   pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
-  const bool isB = (int)blockIdx.x < g.nbB;
-  const CUtensorMap* tm_p = isB ? &tm_pb : &tm_pa;
-  const CUtensorMap* tm_q = isB ? &tm_qb : &tm_qa;
+  int jx = 0;
+  while (jx + 1 < ga.n_jobs && (int)blockIdx.x >= ga.job[jx + 1].first) ++jx;
+  const LgJob& g = ga.job[jx];
+  const LgMaps& maps = ga.maps[jx];
+  const int bx = (int)blockIdx.x - g.first;
+  const bool isB = bx < g.nbB;
+  const CUtensorMap* tm_p = isB ? &maps.pb : &maps.pa;
+  const CUtensorMap* tm_q = isB ? &maps.qb : &maps.qa;
   const int C = isB ? g.N : g.K;
-  const int j0 = (isB ? (int)blockIdx.x : (int)blockIdx.x - g.nbB) * 128;
-  const int m_begin = blockIdx.y * g.tps, m_end = min(g.M, m_begin + g.tps);
+  const int j0 = (isB ? bx : bx - g.nbB) * 128;
+  const int m_begin = blockIdx.y * ga.tps, m_end = min(ga.M, m_begin + ga.tps);
   const int nchunks = (m_end - m_begin + 63) / 64;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < LG_NS; ++i) {
-      mbar_init(&full[i], 3);  // three producer threads
-      mbar_init(&ready[i], 4);
+      mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
     mbar_init(done, 1);
@@ -103,95 +111,52 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   pdl_wait();
 
-  if (warp == 4 || warp >= 6) {
-    // three producer threads, one TMA instruction per stage each (an instruction costs its thread about 0.1 us)
+  if (warp == 4) {
     if (elect_one()) {
-      const int which = warp == 4 ? 0 : warp - 5;  // 0, 1: the two 64-column panels of Big; 2: the Small tile
+      int s = 0;
+      uint32_t ph = 0;
       for (int ch = 0; ch < nchunks; ++ch) {
-        const int s = ch % LG_NS;
-        if (!mbar_wait(&empty[s], (((uint32_t)(ch / LG_NS)) & 1) ^ 1, status, SITE_LG_FREE)) break;
+        if (!mbar_wait(&empty[s], ph ^ 1, status, SITE_LG_FREE)) break;
         const int mrow = m_begin + ch * 64;
-        mbar_expect_tx(&full[s], 8192);
-        if (which == 2) tma_load_2d(sm + s * LG_STAGE + LG_Q_BYTES, tm_p, 0, mrow, &full[s]);
-        else tma_load_2d(sm + s * LG_STAGE + which * 8192, tm_q, j0 + which * 64, mrow, &full[s]);
+        uint8_t* dst = sm + s * LG_STAGE;
+        mbar_expect_tx(&full[s], LG_STAGE);
+        tma_load_2d(dst, tm_q, j0, mrow, &full[s]);
+        tma_load_2d(dst + 8192, tm_q, j0 + 64, mrow, &full[s]);
+        tma_load_2d(dst + LG_Q_BYTES, tm_p, 0, mrow, &full[s]);
+        if (++s == LG_NS) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == 5) {
     if (elect_one()) {
       const uint32_t idesc = umma_idesc(0, 0, 1, 1, 128, 64);
-      const uint32_t s0 = smem_u32(sm);
+      const uint64_t a0 = umma_desc_sw128(smem_u32(sm), 8192, 1024), b0 = umma_desc_sw128(smem_u32(sm) + LG_Q_BYTES, 8192, 1024);
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
-      for (int ch = 0; ch < nchunks && ok; ++ch) {
-        const int s = ch % LG_NS;
-        if (!mbar_wait(&ready[s], ((uint32_t)(ch / LG_NS)) & 1, status, SITE_LG_READY)) { ok = false; break; }
+      for (int ch = 0; ch < nchunks; ++ch) {
+        if (!mbar_wait(&full[s], ph, status, SITE_LG_FULL)) { ok = false; break; }
         tc_fence_after();
+        const uint32_t off = (uint32_t)s * (LG_STAGE >> 4);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint64_t ad = umma_desc_sw128(s0 + s * LG_STAGE + kk * 2048, 8192, 1024);
-          const uint64_t bd = umma_desc_sw128(s0 + s * LG_STAGE + LG_Q_BYTES + kk * 2048, 8192, 1024);
-          umma_f16(tmem_base, ad, bd, idesc, (ch | kk) != 0);
-        }
+        for (int kk = 0; kk < 4; ++kk)
+          umma_f16_split<false>(tmem_base, (uint32_t)a0 + off + kk * (2048 >> 4), (uint32_t)(a0 >> 32), (uint32_t)b0 + off + kk * (2048 >> 4),
+                                (uint32_t)(b0 >> 32), idesc, (uint32_t)((ch | kk) != 0));
         umma_commit(&empty[s]);
+        if (++s == LG_NS) { s = 0; ph ^= 1; }
       }
       if (ok) umma_commit(done);
     }
   } else {
-    // ---- 128 threads: factors of the split, Small tiles scaled in place, then the epilogue
-    const int tid = threadIdx.x;
-    // out_mul: what the split's sums are multiplied by at the end (the split's largest factor)
-    float out_mul = 1.0f;
-    if (g.pscale) {
-      // Largest factor of the split (factors are >= 0), rounded up to a power of two so that
-      // dividing by it changes no mantissa.  (Lifting the rows further, to the top of f16's range by
-      // the largest magnitude of the split's Small rows, was tried: it needs a pass over those
-      // rows before the first tile can be scaled, 6 us of a 22 us launch, and changed no digit of
-      // the shards-against-whole-batch check once the attention backward weighed rows per sequence.)
-      float v = 0.f;
-      for (int m = m_begin + tid; m < m_end; m += 128) v = fmaxf(v, g.pscale[m]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-      if (lane == 0) s_red[warp] = v;
-      named_barrier_sync(1, 128);
-      float lmax = fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3]));
-      lmax = __int_as_float((__float_as_int(lmax) + 0x007FFFFF) & 0x7F800000);
-      const float inv = lmax > 0.f ? 1.0f / lmax : 0.f;
-      out_mul = lmax;
-      for (int m = tid; m < nchunks * 64; m += 128) s_scale[m] = (m_begin + m < m_end) ? g.pscale[m_begin + m] * inv : 0.f;
-      named_barrier_sync(1, 128);
-    }
-    bool ok = true;
-    for (int ch = 0; ch < nchunks && ok; ++ch) {
-      const int s = ch % LG_NS;
-      if (!mbar_wait(&full[s], ((uint32_t)(ch / LG_NS)) & 1, status, SITE_LG_FULL)) { ok = false; break; }
-      if (g.pscale) {
-        uint8_t* pt = sm + s * LG_STAGE + LG_Q_BYTES;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int e = tid + k * 128;  // 16-byte unit; its token row is e / 8 whatever the swizzle
-          const float f = s_scale[ch * 64 + (e >> 3)];
-          uint4* ptr = (uint4*)(pt + e * 16);
-          uint4 v = *ptr;
-          __half2* h2 = (__half2*)&v;
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 x = __half22float2(h2[q]);
-            h2[q] = __floats2half2_rn(x.x * f, x.y * f);
-          }
-          *ptr = v;
-        }
-        fence_proxy_async_smem();
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ready[s]);
-    }
-    if (ok && mbar_wait(done, 0, status, SITE_LG_DONE)) {
+    // ---- 128 threads: the epilogue
+    const float out_mul = g.top ? g.top[blockIdx.y] : 1.0f;  // what the split's sums are multiplied by
+    if (mbar_wait(done, 0, status, SITE_LG_DONE)) {
       tc_fence_after();
       uint32_t v[64];
       tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
       if (g.r > 32) tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + 32, v + 32);
       tmem_ld_wait();
       const int j = j0 + warp * 32 + lane;
-      if (g.direct) {
+      if (ga.direct) {
         float* mine = (float*)sm + warp * 32 + lane;
 #pragma unroll
         for (int i = 0; i < 64; ++i)
@@ -209,9 +174,9 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
   }
   tc_fence_before();
   __syncwarp();
-  if (g.direct && gridDim.y > 1) cluster_sync_all();  // every split's sums are in its CTA's shared memory
+  if (ga.direct && gridDim.y > 1) cluster_sync_all();  // every split's sums are in its CTA's shared memory
   else __syncthreads();
-  if (g.direct && *(volatile int*)status == 0) {
+  if (ga.direct && *(volatile int*)status == 0) {
     const int n_cta = (int)gridDim.y, ncol = min(128, C - j0);
     auto add_splits = [&](int i, int col, float* dst) {
       const uint32_t a = smem_u32(sm) + (uint32_t)(i * LG_PITCH + col) * 4u;
@@ -230,17 +195,76 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
       // a member owns whole column tiles of dB (its rows start on a multiple of 128) and r rows of dA
       if (isB && (j0 < mb.row_off || j0 >= mb.row_off + mb.rows)) continue;
       const int items = ncol * mb.r, per = (items + n_cta - 1) / n_cta, end = min(items, ((int)blockIdx.y + 1) * per);
-      for (int e = (int)blockIdx.y * per + threadIdx.x; e < end; e += 256) {
+      for (int e = (int)blockIdx.y * per + threadIdx.x; e < end; e += LG_THREADS) {
         if (isB) add_splits(mb.rank_off + e % mb.r, e / mb.r, mb.gb + (size_t)(j0 - mb.row_off) * mb.r + e);
         else add_splits(mb.rank_off + e / ncol, e % ncol, mb.ga + (size_t)(e / ncol) * g.K + j0 + e % ncol);
       }
     }
   }
   __syncwarp();
-  if (g.direct && gridDim.y > 1) cluster_sync_all();  // nobody leaves while its shared memory may still be read
+  if (ga.direct && gridDim.y > 1) cluster_sync_all();  // nobody leaves while its shared memory may still be read
   if (warp == 5) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 64);
+  }
+}
+
+// What the main kernel reads instead of Hs and Gs: row m times factor_m / (its split's largest factor).
+struct LgScaleJob {
+  const __half *hs, *gs;
+  const float* pscale;
+  __half *hs_out, *gs_out;
+  float* top;  // [splits]
+};
+struct LgScaleArgs {
+  LgScaleJob job[LORA_GRAD_JOBS];
+  int M, tps;
+};
+// one block per (64 tokens, job); a split is a multiple of 64 tokens
+__global__ void __launch_bounds__(256) lora_scale_small_kernel(const LgScaleArgs a) {
+  pdl_entry();
+  __shared__ float s_red[8];
+  const LgScaleJob& g = a.job[blockIdx.y];
+  const int m0 = blockIdx.x * 64, split = m0 / a.tps, m_begin = split * a.tps, m_end = min(a.M, m_begin + a.tps);
+  const int rows = min(64, a.M - m0), tid = threadIdx.x;
+  uint4 v[2][2];  // this thread's 16-byte units tid and tid + 256 of the 64 x 64 tile, of Hs and of Gs
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int e = tid + k * 256;
+    if ((e >> 3) < rows) {
+      v[0][k] = ((const uint4*)(g.hs + (size_t)m0 * 64))[e];
+      v[1][k] = ((const uint4*)(g.gs + (size_t)m0 * 64))[e];
+    }
+  }
+  // largest factor of the split (factors are >= 0), rounded up to a power of two so that dividing by it
+  // changes no mantissa
+  float mx = 0.f;
+  for (int m = m_begin + tid; m < m_end; m += 256) mx = fmaxf(mx, g.pscale[m]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) s_red[tid >> 5] = mx;
+  __syncthreads();
+  mx = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) mx = fmaxf(mx, s_red[k]);
+  mx = __int_as_float((__float_as_int(mx) + 0x007FFFFF) & 0x7F800000);
+  const float inv = mx > 0.f ? 1.0f / mx : 0.f;
+  if (m0 == m_begin && tid == 0) g.top[split] = mx;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int e = tid + k * 256;
+    if ((e >> 3) >= rows) continue;
+    const float f = g.pscale[m0 + (e >> 3)] * inv;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      __half2* h2 = (__half2*)&v[q][k];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 x = __half22float2(h2[i]);
+        h2[i] = __floats2half2_rn(x.x * f, x.y * f);
+      }
+      ((uint4*)((q == 0 ? g.hs_out : g.gs_out) + (size_t)m0 * 64))[e] = v[q][k];
+    }
   }
 }
 
@@ -249,40 +273,83 @@ lora_grads_tc_kernel(const __grid_constant__ CUtensorMap tm_pb, const __grid_con
 // Tokens per split of the tcgen05 contraction: fixed by the token count's range only.
 int lora_grads_tc_tokens_per_split(int M) { return M >= 4096 ? 1024 : M >= 2048 ? 512 : M >= 1024 ? 256 : M >= 512 ? 128 : 64; }
 // whether the splits fit one cluster (of the portable size), which then adds them itself
-bool lora_grads_tc_direct(int M) {
+static bool lora_grads_tc_direct(int M) {
   const int tps = lora_grads_tc_tokens_per_split(M);
   return (M + tps - 1) / tps <= 8;
 }
 
-// Up to eight splits: adds dB and dA into the gradients of the table's members, which is all there is to
-// do.  More: launches the product kernel only and leaves partial sums, partB / partA: [splits][r x N] /
-// [splits][r x K] with splits = ceil(M / lora_grads_tc_tokens_per_split(M)), for the caller to add.
-// 0: launched; 1: shape not covered; 3: launch failure.
-int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy, const __half* gs, const __half* x16,
-                         const float* dscale, int M, int N, int K, int r, const LoraGroupTable& t, float* partB, float* partA) {
-  if (M <= 0) return 0;
-  if (r <= 0 || r > 64 || N % 8 != 0 || K % 8 != 0 || ld_dy % 8 != 0) return 1;
-  if (((uintptr_t)hs | (uintptr_t)dy16 | (uintptr_t)gs | (uintptr_t)x16) & 15) return 1;
+bool lora_grads_tc_takes(const LoraGradJob& j) {
+  return j.r > 0 && j.r <= 64 && j.N % 8 == 0 && j.K % 8 == 0 && j.ld_dy % 8 == 0 && j.t.n >= 1 && j.t.n <= 3 &&
+         (((uintptr_t)j.hs | (uintptr_t)j.dy | (uintptr_t)j.gs | (uintptr_t)j.x) & 15) == 0;
+}
+static int lora_grads_splits(int M) {
+  const int tps = lora_grads_tc_tokens_per_split(M);
+  return (M + tps - 1) / tps;
+}
+// per job: the scaled Hs and Gs, the splits' largest factors, and the partial sums if they go through memory
+size_t lora_grads_tc_workspace_floats(const LoraGradJob* jobs, int n, int M) {
+  const size_t splits = (size_t)lora_grads_splits(M);
+  size_t f = 0;
+  for (int j = 0; j < n; ++j) {
+    f += (size_t)M * 64 + (splits + 63) / 64 * 64;
+    if (!lora_grads_tc_direct(M)) f += splits * jobs[j].r * ((size_t)jobs[j].N + (size_t)jobs[j].K);
+  }
+  return f;
+}
+
+// One launch for all the jobs (a block's linears): a launch per linear left half of the GPU idle at 1024
+// tokens (152 CTAs of 296 places, 10.6 us each) and ended in a nearly empty wave at 8192.
+int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float* ws) {
+  if (M <= 0 || n <= 0) return 0;
+  if (n > LORA_GRAD_JOBS) return 3;
   static bool attr = false;
   if (!attr) {
     if (cudaFuncSetAttribute(lora_grads_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LG_TOTAL) != cudaSuccess) return 3;
     attr = true;
   }
-  CUtensorMap tpb, tqb, tpa, tqa;
-  if (tensor_map_f16_2d_ld(c, &tpb, hs, (uint64_t)M, 64, 64, 64, 64)) return 3;
-  if (tensor_map_f16_2d_ld(c, &tqb, dy16, (uint64_t)M, (uint64_t)N, (uint64_t)ld_dy, 64, 64)) return 3;
-  if (tensor_map_f16_2d_ld(c, &tpa, gs, (uint64_t)M, 64, 64, 64, 64)) return 3;
-  if (tensor_map_f16_2d_ld(c, &tqa, x16, (uint64_t)M, (uint64_t)K, (uint64_t)K, 64, 64)) return 3;
-  LoraGradTcArgs g;
-  g.pscale = dscale;
-  g.M = M; g.N = N; g.K = K; g.r = r;
-  g.nbB = (N + 127) / 128;
+  LgArgs g;
+  g.n_jobs = n;
+  g.M = M;
   g.tps = lora_grads_tc_tokens_per_split(M);
-  g.partB = partB;
-  g.partA = partA;
-  const int splits = (M + g.tps - 1) / g.tps;
   g.direct = lora_grads_tc_direct(M) ? 1 : 0;
-  g.t = t;
+  const int splits = lora_grads_splits(M);
+  LgScaleArgs sa;
+  sa.M = M;
+  sa.tps = g.tps;
+  int tiles = 0, n_scaled = 0;
+  for (int j = 0; j < n; ++j) {
+    const LoraGradJob& q = jobs[j];
+    const __half *hs = q.hs, *gs = q.gs;
+    LgJob& t = g.job[j];
+    t.top = nullptr;
+    if (q.dscale) {
+      LgScaleJob& w = sa.job[n_scaled++];
+      w = LgScaleJob{q.hs, q.gs, q.dscale, (__half*)ws, (__half*)ws + (size_t)M * 64, ws + (size_t)M * 64};
+      hs = w.hs_out;
+      gs = w.gs_out;
+      t.top = w.top;
+    }
+    ws += (size_t)M * 64 + ((size_t)splits + 63) / 64 * 64;
+    LgMaps& m = g.maps[j];
+    if (tensor_map_f16_2d_ld(c, &m.pb, hs, (uint64_t)M, 64, 64, 64, 64)) return 3;
+    if (tensor_map_f16_2d_ld(c, &m.qb, q.dy, (uint64_t)M, (uint64_t)q.N, (uint64_t)q.ld_dy, 64, 64)) return 3;
+    if (tensor_map_f16_2d_ld(c, &m.pa, gs, (uint64_t)M, 64, 64, 64, 64)) return 3;
+    if (tensor_map_f16_2d_ld(c, &m.qa, q.x, (uint64_t)M, (uint64_t)q.K, (uint64_t)q.K, 64, 64)) return 3;
+    t.N = q.N;
+    t.K = q.K;
+    t.r = q.r;
+    t.first = tiles;
+    t.nbB = (q.N + 127) / 128;
+    t.t = q.t;
+    t.partB = ws;
+    t.partA = ws + (size_t)splits * q.r * q.N;
+    if (!g.direct) ws = t.partA + (size_t)splits * q.r * q.K;
+    tiles += t.nbB + (q.K + 127) / 128;
+  }
+  if (n_scaled > 0) {
+    pdl(lora_scale_small_kernel, dim3((M + 63) / 64, n_scaled), 256, 0, c->stream)(sa);
+    RT_COUNT_LAUNCH(1);
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -291,14 +358,16 @@ int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld
   at[1].val.clusterDim.x = 1;
   at[1].val.clusterDim.y = (unsigned)splits;
   at[1].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)(g.nbB + (K + 127) / 128), (unsigned)splits);
-  cfg.blockDim = dim3(256);
+  cfg.gridDim = dim3((unsigned)tiles, (unsigned)splits);
+  cfg.blockDim = dim3(LG_THREADS);
   cfg.dynamicSmemBytes = LG_TOTAL;
   cfg.stream = c->stream;
   cfg.attrs = at;
   cfg.numAttrs = g.direct && splits > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, lora_grads_tc_kernel, tpb, tqb, tpa, tqa, g, c->status_dev) != cudaSuccess) return 3;
+  if (cudaLaunchKernelEx(&cfg, lora_grads_tc_kernel, g, c->status_dev) != cudaSuccess) return 3;
   RT_COUNT_LAUNCH(1);
+  if (!g.direct)
+    for (int j = 0; j < n; ++j) launch_lora_grads_group_reduce(g.job[j].partB, g.job[j].partA, splits, jobs[j].N, jobs[j].K, jobs[j].r, jobs[j].t, c->stream);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -71,7 +71,6 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   uint64_t* empty = bars + NS;   // [NS]
   uint64_t* done = bars + 2 * NS;
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * NS + 2);
-  pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int rank = n_ctas > 1 ? (int)cluster_ctarank() : 0;
   const int m0 = (int)(blockIdx.x / n_ctas) * TN;
@@ -96,6 +95,9 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   pdl_wait();
+  // Only now: the matmul that follows (QGemmArgs::late_wait) takes everything older than this kernel as
+  // complete once it runs, and waits for this kernel alone, before the last step of its contraction.
+  pdl_launch_dependents();
 
   bool ok = true;
   if (warp == 2) {

@@ -81,39 +81,10 @@ static __half* lowrank_buf(rt_ctx* c, DevBuf& b, int& cur_rank, int M, int rank)
   return b.as<__half>();
 }
 
-// out[M x 64] = X[M x K] . Wt[r x K]^T: the tcgen05 stream kernel, or (return 1) a shape it does not take
-static int lowrank_product(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64) {
-  return launch_lowrank_tc(c, X, Wt, M, K, r, out64);
-}
-
-static QWeight dense_view(const __half* p, int rows, int cols) {
-  QWeight w;
-  w.fmt = GGML_F16;
-  w.rows = rows;
-  w.cols = cols;
-  w.dense16 = (void*)p;
-  return w;
-}
-
 rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out) {
-  rt_ctx* c = l->ctx;
   lora_refresh(l);
-  {
-    const int rc0 = lowrank_product(c, x16, l->lora.a_s, M, l->in_dim(), l->lora.rank, hs_out);
-    if (rc0 == 0) return RT_OK;
-    if (rc0 != 1) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
-  }
-  QGemmArgs ha;  // Hs = X . (sA)^T  (general shapes: through the big kernel)
-  ha.dir = QG_FWD;
-  ha.act = x16;
-  ha.act_f16 = 1;
-  ha.M = M;
-  ha.out = hs_out;
-  ha.out_dtype = OUT_F16;
-  ha.ld_out = 64;
-  ha.aux = 1;
-  int rc = qgemm_launch(c, dense_view(l->lora.a_s, l->lora.rank, l->in_dim()), ha);
-  if (rc) return c->fail(rc, "lora H matmul launch failed");
+  if (launch_lowrank_tc(l->ctx, x16, l->lora.a_s, M, l->in_dim(), l->lora.rank, hs_out))
+    return l->ctx->fail(RT_ERR_CUDA, "lora H kernel launch failed");
   return RT_OK;
 }
 
@@ -136,13 +107,32 @@ rt_status linear_forward_dev(rt_linear* l, LinearScratch& sc, const __half* x16,
     const int r = l->lora.rank;
     __half* hs = hs_keep ? hs_keep : lowrank_buf(c, sc.hs, sc.hs_rank, M, r);
     if (!hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    if (!(hs_keep && hs_ready)) RT_TRY(linear_lora_h(l, x16, M, hs));
+    if (!(hs_keep && hs_ready)) {
+      RT_TRY(linear_lora_h(l, x16, M, hs));
+      a.late_wait = 1;
+    }
     a.lora.act = hs;
     a.lora.w = l->lora.bp;
     a.lora.rank = r;
   }
   int rc = frozen_matmul_launch(c, l->w->w, a);
   if (rc) return c->fail(rc, "frozen forward matmul launch failed");
+  return RT_OK;
+}
+
+// The adapter gradients of one product: dB, dA of every member of `t` from Hs, dY, Gs and X.
+static rt_status lora_grads_add(rt_ctx* c, LinearScratch& sc, const LoraGradJob& j, int M) {
+  if (!lora_grads_tc_takes(j)) return c->fail(RT_ERR_BAD_SHAPE, "adapter gradients: unsupported shape");
+  sc.jobs[sc.n_jobs++] = j;
+  return sc.defer && sc.n_jobs < LORA_GRAD_JOBS ? RT_OK : lora_grads_flush(c, sc, M);
+}
+rt_status lora_grads_flush(rt_ctx* c, LinearScratch& sc, int M) {
+  const int n = sc.n_jobs;
+  sc.n_jobs = 0;
+  if (n == 0) return RT_OK;
+  if (!sc.grad_ws.reserve(lora_grads_tc_workspace_floats(sc.jobs, n, M) * sizeof(float)))
+    return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
+  if (launch_lora_grads_tc(c, sc.jobs, n, M, sc.grad_ws.as<float>())) return c->fail(RT_ERR_CUDA, "lora gradient kernel launch failed");
   return RT_OK;
 }
 
@@ -162,92 +152,28 @@ rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16
   a.out_dtype = unscaled_f16_out ? OUT_F16 : OUT_F32;
   a.accumulate = accumulate;
   a.row_scale = unscaled_f16_out ? nullptr : dscale;
-  if (l->lora_active()) {
+  const bool lora = l->lora_active();
+  LoraGradJob job;
+  if (lora) {
     lora_refresh(l);
     const int r = l->lora.rank;
     __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(c, sc.hs, sc.hs_rank, M, r);
-    __half* gs = lowrank_buf(c, sc.gs, sc.gs_rank, M, r);
+    __half* gs = lowrank_buf(c, sc.gs[sc.n_jobs], sc.gs_rank[sc.n_jobs], M, r);
     if (!hs || !gs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     // Hs = X . (sA)^T: recomputed as src/linear.rs:105 does, unless the caller kept it
     if (!hs_saved) RT_TRY(linear_lora_h(l, x16, M, hs));
-    int rc = lowrank_product(c, dy16, l->lora.bt_s, M, N, r, gs);
-    if (rc > 1) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
-    const bool g_done = rc == 0;
-    QGemmArgs ga;  // Gs = dY~ . (sB)   (unit rows: the row scale is applied where Gs is consumed)
-    ga.dir = QG_FWD;
-    ga.act = dy16;
-    ga.act_f16 = 1;
-    ga.M = M;
-    ga.out = gs;
-    ga.out_dtype = OUT_F16;
-    ga.ld_out = 64;
-    ga.aux = 1;
-    if (!g_done) {
-      rc = qgemm_launch(c, dense_view(l->lora.bt_s, r, N), ga);
-      if (rc) return c->fail(rc, "lora G matmul launch failed");
-    }
-    // gb[N x r] += dY^T . Hs ; ga[r x K] += Gs^T . X   on the tensor cores, contraction over tokens.
-    // The per-token scales of dY move onto the skinny operand (rows * scale / max), the max onto the result.
-    const __half *hs_c = hs, *gs_c = gs;
-    const float* alpha = nullptr;
-    const size_t wsf2 = lora_grads_workspace_floats(M, N, K, r);
-    if (!sc.grad_ws.reserve(wsf2 * sizeof(float))) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    int rb = launch_lora_grads(c, hs, dy16, N, gs, x16, dscale, M, N, K, r, l->lora.gb, l->lora.ga, sc.grad_ws.as<float>(), c->stream);
-    if (rb > 1) return c->fail(RT_ERR_CUDA, "lora gradient kernel launch failed");
-    int ra = rb;
-    if (rb == 1) {  // shapes the fused kernels do not cover: one product at a time
-      if (dscale) {
-        if (!sc.smax.reserve(16)) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-        launch_rowscale_max(dscale, M, sc.smax.as<float>(), c->stream);
-        alpha = sc.smax.as<float>();
-      }
-      const size_t wsf = tok_contract_workspace_floats(M, K > N ? K : N, r);
-      if (!sc.grad_ws.reserve(wsf * sizeof(float))) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-      rb = launch_tok_contract(hs, dy16, dscale, M, N, r, 1, (size_t)r, alpha, l->lora.gb, sc.grad_ws.as<float>(), c->stream);
-      ra = launch_tok_contract(gs, x16, dscale, M, K, r, (size_t)K, 1, alpha, l->lora.ga, sc.grad_ws.as<float>(), c->stream);
-      if (rb > 1 || ra > 1) return c->fail(RT_ERR_CUDA, "lora gradient kernel launch failed");
-    }
-    if (dscale && (rb == 1 || ra == 1)) {  // general shapes go through the big kernel and need scaled copies
-      __half* hs2 = lowrank_buf(c, sc.hs2, sc.hs2_rank, M, r);
-      __half* gs2 = lowrank_buf(c, sc.gs2, sc.gs2_rank, M, r);
-      if (!hs2 || !gs2) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-      launch_scale_lowrank_rows(hs, dscale, sc.smax.as<float>(), M, hs2, c->stream);
-      launch_scale_lowrank_rows(gs, dscale, sc.smax.as<float>(), M, gs2, c->stream);
-      hs_c = hs2;
-      gs_c = gs2;
-    }
-    QGemmArgs ta;
-    ta.dir = QG_BWD;
-    ta.tok_mode = 1;
-    ta.act_f16 = 1;
-    ta.M = r;
-    ta.out_dtype = OUT_F32;
-    ta.accumulate = 1;
-    ta.alpha_dev = alpha;
-    ta.aux = 1;
-    ta.act = hs_c;  // dB[n, i] += sum_m dY[m, n] Hs[m, i]
-    ta.out = l->lora.gb;
-    ta.out_s_tok = 1;
-    ta.out_s_row = (size_t)r;
-    if (rb == 1) {
-      rc = qgemm_launch(c, dense_view(dy16, M, N), ta);
-      if (rc) return c->fail(rc, "lora dB matmul launch failed");
-    }
-    ta.act = gs_c;  // dA[i, k] += sum_m Gs[m, i] X[m, k]
-    ta.out = l->lora.ga;
-    ta.out_s_tok = (size_t)K;
-    ta.out_s_row = 1;
-    if (ra == 1) {
-      rc = qgemm_launch(c, dense_view(x16, M, K), ta);
-      if (rc) return c->fail(rc, "lora dA matmul launch failed");
-    }
+    // Gs = dY~ . (sB)   (unit rows: the row scale is applied where Gs is consumed)
+    if (launch_lowrank_tc(c, dy16, l->lora.bt_s, M, N, r, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
     a.lora.act = gs;
     a.lora.w = l->lora.a_h;
     a.lora.rank = r;
+    a.late_wait = 1;
+    // gb[N x r] += dY^T . Hs ; ga[r x K] += Gs^T . X   on the tensor cores, contraction over tokens
+    job = LoraGradJob{hs, dy16, gs, x16, dscale, N, N, K, r, {{{l->lora.gb, l->lora.ga, 0, N, 0, r}}, 1}};
   }
   int rc = frozen_matmul_launch(c, l->w->w, a);
   if (rc) return c->fail(rc, "frozen backward matmul launch failed");
-  return RT_OK;
+  return lora ? lora_grads_add(c, sc, job, M) : RT_OK;
 }
 
 
@@ -370,8 +296,10 @@ rt_status group_forward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, i
     group_refresh(g, c->stream);
     __half* hs = hs_keep ? hs_keep : lowrank_buf(c, sc.hs, sc.hs_rank, M, g.rank_total);
     if (!hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    if (!(hs_keep && hs_ready) && lowrank_product(c, x16, g.a_s, M, g.w.cols, g.rank_total, hs))
-      return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
+    if (!(hs_keep && hs_ready)) {
+      if (launch_lowrank_tc(c, x16, g.a_s, M, g.w.cols, g.rank_total, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
+      a.late_wait = 1;
+    }
     a.lora.act = hs;
     a.lora.w = g.bp;
     a.lora.rank = g.rank_total;
@@ -399,35 +327,29 @@ rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, 
   a.row_scale = dscale;
   bool any;
   group_lora_on(g, &any);
+  LoraGradJob job;
   if (any) {
     group_refresh(g, c->stream);
     const int R = g.rank_total;
     __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(c, sc.hs, sc.hs_rank, M, R);
-    __half* gs = lowrank_buf(c, sc.gs, sc.gs_rank, M, R);
+    __half* gs = lowrank_buf(c, sc.gs[sc.n_jobs], sc.gs_rank[sc.n_jobs], M, R);
     if (!hs || !gs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    if (!hs_saved && lowrank_product(c, x16, g.a_s, M, K, R, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
-    if (lowrank_product(c, dy16, g.bt_s, M, NT, R, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
-    if (!sc.grad_ws.reserve(lora_grads_workspace_floats(M, NT, K, R) * sizeof(float)))
-      return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    float *gbp[3], *gap[3];
-    int roff[3], rws[3], koff[3], rk[3], nm = 0;
+    if (!hs_saved && launch_lowrank_tc(c, x16, g.a_s, M, K, R, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
+    if (launch_lowrank_tc(c, dy16, g.bt_s, M, NT, R, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
+    job = LoraGradJob{hs, dy16, gs, x16, dscale, NT, NT, K, R, {}};
+    job.t.n = 0;
     for (int i = 0; i < g.n; ++i) {
       rt_linear* l = g.lin[i];
-      if (!l->has_lora) continue;
-      gbp[nm] = l->lora.gb; gap[nm] = l->lora.ga;
-      roff[nm] = g.row_off[i]; rws[nm] = l->out_dim(); koff[nm] = g.rank_off[i]; rk[nm] = l->lora.rank;
-      ++nm;
+      if (l->has_lora) job.t.m[job.t.n++] = LoraGroupMember{l->lora.gb, l->lora.ga, g.row_off[i], l->out_dim(), g.rank_off[i], l->lora.rank};
     }
-    if (launch_lora_grads_group(c, hs, dy16, gs, x16, dscale, M, NT, K, R, nm, gbp, gap, roff, rws, koff, rk,
-                                sc.grad_ws.as<float>(), c->stream))
-      return c->fail(RT_ERR_CUDA, "lora gradient kernel launch failed");
     a.lora.act = gs;
     a.lora.w = g.a_h;
     a.lora.rank = R;
+    a.late_wait = 1;
   }
   int rc = qgemm_launch(c, g.w, a);
   if (rc) return c->fail(rc, "frozen backward matmul launch failed");
-  return RT_OK;
+  return any ? lora_grads_add(c, sc, job, M) : RT_OK;
 }
 
 // tensor.rs:155-199 Rng, host side, for Lora::new's A ~ U(-1/sqrt(in), 1/sqrt(in))
@@ -679,10 +601,10 @@ void rt_model_destroy(rt_model* m) {
   if (m->embed) rt_frozen_destroy(m->embed);
   for (void* p : m->owned) cudaFree(p);
   DevBuf* bufs[] = {&m->P, &m->G, &m->Mo, &m->Vo, &m->opt_scalars, &m->inv_freq, &m->rope_cos, &m->rope_sin,
-                    &m->lsc.hs, &m->lsc.gs, &m->lsc.hs2, &m->lsc.gs2, &m->lsc.smax, &m->lsc.grad_ws, &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
+                    &m->lsc.hs, &m->lsc.gs[0], &m->lsc.gs[1], &m->lsc.gs[2], &m->lsc.gs[3], &m->lsc.grad_ws, &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
                     &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw, &m->q16, &m->k16, &m->v16, &m->o16, &m->lse,
                     &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16, &m->sc_y, &m->dhm, &m->dg16, &m->du16,
-                    &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->amax, &m->dq, &m->dk, &m->dv, &m->dq16, &m->dk16,
+                    &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq, &m->dk, &m->dv, &m->dq16, &m->dk16,
                     &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs,
                     &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) b->release();
@@ -880,7 +802,7 @@ rt_status rt_model_finalize(rt_model* m) {
       if (!b.lin[i]) { snprintf(buf, sizeof buf, "blk.%d.%s.weight missing", li, LIN_NAMES[i]); return c->fail(RT_ERR_BAD_ARG, buf); }
   }
   // opt_scalars: [0,1024) f64 partials, [1024] f64 sum, then one f32 norm
-  if (!m->opt_scalars.reserve(1025 * sizeof(double) + 16) || !m->amax.reserve(16)) return c->fail(RT_ERR_CUDA, "out of device memory");
+  if (!m->opt_scalars.reserve(1025 * sizeof(double) + 16)) return c->fail(RT_ERR_CUDA, "out of device memory");
   if (!m->finalized) {
     const char* e = getenv("RT_B200_NO_GROUPS");  // measurement aid: one matmul per projection
     if (!(e && e[0] == '1'))
@@ -1046,12 +968,13 @@ static bool ensure_tokens(rt_model* m, int M) {
   ok &= m->n1.reserve(T * d * 2 * L) && m->n2.reserve(T * d * 2 * L);
   ok &= m->q_raw.reserve(T * (qd + 2 * kvd) * 4 * L);  // q | k | v before RoPE
   ok &= m->q16.reserve(T * qd * 2 * L) && m->k16.reserve(T * kvd * 2 * L) && m->v16.reserve(T * kvd * 2 * L) && m->o16.reserve(T * qd * 2 * L);
-  ok &= m->lse.reserve(T * g.n_heads * 4 * L) && m->delta.reserve(attn_delta_floats(M, g.n_heads) * 4);
+  ok &= m->lse.reserve(T * g.n_heads * 4 * L) && m->delta.reserve(attn_bwd_work_floats(M, g.n_heads) * 4);
   ok &= m->g16.reserve(T * ff * 2 * 2 * L) && m->hm16.reserve(T * ff * 2 * L);  // gate | up
   ok &= m->dx.reserve(T * d * 4) && m->dy16.reserve(T * d * 2) && m->sc_y.reserve(T * 4);
   ok &= m->dhm.reserve(T * ff * 2) && m->dg16.reserve(T * ff * 2 * 2);  // d(gate) | d(up)
   ok &= m->sc_g.reserve(T * 4) && m->sc_u.reserve(T * 4) && m->dn.reserve(T * d * 4);
-  ok &= m->dO16.reserve(T * qd * 2) && m->amax.reserve(2 * T * 4 + 16);  // amax: per token, its sequence's largest factor, then its weight against it
+  ok &= m->dy16o.reserve(T * d * 2) && m->sc_yo.reserve(T * 4);  // the gradient in front of the attention's output projection
+  ok &= m->dO16.reserve(T * qd * 2);
   ok &= m->dq.reserve(T * qd * 4) && m->dk.reserve(T * kvd * 4) && m->dv.reserve(T * kvd * 4);
   ok &= m->dq16.reserve(T * (qd + 2 * kvd) * 2);  // d(q) | d(k) | d(v)
   ok &= m->sc_q.reserve(T * 4) && m->sc_k.reserve(T * 4) && m->sc_v.reserve(T * 4);
@@ -1202,6 +1125,8 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   __half* dy16 = m->dy16.as<__half>();
   float* sc_y = m->sc_y.as<float>();
 #define HS(i) (b.lin[i]->lora_active() ? A.hs[i] : nullptr)
+  m->lsc.defer = true;  // the block's adapter gradients are one launch at its end
+  m->lsc.n_jobs = 0;
   // Mlp::backward (src/model.rs:120-134)
   // d(hm) leaves the matmul as f16 rows still lacking sc_y: SwiGLU's backward folds the factor into its own scales
   RT_TRY(linear_backward_dev(b.lin[6], m->lsc, A.hm16, dy16, sc_y, M, m->dhm.p, 0, HS(6), true));
@@ -1217,15 +1142,14 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
     RT_TRY(linear_backward_dev(b.lin[5], m->lsc, A.n2, du16, m->sc_u.as<float>(), M, m->dn.as<float>(), 1, HS(5)));
   }
   // dh = dy + rmsnorm_backward(h, post_norm, dn2)
-  launch_rmsnorm_bwd(A.h, b.post_norm, m->dn.as<float>(), dx, M, d, g.rms_eps, dx, dy16, sc_y, st);
+  __half* dy16o = m->dy16o.as<__half>();
+  float* sc_yo = m->sc_yo.as<float>();
+  launch_rmsnorm_bwd(A.h, b.post_norm, m->dn.as<float>(), dx, M, d, g.rms_eps, dx, dy16o, sc_yo, st);
   // Attention::backward (src/attention.rs:246-367)
-  // d(attention output) leaves the matmul as f16 rows still lacking sc_y; the attention backward
-  // takes the factors per query row (in amax, for every token, the largest one of its own sequence:
-  // nothing a sequence's backward sees may depend on its batch mates)
-  RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16, sc_y, M, m->dO16.p, 0, HS(3), true));
-  launch_rowscale_seqmax(sc_y, m->seq_start, M, m->amax.as<float>(), st);
-  if (launch_attn_bwd_tc(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(), m->amax.as<float>(), sc_y, A.lse, m->attn_batch(M),
-                         g.n_heads, g.n_kv_heads, g.head_dim, m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
+  // d(attention output) leaves the matmul as f16 rows still lacking sc_yo; the attention backward takes the factors per query row
+  RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16o, sc_yo, M, m->dO16.p, 0, HS(3), true));
+  if (launch_attn_bwd_tc(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(), sc_yo, A.lse, m->attn_batch(M), g.n_heads, g.n_kv_heads,
+                         g.head_dim, m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
   const size_t qd = (size_t)g.n_heads * g.head_dim, kvd = (size_t)g.n_kv_heads * g.head_dim;
   __half* dq16 = m->dq16.as<__half>();
@@ -1242,6 +1166,8 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
     RT_TRY(linear_backward_dev(b.lin[1], m->lsc, A.n1, dk16, m->sc_k.as<float>(), M, m->dn.as<float>(), 1, HS(1)));
     RT_TRY(linear_backward_dev(b.lin[2], m->lsc, A.n1, dv16, m->sc_v.as<float>(), M, m->dn.as<float>(), 1, HS(2)));
   }
+  m->lsc.defer = false;
+  RT_TRY(lora_grads_flush(c, m->lsc, M));  // before dy16, the first of the gradients it reads, is overwritten
   // dx = dh + rmsnorm_backward(x, input_norm, dn1)
   launch_rmsnorm_bwd(x_in, b.input_norm, m->dn.as<float>(), dx, M, d, g.rms_eps, dx, dy16, sc_y, st);
 #undef HS
@@ -1405,10 +1331,10 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
 static uint64_t buffer_signature(rt_model* m) {
   uint64_t h = 1469598103934665603ull;
   auto mix = [&](const void* p) { h = (h ^ (uint64_t)(uintptr_t)p) * 1099511628211ull; };
-  DevBuf* bufs[] = {&m->P, &m->G, &m->rope_cos, &m->rope_sin, &m->lsc.hs, &m->lsc.gs, &m->lsc.hs2, &m->lsc.gs2, &m->lsc.smax, &m->lsc.grad_ws,
+  DevBuf* bufs[] = {&m->P, &m->G, &m->rope_cos, &m->rope_sin, &m->lsc.hs, &m->lsc.gs[0], &m->lsc.gs[1], &m->lsc.gs[2], &m->lsc.gs[3], &m->lsc.grad_ws,
                     &m->batch, &m->results, &m->x, &m->ckpt, &m->h, &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw,
                     &m->q16, &m->k16, &m->v16, &m->o16, &m->lse, &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16,
-                    &m->sc_y, &m->dhm, &m->dg16, &m->du16, &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->amax, &m->dq,
+                    &m->sc_y, &m->dhm, &m->dg16, &m->du16, &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq,
                     &m->dk, &m->dv, &m->dq16, &m->dk16, &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs, &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) mix(b->p);
   for (int i = 0; i < 7; ++i) mix(m->hs_keep[i].p);

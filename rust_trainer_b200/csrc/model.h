@@ -54,8 +54,13 @@ struct rt_linear {
 
 // Scratch shared by every Linear call on a ctx (one call at a time per ctx).
 struct LinearScratch {
-  DevBuf hs, gs, hs2, gs2, smax, grad_ws;
-  int hs_rank = -1, gs_rank = -1, hs2_rank = -1, gs2_rank = -1;
+  DevBuf hs, gs[rt::LORA_GRAD_JOBS], grad_ws;
+  int hs_rank = -1, gs_rank[rt::LORA_GRAD_JOBS] = {-1, -1, -1, -1};
+  // Adapter gradients wait here for the other linears of their block (`defer`), to be computed by one
+  // launch: what they read has to stay in place until lora_grads_flush.
+  bool defer = false;
+  int n_jobs = 0;
+  rt::LoraGradJob jobs[rt::LORA_GRAD_JOBS];
 };
 
 namespace rt {
@@ -71,6 +76,8 @@ rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out);
 rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16, const __half* dy16,
                               const float* dscale, int M, void* dx, int accumulate,
                               const __half* hs_saved = nullptr, bool unscaled_f16_out = false);
+// computes the adapter gradients that are waiting in `sc`
+rt_status lora_grads_flush(rt_ctx* c, LinearScratch& sc, int M);
 rt_status lora_refresh(rt_linear* l);
 }  // namespace rt
 
@@ -135,7 +142,7 @@ struct rt_model {
   // q_raw holds q|k|v before RoPE (three regions, or one matrix with q, k, v as column slices when the
   // block runs them as a group); g16 holds gate|up the same way; dq16, dg16 likewise for the gradients
   DevBuf x, ckpt, h, n1, n2, q_raw, k_raw, v_raw, q16, k16, v16, o16, lse, delta, g16, u16, hm16;
-  DevBuf dx, dy16, sc_y, dhm, dg16, du16, sc_g, sc_u, dn, d_o, dO16, amax, dq, dk, dv, dq16, dk16, dv16, sc_q, sc_k, sc_v;
+  DevBuf dx, dy16, sc_y, dhm, dg16, du16, sc_g, sc_u, dn, d_o, dO16, dy16o, sc_yo, dq, dk, dv, dq16, dk16, dv16, sc_q, sc_k, sc_v;
   DevBuf xs, ns16, logits, dl16, sc_l, dns, dxs;
   DevBuf argmax;            // per target, the greedy token of the last pass that asked for it
   bool want_argmax = false;

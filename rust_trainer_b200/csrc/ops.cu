@@ -1572,135 +1572,6 @@ void launch_lora_refresh(const float* a, const float* b, int r, int K, int N, fl
   { lora_refresh_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, r, K, N, s, a_s, a_h, bp, bt_s); RT_COUNT_LAUNCH(1); }
 }
 
-// Token-contraction for the LoRA gradients (reference src/linear.rs:108-116):
-//   part[split][i, j] = sum_{m in split} pscale[m] * P[m, i] * qscale[m] * Q[m, j],  i < r, j < C
-// P is [M x 64] f16, Q is [M x C] f16.  A second kernel adds the splits, in order, into
-// out[i*so_i + j*so_j] (deterministic: no float atomics).
-//   dA: P = Gs (unit rows, pscale = row scale of dY), Q = X        -> ga[r x K]: so_i = K, so_j = 1
-//   dB: P = Hs,                       Q = dY (qscale = its scale)  -> gb[N x r]: so_i = 1, so_j = r
-constexpr int LG_TOK = 32;
-__global__ void __launch_bounds__(256)
-lora_grad_partial_kernel(const __half* __restrict__ P, const __half* __restrict__ Q, const float* __restrict__ pscale,
-                         const float* __restrict__ qscale, int M, int C, int r, int tokens_per_split,
-                         float* __restrict__ part) {
-  __shared__ float sP[LG_TOK][65];
-  __shared__ float sQ[LG_TOK][64];
-  const int j0 = blockIdx.x * 64;
-  const int m_begin = blockIdx.y * tokens_per_split;
-  const int m_end = min(M, m_begin + tokens_per_split);
-  const int tj = threadIdx.x & 63, ti = threadIdx.x >> 6;  // column, row group (4 groups)
-  float acc[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) acc[k] = 0.f;
-  const int rows_per = (r + 3) / 4;  // <= 16
-  for (int m0 = m_begin; m0 < m_end; m0 += LG_TOK) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < LG_TOK * 64; e += 256) {
-      const int mm = e >> 6, c = e & 63, m = m0 + mm;
-      float pv = 0.f, qv = 0.f;
-      if (m < m_end) {
-        const float sc = (pscale ? pscale[m] : 1.f) * (qscale ? qscale[m] : 1.f);
-        if (c < r) pv = __half2float(P[(size_t)m * 64 + c]) * sc;
-        if (j0 + c < C) qv = __half2float(Q[(size_t)m * C + j0 + c]);
-      }
-      sP[mm][c] = pv;
-      sQ[mm][c] = qv;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int mm = 0; mm < LG_TOK; ++mm) {
-      const float q = sQ[mm][tj];
-#pragma unroll
-      for (int k = 0; k < 16; ++k)
-        if (k < rows_per) acc[k] += sP[mm][ti + 4 * k] * q;
-    }
-  }
-  float* dst = part + (size_t)blockIdx.y * r * C;
-  for (int k = 0; k < rows_per; ++k) {
-    const int i = ti + 4 * k;
-    if (i < r && j0 + tj < C) dst[(size_t)i * C + j0 + tj] = acc[k];
-  }
-}
-__global__ void lora_grad_reduce_kernel(const float* __restrict__ part, int splits, int C, int r, size_t so_i,
-                                        size_t so_j, float* __restrict__ out) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)r * C) return;
-  const int i = (int)(e / C), j = (int)(e % C);
-  float s = 0.f;
-  for (int k = 0; k < splits; ++k) s += part[(size_t)k * r * C + e];
-  out[i * so_i + j * so_j] += s;
-}
-size_t lora_grad_workspace_floats(int M, int C, int r) {
-  int splits = (M + 511) / 512;
-  if (splits < 1) splits = 1;
-  return (size_t)splits * r * C;
-}
-void launch_lora_grad(const __half* P, const __half* Q, const float* pscale, const float* qscale, int M, int C, int r,
-                      size_t so_i, size_t so_j, float* out, float* workspace, cudaStream_t st) {
-  if (M <= 0 || r <= 0) return;
-  int splits = (M + 511) / 512;
-  if (splits < 1) splits = 1;
-  const int tps = ((M + splits - 1) / splits + LG_TOK - 1) / LG_TOK * LG_TOK;
-  splits = (M + tps - 1) / tps;
-  dim3 grid((C + 63) / 64, splits);
-  { lora_grad_partial_kernel<<<grid, 256, 0, st>>>(P, Q, pscale, qscale, M, C, r, tps, workspace); RT_COUNT_LAUNCH(1); }
-  const size_t n = (size_t)r * C;
-  { lora_grad_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(workspace, splits, C, r, so_i, so_j, out); RT_COUNT_LAUNCH(1); }
-}
-
-// Largest per-token scale of a backward input, and a [M x 64] low-rank operand with each row
-// multiplied by scale[m] / max: the token contractions dA, dB need ONE common scale, so the
-// per-row factors move onto the skinny operand and the common factor onto the result.
-__global__ void rowscale_max_kernel(const float* __restrict__ sc, int M, float* __restrict__ out) {
-  pdl_entry();
-  float m = 0.f;
-  for (int i = threadIdx.x; i < M; i += blockDim.x) m = fmaxf(m, sc[i]);
-  m = block_max(m);
-  // rounded up to a power of two: dividing by it changes no mantissa, so what a row rounds to in
-  // f16 does not depend on which other rows share the batch (N ranks on shards of a batch then
-  // reproduce one rank on the whole of it up to the order of f32 sums)
-  if (threadIdx.x == 0) out[0] = m > 0.f ? __int_as_float((__float_as_int(m) + 0x007FFFFF) & 0x7F800000) : 1.f;
-}
-__global__ void scale_lowrank_rows_kernel(const __half* __restrict__ in, const float* __restrict__ sc,
-                                          const float* __restrict__ smax, int M, __half* __restrict__ out) {
-  const size_t e = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  if (e >= (size_t)M * 64) return;
-  const float f = sc[e >> 6] / smax[0];
-  float2 v = __half22float2(*(const __half2*)(in + e));
-  *(__half2*)(out + e) = __floats2half2_rn(v.x * f, v.y * f);
-}
-// The same per SEQUENCE: out[m] = largest scale among the tokens of m's sequence (seq_start[m] =
-// first token of it), rounded up to a power of two; 1 where the whole sequence is zero; and
-// out[M + m] = sc[m] / out[m], the weight of row m among its sequence's rows.  A sequence's
-// backward then never sees a number that depends on its batch mates.  One block:
-// the slot of a sequence is out[first token]; converting a slot is idempotent, so a reader may
-// meet it before or after its own token converted it.
-__global__ void rowscale_seqmax_kernel(const float* __restrict__ sc, const int* __restrict__ seq_start, int M,
-                                       float* __restrict__ out) {
-  pdl_entry();
-  for (int i = threadIdx.x; i < M; i += blockDim.x) out[i] = 0.f;
-  __syncthreads();
-  for (int i = threadIdx.x; i < M; i += blockDim.x) atomicMax((int*)out + seq_start[i], __float_as_int(fmaxf(sc[i], 0.f)));
-  __syncthreads();
-  for (int i = threadIdx.x; i < M; i += blockDim.x) {
-    const float m = out[seq_start[i]];
-    const float top = m > 0.f ? __int_as_float((__float_as_int(m) + 0x007FFFFF) & 0x7F800000) : 1.f;
-    out[i] = top;
-    out[M + i] = fmaxf(sc[i], 0.f) / top;
-  }
-}
-void launch_rowscale_seqmax(const float* sc, const int* seq_start, int M, float* out, cudaStream_t st) {
-  if (M > 0) { pdl(rowscale_seqmax_kernel, 1, 1024, 0, st)(sc, seq_start, M, out); RT_COUNT_LAUNCH(1); }
-}
-void launch_rowscale_max(const float* sc, int M, float* out, cudaStream_t st) {
-  if (M > 0) { pdl(rowscale_max_kernel, 1, 1024, 0, st)(sc, M, out); RT_COUNT_LAUNCH(1); }
-}
-void launch_scale_lowrank_rows(const __half* in, const float* sc, const float* smax, int M, __half* out, cudaStream_t st) {
-  if (M <= 0) return;
-  const size_t threads = (size_t)M * 32;
-  { scale_lowrank_rows_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(in, sc, smax, M, out); RT_COUNT_LAUNCH(1); }
-}
-
 // ------------------------------------------------------------------ optimiser (reference src/optim.rs:48-90)
 // Sum of squares in f64: fixed-size blocks write partials, one block adds them in order.
 __global__ void sumsq_partial_kernel(const float* __restrict__ g, size_t n, double* __restrict__ part) {
@@ -1750,35 +1621,6 @@ void launch_adamw(float* p, float* g, float* m, float* v, size_t n, const double
   if (n == 0) return;
   { adamw_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, g, m, v, n, sumsq, max_norm, lr, beta1, beta2, eps, wd,
                                                              bc1, bc2, norm_out); RT_COUNT_LAUNCH(1); }
-}
-
-// ------------------------------------------------------------------ misc
-__global__ void absmax_kernel(const float* __restrict__ x, size_t n, float* __restrict__ out) {
-  float m = 0.f;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(x[i]));
-  m = block_max(m);
-  if (threadIdx.x == 0) atomicMax((int*)out, __float_as_int(m));  // non-negative floats order like ints
-}
-// y16 = x / max(amax, tiny); inv/scale read on device
-__global__ void scale_to_f16_kernel(const float* __restrict__ x, size_t n, const float* __restrict__ amax,
-                                    __half* __restrict__ y) {
-  const float a = amax[0];
-  const float inv = a > 0.f ? 1.f / a : 1.f;
-  size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-  if (i + 1 < n) {
-    float2 v = *(const float2*)(x + i);
-    *(__half2*)(y + i) = __floats2half2_rn(v.x * inv, v.y * inv);
-  } else if (i < n) y[i] = __float2half_rn(x[i] * inv);
-}
-void launch_global_normalize(const float* x, size_t n, float* amax_dev, __half* y16, cudaStream_t st) {
-  if (n == 0) return;
-  cudaMemsetAsync(amax_dev, 0, sizeof(float), st);
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 1184) blocks = 1184;
-  { absmax_kernel<<<blocks, 256, 0, st>>>(x, n, amax_dev); RT_COUNT_LAUNCH(1); }
-  size_t threads = (n + 1) / 2;
-  { scale_to_f16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(x, n, amax_dev, y16); RT_COUNT_LAUNCH(1); }
 }
 
 }  // namespace rt

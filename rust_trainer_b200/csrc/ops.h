@@ -59,24 +59,13 @@ inline unsigned lora_refresh_job_blocks(const LoraRefreshJob& j) {
   return (unsigned)(((na > nb ? na : nb) + 255) / 256);
 }
 void launch_lora_refresh_table(const LoraRefreshJob* jobs_dev, int n_jobs, unsigned total_blocks, cudaStream_t st);
-size_t lora_grad_workspace_floats(int M, int C, int r);
-void launch_lora_grad(const __half* P, const __half* Q, const float* pscale, const float* qscale, int M, int C, int r,
-                      size_t so_i, size_t so_j, float* out, float* workspace, cudaStream_t st);
-void launch_rowscale_max(const float* sc, int M, float* out, cudaStream_t st);
-// out[m] = largest sc of m's sequence (power of two, 1 for an all-zero sequence), out[M + m] = sc[m] / out[m]
-void launch_rowscale_seqmax(const float* sc, const int* seq_start, int M, float* out, cudaStream_t st);
-void launch_scale_lowrank_rows(const __half* in, const float* sc, const float* smax, int M, __half* out, cudaStream_t st);
 void launch_sumsq(const float* g, size_t n, double* part, double* out, cudaStream_t st);
 void launch_adamw(float* p, float* g, float* m, float* v, size_t n, const double* sumsq, float max_norm, float lr,
                   float beta1, float beta2, float eps, float wd, float bc1, float bc2, float* norm_out,
                   cudaStream_t st);
-void launch_global_normalize(const float* x, size_t n, float* amax_dev, __half* y16, cudaStream_t st);
 
-// ---- lora_kernels.cu: skinny low-rank products (return 1 when the shape is not supported)
 // ---- lowrank_tc.cu: out64[M x 64] (f16, zero from column r up) = X[M x K] . Wt[r x K]^T on tcgen05; 1 = shape not taken
 int launch_lowrank_tc(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64);
-size_t tok_contract_workspace_floats(int M, int C, int r);
-size_t lora_grads_workspace_floats(int M, int N, int K, int r);
 // A linear's (or a stacked group's) adapters as the token contractions see them: member j owns rows
 // rank_off..+r of the rank axis and columns row_off..+rows of dY.
 struct LoraGroupMember {
@@ -87,40 +76,42 @@ struct LoraGroupTable {
   LoraGroupMember m[3];
   int n;
 };
-// lora_grads_tc.cu: the product kernel on tcgen05 (splits of lora_grads_tc_tokens_per_split(M) tokens)
+// lora_grads_tc.cu: the gradients of one linear, or of a stacked group, on tcgen05.  Hs, Gs: [M x 64];
+// dY: [M x N] f16 rows with one factor each (or null); X: [M x K].
+struct LoraGradJob {
+  const __half *hs, *dy, *gs, *x;
+  const float* dscale;
+  int ld_dy, N, K, r;
+  LoraGroupTable t;
+};
+constexpr int LORA_GRAD_JOBS = 4;  // jobs of one launch: the linears of a block
 int lora_grads_tc_tokens_per_split(int M);
-bool lora_grads_tc_direct(int M);
-int launch_lora_grads_tc(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy, const __half* gs, const __half* x16,
-                         const float* dscale, int M, int N, int K, int r, const LoraGroupTable& t, float* partB, float* partA);
-int launch_lora_grads_group(rt_ctx* c, const __half* hs, const __half* dy16, const __half* gs, const __half* x16, const float* dscale,
-                            int M, int NT, int K, int R, int n, float* const* gb, float* const* ga, const int* row_off,
-                            const int* rows, const int* rank_off, const int* rank, float* workspace, cudaStream_t st);
-int launch_lora_grads(rt_ctx* c, const __half* hs, const __half* dy16, int ld_dy, const __half* gs, const __half* x16, const float* dscale,
-                      int M, int N, int K, int r, float* gb, float* ga, float* workspace, cudaStream_t st);
-// pscale (optional): P's rows are multiplied by pscale[m] / alpha_dev[0] on the fly; alpha_dev[0] then scales the result
-int launch_tok_contract(const __half* P, const __half* Q, const float* pscale, int M, int C, int r, size_t so_i, size_t so_j,
-                        const float* alpha_dev, float* out, float* workspace, cudaStream_t st);
+bool lora_grads_tc_takes(const LoraGradJob& j);
+size_t lora_grads_tc_workspace_floats(const LoraGradJob* jobs, int n, int M);
+// adds dB and dA of the jobs into the gradients of their tables' members; 0 or 3 (launch failure)
+int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float* workspace);
+// adds partial sums [splits][r x N] and [splits][r x K] into the table's members, splits in order
+void launch_lora_grads_group_reduce(const float* partB, const float* partA, int splits, int N, int K, int r, const LoraGroupTable& t,
+                                    cudaStream_t st);
 
 // ---- attention_tc.cu: causal GQA attention over a concatenation of independent sequences, on
 // tcgen05 / TMEM / TMA (waits report through the ctx status word).
 // q [M x nh x hd], k/v [M x nkv x hd] f16 (q unscaled; the kernels apply 1/sqrt(hd)).
 // seq_start[m] = index of the first token of m's sequence; gap [M x 2] or null; lse is [nh x M].
-// Backward: dO row i stands for do_scale[0] * dO16[i], or, with row_scale, for row_scale[i] *
-// dO16[i] (then do_scale is the array [2 M] of launch_rowscale_seqmax: for each token a power of two >=
-// the largest row_scale of its own sequence, then each row's weight against it); outputs are true-scale f32.
+// Backward: dO row i stands for row_scale[i] * dO16[i]; outputs are true-scale f32.
 // What the kernels need to know of a batch, all on the device.  tiles_q: its 128-token tiles as query tiles,
 // longest loops first; tiles_k: as key tiles, pairs (tile, end of the sequence holding its last key).
 struct AttnBatch {
   const int *seq_start, *gap, *tiles_q, *tiles_k;
   int M;
 };
-// floats of the `delta` workspace of the backward
-size_t attn_delta_floats(int M, int nh);
+// floats of the backward's workspace
+size_t attn_bwd_work_floats(int M, int nh);
 // fills the two tile lists (host memory, n and 2 n ints for n = ceil(M / 128) tiles) from seq_start (host memory)
 void attn_plan_tiles(const int* seq_start, int M, int* tiles_q, int* tiles_k);
 int launch_attn_bwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const __half* o, const __half* dO16,
-                       const float* do_scale, const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, int hd,
-                       float* delta, float* dq, float* dk, float* dv);
+                       const float* row_scale, const float* lse, const AttnBatch& b, int nh, int nkv, int hd, float* work, float* dq,
+                       float* dk, float* dv);
 int launch_attn_fwd_tc(rt_ctx* c, const __half* q, const __half* k, const __half* v, const AttnBatch& b, int nh, int nkv, int hd,
                        __half* o, float* lse);
 

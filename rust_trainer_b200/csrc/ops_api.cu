@@ -226,9 +226,9 @@ rt_status rt_op_attention_backward(rt_ctx* c, const float* q, const float* k, co
   attn_plan_tiles(seq_start, (int)M, tq.data(), tk.data());
   int *tqd = t.up(tq.data(), nt, c->stream), *tkd = t.up(tk.data(), 2 * nt, c->stream);
   __half *q16 = t.get<__half>(nq), *k16 = t.get<__half>(nk), *v16 = t.get<__half>(nk), *o16 = t.get<__half>(nq), *do16 = t.get<__half>(nq);
-  float *lsed = t.get<float>(M * nh), *delta = t.get<float>(attn_delta_floats((int)M, nh)), *sc = t.get<float>(M), *amax = t.get<float>(2 * M + 4);
+  float *lsed = t.get<float>(M * nh), *delta = t.get<float>(attn_bwd_work_floats((int)M, nh)), *sc = t.get<float>(M);
   float *dqd = t.get<float>(nq), *dkd = t.get<float>(nk), *dvd = t.get<float>(nk);
-  if (!qd || !kd || !vd || !dod || !ss || !tqd || !tkd || !q16 || !k16 || !v16 || !o16 || !do16 || !lsed || !delta || !sc || !amax || !dqd || !dkd || !dvd)
+  if (!qd || !kd || !vd || !dod || !ss || !tqd || !tkd || !q16 || !k16 || !v16 || !o16 || !do16 || !lsed || !delta || !sc || !dqd || !dkd || !dvd)
     return c->fail(RT_ERR_CUDA, "out of device memory");
   launch_f32_to_16(qd, q16, nq, true, c->stream);
   launch_f32_to_16(kd, k16, nk, true, c->stream);
@@ -238,8 +238,7 @@ rt_status rt_op_attention_backward(rt_ctx* c, const float* q, const float* k, co
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   // dO as the model passes it: f16 rows divided by their largest magnitude, factors beside them
   launch_normalize_rows(dod, (int)M, nh * hd, do16, sc, c->stream);
-  launch_rowscale_seqmax(sc, ss, (int)M, amax, c->stream);
-  if (launch_attn_bwd_tc(c, q16, k16, v16, o16, do16, amax, sc, lsed, ab, nh, nkv, hd, delta, dqd, dkd, dvd))
+  if (launch_attn_bwd_tc(c, q16, k16, v16, o16, do16, sc, lsed, ab, nh, nkv, hd, delta, dqd, dkd, dvd))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
   RT_CUDA(c, cudaMemcpyAsync(dq, dqd, nq * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   RT_CUDA(c, cudaMemcpyAsync(dk, dkd, nk * sizeof(float), cudaMemcpyDeviceToHost, c->stream));

@@ -100,6 +100,7 @@ struct KParams {
   const float* bias;
   uint32_t idesc;
   int* status;
+  int late_wait;  // see QGemmArgs
   int tma_out;  // 16-bit output that TMA can address: staged in shared memory and stored by TMA
 };
 
@@ -325,7 +326,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   // barriers, TMEM and descriptors are set up; from here on the kernel reads what its predecessor wrote
-  pdl_wait();
+  if (!p.late_wait) pdl_wait();
 
   // One [32 tokens x 32 features] block of a 16-bit output -> staging -> TMA store.  `stage_base` is
   // private to the calling warp; a block of it is reused only after the store that read it is done.
@@ -529,6 +530,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
               }
             }
           } else {
+            if (p.late_wait) pdl_wait();
             load2d(a_dst, &tm_lact, 0, m_cta);
             if (p.dir == QG_FWD) {
               load2d(w_dst, &tm_lw, 0, r0);
@@ -1021,6 +1023,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   const int kfmt = !is16 ? w.fmt : p.conv16 ? QF_16CONV : QF_16;
   p.row_scale = a.row_scale;
   p.residual = a.residual;
+  p.late_wait = a.late_wait && a.lora.rank > 0 ? 1 : 0;
   p.dir = a.dir;
   p.out_rows = out_rows;
   p.M = a.M;

@@ -64,6 +64,9 @@ struct QGemmArgs {
   // cached or allocated on the way); a launch that needs more fails with RT_ERR_TOO_LARGE
   float* fixed_part = nullptr;
   size_t fixed_part_floats = 0;
+  // The launch right before this one is the low-rank stream that produces lora.act: a programmatic launch
+  // may start at once and waits for it only where it reads that.
+  int late_wait = 0;
   int aux = 0;                         // 1: a skinny LoRA helper product (kept apart in the profile)
 };
 
