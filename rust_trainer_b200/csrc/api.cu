@@ -59,7 +59,7 @@ static void ctx_register(const rt_ctx* c, bool live) {
 
 int frozen_matmul_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   int rc = qgemm_launch(ctx, w, a);
-  if (rc || !w.dense16_lo || a.out_dtype != OUT_F32 || a.tok_mode) return rc;
+  if (rc || !w.dense16_lo || a.out_dtype != OUT_F32) return rc;
   QWeight lo = w;
   lo.dense16 = w.dense16_lo;
   lo.dense16_lo = nullptr;

@@ -22,7 +22,7 @@ struct rt_ctx {
   double prof_flops = 0, prof_bytes = 0;
   // encoded TMA descriptors, keyed by (base, rows, cols, box, type): the same buffers recur every layer
   std::map<std::tuple<const void*, uint64_t, uint64_t, uint32_t, uint32_t, bool>, CUtensorMap> tmap_cache;
-  struct ProfRec { int cls, M, rows, contract; };  // cls: 0 fwd, 1 bwd, 2 skinny LoRA helper, 3 token contraction
+  struct ProfRec { int cls, M, rows, contract; };  // cls: 0 fwd, 1 bwd
   std::vector<ProfRec> prof_recs;
   // data-parallel communicator (an ncclComm_t once rt_comm_init_rank has run; a world of one otherwise)
   void* comm = nullptr;

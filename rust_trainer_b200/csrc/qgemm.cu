@@ -25,7 +25,6 @@
 
 namespace rt {
 
-constexpr int W_STAGE = 16384;        // 128 x 64 x 16-bit
 
 // The kernel is compiled per launch kind and weight format (one switch on the host instead of one
 // per unpacked unit on the device).
@@ -33,6 +32,7 @@ enum QKind : int {
   QK_PAIR = 0,    // a CTA pair per tile of 256 weight rows x up to 256 tokens
   QK_WIDE = 1,    // one CTA per tile of 128 weight rows x up to 256 tokens (16-bit weights only)
   QK_NARROW = 2,  // one CTA per tile of 128 weight rows x up to 64 tokens
+  QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
 };
 // Weight formats as the kernel sees them: ggml's ids for packed weights, and two 16-bit cases.
 constexpr int QF_16 = 0;       // 16-bit weights of the activations' type, straight from TMA
@@ -41,7 +41,11 @@ constexpr int QF_16CONV = 1;   // 16-bit weights of the other 16-bit type, conve
 // Shared-memory plan of one CTA.
 template <int KIND, int FMT>
 struct QCfg {
-  static constexpr bool PAIR = KIND == QK_PAIR;
+  static constexpr bool PAIR = KIND == QK_PAIR, HALF = KIND == QK_HALF;
+  // Weight rows of the CTA's tile.  The MMA always takes 128: a half tile's upper 64 are whatever follows it in
+  // shared memory, and their accumulator lanes are not read.
+  static constexpr int ROWS = HALF ? 64 : 128, BRICKS = ROWS / 64;
+  static constexpr int W_SUB = ROWS * 128;  // bytes of a [ROWS x 64] 16-bit weight tile
   static constexpr bool PACKED = FMT > QF_16CONV;
   // Unpack warps.  Sixteen for packed weights: one unpack pass is a chain of dependent operations
   // (codes -> convert -> swizzled store -> fence -> arrive), so what counts is how many passes are
@@ -49,14 +53,21 @@ struct QCfg {
   // 406 us against 363.)  Without unpacking eight warps stay, to help with the last tile's epilogue.
   static constexpr int NUW = PACKED ? 16 : 8;
   static constexpr int THREADS = 32 * (7 + NUW);  // + activation / brick producers, MMA, 4 epilogue warps
-  // 64-element contraction steps per stage.  Two for narrow tiles: their MMAs are short, and one hand-off
-  // between the roles costs about 500 cycles whatever it hands over.
-  static constexpr int KS = KIND == QK_NARROW ? 2 : 1;
-  // Activation / unpacked-weight stages and packed-brick stages: as many as fit beside the epilogue
-  // staging.  NS <= NR + 1 is part of the phase rule below.
-  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : PACKED ? 3 : 4;
-  static constexpr int NR = !PACKED ? 0 : PAIR ? 4 : 3;
-  static constexpr int RAW_STAGE = PACKED ? KS * 2 * fmt_brick_bytes(FMT) : 0;
+  // 64-element contraction steps per stage.  Two for narrow and half tiles: their MMAs are short, and one
+  // hand-off between the roles costs about 500 cycles whatever it hands over.
+  static constexpr int KS = KIND == QK_NARROW || HALF ? 2 : 1;
+  // Activation / unpacked-weight stages, and packed-brick stages in the room that is left beside them and
+  // the epilogue staging.
+  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : HALF ? 4 : PACKED ? 3 : 4;
+  static constexpr int RAW_STAGE = PACKED ? KS * BRICKS * fmt_brick_bytes(FMT) : 0;
+  static constexpr int ACT_SUB = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
+  static constexpr int ACT_STAGE = KS * ACT_SUB;
+  static constexpr int W_BYTES = KS * W_SUB;               // unpacked weights of a stage
+  // Epilogue staging of 16-bit outputs per warp: three blocks of [32 tokens x 32 features], 2 KB each.
+  static constexpr int OUT_BUFS = 3, OUT_WARP = OUT_BUFS * 2048;
+  static constexpr int SMEM_MAX = 232448, SMEM_REST = 4 * OUT_WARP + 512 + 2 * 1024;  // staging, barriers, alignment
+  static constexpr int NR_FIT = PACKED ? (SMEM_MAX - SMEM_REST - NS * (ACT_STAGE + W_BYTES)) / (RAW_STAGE ? RAW_STAGE : 1) : 0;
+  static constexpr int NR = NR_FIT > 8 ? 8 : NR_FIT;
   // The unpack warps work as UG groups on alternate stages.  Waits are by phase parity,
   // which is only sound while a waiter cannot run two phases ahead of its barrier: UG <= NS keeps a
   // group from reaching a stage before the use two back has been released, and NS <= NR + 1 keeps a
@@ -67,18 +78,13 @@ struct QCfg {
   static constexpr int UTG = NUW * 32 / UG;                // threads per group
   static_assert(UG <= NS && (!PACKED || NS <= NR + 1), "unpack groups would alias barrier phases");
   static_assert(!PACKED || UTG == KS * 128, "a thread of a group owns one unit of each half of a weight tile");
-  static constexpr int W_BYTES = KS * W_STAGE;             // unpacked weights of a stage
-  static constexpr int ACT_SUB = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
-  static constexpr int ACT_STAGE = KS * ACT_SUB;
   static constexpr int OFF_W = NS * ACT_STAGE;
   static constexpr int OFF_RAW = OFF_W + NS * W_BYTES;
-  static constexpr int OFF_OUT = OFF_RAW + NR * RAW_STAGE;
-  // Epilogue staging of 16-bit outputs per warp: three blocks of [32 tokens x 32 features], 2 KB each.
-  static constexpr int OUT_BUFS = 3, OUT_WARP = OUT_BUFS * 2048;
+  static constexpr int OFF_OUT = (OFF_RAW + NR * RAW_STAGE + 1023) / 1024 * 1024;  // (a swizzled store's source starts on its pattern)
   static constexpr int OFF_BAR = OFF_OUT + 4 * OUT_WARP;
-  static constexpr int N_BARS = 3 * NS + 2 * NR + 4;
+  static constexpr int N_BARS = 3 * NS + 2 * NR + 5;
   static constexpr int SMEM_BYTES = OFF_BAR + N_BARS * 8 + 16 + 1024;
-  static_assert(SMEM_BYTES <= 232448, "shared memory plan exceeds one SM");
+  static_assert(SMEM_BYTES <= SMEM_MAX && N_BARS * 8 + 16 <= 512, "shared memory plan exceeds one SM");
   static_assert(OFF_RAW >= 11 * 8192, "the last tile's helpers stage in the operand stages");
 };
 
@@ -90,8 +96,7 @@ struct KParams {
   int dir, out_rows, M, TN;
   int n_main, lora_mmas;
   int n_splits, steps_per_split;  // work item = (tile, piece of the contraction); partial results go to `part`
-  int b_mn;                       // token-contraction mode: the B operand is MN-major (tile rows = contraction)
-  float* part;                    // [n_splits][M][out_rows] f32 partials when n_splits > 1 or b_mn
+  float* part;                    // [n_splits][M][out_rows] f32 partials when n_splits > 1
   int n_row_tiles, n_tok_tiles;   // a row tile is 128 weight rows, 256 for a CTA pair
   void* out;
   int out_dtype, accumulate, ld_out;
@@ -251,6 +256,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   uint64_t* raw_empty = raw_full + NR;     // [NR]
   uint64_t* acc_full = raw_empty + NR;     // [2]                                                 (every CTA)
   uint64_t* acc_empty = acc_full + 2;      // [2]                                                 (leader's is used)
+  uint64_t* last_full = acc_empty + 2;     // the last tile's accumulator is complete: what its helpers wait for (they
+                                           // have not followed acc_full's phases)                (every CTA)
   uint32_t* tmem_slot = (uint32_t*)(bars + C::N_BARS);
   pdl_launch_dependents();
 
@@ -294,7 +301,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   (void)split; (void)n_main_st
 // first weight row (output feature) of this CTA's half of the tile, first token of the tile
 #define QG_TILE_ORIGIN()                                                                      \
-  const int r0 = (tile % p.n_row_tiles) * (128 * n_cta) + (int)rank * 128;                    \
+  const int r0 = (tile % p.n_row_tiles) * (C::ROWS * n_cta) + (int)rank * 128;                \
   const int m0 = (tile / p.n_row_tiles) * p.TN
 
   if (threadIdx.x == 0) {
@@ -309,6 +316,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     }
     for (int i = 0; i < NR; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], UTG / 32); }  // per warp
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4 * n_cta); }  // per epilogue warp
+    mbar_init(last_full, 1);
     mbar_fence_init();
     prefetch_tmap(&tm_act);
     if (IS16) prefetch_tmap(&tm_w16);
@@ -471,13 +479,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   const int q_res = warp & 3;
   const int q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
   auto tail_helper = [&](int turn, int hslot) {
-    if (n_my == 0) return;
+    if (n_my == 0 || q_res * 32 >= C::ROWS) return;
     const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
     QG_ITEM_DECODE(item);
     (void)s_begin; (void)n_steps; (void)s_main;
     QG_TILE_ORIGIN();
     const int acc = tc_last & 1;
-    if (!mbar_wait(&acc_full[acc], (uint32_t)((tc_last >> 1) & 1), p.status, 402)) return;
+    if (!mbar_wait(last_full, 0, p.status, 402)) return;
     tc_fence_after();
     uint32_t cnt = 0;
     for (int c = turn; c < p.TN / 32; c += q_turns) {
@@ -505,7 +513,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
           uint8_t* w_dst = sW + st * C::W_BYTES;
           // the leader's barrier counts the bytes both CTAs will bring
           if (rank == 0)
-            mbar_expect_tx(&full[st], (uint32_t)subs * ((uint32_t)p.TN * 128u + ((IS16 || lora) ? (uint32_t)(W_STAGE * n_cta) : 0u)));
+            mbar_expect_tx(&full[st], (uint32_t)subs * ((uint32_t)p.TN * 128u + ((IS16 || lora) ? (uint32_t)(C::W_SUB * n_cta) : 0u)));
           const uint32_t fbar = PAIR ? mapa_u32(smem_u32(&full[st]), 0) : 0u;
           auto load2d = [&](void* dst, const CUtensorMap* map, int x, int y) {
             if (PAIR) tma_load_2d_pair(dst, map, x, y, fbar);
@@ -516,28 +524,23 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
             for (int u = 0; u < KS; ++u) {
               if (u >= subs) break;
               const int s = s_begin + si * KS + u;
-              if (p.b_mn) load2d(a_dst + u * C::ACT_SUB, &tm_act, 0, s * 64);  // [64 contraction rows x 64]
-              else load2d(a_dst + u * C::ACT_SUB, &tm_act, s * 64, m_cta);
+              load2d(a_dst + u * C::ACT_SUB, &tm_act, s * 64, m_cta);
               if (IS16) {
-                uint8_t* w = w_dst + u * W_STAGE;
-                if (p.dir == QG_FWD) {
-                  load2d(w, &tm_w16, s * 64, r0);
-                  load2d(w + 8192, &tm_w16, s * 64, r0 + 64);
-                } else {
-                  load2d(w, &tm_w16, r0, s * 64);
-                  load2d(w + 8192, &tm_w16, r0 + 64, s * 64);
+#pragma unroll
+                for (int b = 0; b < C::BRICKS; ++b) {
+                  uint8_t* w = w_dst + u * C::W_SUB + b * 8192;
+                  if (p.dir == QG_FWD) load2d(w, &tm_w16, s * 64, r0 + b * 64);
+                  else load2d(w, &tm_w16, r0 + b * 64, s * 64);
                 }
               }
             }
           } else {
             if (p.late_wait) pdl_wait();
             load2d(a_dst, &tm_lact, 0, m_cta);
-            if (p.dir == QG_FWD) {
-              load2d(w_dst, &tm_lw, 0, r0);
-              load2d(w_dst + 8192, &tm_lw, 0, r0 + 64);
-            } else {
-              load2d(w_dst, &tm_lw, r0, 0);
-              load2d(w_dst + 8192, &tm_lw, r0 + 64, 0);
+#pragma unroll
+            for (int b = 0; b < C::BRICKS; ++b) {
+              if (p.dir == QG_FWD) load2d(w_dst + b * 8192, &tm_lw, 0, r0 + b * 64);
+              else load2d(w_dst + b * 8192, &tm_lw, r0 + b * 64, 0);
             }
           }
           if (++st == NS) { st = 0; ph ^= 1; }
@@ -556,10 +559,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       // Descriptors: the high words are fixed for the launch, the low words are address >> 4 plus
       // the leading-dimension field; a stage or a K step of 16 only adds a constant to them.
       const uint64_t a_d0 = (p.dir == QG_FWD) ? umma_desc_sw128(smem_u32(sW), 16, 1024) : umma_desc_sw128(smem_u32(sW), 8192, 1024);
-      const uint64_t b_d0 = p.b_mn ? umma_desc_sw128(smem_u32(sAct), 8192, 1024) : umma_desc_sw128(smem_u32(sAct), 16, 1024);
+      const uint64_t b_d0 = umma_desc_sw128(smem_u32(sAct), 16, 1024);
       const uint32_t a_hi = (uint32_t)(a_d0 >> 32), b_hi = (uint32_t)(b_d0 >> 32);
       const uint32_t a_k = (p.dir == QG_FWD) ? (32u >> 4) : (2048u >> 4);  // low-word step per K = 16
-      const uint32_t b_k = p.b_mn ? (2048u >> 4) : (32u >> 4);
+      constexpr uint32_t b_k = 32u >> 4;
       const uint32_t idesc = p.idesc;
       for (int item = worker; item < n_items && ok; item += n_workers, ++tcount) {
         QG_ITEM_DECODE(item);
@@ -590,7 +593,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
 #pragma unroll
           for (int u = 0; u < KS; ++u) {
             if (u > 0 && s * KS + u >= s_main) break;
-            const uint32_t au = a_lo + u * (W_STAGE >> 4), bu = b_lo + u * (C::ACT_SUB >> 4);
+            const uint32_t au = a_lo + u * (C::W_SUB >> 4), bu = b_lo + u * (C::ACT_SUB >> 4);
             umma_f16_split<PAIR>(d_tmem, au, a_hi, bu, b_hi, idesc, (uint32_t)(u != 0 || s != 0));
             umma_f16_split<PAIR>(d_tmem, au + a_k, a_hi, bu + b_k, b_hi, idesc, 1u);
             umma_f16_split<PAIR>(d_tmem, au + 2 * a_k, a_hi, bu + 2 * b_k, b_hi, idesc, 1u);
@@ -610,6 +613,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         if (ok) {
           if (PAIR) umma_commit_pair(&acc_full[acc], 3);
           else umma_commit(&acc_full[acc]);
+          if (item + n_workers >= n_items) {
+            if (PAIR) umma_commit_pair(last_full, 3);
+            else umma_commit(last_full);
+          }
         }
       }
     }
@@ -624,7 +631,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       const int grp = t / UTG, tg = t % UTG;
       const UnitDst ud(tg & 127);
       const uint32_t w_base = smem_u32(sW);
-      constexpr int BB = PACKED ? C::RAW_STAGE / (2 * KS) : 0;  // bytes of a brick
+      constexpr int BB = PACKED ? C::RAW_STAGE / (C::BRICKS * KS) : 0;  // bytes of a brick
       int st = 0, rs = 0, turn = 0;  // ring positions of the current step, and the group whose step it is
       uint32_t ph = 0, rph = 0;
       bool ok = true;
@@ -641,7 +648,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
               // (element-wise, so the swizzled placement is untouched)
               if (!mbar_wait(&full[st], ph, p.status, 203)) { ok = false; break; }
               uint4* tile16 = (uint4*)(sW + st * C::W_BYTES);
-              for (int i = 0; i < subs * 1024 / UTG; ++i) {
+              for (int i = 0; i < subs * (C::W_SUB / 16) / UTG; ++i) {
                 uint4 v = tile16[tg + i * UTG];
                 uint32_t* w = (uint32_t*)&v;
 #pragma unroll
@@ -664,15 +671,15 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
               // two halves of the group.
               const int u = tg >> 7;
               if (u < subs) {
-                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : 2 * u * BB);
+                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : C::BRICKS * u * BB);
                 const int next = p.dir == QG_FWD ? KS * BB : BB;
-                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * W_STAGE;
+                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB;
                 if (p.act_f16) {
 #pragma unroll
-                  for (int b = 0; b < 2; ++b) unpack_unit<FMT, false>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, false>(raw + b * next, tg & 127, dst + b * 8192, ud);
                 } else {
 #pragma unroll 1
-                  for (int b = 0; b < 2; ++b) unpack_unit<FMT, true>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, true>(raw + b * next, tg & 127, dst + b * 8192, ud);
                 }
               }
               fence_proxy_async_smem();
@@ -702,7 +709,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       int rs = 0;
       uint32_t rph = 0;
       bool ok = true;
-      constexpr uint32_t bb = (uint32_t)C::RAW_STAGE / (2 * KS);
+      constexpr uint32_t bb = (uint32_t)C::RAW_STAGE / (C::BRICKS * KS);
       for (int item = worker; item < n_items && ok; item += n_workers) {
         QG_ITEM_DECODE(item);
         (void)n_steps;
@@ -710,7 +717,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         (void)m0;
         // a pair's second half may lie past the last brick row: it then works on the last one again
         // (its results are not stored)
-        const int br = min(r0 >> 6, p.nb - 2);
+        const int br = min(r0 >> 6, p.nb - C::BRICKS);
         const uint8_t* b0 = p.bricks + (p.dir == QG_FWD ? ((size_t)br * p.nbk + s_begin) * bb : ((size_t)s_begin * p.nbk + br) * bb);
         const size_t b1 = p.dir == QG_FWD ? (size_t)p.nbk * bb : (size_t)bb;    // the tile's second brick
         const size_t step = p.dir == QG_FWD ? (size_t)bb : (size_t)p.nbk * bb;  // the next contraction step
@@ -718,13 +725,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
           if (!mbar_wait(&raw_empty[rs], rph ^ 1, p.status, 102)) { ok = false; break; }
           const uint32_t subs = KS == 1 ? 1u : (uint32_t)min(KS, s_main - si * KS);
           uint8_t* dst = sRaw + rs * C::RAW_STAGE;
-          mbar_expect_tx(&raw_full[rs], subs * 2 * bb);
+          mbar_expect_tx(&raw_full[rs], subs * C::BRICKS * bb);
           if (p.dir == QG_FWD) {  // a brick row's steps are adjacent
             bulk_load_1d(dst, b0, subs * bb, &raw_full[rs]);
-            bulk_load_1d(dst + KS * bb, b0 + b1, subs * bb, &raw_full[rs]);
+            if (C::BRICKS > 1) bulk_load_1d(dst + KS * bb, b0 + b1, subs * bb, &raw_full[rs]);
           } else {  // column neighbours are adjacent
-            bulk_load_1d(dst, b0, 2 * bb, &raw_full[rs]);
-            if (KS > 1 && subs > 1) bulk_load_1d(dst + 2 * bb, b0 + step, 2 * bb, &raw_full[rs]);
+            bulk_load_1d(dst, b0, C::BRICKS * bb, &raw_full[rs]);
+            if (KS > 1 && subs > 1) bulk_load_1d(dst + C::BRICKS * bb, b0 + step, C::BRICKS * bb, &raw_full[rs]);
           }
           if (++rs == NR) { rs = 0; rph ^= 1; }
         }
@@ -745,7 +752,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       if (!mbar_wait(&acc_full[acc], aph, p.status, 401)) break;
       tc_fence_after();
       const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
-      for (int c = 0; c < p.TN / 32; c += stride) {
+      for (int c = wq * 32 < C::ROWS ? 0 : p.TN; c < p.TN / 32; c += stride) {
         if (p.tma_out) tma_chunk(acc, wq, c, r0, m0, sOut + wq * C::OUT_WARP, out_chunk);
         else direct_chunk(acc, wq, c, r0, m0, split);
       }
@@ -777,13 +784,11 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   }
 }
 
-// Sums split-K partials in split order (deterministic) and applies the epilogue the fused path
-// would have applied: per-token scale, scalar factor, bias, accumulate.  Output is f32 at
-// out[tok * s_tok + row * s_row].
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int M, int R, float* __restrict__ out,
-                                     size_t s_tok, size_t s_row, const float* __restrict__ row_scale,
-                                     const float* __restrict__ alpha_dev, const float* __restrict__ bias,
-                                     int accumulate, const float* __restrict__ residual) {
+// Sums the pieces' partials in order (deterministic) and applies the epilogue the fused path would have
+// applied: per-token scale, bias, accumulate or residual.  Output is f32 with row pitch ld.
+__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int M, int R, float* __restrict__ out, size_t ld,
+                                     const float* __restrict__ row_scale, const float* __restrict__ bias, int accumulate,
+                                     const float* __restrict__ residual) {
   pdl_entry();
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = (size_t)M * R;
@@ -792,12 +797,11 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
   float v = 0.f;
   for (int k = 0; k < splits; ++k) v += part[(size_t)k * n + e];
   if (row_scale) v *= row_scale[tok];
-  if (alpha_dev) v *= alpha_dev[0];
   if (bias) v += bias[row];
-  float* o = out + tok * s_tok + row * s_row;
-  if (accumulate) v += *o;
-  if (residual) v += residual[tok * s_tok + row * s_row];
-  *o = v;
+  const size_t at = tok * ld + row;
+  if (accumulate) v += out[at];
+  if (residual) v += residual[at];
+  out[at] = v;
 }
 
 // ------------------------------------------------------------------ host side
@@ -817,8 +821,8 @@ template <int KIND, int FMT>
 static QKernel qkernel() {
   return {(const void*)qgemm_kernel<KIND, FMT>, QCfg<KIND, FMT>::THREADS, QCfg<KIND, FMT>::SMEM_BYTES};
 }
-// fmt: a packed ggml format, QF_16 or QF_16CONV.  The wide single-CTA kernel only serves 16-bit weights
-// (token contractions and converted weights): packed weights and plain ones run as pairs or narrow tiles.
+// fmt: a packed ggml format, QF_16 or QF_16CONV.  The wide single-CTA kernel only serves converted
+// 16-bit weights: the others' wide tiles run as pairs.
 static QKernel qkernel_for(int kind, int fmt) {
   if (kind == QK_PAIR) switch (fmt) {
       case QF_16: return qkernel<QK_PAIR, QF_16>();
@@ -835,8 +839,15 @@ static QKernel qkernel_for(int kind, int fmt) {
       case GGML_Q4_K: return qkernel<QK_NARROW, GGML_Q4_K>();
       case GGML_Q6_K: return qkernel<QK_NARROW, GGML_Q6_K>();
     }
+  if (kind == QK_HALF) switch (fmt) {
+      case QF_16: return qkernel<QK_HALF, QF_16>();
+      case QF_16CONV: return qkernel<QK_HALF, QF_16CONV>();
+      case GGML_Q4_0: return qkernel<QK_HALF, GGML_Q4_0>();
+      case GGML_Q8_0: return qkernel<QK_HALF, GGML_Q8_0>();
+      case GGML_Q4_K: return qkernel<QK_HALF, GGML_Q4_K>();
+      case GGML_Q6_K: return qkernel<QK_HALF, GGML_Q6_K>();
+    }
   if (kind == QK_WIDE) switch (fmt) {
-      case QF_16: return qkernel<QK_WIDE, QF_16>();
       case QF_16CONV: return qkernel<QK_WIDE, QF_16CONV>();
     }
   return {nullptr, 0, 0};
@@ -853,7 +864,7 @@ int qgemm_init() {
       return RT_ERR_CUDA;
     g_encode = (PFN_encodeTiled)fn;
   }
-  for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW})
+  for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF})
     for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K}) {
       const QKernel k = qkernel_for(kind, fmt);
       if (k.fn && cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem) != cudaSuccess) return RT_ERR_CUDA;
@@ -967,19 +978,19 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 // (us, 64 contraction elements) are fitted to sweeps over both kernels and all widths (eight weight shapes
 // of 128..151936 rows, 1..8192 tokens): about 0.33 for a pair while the single-thread roles and the unpack
 // passes set the pace, more from about 64 tokens of width per CTA on, when the MMAs do; 0.25 for narrow
-// tiles, which hand over two steps at a time.
-// Narrow tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
-// backward at 1024 tokens 31 us (44 on pairs of 128 tokens before), 1024x1024 at 157 tokens 10 us (15).
+// tiles, which hand over two steps at a time, and 0.17 for half tiles, whose unpack passes are half as long.
+// Narrow and half tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
+// backward at 1024 tokens 29 us (44 on pairs of 128 tokens before), 8192x3072 Q6_K backward at 24 tokens 30 us
+// (43 on narrow tiles, 91 before), 1024x2048 at 157 tokens 9.6 us (12).
 // The choice changes no result: an output element's contraction is one chain in any tile.
 struct QPlan {
   int kind, TN;
 };
-static QPlan qgemm_plan(int kfmt, bool tok_mode, int M, int out_rows, int n_splits, int steps, int num_sms) {
-  if (tok_mode) return {QK_WIDE, 64};
+static QPlan qgemm_plan(int kfmt, int M, int out_rows, int n_splits, int steps, int num_sms) {
   QPlan best = {QK_NARROW, 64};
   double best_cost = -1;
   auto consider = [&](int kind, int tn, double step_us) {
-    const int rows = kind == QK_PAIR ? 256 : 128;
+    const int rows = kind == QK_PAIR ? 256 : kind == QK_HALF ? 64 : 128;
     const long tiles = (long)((out_rows + rows - 1) / rows) * ((M + tn - 1) / tn) * n_splits;
     const long workers = kind == QK_PAIR ? g_pair_workers : num_sms;
     const double cost = (double)((tiles + workers - 1) / workers) * (steps * step_us + 0.5);
@@ -987,6 +998,8 @@ static QPlan qgemm_plan(int kfmt, bool tok_mode, int M, int out_rows, int n_spli
   };
   if (M > 32) consider(QK_NARROW, 64, 0.25);
   consider(QK_NARROW, 32, 0.25);
+  if (M > 32) consider(QK_HALF, 64, 0.16);
+  consider(QK_HALF, 32, 0.155);
   if (kfmt == QF_16CONV) {
     for (int tn = 256; tn >= 128; tn -= 32) consider(QK_WIDE, tn, 0.25 + 0.0012 * tn);
   } else if (g_pair_workers > 0 && M > 64) {
@@ -1009,8 +1022,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   const bool is16 = fmt_is_16bit(w.fmt);
   const int contract = a.dir == QG_FWD ? w.cols : w.rows;
   const int out_rows = a.dir == QG_FWD ? w.rows : w.cols;
-  if ((!a.tok_mode && contract % 8 != 0) || (is16 && w.cols % 8 != 0)) return RT_ERR_BAD_SHAPE;
-  if (a.tok_mode && (!is16 || a.dir != QG_BWD || a.M > 64 || a.lora.rank > 0 || a.out_dtype != OUT_F32)) return RT_ERR_BAD_ARG;
+  if (contract % 8 != 0 || (is16 && w.cols % 8 != 0)) return RT_ERR_BAD_SHAPE;
   if ((a.accumulate || a.residual) && a.out_dtype != OUT_F32) return RT_ERR_BAD_ARG;
   if (a.lora.rank > 64 || (a.lora.rank > 0 && (!a.lora.act || !a.lora.w))) return RT_ERR_BAD_ARG;
 
@@ -1046,31 +1058,22 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   // in pieces of a FIXED 8192 elements whose f32 partial sums are added afterwards: the error of
   // one chain grows with its length (about 3e-4 relative over 150 000 elements).
   p.steps_per_split = p.n_main;
-  if (!a.tok_mode && a.out_dtype == OUT_F32 && p.n_main > 256) p.steps_per_split = 128;
-  if (a.tok_mode) {
-    const int n_tiles = (out_rows + 127) / 128;
-    int splits = num_sms / n_tiles;
-    if (splits > p.n_main / 4) splits = p.n_main / 4;
-    if (splits < 1) splits = 1;
-    p.steps_per_split = (p.n_main + splits - 1) / splits;
-  }
+  if (a.out_dtype == OUT_F32 && p.n_main > 256) p.steps_per_split = 128;
   p.n_splits = (p.n_main + p.steps_per_split - 1) / p.steps_per_split;
-  p.b_mn = a.tok_mode ? 1 : 0;
 
-  const QPlan plan = qgemm_plan(kfmt, a.tok_mode != 0, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms);
+  const QPlan plan = qgemm_plan(kfmt, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms);
   const bool pair = plan.kind == QK_PAIR;
   p.TN = plan.TN;
-  p.n_row_tiles = (out_rows + (pair ? 255 : 127)) / (pair ? 256 : 128);
+  const int tile_rows = pair ? 256 : plan.kind == QK_HALF ? 64 : 128;
+  p.n_row_tiles = (out_rows + tile_rows - 1) / tile_rows;
   p.n_tok_tiles = (a.M + p.TN - 1) / p.TN;
   const int tn_cta = pair ? p.TN / 2 : p.TN;  // each CTA of a pair fetches its half of the token tile
   // tcgen05.mma kind::f16 needs A and B of ONE 16-bit type (f16 x bf16 is an illegal instruction).
   const int ab_fmt = a.act_f16 ? 0 : 1;
-  p.idesc = a.tok_mode ? umma_idesc(ab_fmt, ab_fmt, 1, 1, 128, 64)
-                       : umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, pair ? 256 : 128, p.TN);
+  p.idesc = umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, pair ? 256 : 128, p.TN);
 
   CUtensorMap tm_act, tm_w16, tm_lact, tm_lw;
-  int rc = a.tok_mode ? make_map(&tm_act, a.act, (uint64_t)contract, 64, 64, 64, !a.act_f16)
-                      : make_map(&tm_act, a.act, (uint64_t)a.M, (uint64_t)contract, 64, (uint32_t)tn_cta, !a.act_f16);
+  int rc = make_map(&tm_act, a.act, (uint64_t)a.M, (uint64_t)contract, 64, (uint32_t)tn_cta, !a.act_f16);
   if (rc) return rc;
   tm_w16 = tm_act;
   tm_lact = tm_act;
@@ -1087,7 +1090,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     if (rc) return rc;
   }
   p.part = nullptr;
-  if (p.n_splits > 1 || a.tok_mode) {
+  if (p.n_splits > 1) {
     const size_t need = (size_t)p.n_splits * a.M * out_rows;
     if (a.fixed_part) {
       if (need > a.fixed_part_floats) return RT_ERR_TOO_LARGE;
@@ -1143,16 +1146,15 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   RT_COUNT_LAUNCH(1);
   if (p.part) {
     const size_t n = (size_t)a.M * out_rows;
-    const size_t s_tok = a.tok_mode ? a.out_s_tok : (size_t)p.ld_out, s_row = a.tok_mode ? a.out_s_row : 1;
-    pdl(splitk_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, st)(p.part, p.n_splits, a.M, out_rows, (float*)a.out, s_tok,
-                                                                    s_row, a.row_scale, a.alpha_dev, p.bias, a.accumulate, a.residual);
+    pdl(splitk_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, st)(p.part, p.n_splits, a.M, out_rows, (float*)a.out, (size_t)p.ld_out,
+                                                                    a.row_scale, p.bias, a.accumulate, a.residual);
     RT_COUNT_LAUNCH(1);
   }
   if (e1) {
     cudaEventRecord(e1, st);
     const double out_bytes = a.out_dtype == OUT_F32 ? 4.0 : 2.0;
     ctx->prof_flops += 2.0 * (double)a.M * (double)w.rows * (double)w.cols;
-    ctx->prof_recs.push_back({a.tok_mode ? 3 : (a.aux ? 2 : a.dir), a.M, out_rows, contract});
+    ctx->prof_recs.push_back({a.dir, a.M, out_rows, contract});
     ctx->prof_bytes += (double)w.dev_nbytes + 2.0 * (double)a.M * contract + out_bytes * (double)a.M * out_rows * (a.accumulate || a.residual ? 2.0 : 1.0);
   }
   return cudaGetLastError() == cudaSuccess ? RT_OK : RT_ERR_CUDA;

@@ -55,11 +55,6 @@ struct QGemmArgs {
   const float* bias = nullptr;         // forward only, per output feature
   const float* row_scale = nullptr;    // optional per-token factor on the result (before bias)
   LoraSide lora;
-  // token-contraction mode (LoRA gradients): out[i*out_s_tok + j*out_s_row] (+)= alpha * sum_m P[m,i] * Q[m,j]
-  // with Q = the dense 16-bit `w` [tokens x C], P = act [tokens x 64], M = rank (i < M), dir = QG_BWD
-  int tok_mode = 0;
-  size_t out_s_tok = 0, out_s_row = 1;
-  const float* alpha_dev = nullptr;    // optional device scalar factor (split-K / token mode only)
   // split-K partials go to this caller-provided buffer instead of ctx scratch (and nothing is
   // cached or allocated on the way); a launch that needs more fails with RT_ERR_TOO_LARGE
   float* fixed_part = nullptr;
@@ -67,7 +62,6 @@ struct QGemmArgs {
   // The launch right before this one is the low-rank stream that produces lora.act: a programmatic launch
   // may start at once and waits for it only where it reads that.
   int late_wait = 0;
-  int aux = 0;                         // 1: a skinny LoRA helper product (kept apart in the profile)
 };
 
 int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a);
