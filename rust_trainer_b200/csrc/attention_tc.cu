@@ -264,7 +264,11 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[b]);
     }
-    if (ok && mbar_wait(pv_done, (uint32_t)(ntiles - 1) & 1, status, SITE_PVDONE)) {
+    // the last product's phase, and the one before it first: a warp that never rescaled may be here while a
+    // slower warp still owes the tile before (its S came after the product two before, no later one), and
+    // a parity alone does not tell the last phase from the one two before
+    if (ok && (ntiles < 2 || mbar_wait(pv_done, (uint32_t)ntiles & 1, status, SITE_PVDONE)) &&
+        mbar_wait(pv_done, (uint32_t)(ntiles - 1) & 1, status, SITE_PVDONE)) {
       // O / l as f16 into Q's shared memory (every product that read Q has completed), in the
       // layout of a swizzled TMA box, then one bulk store per 64-column panel: rows past the end of
       // the batch are clipped by the tensor map

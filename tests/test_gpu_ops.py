@@ -213,3 +213,17 @@ def test_attention_backward_of_a_sequence_ignores_its_batch_mates(ctx, lens, nh,
                 assert np.array_equal(w[a:b], s), (i, float(np.abs(w[a:b] - s).max()))
             else:
                 assert rel_l2(w[a:b], s) < 1e-5, (i, rel_l2(w[a:b], s))
+
+
+@pytest.mark.parametrize("lens,nh,nkv,hd", [([512] * 16, 16, 8, 128), ([64] * 3 + [449, 700], 14, 2, 64)], ids=["equal", "ragged"])
+def test_attention_gives_the_same_bits_every_time(ctx, lens, nh, nkv, hd):
+    """Every output element has one writer and one order of sums, so a repeated call returns the same bits; a wait that
+    takes one phase of a barrier for another shows here (32 rows of O at a time) before it shows in a tolerance."""
+    rng = np.random.default_rng(5)
+    M = sum(lens)
+    q, k, v, do = (rng.standard_normal((M, n, hd)).astype(np.float32) for n in (nh, nkv, nkv, nh))
+    ss = _seq_start(lens)
+    first = ops.attention(ctx, q, k, v, ss) + ops.attention_backward(ctx, q, k, v, do, ss)
+    for _ in range(6):
+        again = ops.attention(ctx, q, k, v, ss) + ops.attention_backward(ctx, q, k, v, do, ss)
+        assert all(np.array_equal(a, b) for a, b in zip(first, again))
