@@ -29,12 +29,13 @@
 #include "rt_internal.h"
 #include <cuda_fp16.h>
 #include <stdint.h>
+#include <algorithm>
 
 namespace rt {
 
 namespace {
 
-constexpr int LG_NS = 4, LG_THREADS = 192;
+constexpr int LG_NS = 3, LG_THREADS = 192, LG_CTAS_PER_SM = 3;
 constexpr uint32_t LG_Q_BYTES = 2 * 64 * 128, LG_P_BYTES = 64 * 128, LG_STAGE = LG_Q_BYTES + LG_P_BYTES;
 constexpr uint32_t LG_OFF_BAR = LG_NS * LG_STAGE;
 constexpr uint32_t LG_TOTAL = LG_OFF_BAR + 256 + 1024;
@@ -66,7 +67,7 @@ __device__ __forceinline__ float ld_cluster_f1(uint32_t cluster_addr) {
   return v;
 }
 
-__global__ void __launch_bounds__(LG_THREADS, 2)
+__global__ void __launch_bounds__(LG_THREADS, LG_CTAS_PER_SM)
 lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -270,29 +271,36 @@ __global__ void __launch_bounds__(256) lora_scale_small_kernel(const LgScaleArgs
 
 }  // namespace
 
-// Tokens per split of the tcgen05 contraction: fixed by the token count's range only.
-int lora_grads_tc_tokens_per_split(int M) { return M >= 4096 ? 1024 : M >= 2048 ? 512 : M >= 1024 ? 256 : M >= 512 ? 128 : 64; }
-// whether the splits fit one cluster (of the portable size), which then adds them itself
-static bool lora_grads_tc_direct(int M) {
-  const int tps = lora_grads_tc_tokens_per_split(M);
-  return (M + tps - 1) / tps <= 8;
+// Tokens per split: at most 1024 (the tensor core's accumulator error grows with a chain's length), fewer
+// while the column tiles alone leave places on the GPU, a multiple of 64.
+static int lora_grads_tokens_per_split(int M, int tiles, int num_sms) {
+  const int want = std::max((M + 1023) / 1024, std::min(8, LG_CTAS_PER_SM * num_sms / std::max(1, tiles)));
+  return ((M + want - 1) / want + 63) / 64 * 64;
 }
-
+struct LgPlan {
+  int tiles, tps, splits;
+  bool direct;  // the splits fit one cluster (of the portable size), which then adds them itself
+};
+static LgPlan lora_grads_plan(const LoraGradJob* jobs, int n, int M, int num_sms) {
+  LgPlan p;
+  p.tiles = 0;
+  for (int j = 0; j < n; ++j) p.tiles += (jobs[j].N + 127) / 128 + (jobs[j].K + 127) / 128;
+  p.tps = lora_grads_tokens_per_split(M, p.tiles, num_sms);
+  p.splits = (M + p.tps - 1) / p.tps;
+  p.direct = p.splits <= 8;
+  return p;
+}
 bool lora_grads_tc_takes(const LoraGradJob& j) {
   return j.r > 0 && j.r <= 64 && j.N % 8 == 0 && j.K % 8 == 0 && j.ld_dy % 8 == 0 && j.t.n >= 1 && j.t.n <= 3 &&
          (((uintptr_t)j.hs | (uintptr_t)j.dy | (uintptr_t)j.gs | (uintptr_t)j.x) & 15) == 0;
 }
-static int lora_grads_splits(int M) {
-  const int tps = lora_grads_tc_tokens_per_split(M);
-  return (M + tps - 1) / tps;
-}
 // per job: the scaled Hs and Gs, the splits' largest factors, and the partial sums if they go through memory
-size_t lora_grads_tc_workspace_floats(const LoraGradJob* jobs, int n, int M) {
-  const size_t splits = (size_t)lora_grads_splits(M);
+size_t lora_grads_tc_workspace_floats(rt_ctx* c, const LoraGradJob* jobs, int n, int M) {
+  const LgPlan p = lora_grads_plan(jobs, n, M, c->num_sms);
   size_t f = 0;
   for (int j = 0; j < n; ++j) {
-    f += (size_t)M * 64 + (splits + 63) / 64 * 64;
-    if (!lora_grads_tc_direct(M)) f += splits * jobs[j].r * ((size_t)jobs[j].N + (size_t)jobs[j].K);
+    f += (size_t)M * 64 + ((size_t)p.splits + 63) / 64 * 64;
+    if (!p.direct) f += (size_t)p.splits * jobs[j].r * ((size_t)jobs[j].N + (size_t)jobs[j].K);
   }
   return f;
 }
@@ -310,9 +318,10 @@ int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float
   LgArgs g;
   g.n_jobs = n;
   g.M = M;
-  g.tps = lora_grads_tc_tokens_per_split(M);
-  g.direct = lora_grads_tc_direct(M) ? 1 : 0;
-  const int splits = lora_grads_splits(M);
+  const LgPlan plan = lora_grads_plan(jobs, n, M, c->num_sms);
+  const int splits = plan.splits;
+  g.tps = plan.tps;
+  g.direct = plan.direct ? 1 : 0;
   LgScaleArgs sa;
   sa.M = M;
   sa.tps = g.tps;

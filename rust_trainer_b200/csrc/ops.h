@@ -85,9 +85,8 @@ struct LoraGradJob {
   LoraGroupTable t;
 };
 constexpr int LORA_GRAD_JOBS = 4;  // jobs of one launch: the linears of a block
-int lora_grads_tc_tokens_per_split(int M);
 bool lora_grads_tc_takes(const LoraGradJob& j);
-size_t lora_grads_tc_workspace_floats(const LoraGradJob* jobs, int n, int M);
+size_t lora_grads_tc_workspace_floats(rt_ctx* c, const LoraGradJob* jobs, int n, int M);
 // adds dB and dA of the jobs into the gradients of their tables' members; 0 or 3 (launch failure)
 int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float* workspace);
 // adds partial sums [splits][r x N] and [splits][r x K] into the table's members, splits in order
