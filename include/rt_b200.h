@@ -68,6 +68,13 @@ const char* rt_last_error(const rt_ctx* ctx);
 rt_status rt_ctx_synchronize(rt_ctx* ctx);
 /* The CUDA stream (cudaStream_t) every call on this ctx is issued on. */
 void* rt_ctx_stream(rt_ctx* ctx);
+/* Page-locked host memory for results: the copies that the host-buffer calls make into it run at the
+ * link's rate, and it has no first-touch faults.  Blocks come from a pool of the process (256 MB at
+ * most; safe from any thread) and go back to it; NULL when the pool is full or nothing can be locked:
+ * then use ordinary memory, which every call takes as well.  A block may outlive the context; the
+ * pool's free blocks are unlocked with the last context. */
+void* rt_host_alloc(rt_ctx* ctx, size_t bytes);
+void rt_host_free(void* block);
 /* Issue all later calls on `cuda_stream` (a cudaStream_t of the same device) instead of the
  * stream the ctx created, so a host that owns its streams can order and time the work. */
 rt_status rt_ctx_set_stream(rt_ctx* ctx, void* cuda_stream);

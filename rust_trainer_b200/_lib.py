@@ -55,6 +55,8 @@ def _declare(L: C.CDLL) -> None:
         "rt_last_error": (C.c_char_p, [vp]),
         "rt_ctx_synchronize": (i32, [vp]),
         "rt_ctx_stream": (vp, [vp]),
+        "rt_host_alloc": (vp, [vp, sz]),
+        "rt_host_free": (None, [vp]),
         "rt_ctx_set_stream": (i32, [vp, vp]),
         "rt_frozen_forward_dev": (i32, [vp, vp, C.c_int, sz, vp, C.c_int, C.c_int]),
         "rt_frozen_backward_input_dev": (i32, [vp, vp, C.c_int, sz, vp, C.c_int, C.c_int]),

@@ -9,6 +9,7 @@
 #include <vector>
 #include <mutex>
 #include <set>
+#include <iterator>
 
 void* rt_ctx::get_scratch(int slot, size_t bytes) {
   if (bytes <= scratch_bytes[slot]) return scratch[slot];
@@ -55,6 +56,73 @@ static void ctx_register(const rt_ctx* c, bool live) {
   std::lock_guard<std::mutex> lock(g_ctx_mutex);
   if (live) g_live_ctx.insert(c);
   else g_live_ctx.erase(c);
+}
+static bool ctx_any() {
+  std::lock_guard<std::mutex> lock(g_ctx_mutex);
+  return !g_live_ctx.empty();
+}
+
+// Page-locked result blocks.  What it is for: 1.5 MB of results into fresh ordinary memory cost 80 us more
+// than into locked memory (the driver's staging copy, and 375 page faults of the allocation), twice what
+// the matmul behind them takes.  Sizes are rounded up to an eighth of their power of two, so that calls of
+// nearly the same size reuse each other's blocks; when the limit is reached, free blocks of other sizes go first.
+namespace {
+struct HostPool {
+  static constexpr size_t LIMIT = (size_t)256 << 20;
+  std::mutex mutex;
+  std::multimap<size_t, void*> idle;
+  std::map<void*, size_t> used;
+  size_t total = 0;  // locked, idle or used
+};
+HostPool& host_pool() {
+  static HostPool* p = new HostPool;  // never destroyed: blocks come back from interpreters that are shutting down
+  return *p;
+}
+void host_pool_trim_locked(HostPool& hp, size_t down_to) {
+  while (hp.total > down_to && !hp.idle.empty()) {
+    auto it = std::prev(hp.idle.end());
+    cudaFreeHost(it->second);
+    hp.total -= it->first;
+    hp.idle.erase(it);
+  }
+}
+}  // namespace
+static void* host_pool_take(size_t bytes) {
+  HostPool& hp = host_pool();
+  size_t unit = 4096;
+  while (unit * 16 < bytes) unit *= 2;
+  const size_t size = (bytes + unit - 1) / unit * unit;
+  std::lock_guard<std::mutex> lock(hp.mutex);
+  auto it = hp.idle.find(size);
+  void* p = nullptr;
+  if (it != hp.idle.end()) {
+    p = it->second;
+    hp.idle.erase(it);
+  } else {
+    if (size > HostPool::LIMIT) return nullptr;
+    host_pool_trim_locked(hp, HostPool::LIMIT - size);
+    if (hp.total + size > HostPool::LIMIT) return nullptr;
+    if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    hp.total += size;
+  }
+  hp.used[p] = size;
+  return p;
+}
+static void host_pool_give(void* p) {
+  HostPool& hp = host_pool();
+  std::lock_guard<std::mutex> lock(hp.mutex);
+  auto it = hp.used.find(p);
+  if (it == hp.used.end()) return;
+  hp.idle.emplace(it->second, p);
+  hp.used.erase(it);
+}
+static void host_pool_trim() {
+  HostPool& hp = host_pool();
+  std::lock_guard<std::mutex> lock(hp.mutex);
+  host_pool_trim_locked(hp, 0);
 }
 
 int frozen_matmul_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
@@ -121,6 +189,16 @@ void rt_ctx_destroy(rt_ctx* c) {
   if (c->status_host) cudaFreeHost(c->status_host);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;
+  if (!rt::ctx_any()) rt::host_pool_trim();
+}
+
+void* rt_host_alloc(rt_ctx* c, size_t bytes) {
+  if (!c || bytes == 0 || cudaSetDevice(c->device) != cudaSuccess) return nullptr;
+  return rt::host_pool_take(bytes);
+}
+
+void rt_host_free(void* p) {
+  if (p) rt::host_pool_give(p);
 }
 
 const char* rt_last_error(const rt_ctx* c) { return c ? c->err.c_str() : "null context"; }

@@ -130,7 +130,7 @@ rt_status lora_grads_flush(rt_ctx* c, LinearScratch& sc, int M) {
   const int n = sc.n_jobs;
   sc.n_jobs = 0;
   if (n == 0) return RT_OK;
-  if (!sc.grad_ws.reserve(lora_grads_tc_workspace_floats(sc.jobs, n, M) * sizeof(float)))
+  if (!sc.grad_ws.reserve(lora_grads_tc_workspace_floats(c, sc.jobs, n, M) * sizeof(float)))
     return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
   if (launch_lora_grads_tc(c, sc.jobs, n, M, sc.grad_ws.as<float>())) return c->fail(RT_ERR_CUDA, "lora gradient kernel launch failed");
   return RT_OK;
@@ -490,6 +490,7 @@ rt_status rt_linear_forward(rt_linear* l, const float* x_host, size_t t, float* 
   float* yf = (float*)c->get_scratch(2, t * N * sizeof(float));
   if (!xf || !xh || !yf) return c->fail(RT_ERR_CUDA, "out of device memory");
   RT_CUDA(c, cudaMemcpyAsync(xf, x_host, t * K * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  const PdlScope pdl_scope(t);
   launch_f32_to_16(xf, xh, t * K, true, c->stream);
   rt_status st = linear_forward_dev(l, ctx_scratch(c), xh, (int)t, yf, RT_DT_F32, 0);
   if (st) return st;
@@ -512,6 +513,7 @@ rt_status rt_linear_backward(rt_linear* l, const float* x_host, const float* dy_
   __half* dyh = (__half*)(s1 + (t * K * sizeof(__half) + 255) / 256 * 256);
   float* dsc = (float*)((uint8_t*)dyh + (t * N * sizeof(__half) + 255) / 256 * 256);
   RT_CUDA(c, cudaMemcpyAsync(xf, x_host, t * K * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+  const PdlScope pdl_scope(t);
   launch_f32_to_16(xf, xh, t * K, true, c->stream);
   RT_CUDA(c, cudaMemcpyAsync(xf, dy_host, t * N * sizeof(float), cudaMemcpyHostToDevice, c->stream));
   launch_normalize_rows(xf, (int)t, (int)N, dyh, dsc, c->stream);

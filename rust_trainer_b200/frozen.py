@@ -20,6 +20,18 @@ def _fp(a: np.ndarray):
     return a.ctypes.data_as(_F32P)
 
 
+class _HostBlock:
+    """One page-locked block (rt_host_alloc) seen as a float32 array; goes back when the last view of it does."""
+
+    def __init__(self, ptr: int, shape: tuple):
+        self._ptr = ptr
+        self._free = lib().rt_host_free
+        self.__array_interface__ = dict(shape=shape, typestr="<f4", data=(ptr, False), version=3)
+
+    def __del__(self):
+        self._free(self._ptr)
+
+
 class Context:
     """One per GPU (rt_ctx): device, stream and scratch memory."""
 
@@ -36,6 +48,16 @@ class Context:
 
     def synchronize(self) -> None:
         self.check(lib().rt_ctx_synchronize(self._h))
+
+    def result(self, shape: tuple) -> np.ndarray:
+        """An uninitialised float32 array for a result.  Page-locked from 64 KB up (below, the driver's own
+        staging costs less than the bookkeeping), ordinary memory when the library has no locked block to give."""
+        nbytes = 4 * int(np.prod(shape, dtype=np.int64))
+        if nbytes >= 65536:
+            ptr = lib().rt_host_alloc(self._h, nbytes)
+            if ptr:
+                return np.asarray(_HostBlock(ptr, shape))
+        return np.empty(shape, dtype=np.float32)
 
     @property
     def stream(self) -> int:
@@ -142,7 +164,7 @@ class Frozen:
         x = np.ascontiguousarray(x, dtype=np.float32)
         if x.size != t * self.in_dim():
             raise RtError(1, f"forward: x has {x.size} elements, expected {t}*{self.in_dim()}")
-        y = np.empty((t, self.out_dim()), dtype=np.float32)
+        y = self.ctx.result((t, self.out_dim()))
         self.ctx.check(lib().rt_frozen_forward(self._h, _fp(x), t, _fp(y)))
         return y
 

@@ -52,7 +52,7 @@ class Linear:
         x = np.ascontiguousarray(x, dtype=np.float32)
         if x.size != t * self.in_dim():
             raise RtError(1, f"{self.name}: input shape")
-        y = np.empty((t, self.out_dim()), dtype=np.float32)
+        y = self.ctx.result((t, self.out_dim()))
         self.ctx.check(lib().rt_linear_forward(self._h, _fp(x), t, _fp(y)))
         return y
 
@@ -62,7 +62,7 @@ class Linear:
         dy = np.ascontiguousarray(dy, dtype=np.float32)
         if x.size != t * self.in_dim() or dy.size != t * self.out_dim():
             raise RtError(1, f"{self.name}: backward shape")
-        dx = np.empty((t, self.in_dim()), dtype=np.float32)
+        dx = self.ctx.result((t, self.in_dim()))
         self.ctx.check(lib().rt_linear_backward(self._h, _fp(x), _fp(dy), t, _fp(dx)))
         return dx
 

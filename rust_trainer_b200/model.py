@@ -153,7 +153,7 @@ class Model:
         tp = np.ascontiguousarray(target_pos, dtype=np.int32)
         tt = np.ascontiguousarray(target_tok, dtype=np.int32)
         logp = np.empty(tp.size, dtype=np.float32)
-        logits = np.empty((tp.size, self.cfg["vocab"]), dtype=np.float32) if want_logits else None
+        logits = self.ctx.result((tp.size, self.cfg["vocab"])) if want_logits else None
         hits = C.c_int32()
         self.ctx.check(lib().rt_model_score(self._h, _ip(toks), _ip(offs), len(seqs), _ip(tp), _ip(tt), tp.size, _fp(logp),
                                             C.byref(hits), None if logits is None else _fp(logits)))
