@@ -7,6 +7,7 @@
 #include "ctx.h"
 #include "ops.h"
 #include "pdl.cuh"
+#include <algorithm>
 
 namespace rt {
 
@@ -1423,34 +1424,87 @@ __global__ void ce_row_kernel(const float* __restrict__ logits, int v, const int
     }
   }
 }
-// The same for rows whose length is a multiple of 4: 128-bit loads, and the maximum and the sum
-// found in ONE pass (each thread keeps a running maximum and rescales its partial sum when the
-// maximum moves; the partial sums meet in f64), so the logits are read twice instead of three
-// times.
-__global__ void __launch_bounds__(1024)
+// The same for rows whose length is a multiple of 4: 128-bit loads, the maximum and the sum found in ONE
+// pass (each thread keeps a running maximum and rescales its partial sum when the maximum moves; the partial
+// sums meet in f64).  What the chip can hold of the row's exponentials stays there for the second pass: five
+// float4 per thread in registers and twelve in shared memory, each chunk of them relative to the running
+// maximum it met (one factor per chunk brings them to the row's); the rest, half of 151936 columns, is
+// still in L2, with one block per SM, and is read and exponentiated again.  What bounds it: the stream of
+// logits in and gradients out, 0.93 GB for 1024 rows of 151936 columns (141 us at the copy rate), and
+// the exponentials.  1024 rows: 262 us with everything read twice by two blocks per SM, 201 so, 246 keeping the
+// logits instead of the exponentials, 247 as two blocks of 512 threads, 274 as a cluster of eight
+// blocks that reads each logit once into registers (nothing runs under its reductions).
+constexpr int CE_THREADS = 1024, CE_REG4 = 5, CE_CHUNK_BYTES = 4 * CE_THREADS * 16;
+__global__ void __launch_bounds__(CE_THREADS, 1)
 ce_row_vec_kernel(const float* __restrict__ logits, int v, const int* __restrict__ target,
                   const float* __restrict__ weight, float* __restrict__ logp, int* __restrict__ hits,
-                  __half* __restrict__ d16, float* __restrict__ scale, int* __restrict__ argmax, int* status) {
+                  __half* __restrict__ d16, float* __restrict__ scale, int* __restrict__ argmax, int* status, int n_chunks) {
+  extern __shared__ float4 s_row[];  // [n_chunks <= 3][4][CE_THREADS]
   pdl_entry();
   const size_t r = blockIdx.x;
   const float4* row4 = (const float4*)(logits + r * v);
-  const int n4 = v >> 2;
+  const int n4 = v >> 2, tid = threadIdx.x;
   const int tgt = target[r];
   if (tgt < 0 || tgt >= v) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_BAD_INDEX);
+    if (tid == 0) atomicCAS(status, 0, RT_ERR_BAD_INDEX);
     return;
   }
+  const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
   float mt = -INFINITY, st = 0.f;
-  for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-    const float4 x = row4[i];
-    const float cm = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w));
+  auto max4 = [](const float4& x) { return fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w)); };
+  auto take = [&](float cm) {  // a chunk's maximum joins the running one
     if (cm > mt) { st *= expf(mt - cm); mt = cm; }  // expf(-inf) = 0 on the first chunk
-    st += expf(x.x - mt) + expf(x.y - mt) + expf(x.z - mt) + expf(x.w - mt);
+    return mt > -INFINITY ? mt : 0.f;
+  };
+  auto exp4 = [](const float4& x, float ref) { return make_float4(expf(x.x - ref), expf(x.y - ref), expf(x.z - ref), expf(x.w - ref)); };
+  auto add4 = [&](const float4& e) { st += (e.x + e.y) + (e.z + e.w); };
+  float4 keep[CE_REG4];
+#pragma unroll
+  for (int k = 0; k < CE_REG4; ++k) {
+    const int i = tid + k * CE_THREADS;
+    keep[k] = i < n4 ? __ldcs(row4 + i) : none;
+  }
+  float cm = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < CE_REG4; ++k) cm = fmaxf(cm, max4(keep[k]));
+  const float ref0 = take(cm);
+#pragma unroll
+  for (int k = 0; k < CE_REG4; ++k) {
+    keep[k] = exp4(keep[k], ref0);
+    add4(keep[k]);
+  }
+  float ref[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    ref[c] = 0.f;
+    if (c >= n_chunks) continue;
+    float4 x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = (CE_REG4 + c * 4 + k) * CE_THREADS + tid;
+      x[k] = i < n4 ? __ldcs(row4 + i) : none;
+    }
+    ref[c] = take(fmaxf(fmaxf(max4(x[0]), max4(x[1])), fmaxf(max4(x[2]), max4(x[3]))));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 e = exp4(x[k], ref[c]);
+      add4(e);
+      s_row[(c * 4 + k) * CE_THREADS + tid] = e;
+    }
+  }
+  const int i_rest = (CE_REG4 + n_chunks * 4) * CE_THREADS + tid;
+  for (int i0 = i_rest; i0 < n4; i0 += 4 * CE_THREADS) {
+    float4 x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[k] = i0 + k * CE_THREADS < n4 ? row4[i0 + k * CE_THREADS] : none;
+    const float rf = take(fmaxf(fmaxf(max4(x[0]), max4(x[1])), fmaxf(max4(x[2]), max4(x[3]))));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) add4(exp4(x[k], rf));
   }
   const float m = block_max(mt);
   const double s = block_sum_d(mt > -INFINITY ? (double)st * (double)expf(mt - m) : 0.0);
   const float tl = logits[r * v + tgt];
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     logp[r] = tl - (m + (float)log(s));
     if (tl >= m) atomicAdd(hits, 1);
     if (scale) scale[r] = weight[r];
@@ -1460,24 +1514,50 @@ ce_row_vec_kernel(const float* __restrict__ logits, int v, const int* __restrict
     const float inv = (float)(1.0 / s);
     uint2* out = (uint2*)(d16 + r * v);
     const int t4 = tgt >> 2, tk = tgt & 3;
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-      const float4 x = row4[i];
-      float p0 = expf(x.x - m) * inv, p1 = expf(x.y - m) * inv, p2 = expf(x.z - m) * inv, p3 = expf(x.w - m) * inv;
+    auto put = [&](int i, const float4& e, float f) {
+      float p0 = e.x * f, p1 = e.y * f, p2 = e.z * f, p3 = e.w * f;
       if (i == t4) {
         if (tk == 0) p0 -= 1.0f; else if (tk == 1) p1 -= 1.0f; else if (tk == 2) p2 -= 1.0f; else p3 -= 1.0f;
       }
       const __half2 a = __floats2half2_rn(p0, p1), b = __floats2half2_rn(p2, p3);
-      out[i] = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+      __stcs(out + i, make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b));
+    };
+    for (int i0 = i_rest; i0 < n4; i0 += 4 * CE_THREADS) {
+      float4 x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i0 + k * CE_THREADS < n4) x[k] = __ldcs(row4 + i0 + k * CE_THREADS);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i0 + k * CE_THREADS < n4) put(i0 + k * CE_THREADS, exp4(x[k], m), inv);
     }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (c >= n_chunks) continue;
+      const float f = expf(ref[c] - m) * inv;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = (CE_REG4 + c * 4 + k) * CE_THREADS + tid;
+        if (i < n4) put(i, s_row[(c * 4 + k) * CE_THREADS + tid], f);
+      }
+    }
+    const float f0 = expf(ref0 - m) * inv;
+#pragma unroll
+    for (int k = 0; k < CE_REG4; ++k)
+      if (tid + k * CE_THREADS < n4) put(tid + k * CE_THREADS, keep[k], f0);
   }
 }
 void launch_ce_rows(const float* logits, int rows, int v, const int* target, const float* weight, float* logp, int* hits,
                     __half* d16, float* scale, int* argmax, int* status, cudaStream_t st) {
   if (rows <= 0) return;
-  if ((v & 3) == 0 && ((uintptr_t)logits & 15) == 0 && (d16 == nullptr || ((uintptr_t)d16 & 7) == 0))
-    pdl(ce_row_vec_kernel, rows, 1024, 0, st)(logits, v, target, weight, logp, hits, d16, scale, argmax, status);
-  else
+  if ((v & 3) == 0 && ((uintptr_t)logits & 15) == 0 && (d16 == nullptr || ((uintptr_t)d16 & 7) == 0)) {
+    static const bool attr = cudaFuncSetAttribute(ce_row_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * CE_CHUNK_BYTES) == cudaSuccess;
+    const int left = v / 4 - CE_REG4 * CE_THREADS;  // float4s beyond the registers; a row without gradient is read once and needs no place
+    const int n_chunks = attr && d16 && left > 0 ? std::min(3, (left + 4 * CE_THREADS - 1) / (4 * CE_THREADS)) : 0;
+    pdl(ce_row_vec_kernel, rows, CE_THREADS, n_chunks * CE_CHUNK_BYTES, st)(logits, v, target, weight, logp, hits, d16, scale, argmax, status, n_chunks);
+  } else {
     pdl(ce_row_kernel, rows, 1024, 0, st)(logits, v, target, weight, logp, hits, d16, scale, argmax, status);
+  }
   RT_COUNT_LAUNCH(1);
 }
 
