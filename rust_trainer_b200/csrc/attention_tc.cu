@@ -267,8 +267,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     // the last product's phase, and the one before it first: a warp that never rescaled may be here while a
     // slower warp still owes the tile before (its S came after the product two before, no later one), and
     // a parity alone does not tell the last phase from the one two before
-    if (ok && (ntiles < 2 || mbar_wait(pv_done, (uint32_t)ntiles & 1, status, SITE_PVDONE)) &&
-        mbar_wait(pv_done, (uint32_t)(ntiles - 1) & 1, status, SITE_PVDONE)) {
+    ok = ok && (ntiles < 2 || mbar_wait(pv_done, (uint32_t)ntiles & 1, status, SITE_PVDONE)) &&
+         mbar_wait(pv_done, (uint32_t)(ntiles - 1) & 1, status, SITE_PVDONE);
+    if (ok) {
       // O / l as f16 into Q's shared memory (every product that read Q has completed), in the
       // layout of a swizzled TMA box, then one bulk store per 64-column panel: rows past the end of
       // the batch are clipped by the tensor map
@@ -293,12 +294,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       }
       if (i < M) lse[(size_t)h * M + i] = m_used / LOG2E + logf(l_run);
       fence_proxy_async_smem();
-      named_barrier_sync(1, 128);  // the four softmax warps only
-      if (threadIdx.x == 0) {
-        for (int p = 0; p < L::PAN; ++p) tma_store_2d(&tm_o, h * HD + p * 64, m0, sm + L::OFF_Q + p * L::Q_PANEL);
-        bulk_commit_group();
-        bulk_wait_group_read<0>();  // shared memory may go once the store has read it
-      }
+    }
+    __syncwarp();
+    named_barrier_sync(1, 128);  // the four softmax warps only, also after a wait that gave up
+    if (ok && threadIdx.x == 0) {
+      for (int p = 0; p < L::PAN; ++p) tma_store_2d(&tm_o, h * HD + p * 64, m0, sm + L::OFF_Q + p * L::Q_PANEL);
+      bulk_commit_group();
+      bulk_wait_group_read<0>();  // shared memory may go once the store has read it
     }
   }
 
@@ -613,26 +615,36 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[grp]);
     }
-    // group 0 hands out dK, group 1 dV; each of a row's two threads half of its columns
+    // group 0 hands out dK, group 1 dV; each of a row's two threads half of its columns, into shared memory, from
+    // where a row leaves as one bulk copy (a thread per row storing 16 bytes at a time touched 32 sectors per
+    // instruction, 8000 cycles of a CTA's 17000 outside its items: 16 x 512 tokens, 16 heads on 8, 91 -> 77 us, dQ 73 -> 60)
     if (ok) ok = mbar_wait(pd_done, 0, status, SITE_B_PDDONE);
     if (ok) {
       tc_fence_after();
       // a key row only ever meets queries of its own sequence, so its sums are in units of that sequence's largest factor
       const float top_j = tops[min(j, M - 1)];
       const float sc = n_ctas > 1 ? 1.0f : top_j * (grp == 0 ? 1.0f / DS_BOOST : 1.0f / P_BOOST);
-      float* row = n_ctas > 1 ? (float*)sm + (grp * 128 + r) * L::PITCH : (grp == 0 ? dk : dv) + ((size_t)j * nkv + g) * HD;
+      float* row = (float*)sm + (grp * 128 + r) * L::PITCH;
 #pragma unroll
       for (int cc = 0; cc < HD / 64; ++cc) {
         const int c = hf * (HD / 64) + cc;
         uint32_t a[32];
         tmem_ld32(lane_addr + (grp == 0 ? L::COL_DK : L::COL_DV) + c * 32, a);
         tmem_ld_wait();
-        if (n_ctas > 1 || j < M) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            *(float4*)(row + c * 32 + 4 * k) = make_float4(__uint_as_float(a[4 * k]) * sc, __uint_as_float(a[4 * k + 1]) * sc,
-                                                           __uint_as_float(a[4 * k + 2]) * sc, __uint_as_float(a[4 * k + 3]) * sc);
-        }
+        for (int k = 0; k < 8; ++k)
+          *(float4*)(row + c * 32 + 4 * k) = make_float4(__uint_as_float(a[4 * k]) * sc, __uint_as_float(a[4 * k + 1]) * sc,
+                                                         __uint_as_float(a[4 * k + 2]) * sc, __uint_as_float(a[4 * k + 3]) * sc);
+      }
+      fence_proxy_async_smem();
+    }
+    if (n_ctas == 1) {
+      __syncwarp();
+      named_barrier_sync(1 + grp, 256);  // also after a wait that gave up: nobody is left waiting here
+      if (ok && hf == 0 && j < M) {
+        bulk_store_1d((grp == 0 ? dk : dv) + ((size_t)j * nkv + g) * HD, (float*)sm + (grp * 128 + r) * L::PITCH, HD * 4);
+        bulk_commit_group();
+        bulk_wait_group_read<0>();
       }
     }
   }
@@ -694,6 +706,8 @@ struct DqLayout {
   static constexpr uint32_t OFF_BAR = OFF_V + KV_BYTES;
   static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 768;  // slack as in the forward's layout
   static constexpr uint32_t COL_S = 0, COL_DP = BN, COL_DQ = 2 * BN, TMEM_COLS = 256;
+  static constexpr int PITCH = HD + 4;  // dQ as f32 over the operands once those are used up
+  static_assert(BM * PITCH * 4 <= (int)OFF_BAR, "dQ fits over the operands");
 };
 
 constexpr int DQ_THREADS = 320, DQ_TMA_WARP = 8, DQ_MMA_WARP = 9;  // warps 0-7 compute
@@ -879,25 +893,32 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       if (lane == 0) mbar_arrive(ds_full);
     }
     // each of a row's two threads hands out half of its columns
-    if (ok && mbar_wait(dq_done, 0, status, SITE_Q_DQDONE)) {
+    if (ok) ok = mbar_wait(dq_done, 0, status, SITE_Q_DQDONE);
+    if (ok) {
       tc_fence_after();
       // a query row's gradient carries only that row's factor
       const float sc = (i < M ? row_scale[i] : 0.f) * (1.0f / DS_BOOST);
       constexpr int NC = HD / 2;
       const int c0 = hf * NC;
-      float* qrow = dq + ((size_t)i * nh + h) * HD + c0;
+      float* qrow = (float*)sm + r * L::PITCH + c0;  // a row leaves shared memory as one bulk copy, as in dK/dV
 #pragma unroll
       for (int c = 0; c < NC; c += 16) {
         uint32_t a[16];
         tmem_ld16(lane_addr + L::COL_DQ + c0 + c, a);
         tmem_ld_wait();
-        if (i < M) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            *(float4*)(qrow + c + 4 * k) = make_float4(__uint_as_float(a[4 * k]) * sc, __uint_as_float(a[4 * k + 1]) * sc,
-                                                       __uint_as_float(a[4 * k + 2]) * sc, __uint_as_float(a[4 * k + 3]) * sc);
-        }
+        for (int k = 0; k < 4; ++k)
+          *(float4*)(qrow + c + 4 * k) = make_float4(__uint_as_float(a[4 * k]) * sc, __uint_as_float(a[4 * k + 1]) * sc,
+                                                     __uint_as_float(a[4 * k + 2]) * sc, __uint_as_float(a[4 * k + 3]) * sc);
       }
+      fence_proxy_async_smem();
+    }
+    __syncwarp();
+    named_barrier_sync(1 + quarter, 64);  // the row's two warps; also after a wait that gave up
+    if (ok && hf == 0 && i < M) {
+      bulk_store_1d(dq + ((size_t)i * nh + h) * HD, (float*)sm + r * L::PITCH, HD * 4);
+      bulk_commit_group();
+      bulk_wait_group_read<0>();
     }
   }
 

@@ -61,12 +61,6 @@ struct LgArgs {
 constexpr int LG_PITCH = 129;
 static_assert(64 * LG_PITCH * 4 <= (int)(LG_NS * LG_STAGE), "the sums fit over the stages");
 
-__device__ __forceinline__ float ld_cluster_f1(uint32_t cluster_addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
-  return v;
-}
-
 __global__ void __launch_bounds__(LG_THREADS, LG_CTAS_PER_SM)
 lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -184,7 +178,7 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
       float x[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        if (k < n_cta) x[k] = n_cta > 1 ? ld_cluster_f1(mapa_u32(a, (uint32_t)k)) : ((const float*)sm)[i * LG_PITCH + col];
+        if (k < n_cta) x[k] = n_cta > 1 ? ld_cluster_f32(mapa_u32(a, (uint32_t)k)) : ((const float*)sm)[i * LG_PITCH + col];
       float sum = x[0];
 #pragma unroll
       for (int k = 1; k < 8; ++k)
