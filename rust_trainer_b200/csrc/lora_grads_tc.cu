@@ -3,25 +3,28 @@
 //
 //   dB[n, i] = sum_m dY[m, n] * Hs[m, i]      dA[i, k] = sum_m Gs[m, i] * X[m, k]
 //
-// Both are  part[split][i, c] = sum_{m in split} Small[m, i] * Big[m, c]  with Big = dY or X
-// ([M x C], read ONCE: the kernel is a stream over Big) and Small = Hs or Gs ([M x 64]).  One CTA
-// takes 128 columns of Big and a FIXED range of tokens; the tokens are the MMA's K dimension, so
-// both operands are read MN-major straight from their row-major tiles:
+// Both are sums over tokens of Small[m, i] * Big[m, c] with Big = dY or X ([M x C], read ONCE: the
+// kernel is a stream over Big) and Small = Hs or Gs ([M x 64]).  One CTA takes 128 columns of Big and a
+// range of tokens; the tokens are the MMA's K dimension, so both operands are read MN-major straight from
+// their row-major tiles:
 //   A = Big tile   [64 tokens][128 columns]  (two swizzled panels of 64 columns, TMA)
-//   B = Small tile [64 tokens][64]           (TMA, then scaled in place, see below)
-//   D[column (lane), i] in 64 TMEM columns.
+//   B = Small tile [64 tokens][64]           (TMA)
+//   D[column (lane), i] in 64 TMEM columns, two of them in turn.
 // Warps: 0-3 the epilogue, 4 the TMA producer, 5 issues the MMAs.
+// The range is a row of splits of at most 1024 tokens (the tensor core's accumulator error grows with a
+// chain's length); a split's sums are drained into registers under the next split's products.
 // dY arrives row-normalised with one factor per token.  The factors go onto the Small rows
 // relative to the split's largest factor (rounded up to a power of two, so what a row rounds to
 // does not depend on its split mates), and the largest factor multiplies the split's sums.  A launch of its
 // own does that for all the jobs (scaling each tile in place between its landing and its MMAs, in each
 // of the 40-odd column tiles, was the pipeline's longest link: 100 us for the four jobs of a block at 8192
 // tokens, 320 MB to read).
-// Up to eight splits (every batch of up to 8192 tokens) are one cluster: each CTA leaves its split's sums in
-// shared memory, and the CTAs add them in split order straight into the gradient buffers, each its
-// share of the tile.  (A second launch used to do that from partial sums in memory: 2.6 us per linear
-// and 6.1 per group, 0.5 ms of a 1024-token step.)  More splits go through memory and the reduce
-// kernels of lora_kernels.cu.  Deterministic either way, no atomics.
+// A column tile is one cluster of up to eight CTAs: each leaves its sums in shared memory, and the CTAs add
+// them in token order straight into the gradient buffers, each its share of the tile.  Deterministic, no
+// atomics.  As many CTAs per cluster as fit the GPU at once, so that the launch is one wave: with a CTA for
+// every 1024 tokens the clusters of eight (which leave 28 SMs without one) took 3.4 waves, 84 us
+// for the four jobs of a block at 8192 tokens and 19456 columns in all, at 49 % of the DRAM rate; now 71 (floor 48),
+// 45056 columns 200 -> 154 (floor 112).
 #include "ctx.h"
 #include "ops.h"
 #include "pdl.cuh"
@@ -39,25 +42,23 @@ constexpr int LG_NS = 3, LG_THREADS = 192, LG_CTAS_PER_SM = 3;
 constexpr uint32_t LG_Q_BYTES = 2 * 64 * 128, LG_P_BYTES = 64 * 128, LG_STAGE = LG_Q_BYTES + LG_P_BYTES;
 constexpr uint32_t LG_OFF_BAR = LG_NS * LG_STAGE;
 constexpr uint32_t LG_TOTAL = LG_OFF_BAR + 256 + 1024;
-enum { SITE_LG_FREE = 495, SITE_LG_FULL, SITE_LG_DONE };
+enum { SITE_LG_FREE = 495, SITE_LG_FULL, SITE_LG_DONE, SITE_LG_DRAINED };
 
 struct LgMaps {
   CUtensorMap pb, qb, pa, qa;
 };
 struct LgJob {
-  const float* top;     // [splits] largest factor, or null: the rows carry none
+  const float* top;  // [splits] largest factor, or null: the rows carry none
   int N, K, r;
-  int first, nbB;       // the job's first column tile in the grid, and how many of its tiles are dB's
-  float *partB, *partA; // [splits][r x N], [splits][r x K]
-  LoraGroupTable t;     // of one linear (offsets 0) or of a stacked group
+  int first, nbB;    // the job's first column tile in the grid, and how many of its tiles are dB's
+  LoraGroupTable t;  // of one linear (offsets 0) or of a stacked group
 };
 struct LgArgs {
   LgMaps maps[LORA_GRAD_JOBS];
   LgJob job[LORA_GRAD_JOBS];
-  int n_jobs, M, tps;
-  int direct;  // the splits are one cluster: add into the members' gradients
+  int n_jobs, M, tps, per_cta;  // tokens per split, splits per CTA
 };
-// sums of a split, [rank index][128 columns + 1] f32, over the operand stages once those are used up
+// sums of a CTA, [rank index][128 columns + 1] f32, over the operand stages once those are used up
 constexpr int LG_PITCH = 129;
 static_assert(64 * LG_PITCH * 4 <= (int)(LG_NS * LG_STAGE), "the sums fit over the stages");
 
@@ -69,8 +70,9 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   uint64_t* bars = (uint64_t*)(sm + LG_OFF_BAR);
   uint64_t* full = bars;           // [NS] TMA landed
   uint64_t* empty = bars + LG_NS;  // [NS] MMAs retired
-  uint64_t* done = bars + 2 * LG_NS;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * LG_NS + 2);
+  uint64_t* done = bars + 2 * LG_NS;         // [2] a split's products have completed
+  uint64_t* drained = bars + 2 * LG_NS + 2;  // [2] ... and been read
+  uint32_t* tmem_slot = (uint32_t*)(bars + 2 * LG_NS + 4);
   pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   int jx = 0;
@@ -83,21 +85,24 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   const CUtensorMap* tm_q = isB ? &maps.qb : &maps.qa;
   const int C = isB ? g.N : g.K;
   const int j0 = (isB ? bx : bx - g.nbB) * 128;
-  const int m_begin = blockIdx.y * ga.tps, m_end = min(ga.M, m_begin + ga.tps);
-  const int nchunks = (m_end - m_begin + 63) / 64;
+  const int m_begin = blockIdx.y * ga.per_cta * ga.tps, m_end = min(ga.M, m_begin + ga.per_cta * ga.tps);
+  const int nchunks = (m_end - m_begin + 63) / 64, split_chunks = ga.tps / 64, n_splits = (nchunks + split_chunks - 1) / split_chunks;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < LG_NS; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
-    mbar_init(done, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&done[i], 1);
+      mbar_init(&drained[i], 4);
+    }
     mbar_fence_init();
     prefetch_tmap(tm_p);
     prefetch_tmap(tm_q);
   }
   if (warp == 5) {
-    tmem_alloc(tmem_slot, 64);
+    tmem_alloc(tmem_slot, 128);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -127,41 +132,55 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
       const uint64_t a0 = umma_desc_sw128(smem_u32(sm), 8192, 1024), b0 = umma_desc_sw128(smem_u32(sm) + LG_Q_BYTES, 8192, 1024);
       int s = 0;
       uint32_t ph = 0;
-      bool ok = true;
+      int in_split = 0, sp = 0;
       for (int ch = 0; ch < nchunks; ++ch) {
-        if (!mbar_wait(&full[s], ph, status, SITE_LG_FULL)) { ok = false; break; }
+        if (in_split == 0 && sp >= 2 && !mbar_wait(&drained[sp & 1], ((uint32_t)(sp >> 1) & 1) ^ 1, status, SITE_LG_DRAINED)) break;
+        if (!mbar_wait(&full[s], ph, status, SITE_LG_FULL)) break;
         tc_fence_after();
         const uint32_t off = (uint32_t)s * (LG_STAGE >> 4);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_f16_split<false>(tmem_base, (uint32_t)a0 + off + kk * (2048 >> 4), (uint32_t)(a0 >> 32), (uint32_t)b0 + off + kk * (2048 >> 4),
-                                (uint32_t)(b0 >> 32), idesc, (uint32_t)((ch | kk) != 0));
+          umma_f16_split<false>(tmem_base + (sp & 1) * 64, (uint32_t)a0 + off + kk * (2048 >> 4), (uint32_t)(a0 >> 32), (uint32_t)b0 + off + kk * (2048 >> 4),
+                                (uint32_t)(b0 >> 32), idesc, (uint32_t)((in_split | kk) != 0));
         umma_commit(&empty[s]);
         if (++s == LG_NS) { s = 0; ph ^= 1; }
+        if (++in_split == split_chunks || ch + 1 == nchunks) {
+          umma_commit(&done[sp & 1]);
+          in_split = 0;
+          ++sp;
+        }
       }
-      if (ok) umma_commit(done);
     }
   } else {
-    // ---- 128 threads: the epilogue
-    const float out_mul = g.top ? g.top[blockIdx.y] : 1.0f;  // what the split's sums are multiplied by
-    if (mbar_wait(done, 0, status, SITE_LG_DONE)) {
+    // ---- 128 threads: a column each, its sums over the CTA's splits in registers
+    const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+    float acc[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+    bool ok = true;
+    for (int sp = 0; sp < n_splits && ok; ++sp) {
+      const float mul = g.top ? g.top[blockIdx.y * ga.per_cta + sp] : 1.0f;  // what the split's sums are multiplied by
+      ok = mbar_wait(&done[sp & 1], (uint32_t)(sp >> 1) & 1, status, SITE_LG_DONE);
+      if (!ok) break;
       tc_fence_after();
-      uint32_t v[64];
-      tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
-      if (g.r > 32) tmem_ld32(tmem_base + ((uint32_t)(warp * 32) << 16) + 32, v + 32);
-      tmem_ld_wait();
-      const int j = j0 + warp * 32 + lane;
-      if (ga.direct) {
-        float* mine = (float*)sm + warp * 32 + lane;
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (i < g.r) mine[i * LG_PITCH] = __uint_as_float(v[i]) * out_mul;
-      } else if (j < C) {
-        float* dst = (isB ? g.partB : g.partA) + (size_t)blockIdx.y * g.r * C + j;
+      for (int q = 0; q < 4; ++q) {
+        if (q * 16 >= g.r) break;
+        uint32_t v[16];
+        tmem_ld16(lane_addr + (sp & 1) * 64 + q * 16, v);
+        tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-          if (i < g.r) dst[(size_t)i * C] = __uint_as_float(v[i]) * out_mul;
+        for (int i = 0; i < 16; ++i) acc[q * 16 + i] += __uint_as_float(v[i]) * mul;
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&drained[sp & 1]);
+    }
+    if (ok) {  // every product has completed: the stages are free
+      float* mine = (float*)sm + warp * 32 + lane;
+#pragma unroll
+      for (int i = 0; i < 64; ++i)
+        if (i < g.r) mine[i * LG_PITCH] = acc[i];
     }
   }
   if (*(volatile int*)status != 0) {
@@ -169,11 +188,11 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   }
   tc_fence_before();
   __syncwarp();
-  if (ga.direct && gridDim.y > 1) cluster_sync_all();  // every split's sums are in its CTA's shared memory
+  if (gridDim.y > 1) cluster_sync_all();  // every CTA's sums are in its shared memory
   else __syncthreads();
-  if (ga.direct && *(volatile int*)status == 0) {
+  if (*(volatile int*)status == 0) {
     const int n_cta = (int)gridDim.y, ncol = min(128, C - j0);
-    auto add_splits = [&](int i, int col, float* dst) {
+    auto add_parts = [&](int i, int col, float* dst) {
       const uint32_t a = smem_u32(sm) + (uint32_t)(i * LG_PITCH + col) * 4u;
       float x[8];
 #pragma unroll
@@ -191,16 +210,16 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
       if (isB && (j0 < mb.row_off || j0 >= mb.row_off + mb.rows)) continue;
       const int items = ncol * mb.r, per = (items + n_cta - 1) / n_cta, end = min(items, ((int)blockIdx.y + 1) * per);
       for (int e = (int)blockIdx.y * per + threadIdx.x; e < end; e += LG_THREADS) {
-        if (isB) add_splits(mb.rank_off + e % mb.r, e / mb.r, mb.gb + (size_t)(j0 - mb.row_off) * mb.r + e);
-        else add_splits(mb.rank_off + e / ncol, e % ncol, mb.ga + (size_t)(e / ncol) * g.K + j0 + e % ncol);
+        if (isB) add_parts(mb.rank_off + e % mb.r, e / mb.r, mb.gb + (size_t)(j0 - mb.row_off) * mb.r + e);
+        else add_parts(mb.rank_off + e / ncol, e % ncol, mb.ga + (size_t)(e / ncol) * g.K + j0 + e % ncol);
       }
     }
   }
   __syncwarp();
-  if (ga.direct && gridDim.y > 1) cluster_sync_all();  // nobody leaves while its shared memory may still be read
+  if (gridDim.y > 1) cluster_sync_all();  // nobody leaves while its shared memory may still be read
   if (warp == 5) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 64);
+    tmem_dealloc(tmem_base, 128);
   }
 }
 
@@ -265,38 +284,31 @@ __global__ void __launch_bounds__(256) lora_scale_small_kernel(const LgScaleArgs
 
 }  // namespace
 
-// Tokens per split: at most 1024 (the tensor core's accumulator error grows with a chain's length), fewer
-// while the column tiles alone leave places on the GPU, a multiple of 64.
-static int lora_grads_tokens_per_split(int M, int tiles, int num_sms) {
-  const int want = std::max((M + 1023) / 1024, std::min(8, LG_CTAS_PER_SM * num_sms / std::max(1, tiles)));
-  return ((M + want - 1) / want + 63) / 64 * 64;
-}
 struct LgPlan {
-  int tiles, tps, splits;
-  bool direct;  // the splits fit one cluster (of the portable size), which then adds them itself
+  int tps, splits, per_cta, n_ctas;  // tokens per split, splits, splits per CTA, CTAs per column tile
 };
 static LgPlan lora_grads_plan(const LoraGradJob* jobs, int n, int M, int num_sms) {
+  int tiles = 0;
+  for (int j = 0; j < n; ++j) tiles += (jobs[j].N + 127) / 128 + (jobs[j].K + 127) / 128;
   LgPlan p;
-  p.tiles = 0;
-  for (int j = 0; j < n; ++j) p.tiles += (jobs[j].N + 127) / 128 + (jobs[j].K + 127) / 128;
-  p.tps = lora_grads_tokens_per_split(M, p.tiles, num_sms);
+  // a power of two up to the portable cluster size, while all of the launch's CTAs fit the GPU at once and have 64 tokens
+  p.n_ctas = 1;
+  while (p.n_ctas < 8 && tiles * p.n_ctas * 2 <= LG_CTAS_PER_SM * num_sms && p.n_ctas * 64 < M) p.n_ctas *= 2;
+  const int per = (M + p.n_ctas - 1) / p.n_ctas;  // tokens of a CTA
+  p.per_cta = (per + 1023) / 1024;
+  p.tps = ((per + p.per_cta - 1) / p.per_cta + 63) / 64 * 64;
   p.splits = (M + p.tps - 1) / p.tps;
-  p.direct = p.splits <= 8;
+  p.n_ctas = (p.splits + p.per_cta - 1) / p.per_cta;
   return p;
 }
 bool lora_grads_tc_takes(const LoraGradJob& j) {
   return j.r > 0 && j.r <= 64 && j.N % 8 == 0 && j.K % 8 == 0 && j.ld_dy % 8 == 0 && j.t.n >= 1 && j.t.n <= 3 &&
          (((uintptr_t)j.hs | (uintptr_t)j.dy | (uintptr_t)j.gs | (uintptr_t)j.x) & 15) == 0;
 }
-// per job: the scaled Hs and Gs, the splits' largest factors, and the partial sums if they go through memory
+// per job: the scaled Hs and Gs, and the splits' largest factors
 size_t lora_grads_tc_workspace_floats(rt_ctx* c, const LoraGradJob* jobs, int n, int M) {
   const LgPlan p = lora_grads_plan(jobs, n, M, c->num_sms);
-  size_t f = 0;
-  for (int j = 0; j < n; ++j) {
-    f += (size_t)M * 64 + ((size_t)p.splits + 63) / 64 * 64;
-    if (!p.direct) f += (size_t)p.splits * jobs[j].r * ((size_t)jobs[j].N + (size_t)jobs[j].K);
-  }
-  return f;
+  return (size_t)n * ((size_t)M * 64 + ((size_t)p.splits + 63) / 64 * 64);
 }
 
 // One launch for all the jobs (a block's linears): a launch per linear left half of the GPU idle at 1024
@@ -315,7 +327,7 @@ int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float
   const LgPlan plan = lora_grads_plan(jobs, n, M, c->num_sms);
   const int splits = plan.splits;
   g.tps = plan.tps;
-  g.direct = plan.direct ? 1 : 0;
+  g.per_cta = plan.per_cta;
   LgScaleArgs sa;
   sa.M = M;
   sa.tps = g.tps;
@@ -344,9 +356,6 @@ int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float
     t.first = tiles;
     t.nbB = (q.N + 127) / 128;
     t.t = q.t;
-    t.partB = ws;
-    t.partA = ws + (size_t)splits * q.r * q.N;
-    if (!g.direct) ws = t.partA + (size_t)splits * q.r * q.K;
     tiles += t.nbB + (q.K + 127) / 128;
   }
   if (n_scaled > 0) {
@@ -359,18 +368,16 @@ int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float
   at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = 1;
-  at[1].val.clusterDim.y = (unsigned)splits;
+  at[1].val.clusterDim.y = (unsigned)plan.n_ctas;
   at[1].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)tiles, (unsigned)splits);
+  cfg.gridDim = dim3((unsigned)tiles, (unsigned)plan.n_ctas);
   cfg.blockDim = dim3(LG_THREADS);
   cfg.dynamicSmemBytes = LG_TOTAL;
   cfg.stream = c->stream;
   cfg.attrs = at;
-  cfg.numAttrs = g.direct && splits > 1 ? 2 : 1;
+  cfg.numAttrs = plan.n_ctas > 1 ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, lora_grads_tc_kernel, g, c->status_dev) != cudaSuccess) return 3;
   RT_COUNT_LAUNCH(1);
-  if (!g.direct)
-    for (int j = 0; j < n; ++j) launch_lora_grads_group_reduce(g.job[j].partB, g.job[j].partA, splits, jobs[j].N, jobs[j].K, jobs[j].r, jobs[j].t, c->stream);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -89,9 +89,6 @@ bool lora_grads_tc_takes(const LoraGradJob& j);
 size_t lora_grads_tc_workspace_floats(rt_ctx* c, const LoraGradJob* jobs, int n, int M);
 // adds dB and dA of the jobs into the gradients of their tables' members; 0 or 3 (launch failure)
 int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float* workspace);
-// adds partial sums [splits][r x N] and [splits][r x K] into the table's members, splits in order
-void launch_lora_grads_group_reduce(const float* partB, const float* partA, int splits, int N, int K, int r, const LoraGroupTable& t,
-                                    cudaStream_t st);
 
 // ---- attention_tc.cu: causal GQA attention over a concatenation of independent sequences, on
 // tcgen05 / TMEM / TMA (waits report through the ctx status word).
