@@ -34,6 +34,15 @@ enum QKind : int {
   QK_NARROW = 2,  // one CTA per tile of 128 weight rows x up to 64 tokens
   QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
 };
+// How the results leave: a kernel holds the code of one way only (all of them in one kernel cost the small
+// launches 0.4 us each in instruction fetches and the f16 epilogue of a pair registers, 5 % of the
+// 6144x1024 product at 8192 tokens).
+enum QOut : int {
+  QO_TMA16 = 0,   // 16-bit, staged in shared memory and stored by TMA
+  QO_DIRECT = 1,  // from registers: f32, partial sums, 16-bit that TMA cannot address
+  QO_RES = 2,     // f32 with a residual that comes by asynchronous copies (CTA pairs only: in the few blocks of a
+                  // smaller tile the pipeline gains nothing)
+};
 // Weight formats as the kernel sees them: ggml's ids for packed weights, and two 16-bit cases.
 constexpr int QF_16 = 0;       // 16-bit weights of the activations' type, straight from TMA
 constexpr int QF_16CONV = 1;   // 16-bit weights of the other 16-bit type, converted in place
@@ -106,7 +115,6 @@ struct KParams {
   uint32_t idesc;
   int* status;
   int late_wait;  // see QGemmArgs
-  int tma_out;  // 16-bit output that TMA can address: staged in shared memory and stored by TMA
 };
 
 // ------------------------------------------------------------------ unpackers
@@ -234,7 +242,7 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
 //   bytes that TMA writes and the tensor core reads.  Barriers that gate the MMA (full, acc_empty)
 //   live in the leader and are arrived on from both CTAs; barriers the MMA releases (stage_empty,
 //   acc_full) exist in both CTAs and are signalled by one multicast commit.
-template <int KIND, int FMT>
+template <int KIND, int FMT, int OUT>
 __global__ void __launch_bounds__((QCfg<KIND, FMT>::THREADS), 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w16,
              const __grid_constant__ CUtensorMap tm_lact, const __grid_constant__ CUtensorMap tm_lw,
@@ -321,7 +329,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     prefetch_tmap(&tm_act);
     if (IS16) prefetch_tmap(&tm_w16);
     if (p.lora_mmas > 0) { prefetch_tmap(&tm_lact); prefetch_tmap(&tm_lw); }
-    if (p.tma_out) prefetch_tmap(&tm_out);
+    if (OUT == QO_TMA16) prefetch_tmap(&tm_out);
   }
   if (warp == 1) {
     if (PAIR) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
@@ -426,8 +434,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     const size_t ld = fin_out ? (size_t)p.ld_out : (size_t)p.out_rows;
     const size_t base = fin_out ? (size_t)tok0 * ld + row : ((size_t)split * p.M + tok0) * ld + row;
     float* o = (fin_out ? (float*)p.out : p.part) + base;
-    if (nvalid == 32 && (!fin_out || p.out_dtype == OUT_F32)) {
-      if (fin_out && p.residual) {
+    if (nvalid == 32 && (!fin_out || (p.out_dtype == OUT_F32 && (!PAIR || !p.residual)))) {
+      if (!PAIR && fin_out && p.residual) {
         const float* res = p.residual + base;
 #pragma unroll
         for (int q = 0; q < 32; q += 8) {  // eight loads in flight: what the registers have room for
@@ -446,7 +454,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       }
       return;
     }
-    if (!fin_out || p.out_dtype == OUT_F32) {  // the ragged last block of a batch
+    if (!fin_out || p.out_dtype == OUT_F32) {  // the ragged last block of a batch, a residual of odd pitch
       const bool add = fin_out && p.accumulate;
       const float* res = fin_out && p.residual ? p.residual + base : nullptr;
 #pragma unroll
@@ -469,6 +477,63 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         else o16[(size_t)j * ld] = __float2half_rn(val);
       }
   };
+  // A tile's f32 result with a residual added: the residual's blocks come as asynchronous copies of [16 tokens x
+  // 32 features] into the warp's three staging buffers, three ahead of their use.  (Loaded by the thread
+  // that adds, eight values at a time, their latency made the epilogue longer than the next tile's contraction:
+  // 1024x2048 at 8192 tokens 55.6 us against 32.8 without a residual, 37.3 so.)
+  auto res_issue = [&](int k, int wq, int turn, int turns, int r0, int m0, uint32_t stage) {  // the k-th half block of this warp
+    const int c = turn + (k >> 1) * turns, col = r0 + wq * 32 + (lane & 7) * 4;
+    if (c < p.TN / 32 && col < p.out_rows) {
+      const int tok = m0 + c * 32 + (k & 1) * 16 + (lane >> 3);
+      const float* src = p.residual + (size_t)tok * p.ld_out + col;
+      const uint32_t dst = stage + (uint32_t)(k % 3) * 2048u + (uint32_t)lane * 16u;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (tok + i * 4 < p.M) cp_async_16(dst + i * 512, src + (size_t)(i * 4) * p.ld_out);
+    }
+    cp_async_commit();
+  };
+  auto residual_start = [&](int wq, int turn, int turns, int r0, int m0, uint32_t stage) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) res_issue(k, wq, turn, turns, r0, m0, stage);
+  };
+  auto residual_tile = [&](int acc, int wq, int turn, int turns, int r0, int m0, uint32_t stage) {
+    const int row = r0 + wq * 32 + lane;
+    const bool row_ok = row < p.out_rows;
+    const float bias_v = (p.bias != nullptr && row_ok) ? p.bias[row] : 0.f;
+    int k = 0;
+    for (int c = turn; c < p.TN / 32; c += turns) {
+      const int tok0 = m0 + c * 32, nvalid = min(32, p.M - tok0);
+      uint32_t v[32];
+      tmem_ld32(tmem_base + acc * 256 + ((uint32_t)(wq * 32) << 16) + c * 32, v);
+      const float rs_lane = p.row_scale && lane < nvalid ? p.row_scale[tok0 + lane] : 1.f;
+      tmem_ld_wait();
+      if (p.row_scale) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * __shfl_sync(0xffffffffu, rs_lane, j));
+      }
+      float* o = (float*)p.out + (size_t)tok0 * p.ld_out + row;
+#pragma unroll
+      for (int h = 0; h < 2; ++h, ++k) {
+        cp_async_wait<2>();
+        __syncwarp();
+        const uint32_t buf = stage + (uint32_t)(k % 3) * 2048u + (uint32_t)lane * 4u;
+#pragma unroll
+        for (int q = 0; q < 16; q += 8) {
+          float old[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) old[j] = ld_shared_f32(buf + (q + j) * 128);
+          if (!row_ok) continue;
+#pragma unroll
+          for (int j = 0; j < 8; ++j, o += p.ld_out)
+            if (nvalid == 32 || h * 16 + q + j < nvalid) *o = __uint_as_float(v[h * 16 + q + j]) + bias_v + old[j];
+        }
+        __syncwarp();
+        res_issue(k + 3, wq, turn, turns, r0, m0, stage);
+      }
+    }
+    cp_async_wait<0>();
+  };
   // The epilogue of a CTA's LAST tile has nothing to hide behind, so the warps whose own work
   // is over by then help: every warp with residue q (mod 4) may read TMEM lane quarter q.
   // Quarter q's blocks go round-robin over its epilogue warp (turn 0) and its helpers (turns
@@ -488,8 +553,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     if (!mbar_wait(last_full, 0, p.status, 402)) return;
     tc_fence_after();
     uint32_t cnt = 0;
+    if (OUT == QO_RES) {
+      const uint32_t stage = smem_u32(smem + hslot * 8192);
+      residual_start(q_res, turn, q_turns, r0, m0, stage);
+      residual_tile(acc, q_res, turn, q_turns, r0, m0, stage);
+      return;
+    }
     for (int c = turn; c < p.TN / 32; c += q_turns) {
-      if (p.tma_out) tma_chunk(acc, q_res, c, r0, m0, smem + hslot * 8192, cnt);
+      if (OUT == QO_TMA16) tma_chunk(acc, q_res, c, r0, m0, smem + hslot * 8192, cnt);
       else direct_chunk(acc, q_res, c, r0, m0, split);
     }
     if (lane == 0) bulk_wait_group_read<0>();  // staging may go once read; the writes land by the end of the grid
@@ -749,11 +820,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       QG_TILE_ORIGIN();
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
+      const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
+      const bool mine = wq * 32 < C::ROWS;
+      const uint32_t stage = smem_u32(sOut + wq * C::OUT_WARP);
+      if (OUT == QO_RES && mine) residual_start(wq, 0, stride, r0, m0, stage);
       if (!mbar_wait(&acc_full[acc], aph, p.status, 401)) break;
       tc_fence_after();
-      const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
-      for (int c = wq * 32 < C::ROWS ? 0 : p.TN; c < p.TN / 32; c += stride) {
-        if (p.tma_out) tma_chunk(acc, wq, c, r0, m0, sOut + wq * C::OUT_WARP, out_chunk);
+      if (OUT == QO_RES) {
+        if (mine) residual_tile(acc, wq, 0, stride, r0, m0, stage);
+      } else for (int c = mine ? 0 : p.TN; c < p.TN / 32; c += stride) {
+        if (OUT == QO_TMA16) tma_chunk(acc, wq, c, r0, m0, sOut + wq * C::OUT_WARP, out_chunk);
         else direct_chunk(acc, wq, c, r0, m0, split);
       }
       // the accumulator buffer is free once every epilogue warp of every CTA has read its lanes
@@ -817,39 +893,35 @@ struct QKernel {
   const void* fn;
   int threads, smem;
 };
-template <int KIND, int FMT>
+template <int KIND, int FMT, int OUT>
 static QKernel qkernel() {
-  return {(const void*)qgemm_kernel<KIND, FMT>, QCfg<KIND, FMT>::THREADS, QCfg<KIND, FMT>::SMEM_BYTES};
+  return {(const void*)qgemm_kernel<KIND, FMT, OUT>, QCfg<KIND, FMT>::THREADS, QCfg<KIND, FMT>::SMEM_BYTES};
 }
 // fmt: a packed ggml format, QF_16 or QF_16CONV.  The wide single-CTA kernel only serves converted
 // 16-bit weights: the others' wide tiles run as pairs.
-static QKernel qkernel_for(int kind, int fmt) {
-  if (kind == QK_PAIR) switch (fmt) {
-      case QF_16: return qkernel<QK_PAIR, QF_16>();
-      case GGML_Q4_0: return qkernel<QK_PAIR, GGML_Q4_0>();
-      case GGML_Q8_0: return qkernel<QK_PAIR, GGML_Q8_0>();
-      case GGML_Q4_K: return qkernel<QK_PAIR, GGML_Q4_K>();
-      case GGML_Q6_K: return qkernel<QK_PAIR, GGML_Q6_K>();
+template <int KIND, int OUT>
+static QKernel qkernel_fmt(int fmt) {
+  constexpr bool WIDE = KIND == QK_WIDE, PAIR = KIND == QK_PAIR;
+  if constexpr (!PAIR) {
+    if (fmt == QF_16CONV) return qkernel<KIND, QF_16CONV, OUT>();
+  }
+  if constexpr (!WIDE) switch (fmt) {
+      case QF_16: return qkernel<KIND, QF_16, OUT>();
+      case GGML_Q4_0: return qkernel<KIND, GGML_Q4_0, OUT>();
+      case GGML_Q8_0: return qkernel<KIND, GGML_Q8_0, OUT>();
+      case GGML_Q4_K: return qkernel<KIND, GGML_Q4_K, OUT>();
+      case GGML_Q6_K: return qkernel<KIND, GGML_Q6_K, OUT>();
     }
-  if (kind == QK_NARROW) switch (fmt) {
-      case QF_16: return qkernel<QK_NARROW, QF_16>();
-      case QF_16CONV: return qkernel<QK_NARROW, QF_16CONV>();
-      case GGML_Q4_0: return qkernel<QK_NARROW, GGML_Q4_0>();
-      case GGML_Q8_0: return qkernel<QK_NARROW, GGML_Q8_0>();
-      case GGML_Q4_K: return qkernel<QK_NARROW, GGML_Q4_K>();
-      case GGML_Q6_K: return qkernel<QK_NARROW, GGML_Q6_K>();
-    }
-  if (kind == QK_HALF) switch (fmt) {
-      case QF_16: return qkernel<QK_HALF, QF_16>();
-      case QF_16CONV: return qkernel<QK_HALF, QF_16CONV>();
-      case GGML_Q4_0: return qkernel<QK_HALF, GGML_Q4_0>();
-      case GGML_Q8_0: return qkernel<QK_HALF, GGML_Q8_0>();
-      case GGML_Q4_K: return qkernel<QK_HALF, GGML_Q4_K>();
-      case GGML_Q6_K: return qkernel<QK_HALF, GGML_Q6_K>();
-    }
-  if (kind == QK_WIDE) switch (fmt) {
-      case QF_16CONV: return qkernel<QK_WIDE, QF_16CONV>();
-    }
+  return {nullptr, 0, 0};
+}
+static QKernel qkernel_for(int kind, int fmt, int out) {
+  const bool t = out == QO_TMA16;
+  switch (kind) {
+    case QK_PAIR: return t ? qkernel_fmt<QK_PAIR, QO_TMA16>(fmt) : out == QO_RES ? qkernel_fmt<QK_PAIR, QO_RES>(fmt) : qkernel_fmt<QK_PAIR, QO_DIRECT>(fmt);
+    case QK_WIDE: return t ? qkernel_fmt<QK_WIDE, QO_TMA16>(fmt) : qkernel_fmt<QK_WIDE, QO_DIRECT>(fmt);
+    case QK_NARROW: return t ? qkernel_fmt<QK_NARROW, QO_TMA16>(fmt) : qkernel_fmt<QK_NARROW, QO_DIRECT>(fmt);
+    case QK_HALF: return t ? qkernel_fmt<QK_HALF, QO_TMA16>(fmt) : qkernel_fmt<QK_HALF, QO_DIRECT>(fmt);
+  }
   return {nullptr, 0, 0};
 }
 
@@ -865,15 +937,16 @@ int qgemm_init() {
     g_encode = (PFN_encodeTiled)fn;
   }
   for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF})
-    for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K}) {
-      const QKernel k = qkernel_for(kind, fmt);
+    for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K})
+    for (int out : {(int)QO_TMA16, (int)QO_DIRECT, (int)QO_RES}) {
+      const QKernel k = qkernel_for(kind, fmt, out);
       if (k.fn && cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem) != cudaSuccess) return RT_ERR_CUDA;
     }
   if (g_pair_workers < 0) {
     int dev = 0, sms = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const QKernel k = qkernel_for(QK_PAIR, GGML_Q8_0);  // one CTA per SM in every format
+    const QKernel k = qkernel_for(QK_PAIR, GGML_Q8_0, QO_TMA16);  // one CTA per SM in every format
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1100,13 +1173,14 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
       if (!p.part) return RT_ERR_CUDA;
     }
   }
+  int out_kind = QO_DIRECT;
+  if (pair && !p.part && a.residual && (uintptr_t)a.residual % 16 == 0 && p.ld_out % 4 == 0 && out_rows % 4 == 0) out_kind = QO_RES;
   // 16-bit outputs leave through TMA whenever it can address them (16-byte aligned base and row pitch)
   CUtensorMap tm_out = tm_act;
-  p.tma_out = 0;
   if (!p.part && a.out_dtype != OUT_F32 && (uintptr_t)a.out % 16 == 0 && (uint64_t)p.ld_out % 8 == 0) {
     rc = make_out_map(a.fixed_part ? nullptr : ctx, &tm_out, a.out, (uint64_t)a.M, (uint64_t)out_rows, (uint64_t)p.ld_out, a.out_dtype);
     if (rc) return rc;
-    p.tma_out = 1;
+    out_kind = QO_TMA16;
   }
   const int n_items = p.n_row_tiles * p.n_tok_tiles * p.n_splits;
   const int workers = pair ? g_pair_workers : num_sms;
@@ -1125,7 +1199,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     cudaEventRecord(e0, st);
   }
   {
-    const QKernel k = qkernel_for(plan.kind, kfmt);
+    const QKernel k = qkernel_for(plan.kind, kfmt, out_kind);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
