@@ -310,6 +310,12 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
                "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+               "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+               "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+               : "memory");
+}
 // 16 lanes x 32 consecutive fp32 columns in the accumulator-fragment layout of mma (16 registers):
 // thread i holds, for column block k = 0..3, lane base + i/4 at columns 8k + 2(i%4), +1 in
 // v[4k], v[4k+1] and lane base + i/4 + 8 at the same columns in v[4k+2], v[4k+3].

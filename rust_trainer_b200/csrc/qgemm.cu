@@ -33,6 +33,12 @@ enum QKind : int {
   QK_WIDE = 1,    // one CTA per tile of 128 weight rows x up to 256 tokens (16-bit weights only)
   QK_NARROW = 2,  // one CTA per tile of 128 weight rows x up to 64 tokens
   QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
+  // Narrow tiles of packed weights in the forward direction, with the unpacked weights in TMEM: a thread that owns a
+  // weight row is the TMEM lane the MMA reads it from, and the weight tile no longer passes through shared
+  // memory twice.  1024x3072 at 1024 tokens 18.7 -> 16.5 us, at 640 the same.  (Backward reads the
+  // bricks down their columns: only the shared-memory operand can be read transposed.  Half tiles leave half of the
+  // lanes, and so of the unpack warps, without a row: 25 us.)
+  QK_NARROW_T = 4,
 };
 // How the results leave: a kernel holds the code of one way only (all of them in one kernel cost the small
 // launches 0.4 us each in instruction fetches and the f16 epilogue of a pair registers, 5 % of the
@@ -50,7 +56,8 @@ constexpr int QF_16CONV = 1;   // 16-bit weights of the other 16-bit type, conve
 // Shared-memory plan of one CTA.
 template <int KIND, int FMT>
 struct QCfg {
-  static constexpr bool PAIR = KIND == QK_PAIR, HALF = KIND == QK_HALF;
+  static constexpr bool PAIR = KIND == QK_PAIR, HALF = KIND == QK_HALF, NARROW = KIND == QK_NARROW || KIND == QK_NARROW_T;
+  static constexpr bool TM = KIND == QK_NARROW_T;  // unpacked weights in TMEM
   // Weight rows of the CTA's tile.  The MMA always takes 128: a half tile's upper 64 are whatever follows it in
   // shared memory, and their accumulator lanes are not read.
   static constexpr int ROWS = HALF ? 64 : 128, BRICKS = ROWS / 64;
@@ -61,17 +68,21 @@ struct QCfg {
   // in flight per scheduler.  (Eight warps of twice the work each: 8192x3072 Q6_K at 8192 tokens
   // 406 us against 363.)  Without unpacking eight warps stay, to help with the last tile's epilogue.
   static constexpr int NUW = PACKED ? 16 : 8;
-  static constexpr int THREADS = 32 * (7 + NUW);  // + activation / brick producers, MMA, 4 epilogue warps
+  // + activation / brick producers, MMA, 4 epilogue warps, and one idle where four unpack warps of each residue are needed
+  static constexpr int THREADS = 32 * (7 + NUW + (TM ? 1 : 0));
   // 64-element contraction steps per stage.  Two for narrow and half tiles: their MMAs are short, and one
   // hand-off between the roles costs about 500 cycles whatever it hands over.
-  static constexpr int KS = KIND == QK_NARROW || HALF ? 2 : 1;
+  static constexpr int KS = NARROW || HALF ? 2 : 1;
   // Activation / unpacked-weight stages, and packed-brick stages in the room that is left beside them and
   // the epilogue staging.
-  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : HALF ? 4 : PACKED ? 3 : 4;
+  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : HALF || TM ? 4 : PACKED ? 3 : 4;
   static constexpr int RAW_STAGE = PACKED ? KS * BRICKS * fmt_brick_bytes(FMT) : 0;
   static constexpr int ACT_SUB = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
   static constexpr int ACT_STAGE = KS * ACT_SUB;
-  static constexpr int W_BYTES = KS * W_SUB;               // unpacked weights of a stage
+  static constexpr int W_BYTES = (TM ? 1 : KS) * W_SUB;    // weights of a stage (in TMEM: the low-rank step's only)
+  // TMEM columns of a stage's unpacked weights, beside the two accumulators of up to 64 columns at 0 and 256
+  __device__ static constexpr uint32_t a_col(int st) { return 128u + (uint32_t)(st & 1) * 64u + (uint32_t)(st >> 1) * 256u; }
+  static_assert(!TM || (PACKED && NS <= 4), "four stages fit TMEM");
   // Epilogue staging of 16-bit outputs per warp: three blocks of [32 tokens x 32 features], 2 KB each.
   static constexpr int OUT_BUFS = 3, OUT_WARP = OUT_BUFS * 2048;
   static constexpr int SMEM_MAX = 232448, SMEM_REST = 4 * OUT_WARP + 512 + 2 * 1024;  // staging, barriers, alignment
@@ -156,8 +167,13 @@ __device__ __forceinline__ __half2 code_pair(uint32_t w, uint32_t w8, int p, uin
   return __hsub2(u32_as_h2((src & 0x000F000Fu) | 0x64006400u | more), h2c(1024.f + bias));
 }
 
-template <int FMT, bool WBF16>
-__device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_t tile, const UnitDst& ud) {
+// REGS: the unit's sixteen registers are left in `regs` instead of being stored
+template <int FMT, bool WBF16, bool REGS>
+__device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_t tile, const UnitDst& ud, uint32_t* regs) {
+  auto put = [&](int j, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    if (REGS) { regs[4 * j] = a; regs[4 * j + 1] = b; regs[4 * j + 2] = c; regs[4 * j + 3] = d; }
+    else st_shared_v4(tile + ud.off[j], a, b, c, d);
+  };
   if (FMT == GGML_Q4_0) {
     const uint4 q = *(const uint4*)(brick + t * 16);
     const __half2 d2 = __half2half2(((const __half*)(brick + 2048))[t]);
@@ -168,7 +184,7 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
       uint32_t o[4];
 #pragma unroll
       for (int p = 0; p < 4; ++p) o[p] = fin<WBF16>(__hmul2(code_pair(w[j], w8, p, 0u, 8.f), d2));
-      st_shared_v4(tile + ud.off[j], o[0], o[1], o[2], o[3]);
+      put(j, o[0], o[1], o[2], o[3]);
     }
   } else if (FMT == GGML_Q8_0) {
     const uint4 qa = *(const uint4*)(brick + t * 16);
@@ -183,7 +199,7 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
         const uint32_t x = __byte_perm(w[2 * j + (p >> 1)], 0x64646464u, (p & 1) ? 0x4342 : 0x4140);
         o[p] = fin<WBF16>(__hmul2(__hsub2(u32_as_h2(x), h2c(1152.f)), d2));  // 1024 (magic) + 128 (stored offset)
       }
-      st_shared_v4(tile + ud.off[j], o[0], o[1], o[2], o[3]);
+      put(j, o[0], o[1], o[2], o[3]);
     }
   } else if (FMT == GGML_Q4_K) {
     const uint4 q = *(const uint4*)(brick + t * 16);
@@ -206,7 +222,7 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
         const __half2 qv = code_pair(w[j], w8, p, 0u, 0.f);
         o[p] = fin<WBF16>(__hadd2(__hfma2(qv, dsc, ndm), __hfma2(qv, dsc_lo, ndm_lo)));
       }
-      st_shared_v4(tile + ud.off[j], o[0], o[1], o[2], o[3]);
+      put(j, o[0], o[1], o[2], o[3]);
     }
   } else if (FMT == GGML_Q6_K) {
     const uint4 lo = *(const uint4*)(brick + t * 16);
@@ -229,7 +245,7 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
         const uint32_t more = (p < 2 ? h01 : h23) & ((p & 1) ? 0x03000300u : 0x00300030u);
         o[p] = fin<WBF16>(__hmul2(code_pair(w[j], w8, p, more, 32.f), ds));
       }
-      st_shared_v4(tile + ud.off[j], o[0], o[1], o[2], o[3]);
+      put(j, o[0], o[1], o[2], o[3]);
     }
   }
 }
@@ -248,7 +264,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
              const __grid_constant__ CUtensorMap tm_lact, const __grid_constant__ CUtensorMap tm_lw,
              const __grid_constant__ CUtensorMap tm_out, const KParams p) {
   using C = QCfg<KIND, FMT>;
-  constexpr bool PAIR = C::PAIR, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
+  constexpr bool PAIR = C::PAIR, TM = C::TM, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
   constexpr int NS = C::NS, NR = C::NR, UG = C::UG, UTG = C::UTG, KS = C::KS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -276,8 +292,19 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   // residue (a warp reads TMEM lanes 32 * (warp % 4) ..).
   //   warp 1 MMA | 5 activation producer | 9 packed-brick producer | 0, 2, 3, 13 epilogue | rest unpack
   constexpr int R_PROD = 0, R_MMA = 1, R_UNPACK = 2, R_EPI = 3, R_RAW = 4;
+  // A warp writes TMEM lanes by its residue too, so unpacking into TMEM takes four warps of each:
+  //   warp 1 MMA | 23 activation producer | 22 brick producer | 0, 2, 3, 13 epilogue | 20 idle | rest unpack
+  constexpr int R_IDLE = 5;
   int role = R_UNPACK, uidx = 0;  // uidx: position among the unpack warps, neighbours on different schedulers
-  switch (warp) {
+  if (TM) switch (warp) {
+    case 1: role = R_MMA; break;
+    case 23: role = R_PROD; break;
+    case 22: role = R_RAW; break;
+    case 0: case 2: case 3: case 13: role = R_EPI; break;
+    case 20: role = R_IDLE; break;
+    default: uidx = (warp >> 2) - 1 - ((warp & 3) == 1 && warp > 13 ? 1 : 0); break;  // 0..3 within the residue
+  }
+  else switch (warp) {
     case 1: role = R_MMA; break;
     case 5: role = R_PROD; break;
     case 9: role = R_RAW; break;
@@ -619,7 +646,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       }
     }
     __syncwarp();
-    tail_helper(warp >> 2, warp - 4);
+    if (warp < 15) tail_helper(warp >> 2, warp - 4);
   } else if (role == R_MMA) {
     // ------------------------------------------------------------ MMA issue (the leader's thread only)
     if (rank == 0 && elect_one()) {
@@ -665,6 +692,13 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
           for (int u = 0; u < KS; ++u) {
             if (u > 0 && s * KS + u >= s_main) break;
             const uint32_t au = a_lo + u * (C::W_SUB >> 4), bu = b_lo + u * (C::ACT_SUB >> 4);
+            if (TM) {
+              const uint32_t at = tmem_base + C::a_col(st) + u * 32;
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                umma_f16_ta(d_tmem, at + kk * 8, ((uint64_t)b_hi << 32) | (bu + kk * b_k), idesc, (uint32_t)((u | s | kk) != 0));
+              continue;
+            }
             umma_f16_split<PAIR>(d_tmem, au, a_hi, bu, b_hi, idesc, (uint32_t)(u != 0 || s != 0));
             umma_f16_split<PAIR>(d_tmem, au + a_k, a_hi, bu + b_k, b_hi, idesc, 1u);
             umma_f16_split<PAIR>(d_tmem, au + 2 * a_k, a_hi, bu + 2 * b_k, b_hi, idesc, 1u);
@@ -699,7 +733,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     // flight at a time.
     if (PACKED || CONV) {
       const int t = uidx * 32 + lane;
-      const int grp = t / UTG, tg = t % UTG;
+      const int grp = TM ? uidx >> 1 : t / UTG, tg = TM ? 0 : t % UTG;
       const UnitDst ud(tg & 127);
       const uint32_t w_base = smem_u32(sW);
       constexpr int BB = PACKED ? C::RAW_STAGE / (C::BRICKS * KS) : 0;  // bytes of a brick
@@ -736,7 +770,26 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
               }
               fence_proxy_async_smem();
             }
-            if (PACKED && main_step) {
+            if (TM && main_step) {
+              // one of the group's two warps per lane quarter takes each of the stage's two steps; a thread unpacks the
+              // 64 codes of its weight row, which it is the TMEM lane of
+              if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
+              tc_fence_after();
+              const int row = (warp & 3) * 32 + lane, u = uidx & 1;
+              if (u < subs) {
+                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + u * BB + (row >> 6) * (KS * BB);
+                const uint32_t dst = tmem_base + C::a_col(st) + ((uint32_t)((warp & 3) * 32) << 16) + u * 32;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  uint32_t o[16];
+                  if (p.act_f16) unpack_unit<FMT, false, true>(raw, 2 * (row & 63) + h, 0, ud, o);
+                  else unpack_unit<FMT, true, true>(raw, 2 * (row & 63) + h, 0, ud, o);
+                  tmem_st16(dst + h * 16, o);
+                }
+                tmem_st_wait();
+              }
+              tc_fence_before();
+            } else if (PACKED && main_step) {
               if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
               // two bricks per 64-element tile: brick b fills the 8 KB half b.  A stage of two tiles goes to the
               // two halves of the group.
@@ -747,10 +800,10 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
                 const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB;
                 if (p.act_f16) {
 #pragma unroll
-                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, false>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, false, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
                 } else {
 #pragma unroll 1
-                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, true>(raw + b * next, tg & 127, dst + b * 8192, ud);
+                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, true, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
                 }
               }
               fence_proxy_async_smem();
@@ -809,8 +862,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       }
     }
     __syncwarp();
-    tail_helper(warp >> 2, warp - 4);
-  } else {
+    if (warp < 15) tail_helper(warp >> 2, warp - 4);
+  } else if (role == R_EPI) {
     // ------------------------------------------------------------ epilogue
     const int wq = warp & 3;  // TMEM lane quarter this warp may read
     uint32_t tcount = 0, out_chunk = 0;
@@ -901,12 +954,14 @@ static QKernel qkernel() {
 // 16-bit weights: the others' wide tiles run as pairs.
 template <int KIND, int OUT>
 static QKernel qkernel_fmt(int fmt) {
-  constexpr bool WIDE = KIND == QK_WIDE, PAIR = KIND == QK_PAIR;
-  if constexpr (!PAIR) {
+  constexpr bool WIDE = KIND == QK_WIDE, TM = KIND == QK_NARROW_T;
+  if constexpr (KIND != QK_PAIR && !TM) {
     if (fmt == QF_16CONV) return qkernel<KIND, QF_16CONV, OUT>();
   }
+  if constexpr (!WIDE && !TM) {
+    if (fmt == QF_16) return qkernel<KIND, QF_16, OUT>();
+  }
   if constexpr (!WIDE) switch (fmt) {
-      case QF_16: return qkernel<KIND, QF_16, OUT>();
       case GGML_Q4_0: return qkernel<KIND, GGML_Q4_0, OUT>();
       case GGML_Q8_0: return qkernel<KIND, GGML_Q8_0, OUT>();
       case GGML_Q4_K: return qkernel<KIND, GGML_Q4_K, OUT>();
@@ -920,6 +975,7 @@ static QKernel qkernel_for(int kind, int fmt, int out) {
     case QK_PAIR: return t ? qkernel_fmt<QK_PAIR, QO_TMA16>(fmt) : out == QO_RES ? qkernel_fmt<QK_PAIR, QO_RES>(fmt) : qkernel_fmt<QK_PAIR, QO_DIRECT>(fmt);
     case QK_WIDE: return t ? qkernel_fmt<QK_WIDE, QO_TMA16>(fmt) : qkernel_fmt<QK_WIDE, QO_DIRECT>(fmt);
     case QK_NARROW: return t ? qkernel_fmt<QK_NARROW, QO_TMA16>(fmt) : qkernel_fmt<QK_NARROW, QO_DIRECT>(fmt);
+    case QK_NARROW_T: return t ? qkernel_fmt<QK_NARROW_T, QO_TMA16>(fmt) : qkernel_fmt<QK_NARROW_T, QO_DIRECT>(fmt);
     case QK_HALF: return t ? qkernel_fmt<QK_HALF, QO_TMA16>(fmt) : qkernel_fmt<QK_HALF, QO_DIRECT>(fmt);
   }
   return {nullptr, 0, 0};
@@ -936,7 +992,7 @@ int qgemm_init() {
       return RT_ERR_CUDA;
     g_encode = (PFN_encodeTiled)fn;
   }
-  for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF})
+  for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF, (int)QK_NARROW_T})
     for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K})
     for (int out : {(int)QO_TMA16, (int)QO_DIRECT, (int)QO_RES}) {
       const QKernel k = qkernel_for(kind, fmt, out);
@@ -1051,7 +1107,8 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 // (us, 64 contraction elements) are fitted to sweeps over both kernels and all widths (eight weight shapes
 // of 128..151936 rows, 1..8192 tokens): about 0.33 for a pair while the single-thread roles and the unpack
 // passes set the pace, more from about 64 tokens of width per CTA on, when the MMAs do; 0.25 for narrow
-// tiles, which hand over two steps at a time, and 0.17 for half tiles, whose unpack passes are half as long.
+// tiles, which hand over two steps at a time (0.23 from TMEM, but a fit that says so puts pairs
+// out of work that do it faster), and 0.17 for half tiles, whose unpack passes are half as long.
 // Narrow and half tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
 // backward at 1024 tokens 29 us (44 on pairs of 128 tokens before), 8192x3072 Q6_K backward at 24 tokens 30 us
 // (43 on narrow tiles, 91 before), 1024x2048 at 157 tokens 9.6 us (12).
@@ -1059,7 +1116,7 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 struct QPlan {
   int kind, TN;
 };
-static QPlan qgemm_plan(int kfmt, int M, int out_rows, int n_splits, int steps, int num_sms) {
+static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, int steps, int num_sms) {
   QPlan best = {QK_NARROW, 64};
   double best_cost = -1;
   auto consider = [&](int kind, int tn, double step_us) {
@@ -1069,8 +1126,10 @@ static QPlan qgemm_plan(int kfmt, int M, int out_rows, int n_splits, int steps, 
     const double cost = (double)((tiles + workers - 1) / workers) * (steps * step_us + 0.5);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {kind, tn}; }
   };
-  if (M > 32) consider(QK_NARROW, 64, 0.25);
-  consider(QK_NARROW, 32, 0.25);
+  const bool tm = kfmt > QF_16CONV && dir == QG_FWD;
+  const int narrow = tm ? QK_NARROW_T : QK_NARROW;
+  if (M > 32) consider(narrow, 64, 0.25);
+  consider(narrow, 32, 0.25);
   if (M > 32) consider(QK_HALF, 64, 0.16);
   consider(QK_HALF, 32, 0.155);
   if (kfmt == QF_16CONV) {
@@ -1134,7 +1193,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   if (a.out_dtype == OUT_F32 && p.n_main > 256) p.steps_per_split = 128;
   p.n_splits = (p.n_main + p.steps_per_split - 1) / p.steps_per_split;
 
-  const QPlan plan = qgemm_plan(kfmt, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms);
+  const QPlan plan = qgemm_plan(kfmt, a.dir, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms);
   const bool pair = plan.kind == QK_PAIR;
   p.TN = plan.TN;
   const int tile_rows = pair ? 256 : plan.kind == QK_HALF ? 64 : 128;
