@@ -198,3 +198,48 @@ def test_builtin_f32_and_q8_0_weights(ctx):
     O.frozen_backward_input(0, n, k, w2, dy2, m, ref)
     assert rel_l2(dx, ref) < MATMUL_TOL
     f2.close()
+
+
+@pytest.mark.parametrize("t,n,k,big", [(Q.Q4_0, 320, 704, 2600), (Q.Q8_0, 320, 704, 2600), (Q.Q4_K, 192, 768, 2600), (Q.Q6_K, 1088, 768, 1300),
+                                       (Q.F16, 320, 704, 2600), (Q.BF16, 320, 704, 2600), (Q.F16, 128, 64, 40000)],
+                         ids=lambda v: Q.NAMES.get(v, v) if isinstance(v, int) and v < 64 else str(v))
+def test_a_row_gets_the_same_bits_in_any_batch(ctx, t, n, k, big):
+    """An output element is one accumulation chain whatever tile it falls into, so every tile kind, unpacking into shared memory
+    or into TMEM, has to give the same bits: batches of sizes around the tile edges (32 and 64 tokens; half, narrow and pair
+    tiles; an odd number of 64-element steps; rows that end inside a tile; several tiles per CTA) against one large batch."""
+    rng = np.random.default_rng(n + k)
+    packed = Q.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), t)
+    f = rt.Frozen(ctx, t, n, k, packed)
+    x = rng.standard_normal((big, k)).astype(np.float32)
+    dy = rng.standard_normal((big, n)).astype(np.float32)
+    y = f.forward(x, big)
+    dx = np.zeros((big, k), np.float32)
+    f.backward_input(dy, big, dx)
+    rows = rng.integers(0, big, 64)
+    assert rel_l2(y[rows], O.frozen_forward(t, n, k, packed, x[rows], 64)) < MATMUL_TOL
+    for m in (1, 31, 33, 64, 65, 157, 640, 1100):
+        at = big - m
+        assert np.array_equal(f.forward(x[at:], m), y[at:]), m
+        part = np.zeros((m, k), np.float32)
+        f.backward_input(dy[at:], m, part)
+        assert np.array_equal(part, dx[at:]), m
+    f.close()
+
+
+def test_results_in_locked_memory_are_the_callers(ctx):
+    """Results of 64 KB and more lie in page-locked blocks of a bounded pool: a block is reused only after the last view of it
+    is gone, and past the bound (256 MB) results come in ordinary memory."""
+    rng = np.random.default_rng(0)
+    n, k, m = 4096, 64, 2048  # 32 MB of results
+    f = rt.Frozen.from_f32(ctx, (rng.standard_normal((n, k)) * 0.02).astype(np.float32), Q.Q8_0)
+    xs = [rng.standard_normal((m, k)).astype(np.float32) for _ in range(10)]
+    ys = [f.forward(x, m) for x in xs]  # 320 MB held at once
+    for x, y in zip(xs, ys):
+        assert np.array_equal(f.forward(x, m), y)
+    view = ys[0][5:7]
+    keep = view.copy()
+    del y, ys
+    for x in xs:
+        f.forward(x, m)
+    assert np.array_equal(view, keep)
+    f.close()

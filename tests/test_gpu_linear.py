@@ -92,3 +92,12 @@ def test_shape_errors_are_statuses(ctx):
         lin.forward(np.zeros((2, 63), np.float32), 2)
     lin.close()
     f.close()
+
+
+@pytest.mark.parametrize("t,n,k,m,r", [(Q.Q8_0, 128, 256, 9000, 16), (Q.Q8_0, 128, 3072, 4200, 40), (Q.Q4_0, 192, 512, 2049, 3),
+                                       (Q.F16, 264, 72, 65, 64), (Q.Q4_0, 128, 64, 1025, 16)])
+def test_adapter_streams_at_the_edges_of_their_splits(ctx, t, n, k, m, r):
+    """Low-rank streams and adapter gradients where their split changes: more than eight 1024-token splits, one token past a
+    split and past the 2048 and 4096 tokens at which the streams' tiles grow, contraction pieces of a wide input, ranks that
+    are no multiple of 16, column tiles that end inside a matrix."""
+    test_forward_backward_with_adapter(ctx, t, n, k, m, r)

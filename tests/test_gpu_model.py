@@ -382,3 +382,23 @@ def test_handles_may_outlive_their_context():
     gm.close()
     f.close()
     c2.close()  # twice is fine
+
+
+def test_more_batch_shapes_than_graphs_are_kept(ctx):
+    """Every batch shape gets a graph of its own, the least recently used one giving way past 32: a shape whose graph is gone, or
+    was captured after others were, gives the same bits as the first time."""
+    spec, _, gm = _setup(ctx, "tiny-qwen3", "Q8_0")
+    toks = synth.token_batch(spec, 1, 64, 11)[0]
+
+    def run(n):
+        gm.zero_grad()
+        tp, tt = synth.answer_targets(toks[:n], n // 2)
+        lp, _ = gm.forward_backward([toks[:n]], tp, tt, np.full(tp.size, 1.0 / tp.size, np.float32))
+        return lp.copy(), _gpu_flat(gm, "ga", "gb")
+
+    sizes = list(range(16, 56))
+    first = {n: run(n) for n in sizes}
+    for n in (16, 55, 16, 40, 17):
+        lp, g = run(n)
+        assert np.array_equal(lp, first[n][0]) and np.array_equal(g, first[n][1]), n
+    gm.close()

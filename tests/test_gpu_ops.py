@@ -169,6 +169,13 @@ def test_cross_entropy_rows_at_full_vocabulary(ctx, vocab):
     assert res["hits"] == hits
 
 
+@pytest.mark.parametrize("vocab", [512, 20480, 20484, 36868, 69632, 69636])
+def test_cross_entropy_rows_at_the_edges_of_what_a_block_keeps(ctx, vocab):
+    """Rows that end with the registers (20480 columns), one float4 into a shared-memory chunk, with the last chunk
+    (69632), and one float4 past it."""
+    test_cross_entropy_rows_at_full_vocabulary(ctx, vocab)
+
+
 @pytest.mark.parametrize("ff", [3072, 100])
 def test_swiglu_product_beyond_f16_is_an_error_not_a_nan(ctx, ff):
     """silu(gate) * up is stored in 16 bits as the input of down_proj (the reference keeps f32,
