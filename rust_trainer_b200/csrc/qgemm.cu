@@ -118,6 +118,8 @@ struct KParams {
   int n_splits, steps_per_split;  // work item = (tile, piece of the contraction); partial results go to `part`
   float* part;                    // [n_splits][M][out_rows] f32 partials when n_splits > 1
   int n_row_tiles, n_tok_tiles;   // a row tile is 128 weight rows, 256 for a CTA pair
+  int tok_first;                  // a row tile's token tiles are neighbours, instead of a token tile's row tiles
+  int inner;                      // tiles of a run of neighbours
   void* out;
   int out_dtype, accumulate, ld_out;
   const float* row_scale;  // optional per-token factor applied to the result
@@ -336,8 +338,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   (void)split; (void)n_main_st
 // first weight row (output feature) of this CTA's half of the tile, first token of the tile
 #define QG_TILE_ORIGIN()                                                                      \
-  const int r0 = (tile % p.n_row_tiles) * (C::ROWS * n_cta) + (int)rank * 128;                \
-  const int m0 = (tile / p.n_row_tiles) * p.TN
+  const int t_in = tile % p.inner, t_out = tile / p.inner;                                     \
+  const int r0 = (PAIR && p.tok_first ? t_out : t_in) * (C::ROWS * n_cta) + (int)rank * 128;   \
+  const int m0 = (PAIR && p.tok_first ? t_in : t_out) * p.TN
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) {
@@ -1199,6 +1202,12 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   const int tile_rows = pair ? 256 : plan.kind == QK_HALF ? 64 : 128;
   p.n_row_tiles = (out_rows + tile_rows - 1) / tile_rows;
   p.n_tok_tiles = (a.M + p.TN - 1) / p.TN;
+  // Tiles that run together share a token tile's activations; but weights that do not fit beside them in L2 (126 MB)
+  // come from memory again for every token tile (the head's 151936x1024 in Q8_0 at 1024 tokens: 664 MB read for
+  // 165), so then the token tiles of the same weights run together, while the activations do fit.  128256x3072 in Q6_K at
+  // 1024 tokens 631 -> 609 us; at 87 MB of weights, which stay in L2, the other order is the better one by a little.
+  p.tok_first = p.n_tok_tiles > 1 && w.dev_nbytes > ((size_t)96 << 20) && (size_t)a.M * contract * 2 <= ((size_t)32 << 20) && pair;
+  p.inner = p.tok_first ? p.n_tok_tiles : p.n_row_tiles;
   const int tn_cta = pair ? p.TN / 2 : p.TN;  // each CTA of a pair fetches its half of the token tile
   // tcgen05.mma kind::f16 needs A and B of ONE 16-bit type (f16 x bf16 is an illegal instruction).
   const int ab_fmt = a.act_f16 ? 0 : 1;
