@@ -39,7 +39,7 @@ constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_THRESHOLD = 8.0f;  // log2 units the stale maximum may lag behind
 
 // wait sites reported with RT_ERR_DEVICE_WAIT_TIMEOUT
-enum { SITE_Q = 401, SITE_KFREE, SITE_VFREE, SITE_KFULL, SITE_SFREE, SITE_PFULL, SITE_VFULL, SITE_SFULL, SITE_PVDONE, SITE_END };
+enum { SITE_Q = 401, SITE_KFREE, SITE_VFREE, SITE_KFULL, SITE_SFREE, SITE_PFULL, SITE_VFULL, SITE_SFULL, SITE_PVDONE, SITE_ODONE };
 
 template <int HD>
 struct FwdLayout {
@@ -88,7 +88,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   uint64_t* v_free = bars + 7;   // [2]
   uint64_t* s_full = bars + 9;   // [2]
   uint64_t* p_full = bars + 11;  // [2]
-  uint64_t* pv_done = bars + 13;
+  uint64_t* o_done = bars + 13;  // the last product has completed: one phase, so its parity says which
   uint32_t* tmem_slot = (uint32_t*)(bars + 14);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -108,7 +108,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);   // one arrival per softmax warp
     }
-    mbar_init(pv_done, 1);
+    mbar_init(o_done, 1);
     mbar_fence_init();
     prefetch_tmap(&tm_q);
     prefetch_tmap(&tm_k);
@@ -180,12 +180,14 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
           const uint64_t bd = umma_desc_sw128(sV + b * L::KV_BYTES + kk * 2048, L::KV_PANEL, 1024);
           umma_f16_ta(tmem_base + L::COL_O, tmem_base + L::COL_S + b * BN + kk * 8, bd, idesc_o, (n | kk) != 0);
         }
-        umma_commit(pv_done);
         umma_commit(&v_free[b]);
         if (n + 2 < ntiles && !issue_qk(n + 2)) { ok = false; break; }
       }
       // the last arrivals of the tensor core on this CTA's barriers land before the CTA leaves
-      if (ok) mbar_wait(&v_free[(ntiles - 1) & 1], (uint32_t)((ntiles - 1) >> 1) & 1, status, SITE_END);
+      if (ok) {
+        umma_commit(o_done);
+        mbar_wait(o_done, 0, status, SITE_ODONE);
+      }
     }
   } else {
     // ------------------------------------------------------------ softmax: thread = query row = TMEM lane
@@ -245,8 +247,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       l_run += sum.x + sum.y;
       m_used = m_new;
       if (n > 0 && __any_sync(0xffffffffu, grow && corr != 1.0f)) {
-        // O is at rest once the previous tile's P.V has completed
-        if (!mbar_wait(pv_done, (uint32_t)(n - 1) & 1, status, SITE_PVDONE)) { ok = false; break; }
+        // O is at rest once the previous tile's P.V has completed.  (Its phase of v_free cannot be taken for
+        // another: the one before, of P.V(n - 3), was over before K(n) was loaded, and P.V(n + 1) waits for this warp.)
+        if (!mbar_wait(&v_free[(n - 1) & 1], (uint32_t)((n - 1) >> 1) & 1, status, SITE_PVDONE)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < HD / 32; ++c) {
@@ -264,11 +267,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[b]);
     }
-    // the last product's phase, and the one before it first: a warp that never rescaled may be here while a
-    // slower warp still owes the tile before (its S came after the product two before, no later one), and
-    // a parity alone does not tell the last phase from the one two before
-    ok = ok && (ntiles < 2 || mbar_wait(pv_done, (uint32_t)ntiles & 1, status, SITE_PVDONE)) &&
-         mbar_wait(pv_done, (uint32_t)(ntiles - 1) & 1, status, SITE_PVDONE);
+    // A barrier of its own: between this warp's last P and here none, one or two of the last products may have
+    // completed, and the parity of a barrier that counts them all tells two of these states apart, not three.
+    ok = ok && mbar_wait(o_done, 0, status, SITE_ODONE);
     if (ok) {
       // O / l as f16 into Q's shared memory (every product that read Q has completed), in the
       // layout of a swizzled TMA box, then one bulk store per 64-column panel: rows past the end of
