@@ -615,7 +615,7 @@ void rt_model_destroy(rt_model* m) {
   m->h_batch.release();
   m->h_results.release();
   if (m->batch_sent) cudaEventDestroy(m->batch_sent);
-  for (auto& ge : m->graphs) cudaGraphExecDestroy(ge.exec);
+  m->graphs.for_each([](rt_model::Graph& g) { cudaGraphExecDestroy(g.exec); });
   delete m;
 }
 
@@ -1350,8 +1350,8 @@ static uint64_t buffer_signature(rt_model* m) {
 }
 
 // The staged step replays as ONE CUDA graph once the same shape has run eagerly (the eager run
-// sizes every buffer and encodes every TMA descriptor; capture then records ~3000 launches
-// with no host work between them).
+// sizes every buffer and encodes every TMA descriptor; capture then records the step's launches, 1100
+// for 28 layers, with no host work between them).  Which shapes are captured: graph_cache.h.
 static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) {
   rt_ctx* c = m->ctx;
   RT_CUDA(c, cudaSetDevice(c->device));
@@ -1364,14 +1364,12 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
     return run_staged_body(m, backward, logits_out_host);
   RT_CUDA(c, cudaSetDevice(c->device));
   rt_model::Shape shape{m->staged_tokens, m->staged_targets, backward ? 1 : 0, buffer_signature(m)};
-  for (size_t i = 0; i < m->graphs.size(); ++i)
-    if (m->graphs[i].shape == shape) {
-      std::rotate(m->graphs.begin() + i, m->graphs.begin() + i + 1, m->graphs.end());  // now the most recently used
-      RT_CUDA(c, cudaGraphLaunch(m->graphs.back().exec, c->stream));
-      RT_COUNT_LAUNCH(m->graphs.back().kernels);
-      return RT_OK;
-    }
-  if (std::find(m->seen.begin(), m->seen.end(), shape) != m->seen.end()) {
+  if (rt_model::Graph* g = m->graphs.find(shape)) {
+    RT_CUDA(c, cudaGraphLaunch(g->exec, c->stream));
+    RT_COUNT_LAUNCH(g->kernels);
+    return RT_OK;
+  }
+  if (m->graphs.worth_capturing(shape)) {
     const unsigned long long before = g_launch_count.load();
     cudaGraph_t graph = nullptr;
     RT_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -1382,11 +1380,7 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
     cudaGraphExec_t exec = nullptr;
     if (st == RT_OK && e == cudaSuccess && graph && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
       cudaGraphDestroy(graph);
-      if (m->graphs.size() >= rt_model::MAX_GRAPHS) {
-        cudaGraphExecDestroy(m->graphs.front().exec);
-        m->graphs.erase(m->graphs.begin());
-      }
-      m->graphs.push_back({shape, exec, kernels});
+      if (auto gone = m->graphs.put(shape, {exec, kernels})) cudaGraphExecDestroy(gone->exec);
       RT_CUDA(c, cudaGraphLaunch(exec, c->stream));
       RT_COUNT_LAUNCH(kernels);
       return RT_OK;
@@ -1398,8 +1392,7 @@ static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) 
   }
   rt_status st = run_staged_body(m, backward, nullptr);
   shape.sig = buffer_signature(m);  // the eager run may have sized buffers
-  if (m->seen.size() >= rt_model::MAX_SEEN) m->seen.erase(m->seen.begin());
-  m->seen.push_back(shape);
+  m->graphs.touch(shape);
   return st;
 }
 

@@ -4,6 +4,7 @@
 // tensor resident in HBM.
 #pragma once
 #include "ctx.h"
+#include "graph_cache.h"
 #include "ops.h"
 #include <map>
 #include <string>
@@ -164,16 +165,14 @@ struct rt_model {
   float* logp() const { return results.as<float>() + 4; }
   int staged_tokens = 0, staged_targets = 0;
   bool staged_has_weights = false;
-  // CUDA graphs of the staged step, one per shape of batch once it has run eagerly; least recently used first.
+  // CUDA graphs of the staged step, one per shape of batch once it has run eagerly.
   // A trainer meets several shapes in turn (accumulated batches, a preference update's three passes).
   struct Shape {
     int M, n_targets, backward;
     uint64_t sig;
     bool operator==(const Shape& o) const { return M == o.M && n_targets == o.n_targets && backward == o.backward && sig == o.sig; }
   };
-  struct GraphEntry { Shape shape; cudaGraphExec_t exec; unsigned long long kernels; };
-  static constexpr size_t MAX_GRAPHS = 32, MAX_SEEN = 256;
-  std::vector<GraphEntry> graphs;
-  std::vector<Shape> seen;  // shapes that have run eagerly, oldest first
+  struct Graph { cudaGraphExec_t exec; unsigned long long kernels; };
+  rt::GraphCache<Shape, Graph, 32> graphs;
   int use_graphs = -1;  // -1: decide from the environment on first use
 };
