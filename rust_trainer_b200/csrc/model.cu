@@ -171,9 +171,19 @@ rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16
     // gb[N x r] += dY^T . Hs ; ga[r x K] += Gs^T . X   on the tensor cores, contraction over tokens
     job = LoraGradJob{hs, dy16, gs, x16, dscale, N, N, K, r, {{{l->lora.gb, l->lora.ga, 0, N, 0, r}}, 1}};
   }
+  // The adapter gradients run behind the matmul, which starts under the low-rank stream that way; but a host that is done
+  // with x may have dx written over it, and they read x.
+  const uintptr_t x0 = (uintptr_t)x16, x1 = x0 + (size_t)M * K * sizeof(__half);
+  const uintptr_t d0 = (uintptr_t)dx, d1 = d0 + (size_t)M * K * (unscaled_f16_out ? sizeof(__half) : sizeof(float));
+  const bool dx_over_x = d0 < x1 && x0 < d1;
+  if (lora && dx_over_x) {
+    if (sc.defer) return c->fail(RT_ERR_BAD_ARG, "a gradient over an input that waiting adapter gradients read");
+    RT_TRY(lora_grads_add(c, sc, job, M));
+    a.late_wait = 0;
+  }
   int rc = frozen_matmul_launch(c, l->w->w, a);
   if (rc) return c->fail(rc, "frozen backward matmul launch failed");
-  return lora ? lora_grads_add(c, sc, job, M) : RT_OK;
+  return lora && !dx_over_x ? lora_grads_add(c, sc, job, M) : RT_OK;
 }
 
 

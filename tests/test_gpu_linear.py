@@ -101,3 +101,32 @@ def test_adapter_streams_at_the_edges_of_their_splits(ctx, t, n, k, m, r):
     split and past the 2048 and 4096 tokens at which the streams' tiles grow, contraction pieces of a wide input, ranks that
     are no multiple of 16, column tiles that end inside a matrix."""
     test_forward_backward_with_adapter(ctx, t, n, k, m, r)
+
+
+@pytest.mark.parametrize("t,n,k,m,r", [(Q.Q8_0, 256, 512, 300, 16), (Q.F16, 384, 256, 2500, 8)])
+def test_dx_may_be_written_over_x(ctx, t, n, k, m, r):
+    """On device buffers dx may take the memory of an x that is needed no more: the adapter gradients are those of separate buffers."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    _, _, _, _, f, lin = _make(ctx, rng, t, n, k, r)
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(1)).half().cuda()
+    dy = torch.randn(m, n, generator=torch.Generator().manual_seed(2)).half().cuda()
+
+    def run(x16, dx):
+        lin.zero_grad()
+        torch.cuda.synchronize()
+        ctx.check(rt.lib().rt_linear_backward_dev(lin._h, x16.data_ptr(), dy.data_ptr(), None, m, dx.data_ptr(), 0))
+        ctx.synchronize()
+        got = lin.lora()
+        return dx.clone(), got["ga"].copy(), got["gb"].copy()
+
+    want = run(x, torch.empty(m, k, device="cuda"))
+    for at in (0, m * k // 8 * 8):  # the first or the second half of the result's memory
+        both = torch.empty(m * k, device="cuda")
+        x16 = both.view(torch.float16)[at:at + m * k].view(m, k)
+        x16.copy_(x)
+        got = run(x16, both.view(m, k))
+        assert torch.equal(got[0], want[0]) and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
+    lin.close()
+    f.close()
