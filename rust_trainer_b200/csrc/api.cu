@@ -116,7 +116,12 @@ static void host_pool_give(void* p) {
   std::lock_guard<std::mutex> lock(hp.mutex);
   auto it = hp.used.find(p);
   if (it == hp.used.end()) return;
-  hp.idle.emplace(it->second, p);
+  if (ctx_any()) {  // (asked under the pool's lock: the last context unregisters, then trims under it)
+    hp.idle.emplace(it->second, p);
+  } else {
+    cudaFreeHost(p);
+    hp.total -= it->second;
+  }
   hp.used.erase(it);
 }
 static void host_pool_trim() {

@@ -243,3 +243,35 @@ def test_results_in_locked_memory_are_the_callers(ctx):
         f.forward(x, m)
     assert np.array_equal(view, keep)
     f.close()
+
+
+OUTLIVES = """
+import ctypes as C
+import numpy as np
+import rust_trainer_b200 as rt
+from rust_trainer_b200 import quants as Q
+cudart = C.CDLL("libcudart.so.12")
+def locked(address):
+    attr = (C.c_uint64 * 16)()  # cudaPointerAttributes: the memory's type comes first, 0 for ordinary memory
+    assert cudart.cudaPointerGetAttributes(attr, C.c_void_p(address)) == 0
+    return C.cast(attr, C.POINTER(C.c_int))[0] != 0
+ctx = rt.Context(0)
+f = rt.Frozen.from_f32(ctx, np.ones((1024, 64), np.float32), Q.Q8_0)
+y, z = (f.forward(np.ones((m, 64), np.float32), m) for m in (64, 128))
+at_y, at_z = y.ctypes.data, z.ctypes.data
+assert locked(at_y) and locked(at_z)
+del z
+assert locked(at_z)  # waits in the pool for the next result
+f.close()
+ctx.close()
+assert not locked(at_z) and locked(at_y) and float(y[3, 5]) == float(y[0, 0])
+del y
+assert not locked(at_y)
+"""
+
+
+def test_a_result_that_outlives_its_context_is_unlocked_with_its_last_view():
+    import subprocess
+    import sys
+
+    subprocess.run([sys.executable, "-c", OUTLIVES], check=True, timeout=300)
