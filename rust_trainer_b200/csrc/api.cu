@@ -88,6 +88,7 @@ void host_pool_trim_locked(HostPool& hp, size_t down_to) {
 }
 }  // namespace
 static void* host_pool_take(size_t bytes) {
+  if (bytes > HostPool::LIMIT) return nullptr;  // (the rounding below neither overflows nor passes the limit)
   HostPool& hp = host_pool();
   size_t unit = 4096;
   while (unit * 16 < bytes) unit *= 2;
@@ -99,7 +100,6 @@ static void* host_pool_take(size_t bytes) {
     p = it->second;
     hp.idle.erase(it);
   } else {
-    if (size > HostPool::LIMIT) return nullptr;
     host_pool_trim_locked(hp, HostPool::LIMIT - size);
     if (hp.total + size > HostPool::LIMIT) return nullptr;
     if (cudaHostAlloc(&p, size, cudaHostAllocPortable) != cudaSuccess) {

@@ -275,3 +275,11 @@ def test_a_result_that_outlives_its_context_is_unlocked_with_its_last_view():
     import sys
 
     subprocess.run([sys.executable, "-c", OUTLIVES], check=True, timeout=300)
+
+
+@pytest.mark.parametrize("nbytes", [(256 << 20) + 1, 1 << 60, (1 << 64) - 1])
+def test_locked_memory_past_the_pools_bound_is_refused(ctx, nbytes):
+    assert not rt.lib().rt_host_alloc(ctx._h, nbytes)
+    block = rt.lib().rt_host_alloc(ctx._h, 65536)
+    assert block
+    rt.lib().rt_host_free(block)
