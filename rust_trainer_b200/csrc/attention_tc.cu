@@ -322,11 +322,7 @@ template <int HD>
 int fwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, const AttnBatch& b, int nh, int nkv, __half* o, float* lse) {
   const int M = b.M;
   using L = FwdLayout<HD>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(attn_fwd_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL) != cudaSuccess) return 3;
-    attr = true;
-  }
+  if (!c->raise_smem(attn_fwd_tc_kernel<HD>, L::TOTAL)) return 3;
   CUtensorMap tq, tk, tv, to;
   if (tensor_map_f16_2d(c, &tq, q, (uint64_t)M, (uint64_t)nh * HD, 64, BM)) return 3;
   if (tensor_map_f16_2d(c, &to, o, (uint64_t)M, (uint64_t)nh * HD, 64, BM)) return 3;
@@ -1015,12 +1011,7 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   const int2* gap = (const int2*)b.gap;
   using LK = DkvLayout<HD>;
   using LQ = DqLayout<HD>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(attn_bwd_dkdv_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LK::TOTAL) != cudaSuccess) return 3;
-    if (cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LQ::TOTAL) != cudaSuccess) return 3;
-    attr = true;
-  }
+  if (!c->raise_smem(attn_bwd_dkdv_tc_kernel<HD>, LK::TOTAL) || !c->raise_smem(attn_bwd_dq_tc_kernel<HD>, LQ::TOTAL)) return 3;
   CUtensorMap tq128, tdo128, tk64, tv64, tk128, tv128, tq64, tdo64;
   if (tensor_map_f16_2d(c, &tq128, q, (uint64_t)M, (uint64_t)nh * HD, 64, 128)) return 3;
   if (tensor_map_f16_2d(c, &tdo128, dO, (uint64_t)M, (uint64_t)nh * HD, 64, 128)) return 3;

@@ -3,6 +3,7 @@
 #include "qformat.cuh"
 #include "rt_internal.h"
 #include <map>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -40,6 +41,17 @@ struct rt_ctx {
     return RT_ERR_CUDA;
   }
   void* get_scratch(int slot, size_t bytes);
+  // Lets `kernel` have `bytes` of shared memory, more than a launch gets by itself.  The limit belongs to the
+  // device, so each context raises it for itself, once: a process may use several GPUs.
+  std::set<const void*> smem_raised;
+  template <class Kernel>
+  bool raise_smem(Kernel* kernel, uint32_t bytes) {
+    const void* fn = (const void*)kernel;
+    if (smem_raised.count(fn)) return true;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    smem_raised.insert(fn);
+    return true;
+  }
   // Reads the device status word (after synchronising); maps non-zero to an error.
   rt_status check_device_status(const char* where);
 };

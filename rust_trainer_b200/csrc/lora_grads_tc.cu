@@ -316,11 +316,7 @@ size_t lora_grads_tc_workspace_floats(rt_ctx* c, const LoraGradJob* jobs, int n,
 int launch_lora_grads_tc(rt_ctx* c, const LoraGradJob* jobs, int n, int M, float* ws) {
   if (M <= 0 || n <= 0) return 0;
   if (n > LORA_GRAD_JOBS) return 3;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(lora_grads_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LG_TOTAL) != cudaSuccess) return 3;
-    attr = true;
-  }
+  if (!c->raise_smem(lora_grads_tc_kernel, LG_TOTAL)) return 3;
   LgArgs g;
   g.n_jobs = n;
   g.M = M;

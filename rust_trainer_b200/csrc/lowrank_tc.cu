@@ -217,12 +217,7 @@ lowrank_tc_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 template <int TN, int NS, int PPC>
 int lowrank_launch(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64) {
   using Cfg = LrCfg<TN, NS>;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(lowrank_tc_kernel<TN, NS, PPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::TOTAL) != cudaSuccess)
-      return 3;
-    attr = true;
-  }
+  if (!c->raise_smem(lowrank_tc_kernel<TN, NS, PPC>, Cfg::TOTAL)) return 3;
   CUtensorMap tx, tw;
   if (tensor_map_f16_2d(c, &tx, X, (uint64_t)M, (uint64_t)K, 64, TN)) return 3;
   if (tensor_map_f16_2d(c, &tw, Wt, (uint64_t)r, (uint64_t)K, 64, (uint32_t)((r + 7) & ~7))) return 3;

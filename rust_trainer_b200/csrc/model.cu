@@ -1205,9 +1205,10 @@ static rt_status model_head(rt_model* m, int M, int n_targets, bool backward, fl
     RT_TRY(linear_forward_dev(&head, m->lsc, m->ns16.as<__half>(), R, m->logits.p, RT_DT_F32, 0));
     if (logits_out_host)
       RT_CUDA(c, cudaMemcpyAsync(logits_out_host + (size_t)c0 * V, m->logits.p, (size_t)R * V * 4, cudaMemcpyDeviceToHost, st));
-    launch_ce_rows(m->logits.as<float>(), R, V, m->ttok + c0, m->tw + c0, m->logp() + c0,
-                   m->hits(), backward ? m->dl16.as<__half>() : nullptr, backward ? m->sc_l.as<float>() : nullptr,
-                   m->want_argmax ? m->argmax.as<int>() + c0 : nullptr, c->status_dev, st);
+    if (launch_ce_rows(c, m->logits.as<float>(), R, V, m->ttok + c0, m->tw + c0, m->logp() + c0, m->hits(),
+                       backward ? m->dl16.as<__half>() : nullptr, backward ? m->sc_l.as<float>() : nullptr,
+                       m->want_argmax ? m->argmax.as<int>() + c0 : nullptr))
+      return c->fail(RT_ERR_CUDA, "cross-entropy launch failed");
     if (backward) {
       RT_TRY(linear_backward_dev(&head, m->lsc, m->ns16.as<__half>(), m->dl16.as<__half>(), m->sc_l.as<float>(), R, m->dns.as<float>(), 0));
       launch_rmsnorm_bwd(m->xs.as<float>(), m->final_norm, m->dns.as<float>(), nullptr, R, d, g.rms_eps, m->dxs.as<float>(), nullptr, nullptr, st);

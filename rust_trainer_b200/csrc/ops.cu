@@ -1547,18 +1547,21 @@ ce_row_vec_kernel(const float* __restrict__ logits, int v, const int* __restrict
       if (tid + k * CE_THREADS < n4) put(tid + k * CE_THREADS, keep[k], f0);
   }
 }
-void launch_ce_rows(const float* logits, int rows, int v, const int* target, const float* weight, float* logp, int* hits,
-                    __half* d16, float* scale, int* argmax, int* status, cudaStream_t st) {
-  if (rows <= 0) return;
+int launch_ce_rows(rt_ctx* c, const float* logits, int rows, int v, const int* target, const float* weight, float* logp, int* hits,
+                   __half* d16, float* scale, int* argmax) {
+  if (rows <= 0) return 0;
+  cudaError_t e;
   if ((v & 3) == 0 && ((uintptr_t)logits & 15) == 0 && (d16 == nullptr || ((uintptr_t)d16 & 7) == 0)) {
-    static const bool attr = cudaFuncSetAttribute(ce_row_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * CE_CHUNK_BYTES) == cudaSuccess;
     const int left = v / 4 - CE_REG4 * CE_THREADS;  // float4s beyond the registers; a row without gradient is read once and needs no place
-    const int n_chunks = attr && d16 && left > 0 ? std::min(3, (left + 4 * CE_THREADS - 1) / (4 * CE_THREADS)) : 0;
-    pdl(ce_row_vec_kernel, rows, CE_THREADS, n_chunks * CE_CHUNK_BYTES, st)(logits, v, target, weight, logp, hits, d16, scale, argmax, status, n_chunks);
+    const int n_chunks = d16 && left > 0 ? std::min(3, (left + 4 * CE_THREADS - 1) / (4 * CE_THREADS)) : 0;
+    if (n_chunks > 0 && !c->raise_smem(ce_row_vec_kernel, 3 * CE_CHUNK_BYTES)) return 3;
+    e = pdl(ce_row_vec_kernel, rows, CE_THREADS, n_chunks * CE_CHUNK_BYTES, c->stream)(logits, v, target, weight, logp, hits, d16, scale, argmax,
+                                                                                     c->status_dev, n_chunks);
   } else {
-    pdl(ce_row_kernel, rows, 1024, 0, st)(logits, v, target, weight, logp, hits, d16, scale, argmax, status);
+    e = pdl(ce_row_kernel, rows, 1024, 0, c->stream)(logits, v, target, weight, logp, hits, d16, scale, argmax, c->status_dev);
   }
   RT_COUNT_LAUNCH(1);
+  return e == cudaSuccess ? 0 : 3;
 }
 
 // ------------------------------------------------------------------ LoRA shadows and gradients

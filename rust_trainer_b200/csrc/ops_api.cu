@@ -304,7 +304,8 @@ rt_status rt_op_cross_entropy(rt_ctx* c, const float* logits, size_t rows, size_
   if (!ld || !td || !lp || !hd || (weight && !wd) || (argmax && !am) || (dlogits && (!d16 || !sc)))
     return c->fail(RT_ERR_CUDA, "out of device memory");
   RT_CUDA(c, cudaMemsetAsync(hd, 0, 4, c->stream));
-  launch_ce_rows(ld, (int)rows, (int)vocab, td, wd, lp, hd, d16, sc, am, c->status_dev, c->stream);
+  if (launch_ce_rows(c, ld, (int)rows, (int)vocab, td, wd, lp, hd, d16, sc, am))
+    return c->fail(RT_ERR_CUDA, "cross-entropy launch failed");
   RT_CUDA(c, cudaMemcpyAsync(logp, lp, rows * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   if (hits) RT_CUDA(c, cudaMemcpyAsync(hits, hd, 4, cudaMemcpyDeviceToHost, c->stream));
   if (argmax) RT_CUDA(c, cudaMemcpyAsync(argmax, am, rows * sizeof(int), cudaMemcpyDeviceToHost, c->stream));

@@ -69,3 +69,15 @@ def test_product_never_imports_the_oracle():
     for f in list(pkg.rglob("*.py")) + list(pkg.rglob("*.cu")) + list(pkg.rglob("*.h")) + list(pkg.rglob("*.cuh")):
         src = f.read_text()
         assert "import oracle" not in src and "from oracle" not in src and "liboracle" not in src, f
+
+
+def test_shared_memory_limits_are_raised_per_context():
+    """A kernel's shared-memory limit belongs to the device, so nothing may remember for the process that it was raised: only a
+    context does (rt_ctx::raise_smem), or sets it again at each creation (the matmul's kernels)."""
+    csrc = ROOT / "rust_trainer_b200" / "csrc"
+    at = {f.name: [m.start() for m in re.finditer(r"cudaFuncSetAttribute\(", f.read_text())] for p in ("*.cu", "*.h", "*.cuh") for f in csrc.glob(p)}
+    assert {n: len(v) for n, v in at.items() if v} == {"ctx.h": 1, "qgemm.cu": 1}
+    q = (csrc / "qgemm.cu").read_text()
+    start = q.index("int qgemm_init() {")
+    assert start < at["qgemm.cu"][0] < q.index("\n}\n", start)
+    assert "raise_smem" in (csrc / "ctx.h").read_text()
