@@ -190,6 +190,7 @@ void rt_ctx_destroy(rt_ctx* c) {
   for (cudaEvent_t e : c->prof_events) cudaEventDestroy(e);
   for (int i = 0; i < 4; ++i)
     if (c->scratch[i]) cudaFree(c->scratch[i]);
+  rt::linear_scratch_free(c);
   if (c->status_dev) cudaFree(c->status_dev);
   if (c->status_host) cudaFreeHost(c->status_host);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);

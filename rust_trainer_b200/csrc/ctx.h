@@ -28,6 +28,7 @@ struct rt_ctx {
   // data-parallel communicator (an ncclComm_t once rt_comm_init_rank has run; a world of one otherwise)
   void* comm = nullptr;
   int comm_ranks = 1, comm_rank = 0;
+  struct LinearScratch* linear_scratch = nullptr;  // of linears used outside a model (model.cu)
   // grow-only scratch buffers for the host-pointer entry points
   void* scratch[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t scratch_bytes[4] = {0, 0, 0, 0};

@@ -377,6 +377,12 @@ struct SplitMix {
   float uniform_sym(float bound) { return (uniform() * 2.0f - 1.0f) * bound; }
 };
 
+void linear_scratch_free(rt_ctx* c) {
+  if (c->linear_scratch) c->linear_scratch->release();
+  delete c->linear_scratch;
+  c->linear_scratch = nullptr;
+}
+
 }  // namespace rt
 
 using namespace rt;
@@ -462,9 +468,10 @@ rt_status rt_linear_set_lora_enabled(rt_linear* l, int on) {
   return RT_OK;
 }
 
+// scratch for linears used outside a model: the context's, which frees it
 static LinearScratch& ctx_scratch(rt_ctx* c) {
-  static std::map<rt_ctx*, LinearScratch> m;  // scratch for linears used outside a model
-  return m[c];
+  if (!c->linear_scratch) c->linear_scratch = new LinearScratch;
+  return *c->linear_scratch;
 }
 
 rt_status rt_linear_forward_dev(rt_linear* l, const void* x, size_t t, void* y, int y_dtype, int accumulate) {
@@ -613,13 +620,14 @@ void rt_model_destroy(rt_model* m) {
   if (m->embed) rt_frozen_destroy(m->embed);
   for (void* p : m->owned) cudaFree(p);
   DevBuf* bufs[] = {&m->P, &m->G, &m->Mo, &m->Vo, &m->opt_scalars, &m->inv_freq, &m->rope_cos, &m->rope_sin,
-                    &m->lsc.hs, &m->lsc.gs[0], &m->lsc.gs[1], &m->lsc.gs[2], &m->lsc.gs[3], &m->lsc.grad_ws, &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
+                    &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
                     &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw, &m->q16, &m->k16, &m->v16, &m->o16, &m->lse,
                     &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16, &m->sc_y, &m->dhm, &m->dg16, &m->du16,
                     &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq, &m->dk, &m->dv, &m->dq16, &m->dk16,
                     &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs,
                     &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) b->release();
+  m->lsc.release();
   for (int i = 0; i < 7; ++i) m->hs_keep[i].release();
   m->argmax.release();
   m->h_batch.release();

@@ -53,7 +53,7 @@ struct rt_linear {
   bool lora_active() const { return has_lora && lora_enabled; }
 };
 
-// Scratch shared by every Linear call on a ctx (one call at a time per ctx).
+// Scratch of the Linear calls of a model, or of those on a ctx outside any model (one call at a time per ctx).
 struct LinearScratch {
   DevBuf hs, gs[rt::LORA_GRAD_JOBS], grad_ws;
   int hs_rank = -1, gs_rank[rt::LORA_GRAD_JOBS] = {-1, -1, -1, -1};
@@ -62,6 +62,11 @@ struct LinearScratch {
   bool defer = false;
   int n_jobs = 0;
   rt::LoraGradJob jobs[rt::LORA_GRAD_JOBS];
+  void release() {
+    hs.release();
+    for (DevBuf& g : gs) g.release();
+    grad_ws.release();
+  }
 };
 
 namespace rt {

@@ -24,6 +24,9 @@ void prof_mark(const char* file, int line);  // site_prof.cu
 #define RT_COUNT_LAUNCH(n) (rt::g_launch_count.fetch_add((n), std::memory_order_relaxed))
 #endif
 
+// ---- model.cu: the scratch of linears used outside a model, freed with their context
+void linear_scratch_free(rt_ctx* c);
+
 // ---- repack.cu
 void launch_repack(const uint8_t* raw_dev, const QWeight& w, cudaStream_t st);
 void launch_gather_rows(const QWeight& w, const int* ids_dev, int n, float* out, int* status, cudaStream_t st);

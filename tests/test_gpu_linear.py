@@ -130,3 +130,34 @@ def test_dx_may_be_written_over_x(ctx, t, n, k, m, r):
         assert torch.equal(got[0], want[0]) and np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2])
     lin.close()
     f.close()
+
+
+def test_a_contexts_scratch_goes_with_it():
+    """What linears outside a model work in belongs to their context: it is freed with it, and a later context, which may get the
+    same address and another device, does not find it."""
+    import torch
+
+    def free_bytes():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def use():
+        c = rt.Context(0)
+        f = rt.Frozen.from_f32(c, np.ones((64, 64), np.float32), Q.Q8_0)
+        lin = rt.Linear("l", f)
+        lin.attach_lora(8, 16.0, np.zeros((8, 64), np.float32), np.zeros((64, 8), np.float32))
+        x = torch.zeros(1 << 20, 64, dtype=torch.float16, device="cuda")
+        y = torch.empty(1 << 20, 64, dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        c.check(rt.lib().rt_linear_forward_dev(lin._h, x.data_ptr(), 1 << 20, y.data_ptr(), 2, 0))  # 192 MB of Hs
+        c.synchronize()
+        lin.close()
+        f.close()
+        held = free_bytes()
+        c.close()
+        return held
+
+    use()
+    before = free_bytes()
+    assert use() < before - (100 << 20)
+    assert abs(free_bytes() - before) < 32 << 20
