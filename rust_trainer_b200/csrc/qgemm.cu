@@ -30,7 +30,8 @@ namespace rt {
 // per unpacked unit on the device).
 enum QKind : int {
   QK_PAIR = 0,    // a CTA pair per tile of 256 weight rows x up to 256 tokens
-  QK_WIDE = 1,    // one CTA per tile of 128 weight rows x up to 256 tokens (16-bit weights only)
+  QK_WIDE = 1,    // one CTA per tile of 128 weight rows x up to 256 tokens: converted 16-bit weights, and all
+                  // formats where CTA pairs cannot run or are switched off
   QK_NARROW = 2,  // one CTA per tile of 128 weight rows x up to 64 tokens
   QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
   // Narrow tiles of packed weights in the forward direction, with the unpacked weights in TMEM: a thread that owns a
@@ -63,6 +64,7 @@ struct QCfg {
   static constexpr int ROWS = HALF ? 64 : 128, BRICKS = ROWS / 64;
   static constexpr int W_SUB = ROWS * 128;  // bytes of a [ROWS x 64] 16-bit weight tile
   static constexpr bool PACKED = FMT > QF_16CONV;
+  static constexpr bool WIDE = KIND == QK_WIDE;
   // Unpack warps.  Sixteen for packed weights: one unpack pass is a chain of dependent operations
   // (codes -> convert -> swizzled store -> fence -> arrive), so what counts is how many passes are
   // in flight per scheduler.  (Eight warps of twice the work each: 8192x3072 Q6_K at 8192 tokens
@@ -75,9 +77,9 @@ struct QCfg {
   static constexpr int KS = NARROW || HALF ? 2 : 1;
   // Activation / unpacked-weight stages, and packed-brick stages in the room that is left beside them and
   // the epilogue staging.
-  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : KIND == QK_WIDE ? 3 : HALF || TM ? 4 : PACKED ? 3 : 4;
+  static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : WIDE ? 3 : HALF || TM ? 4 : PACKED ? 3 : 4;
   static constexpr int RAW_STAGE = PACKED ? KS * BRICKS * fmt_brick_bytes(FMT) : 0;
-  static constexpr int ACT_SUB = PAIR ? 16384 : KIND == QK_WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
+  static constexpr int ACT_SUB = PAIR ? 16384 : WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
   static constexpr int ACT_STAGE = KS * ACT_SUB;
   static constexpr int W_BYTES = (TM ? 1 : KS) * W_SUB;    // weights of a stage (in TMEM: the low-rank step's only)
   // TMEM columns of a stage's unpacked weights, beside the two accumulators of up to 64 columns at 0 and 256
@@ -97,7 +99,9 @@ struct QCfg {
   static constexpr int UG = PAIR ? 4 : 2;                  // a power of two
   static constexpr int UTG = NUW * 32 / UG;                // threads per group
   static_assert(UG <= NS && (!PACKED || NS <= NR + 1), "unpack groups would alias barrier phases");
-  static_assert(!PACKED || UTG == KS * 128, "a thread of a group owns one unit of each half of a weight tile");
+  // A thread of a group owns one unit of each half of a weight tile; with a group of twice the threads (wide tiles) of one half.
+  static constexpr int HALVES = WIDE ? 1 : BRICKS;
+  static_assert(!PACKED || UTG == KS * 128 * (BRICKS / HALVES), "the group's threads cover a stage's units");
   static constexpr int OFF_W = NS * ACT_STAGE;
   static constexpr int OFF_RAW = OFF_W + NS * W_BYTES;
   static constexpr int OFF_OUT = (OFF_RAW + NR * RAW_STAGE + 1023) / 1024 * 1024;  // (a swizzled store's source starts on its pattern)
@@ -796,17 +800,17 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
               if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
               // two bricks per 64-element tile: brick b fills the 8 KB half b.  A stage of two tiles goes to the
               // two halves of the group.
-              const int u = tg >> 7;
+              const int u = C::WIDE ? 0 : tg >> 7, half = C::WIDE ? tg >> 7 : 0;
               if (u < subs) {
-                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : C::BRICKS * u * BB);
                 const int next = p.dir == QG_FWD ? KS * BB : BB;
-                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB;
+                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : C::BRICKS * u * BB) + half * next;
+                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB + (uint32_t)half * 8192;
                 if (p.act_f16) {
 #pragma unroll
-                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, false, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+                  for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, false, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
                 } else {
 #pragma unroll 1
-                  for (int b = 0; b < C::BRICKS; ++b) unpack_unit<FMT, true, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+                  for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, true, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
                 }
               }
               fence_proxy_async_smem();
@@ -953,23 +957,22 @@ template <int KIND, int FMT, int OUT>
 static QKernel qkernel() {
   return {(const void*)qgemm_kernel<KIND, FMT, OUT>, QCfg<KIND, FMT>::THREADS, QCfg<KIND, FMT>::SMEM_BYTES};
 }
-// fmt: a packed ggml format, QF_16 or QF_16CONV.  The wide single-CTA kernel only serves converted
-// 16-bit weights: the others' wide tiles run as pairs.
+// fmt: a packed ggml format, QF_16 or QF_16CONV
 template <int KIND, int OUT>
 static QKernel qkernel_fmt(int fmt) {
-  constexpr bool WIDE = KIND == QK_WIDE, TM = KIND == QK_NARROW_T;
+  constexpr bool TM = KIND == QK_NARROW_T;
   if constexpr (KIND != QK_PAIR && !TM) {
     if (fmt == QF_16CONV) return qkernel<KIND, QF_16CONV, OUT>();
   }
-  if constexpr (!WIDE && !TM) {
+  if constexpr (!TM) {
     if (fmt == QF_16) return qkernel<KIND, QF_16, OUT>();
   }
-  if constexpr (!WIDE) switch (fmt) {
-      case GGML_Q4_0: return qkernel<KIND, GGML_Q4_0, OUT>();
-      case GGML_Q8_0: return qkernel<KIND, GGML_Q8_0, OUT>();
-      case GGML_Q4_K: return qkernel<KIND, GGML_Q4_K, OUT>();
-      case GGML_Q6_K: return qkernel<KIND, GGML_Q6_K, OUT>();
-    }
+  switch (fmt) {
+    case GGML_Q4_0: return qkernel<KIND, GGML_Q4_0, OUT>();
+    case GGML_Q8_0: return qkernel<KIND, GGML_Q8_0, OUT>();
+    case GGML_Q4_K: return qkernel<KIND, GGML_Q4_K, OUT>();
+    case GGML_Q6_K: return qkernel<KIND, GGML_Q6_K, OUT>();
+  }
   return {nullptr, 0, 0};
 }
 static QKernel qkernel_for(int kind, int fmt, int out) {
@@ -995,12 +998,17 @@ int qgemm_init() {
       return RT_ERR_CUDA;
     g_encode = (PFN_encodeTiled)fn;
   }
-  for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF, (int)QK_NARROW_T})
-    for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K})
-    for (int out : {(int)QO_TMA16, (int)QO_DIRECT, (int)QO_RES}) {
-      const QKernel k = qkernel_for(kind, fmt, out);
-      if (k.fn && cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem) != cudaSuccess) return RT_ERR_CUDA;
-    }
+  auto raise_smem = [](bool wide) {  // wide tiles of weights that are not converted: only where there are no pairs
+    for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF, (int)QK_NARROW_T})
+      for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K})
+        for (int out : {(int)QO_TMA16, (int)QO_DIRECT, (int)QO_RES}) {
+          if ((kind == QK_WIDE && fmt != QF_16CONV) != wide) continue;
+          const QKernel k = qkernel_for(kind, fmt, out);
+          if (k.fn && cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem) != cudaSuccess) return false;
+        }
+    return true;
+  };
+  if (!raise_smem(false)) return RT_ERR_CUDA;
   if (g_pair_workers < 0) {
     int dev = 0, sms = 0, n = 0;
     cudaGetDevice(&dev);
@@ -1024,6 +1032,7 @@ int qgemm_init() {
     const char* e = getenv("RT_B200_NO_PAIR");
     g_pair_workers = (e && atoi(e)) ? 0 : n;
   }
+  if (g_pair_workers == 0 && !raise_smem(true)) return RT_ERR_CUDA;
   return RT_OK;
 }
 
@@ -1142,6 +1151,8 @@ static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, in
       const double mma = 0.29 + 0.00064 * tn;
       consider(QK_PAIR, tn, mma > 0.335 ? mma : 0.335);
     }
+  } else if (M > 64) {  // without pairs: 8192x3072 Q8_0 at 4096 tokens 171-181 us, 279-341 on 64-token tiles
+    for (int tn = 256; tn >= 96; tn -= 32) consider(QK_WIDE, tn, 0.15 + 0.0012 * tn > 0.35 ? 0.15 + 0.0012 * tn : 0.35);
   }
   return best;
 }
