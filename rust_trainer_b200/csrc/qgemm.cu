@@ -1116,11 +1116,17 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 
 // Which kernel and token-tile width a product gets: the one whose persistent grid is estimated to finish
 // first, rounds of tiles x (contraction steps x the step's time + a tile's fixed time).  The step times
-// (us, 64 contraction elements) are fitted to sweeps over both kernels and all widths (eight weight shapes
-// of 128..151936 rows, 1..8192 tokens): about 0.33 for a pair while the single-thread roles and the unpack
-// passes set the pace, more from about 64 tokens of width per CTA on, when the MMAs do; 0.25 for narrow
-// tiles, which hand over two steps at a time (0.23 from TMEM, but a fit that says so puts pairs
-// out of work that do it faster), and 0.17 for half tiles, whose unpack passes are half as long.
+// (us, 64 contraction elements) are fitted to sweeps over the kernels and all widths: about 0.33 for a pair
+// while the single-thread roles and the unpack passes set the pace, more from about 64 tokens of width per
+// CTA on, when the MMAs do; 0.25 for narrow tiles, which hand over two steps at a time, and 0.16 for half
+// tiles, whose unpack passes are half as long.  They are a fit to what wins, not each kernel's own pace: one
+// round of narrow tiles from TMEM takes 0.23 a step, and a pair's fixed time is rather 1.7 than 0.5.  With
+// that 1.7 the choices below are better (0.6 % off, 13 by more than 10 %), but 2560 -> 9728 at 300 tokens goes to three
+// rounds of narrow tiles, 31 -> 38 us in Q8_0 (0.28 a step) and 36 -> 46 in Q6_K.
+// Against the best kind and width of each of 1434 products (15 shapes of 64..9728 -> 128..8192, both directions,
+// 1..12000 tokens, Q8_0, Q6_K and F16) the choice is 0.8 % off on average and 31 are off by more than 10 %, all
+// of them launches of 5 to 10 us: short contractions that pairs get and narrow tiles finish first (25 % at worst, 64 -> 1024
+// at 1500 tokens 7.2 us against 5.6).
 // Narrow and half tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
 // backward at 1024 tokens 29 us (44 on pairs of 128 tokens before), 8192x3072 Q6_K backward at 24 tokens 30 us
 // (43 on narrow tiles, 91 before), 1024x2048 at 157 tokens 9.6 us (12).
