@@ -2,11 +2,20 @@
 // kernel before it on the stream is still running; it must not touch global memory before
 // pdl_wait(), which returns once that kernel has completed and its writes are visible.  What runs
 // before the wait (barrier init, TMEM allocation, tensor-map prefetch, block scheduling itself)
-// overlaps the predecessor's tail.  Rules kept by every kernel launched this way:
-//   - every CTA executes pdl_wait() before its first global access and before any early return
-//     (a grid counts as complete only when all of it has waited, so ordering stays transitive);
+// overlaps the predecessor's tail.  Rules of the kernels launched this way:
+//   - every CTA executes pdl_wait() before its first access to anything the pass computes and before any
+//     early return (a grid that is complete has then waited, so ordering stays transitive).  What a batch
+//     brings along and no kernel writes (tile lists, where sequences start) may be read before it;
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
 //     every CTA of this one has started.
+// One pair of kernels departs from both.  A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
+// weights, activations and residual without waiting and waits only where it loads the stream's result.  That
+// is sound because of what lowrank_tc_kernel and the matmul keep between them:
+//   - lowrank_tc_kernel triggers only after its own wait, so that everything older than it is complete and
+//     visible once the matmul runs.  Moved to the kernel's entry, the trigger would make a race of this;
+//   - it writes nothing the matmul reads but that result, and the matmul writes nothing it reads;
+//   - at least one CTA of the matmul waits (the last piece of a contraction always ends in the low-rank
+//     step), so that whoever waits for the matmul has waited for the stream.
 // Inside stream capture these launches become programmatic edges of the graph.
 // Used for passes of up to PDL_MAX_TOKENS tokens, whose kernels leave SMs free for the next one's CTAs to
 // start on: the 28-layer 0.6B step 10.67 -> 10.14 ms at 1024 tokens, scoring 157 tokens 3.01 -> 2.84 ms.  At

@@ -62,8 +62,9 @@ struct QGemmArgs {
   // cached or allocated on the way); a launch that needs more fails with RT_ERR_TOO_LARGE
   float* fixed_part = nullptr;
   size_t fixed_part_floats = 0;
-  // The launch right before this one is the low-rank stream that produces lora.act: a programmatic launch
-  // may start at once and waits for it only where it reads that.
+  // The launch right before this one is the low-rank stream that produces lora.act, which lets its successor start
+  // only after its own wait: a programmatic launch may start at once and waits only where it reads that result
+  // (pdl.cuh has the conditions).
   int late_wait = 0;
 };
 
