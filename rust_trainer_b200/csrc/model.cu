@@ -1,5 +1,5 @@
 // C ABI levels 2 and 3: Linear + LoRA and the whole decoder step on the device.
-// The arithmetic lives in qgemm.cu (frozen matmuls), attention.cu and ops.cu; this file is the
+// The arithmetic lives in qgemm.cu (frozen matmuls), attention_tc.cu and ops.cu; this file is the
 // sequencing the reference does in src/linear.rs, src/attention.rs, src/model.rs and
 // src/optim.rs, plus buffer management.
 #include "model.h"
@@ -621,10 +621,10 @@ void rt_model_destroy(rt_model* m) {
   for (void* p : m->owned) cudaFree(p);
   DevBuf* bufs[] = {&m->P, &m->G, &m->Mo, &m->Vo, &m->opt_scalars, &m->inv_freq, &m->rope_cos, &m->rope_sin,
                     &m->batch, &m->results, &m->x, &m->ckpt, &m->h,
-                    &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw, &m->q16, &m->k16, &m->v16, &m->o16, &m->lse,
-                    &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16, &m->sc_y, &m->dhm, &m->dg16, &m->du16,
-                    &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq, &m->dk, &m->dv, &m->dq16, &m->dk16,
-                    &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs,
+                    &m->n1, &m->n2, &m->q_raw, &m->q16, &m->k16, &m->v16, &m->o16, &m->lse,
+                    &m->delta, &m->g16, &m->hm16, &m->dx, &m->dy16, &m->sc_y, &m->dhm, &m->dg16,
+                    &m->sc_g, &m->sc_u, &m->dn, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq, &m->dk, &m->dv, &m->dq16,
+                    &m->sc_q, &m->sc_k, &m->sc_v, &m->xs,
                     &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) b->release();
   m->lsc.release();
@@ -976,8 +976,8 @@ static bool ensure_tokens(rt_model* m, int M) {
   if (m->recompute_policy == 0 && g.n_layers > 1) {
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-      const size_t held = m->n1.bytes + m->n2.bytes + m->q_raw.bytes + m->k_raw.bytes + m->q16.bytes + m->k16.bytes + m->v16.bytes +
-                          m->o16.bytes + m->lse.bytes + m->h.bytes + m->g16.bytes + m->u16.bytes + m->hm16.bytes;
+      const size_t held = m->n1.bytes + m->n2.bytes + m->q_raw.bytes + m->q16.bytes + m->k16.bytes + m->v16.bytes +
+                          m->o16.bytes + m->lse.bytes + m->h.bytes + m->g16.bytes + m->hm16.bytes;
       const size_t need = per_layer * g.n_layers;
       m->store_acts = need <= held || (double)(need - held) <= 0.6 * (double)free_b;
     }
@@ -1353,10 +1353,10 @@ static uint64_t buffer_signature(rt_model* m) {
   uint64_t h = 1469598103934665603ull;
   auto mix = [&](const void* p) { h = (h ^ (uint64_t)(uintptr_t)p) * 1099511628211ull; };
   DevBuf* bufs[] = {&m->P, &m->G, &m->rope_cos, &m->rope_sin, &m->lsc.hs, &m->lsc.gs[0], &m->lsc.gs[1], &m->lsc.gs[2], &m->lsc.gs[3], &m->lsc.grad_ws,
-                    &m->batch, &m->results, &m->x, &m->ckpt, &m->h, &m->n1, &m->n2, &m->q_raw, &m->k_raw, &m->v_raw,
-                    &m->q16, &m->k16, &m->v16, &m->o16, &m->lse, &m->delta, &m->g16, &m->u16, &m->hm16, &m->dx, &m->dy16,
-                    &m->sc_y, &m->dhm, &m->dg16, &m->du16, &m->sc_g, &m->sc_u, &m->dn, &m->d_o, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq,
-                    &m->dk, &m->dv, &m->dq16, &m->dk16, &m->dv16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs, &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
+                    &m->batch, &m->results, &m->x, &m->ckpt, &m->h, &m->n1, &m->n2, &m->q_raw,
+                    &m->q16, &m->k16, &m->v16, &m->o16, &m->lse, &m->delta, &m->g16, &m->hm16, &m->dx, &m->dy16,
+                    &m->sc_y, &m->dhm, &m->dg16, &m->sc_g, &m->sc_u, &m->dn, &m->dO16, &m->dy16o, &m->sc_yo, &m->dq,
+                    &m->dk, &m->dv, &m->dq16, &m->sc_q, &m->sc_k, &m->sc_v, &m->xs, &m->ns16, &m->logits, &m->dl16, &m->sc_l, &m->dns, &m->dxs};
   for (DevBuf* b : bufs) mix(b->p);
   for (int i = 0; i < 7; ++i) mix(m->hs_keep[i].p);
   for (int i = 0; i < 4; ++i) mix(m->ctx->scratch[i]);

@@ -147,15 +147,15 @@ struct rt_model {
   int cap_tokens = 0, cap_targets = 0, cap_head_rows = 0;
   // q_raw holds q|k|v before RoPE (three regions, or one matrix with q, k, v as column slices when the
   // block runs them as a group); g16 holds gate|up the same way; dq16, dg16 likewise for the gradients
-  DevBuf x, ckpt, h, n1, n2, q_raw, k_raw, v_raw, q16, k16, v16, o16, lse, delta, g16, u16, hm16;
-  DevBuf dx, dy16, sc_y, dhm, dg16, du16, sc_g, sc_u, dn, d_o, dO16, dy16o, sc_yo, dq, dk, dv, dq16, dk16, dv16, sc_q, sc_k, sc_v;
+  DevBuf x, ckpt, h, n1, n2, q_raw, q16, k16, v16, o16, lse, delta, g16, hm16;
+  DevBuf dx, dy16, sc_y, dhm, dg16, sc_g, sc_u, dn, dO16, dy16o, sc_yo, dq, dk, dv, dq16, sc_q, sc_k, sc_v;
   DevBuf xs, ns16, logits, dl16, sc_l, dns, dxs;
   DevBuf argmax;            // per target, the greedy token of the last pass that asked for it
   bool want_argmax = false;
   DevBuf refresh_tab;       // device copy of refresh_sent
   std::vector<rt::LoraRefreshJob> refresh_jobs, refresh_sent;
   // A batch travels as one block: laid out in pinned memory, one copy to `batch`, the pointers below into it
-  // (they depend on the block's base, the token and target counts and staged_gap only).  Results come back as
+  // (they depend on the block's base, the token and target counts and whether there are gaps only).  Results come back as
   // one block too: hit count, then log-probabilities.
   DevBuf batch, results;
   PinnedBuf h_batch, h_results;
@@ -165,7 +165,6 @@ struct rt_model {
   rt::AttnBatch attn_batch(int M) const { return {seq_start, gap, tiles_q, tiles_k, M}; }
   int* gap = nullptr;       // per token (first, end) of the key range hidden from it: packed shared-prompt groups, or null
   float* tw = nullptr;
-  bool staged_gap = false;  // the staged batch has such ranges
   int* hits() const { return results.as<int>(); }
   float* logp() const { return results.as<float>() + 4; }
   int staged_tokens = 0, staged_targets = 0;

@@ -53,11 +53,6 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity
       : "memory");
   return ok;
 }
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
 // Bounded wait. Returns false (and records `code` in *status) after ~4e9 SM cycles (about two
 // seconds).  The bound counts this SM's own cycle counter, which nothing outside the kernel can
 // step or re-synchronise.
@@ -161,15 +156,9 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// 2-D tiled store / reduce-add, shared -> global, tracked by bulk async-groups.
+// 2-D tiled store, shared -> global, tracked by bulk async-groups.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)map),
-               "r"(smem_u32(src)), "r"(x), "r"(y)
-               : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, const void* src) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
-                   (uint64_t)map),
                "r"(smem_u32(src)), "r"(x), "r"(y)
                : "memory");
 }
@@ -178,10 +167,6 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 template <int N>
 __device__ __forceinline__ void bulk_wait_group_read() {
   asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void bulk_wait_group() {
-  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -233,21 +218,11 @@ __device__ __forceinline__ void umma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, ui
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One MMA over a CTA pair (M = 256: 128 accumulator rows in each CTA's TMEM; each CTA supplies its
-// 128 rows of A and its half of B's N columns from the same shared-memory offsets).  Issued by
-// ONE thread of the leader CTA.
-__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The issuing thread is a single lane: every instruction it spends on building descriptors is
 // latency the tensor core waits for.  These forms take the two halves of each descriptor, so
-// a K step only adds a constant to the low (address) words.
+// a K step only adds a constant to the low (address) words.  PAIR: one MMA over a CTA pair (M = 256: 128
+// accumulator rows in each CTA's TMEM; each CTA supplies its 128 rows of A and its half of B's N columns
+// from the same shared-memory offsets), issued by ONE thread of the leader CTA.
 template <bool PAIR>
 __device__ __forceinline__ void umma_f16_split(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                                uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {

@@ -946,8 +946,6 @@ typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static PFN_encodeTiled g_encode = nullptr;
 
-size_t qgemm_smem_bytes() { return QCfg<QK_PAIR, GGML_Q8_0>::SMEM_BYTES; }
-
 // Every (kind, format) the dispatch can ask for, with its launch shape.
 struct QKernel {
   const void* fn;

@@ -80,7 +80,6 @@ int tensor_map_f16_2d(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t ro
 // The same with a row pitch of `ld` elements (a column slice of a wider matrix).
 int tensor_map_f16_2d_ld(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                          uint32_t box_cols, uint32_t box_rows);
-size_t qgemm_smem_bytes();
 int qgemm_init();  // resolves the driver entry point for tensor-map encoding; sets smem attributes
 
 }  // namespace rt
