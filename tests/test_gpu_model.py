@@ -385,8 +385,8 @@ def test_handles_may_outlive_their_context():
 
 
 def test_more_batch_shapes_than_graphs_are_kept(ctx):
-    """Every batch shape gets a graph of its own, the least recently used one giving way past 32: a shape whose graph is gone, or
-    was captured after others were, gives the same bits as the first time."""
+    """A batch shape that comes again soon is captured, past 32 distinct ones in between it is not: either way the same bits as the
+    first time."""
     spec, _, gm = _setup(ctx, "tiny-qwen3", "Q8_0")
     toks = synth.token_batch(spec, 1, 64, 11)[0]
 
@@ -399,6 +399,30 @@ def test_more_batch_shapes_than_graphs_are_kept(ctx):
     sizes = list(range(16, 56))
     first = {n: run(n) for n in sizes}
     for n in (16, 55, 16, 40, 17):
+        lp, g = run(n)
+        assert np.array_equal(lp, first[n][0]) and np.array_equal(g, first[n][1]), n
+    gm.close()
+
+
+def test_a_shape_whose_graph_gave_way_gives_the_same_bits(ctx):
+    """Each of 40 shapes twice in a row is captured, and the first eight graphs give way to the last; shapes with a graph, without
+    one and captured again give the bits of the first, eager pass."""
+    spec, _, gm = _setup(ctx, "tiny-qwen3", "Q8_0")
+    toks = synth.token_batch(spec, 1, 64, 11)[0]
+
+    def run(n):
+        gm.zero_grad()
+        tp, tt = synth.answer_targets(toks[:n], n // 2)
+        lp, _ = gm.forward_backward([toks[:n]], tp, tt, np.full(tp.size, 1.0 / tp.size, np.float32))
+        return lp.copy(), _gpu_flat(gm, "ga", "gb")
+
+    run(64)  # buffers of their final size: no graph goes stale
+    sizes = list(range(16, 56))
+    first = {}
+    for n in sizes:
+        first[n] = run(n)
+        run(n)
+    for n in (55, 24, 16, 16, 16, 23, 54):
         lp, g = run(n)
         assert np.array_equal(lp, first[n][0]) and np.array_equal(g, first[n][1]), n
     gm.close()
