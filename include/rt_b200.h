@@ -72,7 +72,7 @@ void* rt_ctx_stream(rt_ctx* ctx);
  * link's rate, and it has no first-touch faults.  Blocks come from a pool of the process (256 MB at
  * most; safe from any thread) and go back to it; NULL when the pool is full or nothing can be locked:
  * then use ordinary memory, which every call takes as well.  A block may outlive the context; the
- * pool's free blocks are unlocked with the last context. */
+ * pool's free blocks are unlocked with the last context, and one that comes back later at once. */
 void* rt_host_alloc(rt_ctx* ctx, size_t bytes);
 void rt_host_free(void* block);
 /* Issue all later calls on `cuda_stream` (a cudaStream_t of the same device) instead of the
@@ -224,7 +224,8 @@ rt_status rt_linear_forward_dev(rt_linear* lin, const void* x_f16_dev, size_t t,
 /* Linear::backward (src/linear.rs:97-121), device form.  dy is passed as f16 rows divided by a
  * per-row positive scale (dy[m,:] = dy_f16[m,:] * dy_row_scale[m]; NULL scale = 1), which keeps
  * 11 significant bits for gradients of any magnitude.  Writes (or, with accumulate, adds to)
- * dx_f32_dev [t x in] and adds dA, dB into the adapter's gradient buffers. */
+ * dx_f32_dev [t x in] and adds dA, dB into the adapter's gradient buffers.  dx may lie over x, which
+ * then is overwritten after its last use; it may not lie over dy or the scales. */
 rt_status rt_linear_backward_dev(rt_linear* lin, const void* x_f16_dev, const void* dy_f16_dev,
                                  const float* dy_row_scale_dev, size_t t, float* dx_f32_dev, int accumulate);
 /* Host-buffer forms with the reference's exact signatures: Linear::forward(x, t) -> y and
