@@ -36,10 +36,15 @@ enum QKind : int {
   QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
   // Narrow tiles of packed weights in the forward direction, with the unpacked weights in TMEM: a thread that owns a
   // weight row is the TMEM lane the MMA reads it from, and the weight tile no longer passes through shared
-  // memory twice.  1024x3072 at 1024 tokens 18.7 -> 16.5 us, at 640 the same.  (Backward reads the
+  // memory twice.  1024x4096 in Q8_0 at 157 tokens 7.0 us, on slim pairs 8.2; at 64 tokens 5.8 and 6.5.  (Backward reads the
   // bricks down their columns: only the shared-memory operand can be read transposed.  Half tiles leave half of the
-  // lanes, and so of the unpack warps, without a row: 25 us.)
+  // lanes, and so of the unpack warps, without a row.)
   QK_NARROW_T = 4,
+  // A CTA pair per tile of 128 weight rows x up to 128 tokens: 64 rows of weights and half of the tokens in each CTA, so that a CTA
+  // unpacks, writes and hands to the tensor core half the weights of a narrow tile for the same number of results.
+  // What bounds a narrow tile is shared memory: 128 rows written and read, 64 tokens written and read, the codes in and out,
+  // about 460 cycles of its 128 bytes a cycle for each 64 contraction elements, against 290 here.
+  QK_SLIM = 5,
 };
 // How the results leave: a kernel holds the code of one way only (all of them in one kernel cost the small
 // launches 0.4 us each in instruction fetches and the f16 epilogue of a pair registers, 5 % of the
@@ -57,11 +62,11 @@ constexpr int QF_16CONV = 1;   // 16-bit weights of the other 16-bit type, conve
 // Shared-memory plan of one CTA.
 template <int KIND, int FMT>
 struct QCfg {
-  static constexpr bool PAIR = KIND == QK_PAIR, HALF = KIND == QK_HALF, NARROW = KIND == QK_NARROW || KIND == QK_NARROW_T;
+  static constexpr bool SLIM = KIND == QK_SLIM, PAIR = KIND == QK_PAIR || SLIM, HALF = KIND == QK_HALF, NARROW = KIND == QK_NARROW || KIND == QK_NARROW_T;
   static constexpr bool TM = KIND == QK_NARROW_T;  // unpacked weights in TMEM
   // Weight rows of the CTA's tile.  The MMA always takes 128: a half tile's upper 64 are whatever follows it in
   // shared memory, and their accumulator lanes are not read.
-  static constexpr int ROWS = HALF ? 64 : 128, BRICKS = ROWS / 64;
+  static constexpr int ROWS = HALF || SLIM ? 64 : 128, BRICKS = ROWS / 64;
   static constexpr int W_SUB = ROWS * 128;  // bytes of a [ROWS x 64] 16-bit weight tile
   static constexpr bool PACKED = FMT > QF_16CONV;
   static constexpr bool WIDE = KIND == QK_WIDE;
@@ -74,12 +79,12 @@ struct QCfg {
   static constexpr int THREADS = 32 * (7 + NUW + (TM ? 1 : 0));
   // 64-element contraction steps per stage.  Two for narrow and half tiles: their MMAs are short, and one
   // hand-off between the roles costs about 500 cycles whatever it hands over.
-  static constexpr int KS = NARROW || HALF ? 2 : 1;
+  static constexpr int KS = NARROW || HALF || SLIM ? 2 : 1;
   // Activation / unpacked-weight stages, and packed-brick stages in the room that is left beside them and
   // the epilogue staging.
   static constexpr int NS = PAIR ? (PACKED ? 5 : 6) : WIDE ? 3 : HALF || TM ? 4 : PACKED ? 3 : 4;
   static constexpr int RAW_STAGE = PACKED ? KS * BRICKS * fmt_brick_bytes(FMT) : 0;
-  static constexpr int ACT_SUB = PAIR ? 16384 : WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
+  static constexpr int ACT_SUB = KIND == QK_PAIR ? 16384 : WIDE ? 32768 : 8192;  // tokens of the CTA's tile x 64 x 16-bit
   static constexpr int ACT_STAGE = KS * ACT_SUB;
   static constexpr int W_BYTES = (TM ? 1 : KS) * W_SUB;    // weights of a stage (in TMEM: the low-rank step's only)
   // TMEM columns of a stage's unpacked weights, beside the two accumulators of up to 64 columns at 0 and 256
@@ -98,10 +103,12 @@ struct QCfg {
   // that lands late cannot be taken for the one after it.
   static constexpr int UG = PAIR ? 4 : 2;                  // a power of two
   static constexpr int UTG = NUW * 32 / UG;                // threads per group
-  static_assert(UG <= NS && (!PACKED || NS <= NR + 1), "unpack groups would alias barrier phases");
+  static_assert(UG <= NS && (!PACKED || (NS <= NR + 1 && UG <= NR)), "unpack groups would alias barrier phases");
   // A thread of a group owns one unit of each half of a weight tile; with a group of twice the threads (wide tiles) of one half.
   static constexpr int HALVES = WIDE ? 1 : BRICKS;
-  static_assert(!PACKED || UTG == KS * 128 * (BRICKS / HALVES), "the group's threads cover a stage's units");
+  // A group of fewer threads than that goes over the stage's 64-element tiles one after the other.
+  static constexpr int PASSES = KS * 128 * (BRICKS / HALVES) / UTG;
+  static_assert(!PACKED || PASSES * UTG == KS * 128 * (BRICKS / HALVES), "the group's threads cover a stage's units");
   static constexpr int OFF_W = NS * ACT_STAGE;
   static constexpr int OFF_RAW = OFF_W + NS * W_BYTES;
   static constexpr int OFF_OUT = (OFF_RAW + NR * RAW_STAGE + 1023) / 1024 * 1024;  // (a swizzled store's source starts on its pattern)
@@ -270,7 +277,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
              const __grid_constant__ CUtensorMap tm_lact, const __grid_constant__ CUtensorMap tm_lw,
              const __grid_constant__ CUtensorMap tm_out, const KParams p) {
   using C = QCfg<KIND, FMT>;
-  constexpr bool PAIR = C::PAIR, TM = C::TM, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
+  constexpr bool PAIR = C::PAIR, SLIM = C::SLIM, TM = C::TM, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
   constexpr int NS = C::NS, NR = C::NR, UG = C::UG, UTG = C::UTG, KS = C::KS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -343,7 +350,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
 // first weight row (output feature) of this CTA's half of the tile, first token of the tile
 #define QG_TILE_ORIGIN()                                                                      \
   const int t_in = tile % p.inner, t_out = tile / p.inner;                                     \
-  const int r0 = (PAIR && p.tok_first ? t_out : t_in) * (C::ROWS * n_cta) + (int)rank * 128;   \
+  const int r0 = (PAIR && p.tok_first ? t_out : t_in) * (C::ROWS * n_cta) + (int)rank * C::ROWS;   \
   const int m0 = (PAIR && p.tok_first ? t_in : t_out) * p.TN
 
   if (threadIdx.x == 0) {
@@ -375,8 +382,16 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  // barriers, TMEM and descriptors are set up; from here on the kernel reads what its predecessor wrote
-  if (!p.late_wait) pdl_wait();
+  // barriers, TMEM and descriptors are set up; from here on the kernel reads what its predecessor wrote.  Packed weights
+  // no kernel of a pass writes: their bricks are fetched and unpacked under the predecessor's end.
+  const bool weights_only = PACKED && (role == R_RAW || role == R_UNPACK);
+  if (!p.late_wait && !weights_only) pdl_wait();
+
+  // Where the 32 accumulator lanes of quarter wq belong.  A slim pair's accumulator has 64 rows in each CTA: lanes 0..63 hold
+  // them for the tile's first half of the tokens, lanes 64..127 for the second, in half as many columns.
+  const int tn_q = SLIM ? p.TN >> 1 : p.TN;  // tokens (columns) of a quarter
+  auto q_row = [&](int wq) { return SLIM ? (wq & 1) * 32 : wq * 32; };
+  auto q_tok = [&](int wq) { return SLIM ? (wq >> 1) * tn_q : 0; };
 
   // One [32 tokens x 32 features] block of a 16-bit output -> staging -> TMA store.  `stage_base` is
   // private to the calling warp; a block of it is reused only after the store that read it is done.
@@ -395,7 +410,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     float2 rs[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int tok = m0 + c * 32 + 8 * k + 2 * (lane & 3);
+      const int tok = m0 + q_tok(wq) + c * 32 + 8 * k + 2 * (lane & 3);
       rs[k] = make_float2(1.f, 1.f);
       if (p.row_scale) {
         rs[k].x = tok < p.M ? p.row_scale[tok] : 0.f;
@@ -406,7 +421,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     if (p.bias) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const int row = r0 + wq * 32 + 8 * e + (lane >> 2);
+        const int row = r0 + q_row(wq) + 8 * e + (lane >> 2);
         bv[e] = row < p.out_rows ? p.bias[row] : 0.f;
       }
     }
@@ -436,7 +451,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {
-      tma_store_2d(&tm_out, r0 + wq * 32, m0 + c * 32, stage);
+      tma_store_2d(&tm_out, r0 + q_row(wq), m0 + q_tok(wq) + c * 32, stage);
       bulk_commit_group();
     }
   };
@@ -449,12 +464,12 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   // instructions per value: whole blocks take straight-line code without a test per value (with one,
   // the same product took 135 us).
   auto direct_chunk = [&](int acc, int wq, int c, int r0, int m0, int split) {
-    if (m0 + c * 32 >= p.M) return;
+    const int tok0 = m0 + q_tok(wq) + c * 32, row = r0 + q_row(wq) + lane;
+    if (tok0 >= p.M) return;
     uint32_t v[32];
     tmem_ld32(tmem_base + acc * 256 + ((uint32_t)(wq * 32) << 16) + c * 32, v);
-    const int tok0 = m0 + c * 32, row = r0 + wq * 32 + lane;
     const bool row_ok = row < p.out_rows;
-    const int nvalid = min(32, p.M - tok0);
+    const int nvalid = min(min(32, tn_q - c * 32), p.M - tok0);
     const bool fin_out = p.part == nullptr;  // partial sums are scaled, biased and added up by the reduce kernel
     float rs_lane = 1.0f;
     if (fin_out && p.row_scale) rs_lane = lane < nvalid ? p.row_scale[tok0 + lane] : 0.f;
@@ -468,8 +483,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     const size_t ld = fin_out ? (size_t)p.ld_out : (size_t)p.out_rows;
     const size_t base = fin_out ? (size_t)tok0 * ld + row : ((size_t)split * p.M + tok0) * ld + row;
     float* o = (fin_out ? (float*)p.out : p.part) + base;
-    if (nvalid == 32 && (!fin_out || (p.out_dtype == OUT_F32 && (!PAIR || !p.residual)))) {
-      if (!PAIR && fin_out && p.residual) {
+    if (nvalid == 32 && (!fin_out || (p.out_dtype == OUT_F32 && (KIND != QK_PAIR || !p.residual)))) {
+      if (KIND != QK_PAIR && fin_out && p.residual) {
         const float* res = p.residual + base;
 #pragma unroll
         for (int q = 0; q < 32; q += 8) {  // eight loads in flight: what the registers have room for
@@ -578,7 +593,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   const int q_res = warp & 3;
   const int q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
   auto tail_helper = [&](int turn, int hslot) {
-    if (n_my == 0 || q_res * 32 >= C::ROWS) return;
+    if (n_my == 0 || (!SLIM && q_res * 32 >= C::ROWS)) return;
+    if (!p.late_wait && weights_only) pdl_wait();
     const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
     QG_ITEM_DECODE(item);
     (void)s_begin; (void)n_steps; (void)s_main;
@@ -593,7 +609,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       residual_tile(acc, q_res, turn, q_turns, r0, m0, stage);
       return;
     }
-    for (int c = turn; c < p.TN / 32; c += q_turns) {
+    for (int c = turn; c * 32 < tn_q; c += q_turns) {
       if (OUT == QO_TMA16) tma_chunk(acc, q_res, c, r0, m0, smem + hslot * 8192, cnt);
       else direct_chunk(acc, q_res, c, r0, m0, split);
     }
@@ -744,91 +760,98 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       const UnitDst ud(tg & 127);
       const uint32_t w_base = smem_u32(sW);
       constexpr int BB = PACKED ? C::RAW_STAGE / (C::BRICKS * KS) : 0;  // bytes of a brick
-      int st = 0, rs = 0, turn = 0;  // ring positions of the current step, and the group whose step it is
+      // A group goes straight from one of its steps to the next, UG further on in the rings: counting through the other
+      // groups' steps took a third of its time (6144x1024 Q4_0 backward at 1024 tokens on narrow tiles 31 -> 26 us).
+      int st = grp, rs = grp, s = grp;  // ring positions of the group's step, and its number within the item
       uint32_t ph = 0, rph = 0;
       bool ok = true;
       for (int item = worker; item < n_items && ok; item += n_workers) {
         QG_ITEM_DECODE(item);
         (void)tile; (void)s_begin;
-        for (int s = 0; s < n_steps; ++s) {
+        for (; s < n_steps; s += UG) {
           const bool main_step = s < n_main_st;
-          if (turn == grp) {
-            const int subs = KS == 1 ? 1 : min(KS, s_main - s * KS);
-            if (!mbar_wait(&stage_empty[st], ph ^ 1, p.status, 201)) { ok = false; break; }
-            if (CONV && main_step) {
-              // the TMA'd 16-bit weight tile has the other 16-bit type: convert it in place
-              // (element-wise, so the swizzled placement is untouched)
-              if (!mbar_wait(&full[st], ph, p.status, 203)) { ok = false; break; }
-              uint4* tile16 = (uint4*)(sW + st * C::W_BYTES);
-              for (int i = 0; i < subs * (C::W_SUB / 16) / UTG; ++i) {
-                uint4 v = tile16[tg + i * UTG];
-                uint32_t* w = (uint32_t*)&v;
+          const int subs = KS == 1 ? 1 : min(KS, s_main - s * KS);
+          if (!mbar_wait(&stage_empty[st], ph ^ 1, p.status, 201)) { ok = false; break; }
+          if (CONV && main_step) {
+            // the TMA'd 16-bit weight tile has the other 16-bit type: convert it in place
+            // (element-wise, so the swizzled placement is untouched)
+            if (!mbar_wait(&full[st], ph, p.status, 203)) { ok = false; break; }
+            uint4* tile16 = (uint4*)(sW + st * C::W_BYTES);
+            for (int i = 0; i < subs * (C::W_SUB / 16) / UTG; ++i) {
+              uint4 v = tile16[tg + i * UTG];
+              uint32_t* w = (uint32_t*)&v;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  if (p.conv16 == 1) {
-                    __nv_bfloat162 b = __float22bfloat162_rn(__half22float2(*(__half2*)&w[j]));
-                    w[j] = *(uint32_t*)&b;
-                  } else {
-                    __half2 h = __float22half2_rn(__bfloat1622float2(*(__nv_bfloat162*)&w[j]));
-                    w[j] = *(uint32_t*)&h;
-                  }
-                }
-                tile16[tg + i * UTG] = v;
-              }
-              fence_proxy_async_smem();
-            }
-            if (TM && main_step) {
-              // one of the group's two warps per lane quarter takes each of the stage's two steps; a thread unpacks the
-              // 64 codes of its weight row, which it is the TMEM lane of
-              if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
-              tc_fence_after();
-              const int row = (warp & 3) * 32 + lane, u = uidx & 1;
-              if (u < subs) {
-                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + u * BB + (row >> 6) * (KS * BB);
-                const uint32_t dst = tmem_base + C::a_col(st) + ((uint32_t)((warp & 3) * 32) << 16) + u * 32;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  uint32_t o[16];
-                  if (p.act_f16) unpack_unit<FMT, false, true>(raw, 2 * (row & 63) + h, 0, ud, o);
-                  else unpack_unit<FMT, true, true>(raw, 2 * (row & 63) + h, 0, ud, o);
-                  tmem_st16(dst + h * 16, o);
-                }
-                tmem_st_wait();
-              }
-              tc_fence_before();
-            } else if (PACKED && main_step) {
-              if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
-              // two bricks per 64-element tile: brick b fills the 8 KB half b.  A stage of two tiles goes to the
-              // two halves of the group.
-              const int u = C::WIDE ? 0 : tg >> 7, half = C::WIDE ? tg >> 7 : 0;
-              if (u < subs) {
-                const int next = p.dir == QG_FWD ? KS * BB : BB;
-                const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : C::BRICKS * u * BB) + half * next;
-                const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB + (uint32_t)half * 8192;
-                if (p.act_f16) {
-#pragma unroll
-                  for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, false, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+              for (int j = 0; j < 4; ++j) {
+                if (p.conv16 == 1) {
+                  __nv_bfloat162 b = __float22bfloat162_rn(__half22float2(*(__half2*)&w[j]));
+                  w[j] = *(uint32_t*)&b;
                 } else {
-#pragma unroll 1
-                  for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, true, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+                  __half2 h = __float22half2_rn(__bfloat1622float2(*(__nv_bfloat162*)&w[j]));
+                  w[j] = *(uint32_t*)&h;
                 }
               }
-              fence_proxy_async_smem();
+              tile16[tg + i * UTG] = v;
             }
-            // one arrival per warp, after every lane's writes are fenced towards the tensor core's
-            // reads; then the brick slot, which every lane has read, goes back to its producer
-            __syncwarp();
-            if (lane == 0) {
-              if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&full[st]), 0));
-              else if (PACKED) mbar_arrive(&full[st]);
-              else mbar_arrive(&w_ready[st]);
-              if (PACKED && main_step) mbar_arrive(&raw_empty[rs]);
-            }
+            fence_proxy_async_smem();
           }
-          turn = (turn + 1) & (UG - 1);
-          if (++st == NS) { st = 0; ph ^= 1; }
-          if (PACKED && main_step && ++rs == NR) { rs = 0; rph ^= 1; }
+          if (TM && main_step) {
+            // one of the group's two warps per lane quarter takes each of the stage's two steps; a thread unpacks the
+            // 64 codes of its weight row, which it is the TMEM lane of
+            if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
+            tc_fence_after();
+            const int row = (warp & 3) * 32 + lane, u = uidx & 1;
+            if (u < subs) {
+              const uint8_t* raw = sRaw + rs * C::RAW_STAGE + u * BB + (row >> 6) * (KS * BB);
+              const uint32_t dst = tmem_base + C::a_col(st) + ((uint32_t)((warp & 3) * 32) << 16) + u * 32;
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                uint32_t o[16];
+                if (p.act_f16) unpack_unit<FMT, false, true>(raw, 2 * (row & 63) + h, 0, ud, o);
+                else unpack_unit<FMT, true, true>(raw, 2 * (row & 63) + h, 0, ud, o);
+                tmem_st16(dst + h * 16, o);
+              }
+              tmem_st_wait();
+            }
+            tc_fence_before();
+          } else if (PACKED && main_step) {
+            if (!mbar_wait(&raw_full[rs], rph, p.status, 202)) { ok = false; break; }
+            // two bricks per 64-element tile: brick b fills the 8 KB half b.  A stage of two tiles goes to the
+            // two halves of the group.
+#pragma unroll
+            for (int pass = 0; pass < C::PASSES; ++pass) {
+              const int u = C::WIDE ? 0 : (tg >> 7) + pass, half = C::WIDE ? tg >> 7 : 0;
+              if (u >= subs) break;
+              const int next = p.dir == QG_FWD ? KS * BB : BB;
+              const uint8_t* raw = sRaw + rs * C::RAW_STAGE + (p.dir == QG_FWD ? u * BB : C::BRICKS * u * BB) + half * next;
+              const uint32_t dst = w_base + (uint32_t)st * C::W_BYTES + (uint32_t)u * C::W_SUB + (uint32_t)half * 8192;
+              if (p.act_f16) {
+#pragma unroll
+                for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, false, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+              } else {
+#pragma unroll 1
+                for (int b = 0; b < C::HALVES; ++b) unpack_unit<FMT, true, false>(raw + b * next, tg & 127, dst + b * 8192, ud, nullptr);
+              }
+            }
+            fence_proxy_async_smem();
+          }
+          // one arrival per warp, after every lane's writes are fenced towards the tensor core's
+          // reads; then the brick slot, which every lane has read, goes back to its producer
+          __syncwarp();
+          if (lane == 0) {
+            if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&full[st]), 0));
+            else if (PACKED) mbar_arrive(&full[st]);
+            else mbar_arrive(&w_ready[st]);
+            if (PACKED && main_step) mbar_arrive(&raw_empty[rs]);
+          }
+          st += UG;
+          if (st >= NS) { st -= NS; ph ^= 1; }
+          if (PACKED) {
+            rs += UG;
+            if (rs >= NR) { rs -= NR; rph ^= 1; }
+          }
         }
+        s -= n_steps;  // the next item's
+        if (PACKED && n_steps > n_main_st && --rs < 0) { rs += NR; rph ^= 1; }  // a low-rank step takes a stage but no bricks
       }
     }
     if (warp < 15) tail_helper(warp >> 2, warp - 4);
@@ -881,14 +904,14 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
       const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
-      const bool mine = wq * 32 < C::ROWS;
+      const bool mine = SLIM || wq * 32 < C::ROWS;
       const uint32_t stage = smem_u32(sOut + wq * C::OUT_WARP);
       if (OUT == QO_RES && mine) residual_start(wq, 0, stride, r0, m0, stage);
       if (!mbar_wait(&acc_full[acc], aph, p.status, 401)) break;
       tc_fence_after();
       if (OUT == QO_RES) {
         if (mine) residual_tile(acc, wq, 0, stride, r0, m0, stage);
-      } else for (int c = mine ? 0 : p.TN; c < p.TN / 32; c += stride) {
+      } else for (int c = mine ? 0 : p.TN; c * 32 < tn_q; c += stride) {
         if (OUT == QO_TMA16) tma_chunk(acc, wq, c, r0, m0, sOut + wq * C::OUT_WARP, out_chunk);
         else direct_chunk(acc, wq, c, r0, m0, split);
       }
@@ -959,7 +982,7 @@ static QKernel qkernel() {
 template <int KIND, int OUT>
 static QKernel qkernel_fmt(int fmt) {
   constexpr bool TM = KIND == QK_NARROW_T;
-  if constexpr (KIND != QK_PAIR && !TM) {
+  if constexpr (KIND != QK_PAIR && KIND != QK_SLIM && !TM) {
     if (fmt == QF_16CONV) return qkernel<KIND, QF_16CONV, OUT>();
   }
   if constexpr (!TM) {
@@ -981,6 +1004,7 @@ static QKernel qkernel_for(int kind, int fmt, int out) {
     case QK_NARROW: return t ? qkernel_fmt<QK_NARROW, QO_TMA16>(fmt) : qkernel_fmt<QK_NARROW, QO_DIRECT>(fmt);
     case QK_NARROW_T: return t ? qkernel_fmt<QK_NARROW_T, QO_TMA16>(fmt) : qkernel_fmt<QK_NARROW_T, QO_DIRECT>(fmt);
     case QK_HALF: return t ? qkernel_fmt<QK_HALF, QO_TMA16>(fmt) : qkernel_fmt<QK_HALF, QO_DIRECT>(fmt);
+    case QK_SLIM: return t ? qkernel_fmt<QK_SLIM, QO_TMA16>(fmt) : qkernel_fmt<QK_SLIM, QO_DIRECT>(fmt);
   }
   return {nullptr, 0, 0};
 }
@@ -997,7 +1021,7 @@ int qgemm_init() {
     g_encode = (PFN_encodeTiled)fn;
   }
   auto raise_smem = [](bool wide) {  // wide tiles of weights that are not converted: only where there are no pairs
-    for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF, (int)QK_NARROW_T})
+    for (int kind : {(int)QK_PAIR, (int)QK_WIDE, (int)QK_NARROW, (int)QK_HALF, (int)QK_NARROW_T, (int)QK_SLIM})
       for (int fmt : {QF_16, QF_16CONV, (int)GGML_Q4_0, (int)GGML_Q8_0, (int)GGML_Q4_K, (int)GGML_Q6_K})
         for (int out : {(int)QO_TMA16, (int)QO_DIRECT, (int)QO_RES}) {
           if ((kind == QK_WIDE && fmt != QF_16CONV) != wide) continue;
@@ -1113,50 +1137,48 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 }
 
 // Which kernel and token-tile width a product gets: the one whose persistent grid is estimated to finish
-// first, rounds of tiles x (contraction steps x the step's time + a tile's fixed time).  The step times
-// (us, 64 contraction elements) are fitted to sweeps over the kernels and all widths: about 0.33 for a pair
-// while the single-thread roles and the unpack passes set the pace, more from about 64 tokens of width per
-// CTA on, when the MMAs do; 0.25 for narrow tiles, which hand over two steps at a time, and 0.16 for half
-// tiles, whose unpack passes are half as long.  They are a fit to what wins, not each kernel's own pace: one
-// round of narrow tiles from TMEM takes 0.23 a step, and a pair's fixed time is rather 1.7 than 0.5.  With
-// that 1.7 the choices below are better (0.6 % off, 13 by more than 10 %), but 2560 -> 9728 at 300 tokens goes to three
-// rounds of narrow tiles, 31 -> 38 us in Q8_0 (0.28 a step) and 36 -> 46 in Q6_K.
-// Against the best kind and width of each of 1434 products (15 shapes of 64..9728 -> 128..8192, both directions,
-// 1..12000 tokens, Q8_0, Q6_K and F16) the choice is 0.8 % off on average and 31 are off by more than 10 %, all
-// of them launches of 5 to 10 us: short contractions that pairs get and narrow tiles finish first (25 % at worst, 64 -> 1024
-// at 1500 tokens 7.2 us against 5.6).
-// Narrow and half tiles win while the wider ones leave SMs idle (few tokens or few output rows): 6144x1024
-// backward at 1024 tokens 29 us (44 on pairs of 128 tokens before), 8192x3072 Q6_K backward at 24 tokens 30 us
-// (43 on narrow tiles, 91 before), 1024x2048 at 157 tokens 9.6 us (12).
+// first: the launch + rounds of tiles x (contraction steps x the step's time + a tile's own time).  The constants (us, 64
+// contraction elements a step) are fitted to times of every kind and width for 576 products (9 shapes of 128..8192 rows and
+// columns, both directions, 3..2048 tokens, four formats, weights from memory, launches that follow each other
+// programmatically); the launches of the pair kinds are given 1 to 2 us more than the fit, which they lose behind other
+// kernels than themselves.  What a step's time stands for: a pair's for its MMAs from about 200 tokens of width on and
+// for the hand-offs between the roles below; a slim pair's for shared memory; the narrow kinds' for one round of unpacking.
+// Slim pairs came in where narrow tiles ran before, at 1024 tokens (Q4_0 | Q6_K, the same unpack loop on both
+// sides): 6144x1024 backward 26.0 -> 18.8 | 30.3 -> 20.5 us, 4096x1024 backward 19.0 -> 14.7 | 21.7 -> 15.8,
+// 1024x3072 forward 14.0 -> 12.3 | 15.7 -> 13.3; 8192x3072 Q6_K backward at 24 tokens 24.5 -> 22.1 (half tiles before).
 // The choice changes no result: an output element's contraction is one chain in any tile.
 struct QPlan {
   int kind, TN;
 };
-static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, int steps, int num_sms) {
+static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, int steps, int num_sms, bool out16) {
   QPlan best = {QK_NARROW, 64};
   double best_cost = -1;
-  auto consider = [&](int kind, int tn, double step_us) {
+  auto consider = [&](int kind, int tn, double step_us, double tile_us, double launch_us) {
     const int rows = kind == QK_PAIR ? 256 : kind == QK_HALF ? 64 : 128;
     const long tiles = (long)((out_rows + rows - 1) / rows) * ((M + tn - 1) / tn) * n_splits;
-    const long workers = kind == QK_PAIR ? g_pair_workers : num_sms;
-    const double cost = (double)((tiles + workers - 1) / workers) * (steps * step_us + 0.5);
+    const long workers = kind == QK_PAIR || kind == QK_SLIM ? g_pair_workers : num_sms;
+    const double cost = launch_us + (double)((tiles + workers - 1) / workers) * (steps * step_us + tile_us);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {kind, tn}; }
   };
-  const bool tm = kfmt > QF_16CONV && dir == QG_FWD;
-  const int narrow = tm ? QK_NARROW_T : QK_NARROW;
-  if (M > 32) consider(narrow, 64, 0.25);
-  consider(narrow, 32, 0.25);
-  if (M > 32) consider(QK_HALF, 64, 0.16);
-  consider(QK_HALF, 32, 0.155);
-  if (kfmt == QF_16CONV) {
-    for (int tn = 256; tn >= 128; tn -= 32) consider(QK_WIDE, tn, 0.25 + 0.0012 * tn);
-  } else if (g_pair_workers > 0 && M > 64) {
-    for (int tn = 256; tn >= 64; tn -= 32) {
-      const double mma = 0.29 + 0.00064 * tn;
-      consider(QK_PAIR, tn, mma > 0.335 ? mma : 0.335);
+  const bool packed = kfmt > QF_16CONV;
+  if (kfmt == QF_16CONV) {  // single CTAs only: their warps convert what TMA brought
+    for (int tn = M > 32 ? 64 : 32; tn >= 32; tn -= 32) {
+      consider(QK_NARROW, tn, 0.25, 0.5, 0);
+      consider(QK_HALF, tn, tn == 64 ? 0.16 : 0.155, 0.5, 0);
     }
+    for (int tn = 256; tn >= 128; tn -= 32) consider(QK_WIDE, tn, 0.25 + 0.0012 * tn, 0.5, 0);
+    return best;
+  }
+  for (int tn = M > 32 ? 64 : 32; tn >= 32; tn -= 32) {
+    if (packed && dir == QG_FWD) consider(QK_NARROW_T, tn, 0.2, 0.4, 2.5);
+    else consider(QK_NARROW, tn, 0.23, 0.7, 2.3);
+    consider(QK_HALF, tn, 0.19, 0.6, 2.1);
+  }
+  if (g_pair_workers > 0) {
+    for (int tn = M > 64 ? 128 : M > 32 || out16 ? 64 : 32; tn >= (out16 ? 64 : 32); tn /= 2) consider(QK_SLIM, tn, 0.16, 0.9, 4.6);
+    for (int tn = 256; tn >= 64 && M > 64; tn -= 32) consider(QK_PAIR, tn, 0.165 + 0.0008 * tn > 0.3 ? 0.165 + 0.0008 * tn : 0.3, 0.4, 5.5);
   } else if (M > 64) {  // without pairs: 8192x3072 Q8_0 at 4096 tokens 171-181 us, 279-341 on 64-token tiles
-    for (int tn = 256; tn >= 96; tn -= 32) consider(QK_WIDE, tn, 0.15 + 0.0012 * tn > 0.35 ? 0.15 + 0.0012 * tn : 0.35);
+    for (int tn = 256; tn >= 96; tn -= 32) consider(QK_WIDE, tn, 0.15 + 0.0012 * tn > 0.35 ? 0.15 + 0.0012 * tn : 0.35, 0.5, 2.4);
   }
   return best;
 }
@@ -1211,22 +1233,23 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   if (a.out_dtype == OUT_F32 && p.n_main > 256) p.steps_per_split = 128;
   p.n_splits = (p.n_main + p.steps_per_split - 1) / p.steps_per_split;
 
-  const QPlan plan = qgemm_plan(kfmt, a.dir, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms);
-  const bool pair = plan.kind == QK_PAIR;
+  const QPlan plan = qgemm_plan(kfmt, a.dir, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms,
+                                a.out_dtype != OUT_F32);
+  const bool pair = plan.kind == QK_PAIR || plan.kind == QK_SLIM;
   p.TN = plan.TN;
-  const int tile_rows = pair ? 256 : plan.kind == QK_HALF ? 64 : 128;
+  const int tile_rows = plan.kind == QK_PAIR ? 256 : plan.kind == QK_HALF ? 64 : 128;
   p.n_row_tiles = (out_rows + tile_rows - 1) / tile_rows;
   p.n_tok_tiles = (a.M + p.TN - 1) / p.TN;
   // Tiles that run together share a token tile's activations; but weights that do not fit beside them in L2 (126 MB)
   // come from memory again for every token tile (the head's 151936x1024 in Q8_0 at 1024 tokens: 664 MB read for
   // 165), so then the token tiles of the same weights run together, while the activations do fit.  128256x3072 in Q6_K at
   // 1024 tokens 631 -> 609 us; at 87 MB of weights, which stay in L2, the other order is the better one by a little.
-  p.tok_first = p.n_tok_tiles > 1 && w.dev_nbytes > ((size_t)96 << 20) && (size_t)a.M * contract * 2 <= ((size_t)32 << 20) && pair;
+  p.tok_first = p.n_tok_tiles > 1 && w.dev_nbytes > ((size_t)96 << 20) && (size_t)a.M * contract * 2 <= ((size_t)32 << 20) && plan.kind == QK_PAIR;
   p.inner = p.tok_first ? p.n_tok_tiles : p.n_row_tiles;
   const int tn_cta = pair ? p.TN / 2 : p.TN;  // each CTA of a pair fetches its half of the token tile
   // tcgen05.mma kind::f16 needs A and B of ONE 16-bit type (f16 x bf16 is an illegal instruction).
   const int ab_fmt = a.act_f16 ? 0 : 1;
-  p.idesc = umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, pair ? 256 : 128, p.TN);
+  p.idesc = umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, plan.kind == QK_PAIR ? 256 : 128, p.TN);
 
   CUtensorMap tm_act, tm_w16, tm_lact, tm_lw;
   int rc = make_map(&tm_act, a.act, (uint64_t)a.M, (uint64_t)contract, 64, (uint32_t)tn_cta, !a.act_f16);
@@ -1257,10 +1280,11 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     }
   }
   int out_kind = QO_DIRECT;
-  if (pair && !p.part && a.residual && (uintptr_t)a.residual % 16 == 0 && p.ld_out % 4 == 0 && out_rows % 4 == 0) out_kind = QO_RES;
+  if (plan.kind == QK_PAIR && !p.part && a.residual && (uintptr_t)a.residual % 16 == 0 && p.ld_out % 4 == 0 && out_rows % 4 == 0) out_kind = QO_RES;
   // 16-bit outputs leave through TMA whenever it can address them (16-byte aligned base and row pitch)
   CUtensorMap tm_out = tm_act;
-  if (!p.part && a.out_dtype != OUT_F32 && (uintptr_t)a.out % 16 == 0 && (uint64_t)p.ld_out % 8 == 0) {
+  const bool out_blocks = plan.kind != QK_SLIM || p.TN >= 64;  // a quarter of the accumulator is whole blocks of 32 tokens
+  if (!p.part && out_blocks && a.out_dtype != OUT_F32 && (uintptr_t)a.out % 16 == 0 && (uint64_t)p.ld_out % 8 == 0) {
     rc = make_out_map(a.fixed_part ? nullptr : ctx, &tm_out, a.out, (uint64_t)a.M, (uint64_t)out_rows, (uint64_t)p.ld_out, a.out_dtype);
     if (rc) return rc;
     out_kind = QO_TMA16;

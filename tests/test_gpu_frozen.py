@@ -226,6 +226,36 @@ def test_a_row_gets_the_same_bits_in_any_batch(ctx, t, n, k, big):
     f.close()
 
 
+@pytest.mark.parametrize("t", [Q.Q4_0, Q.Q8_0, Q.Q6_K], ids=lambda t: Q.NAMES[t])
+@pytest.mark.parametrize("m", [1, 32, 33, 64, 65, 127, 128, 129, 250])
+def test_slim_pair_tiles_at_their_edges(ctx, t, m):
+    """Tiles of 128 weight rows over a CTA pair whose accumulator holds the two halves of the tokens in the two halves of its
+    lanes: tokens that end inside a tile, at its half and inside a block, rows that end inside a tile and inside a CTA's half,
+    an odd number of contraction steps; f32, 16-bit and accumulated results."""
+    import torch
+
+    from rust_trainer_b200._lib import DT_BF16, DT_F16, DT_F32, lib
+
+    L, n, k = lib(), 2 * 128 + 72, 1280 if t == Q.Q6_K else 19 * 64  # long enough for slim pairs to be the choice
+    g = torch.Generator(device="cuda").manual_seed(m)
+    packed = Q.quantize((np.random.default_rng(m).standard_normal((n, k)) * 0.05).astype(np.float32), t)
+    f = rt.Frozen(ctx, t, n, k, packed)
+    x, dy = (torch.randn(m, c, generator=g, device="cuda").half() for c in (k, n))
+    y, dx0 = (torch.randn(m + 1, c, generator=g, device="cuda") for c in (n, k))  # one guard row behind the results
+    y16, dx, guard = torch.full((m + 1, n), 7.0, device="cuda").bfloat16(), dx0.clone(), y[m].clone()
+    torch.cuda.synchronize()
+    ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, m, y.data_ptr(), DT_F32, 0))
+    ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, m, y16.data_ptr(), DT_BF16, 0))
+    ctx.check(L.rt_frozen_backward_input_dev(f._h, dy.data_ptr(), DT_F16, m, dx.data_ptr(), DT_F32, 1))
+    ctx.synchronize()
+    w = torch.from_numpy(O.dequant_rows(t, packed, n, k)).cuda().double()
+    assert rel_l2(y[:m].cpu().numpy(), (x.double() @ w.T).cpu().numpy()) < MATMUL_TOL
+    assert rel_l2((dx - dx0)[:m].cpu().numpy(), (dy.double() @ w).cpu().numpy()) < MATMUL_TOL
+    assert torch.equal(y16[:m], y[:m].bfloat16())
+    assert torch.equal(y[m], guard) and torch.equal(dx[m], dx0[m]) and bool((y16[m] == 7.0).all())
+    f.close()
+
+
 def test_results_in_locked_memory_are_the_callers(ctx):
     """Results of 64 KB and more lie in page-locked blocks of a bounded pool: a block is reused only after the last view of it
     is gone, and past the bound (256 MB) results come in ordinary memory."""
