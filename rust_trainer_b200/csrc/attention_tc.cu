@@ -416,7 +416,6 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   uint8_t* sm = smem_raw + (((raw + 1023u) & ~1023u) - raw);
-  pdl_launch_dependents();
   uint64_t* bars = (uint64_t*)(sm + L::OFF_BAR);
   constexpr int NS = L::NS;
   uint64_t* kv_full = bars + 0;
@@ -462,6 +461,8 @@ attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   pdl_wait();
+  // Only now: the dQ kernel behind this one runs beside it without a wait, and takes everything older as complete (pdl.cuh).
+  pdl_launch_dependents();
 
   bool ok = true;
   if (warp == BWD_TMA_WARP) {
@@ -771,7 +772,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
-  pdl_wait();
+  // no wait here: what this kernel reads was complete before the dK/dV kernel, in front of it, let it start
 
   if (warp == DQ_TMA_WARP) {
     if (elect_one()) {
@@ -919,6 +920,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     }
   }
 
+  pdl_wait();  // for dK/dV: whoever waits for this kernel has waited for both
   if (*(volatile int*)status != 0) {
     for (int k = 0; k < 1000; ++k) __nanosleep(1000);
   }
@@ -1044,8 +1046,11 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
   if (cudaLaunchKernelEx(&cfg, attn_bwd_dkdv_tc_kernel<HD>, tk128, tv128, tq64, tdo64, (const float*)tops, (const float*)query_vecs,
                          b.seq_start, gap, (const int2*)b.tiles_k, M, nh, nkv, hpc, n_ctas, scale, dk, dv, c->status_dev) != cudaSuccess)
     return 3;
-  pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st)(tq128, tdo128, tk64, tv64, row_scale, lse, query_vecs,
-                                                                               b.seq_start, gap, b.tiles_q, M, nh, nkv, scale, dq, c->status_dev);
+  // dQ reads nothing of dK/dV's: it starts as soon as that kernel's last CTAs have, in passes of every size.
+  PdlLaunch dq_launch = pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st);
+  dq_launch.programmatic = true;
+  if (dq_launch(tq128, tdo128, tk64, tv64, row_scale, lse, query_vecs, b.seq_start, gap, b.tiles_q, M, nh, nkv, scale, dq, c->status_dev) != cudaSuccess)
+    return 3;
   RT_COUNT_LAUNCH(3);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }

@@ -8,7 +8,7 @@
 //     brings along and no kernel writes (tile lists, where sequences start) may be read before it;
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
 //     every CTA of this one has started.
-// One pair of kernels departs from both.  A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
+// Two pairs of kernels depart from both.  (1) A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
 // weights, activations and residual without waiting and waits only where it loads the stream's result.  That
 // is sound because of what lowrank_tc_kernel and the matmul keep between them:
 //   - lowrank_tc_kernel triggers only after its own wait, so that everything older than it is complete and
@@ -16,6 +16,9 @@
 //   - it writes nothing the matmul reads but that result, and the matmul writes nothing it reads;
 //   - at least one CTA of the matmul waits (the last piece of a contraction always ends in the low-rank
 //     step), so that whoever waits for the matmul has waited for the stream.
+// (2) The attention's dQ kernel behind its dK/dV kernel, which it needs nothing from (attention_tc.cu): dK/dV triggers only
+// after its own wait, so that what both read is complete and visible; neither writes what the other reads or writes;
+// and every CTA of dQ waits before it ends, so that whoever waits for dQ has waited for both.
 // Inside stream capture these launches become programmatic edges of the graph.
 // Used for passes of up to PDL_MAX_TOKENS tokens, whose kernels leave SMs free for the next one's CTAs to
 // start on: the 28-layer 0.6B step 10.67 -> 10.14 ms at 1024 tokens, scoring 157 tokens 3.01 -> 2.84 ms.  At
@@ -58,6 +61,7 @@ struct PdlLaunch {
   dim3 grid, block;
   size_t smem;
   cudaStream_t st;
+  bool programmatic = pdl_enabled();
   template <typename... A>
   cudaError_t operator()(A&&... a) const {
     cudaLaunchConfig_t cfg = {};
@@ -67,7 +71,7 @@ struct PdlLaunch {
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = programmatic ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<A>(a))...);
