@@ -62,23 +62,13 @@ rt_status lora_refresh(rt_linear* l) {
   return RT_OK;
 }
 
-// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16
-// columns, so columns from `rank` up to the next multiple of 16 must hold zeros (or at least
-// finite values against zero weights; zeros keep it exact).  When the rank is not a multiple of
-// 16 the buffer is cleared on every call: a decision taken from what earlier calls left behind
-// would be frozen into a captured graph and replayed after a different history.  `cur_rank`
-// only records that the buffer has been cleared once since it was (re)allocated.
-static __half* lowrank_buf(rt_ctx* c, DevBuf& b, int& cur_rank, int M, int rank) {
+// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16 columns, and the zeros it needs
+// from the rank on come from lowrank_tc_kernel, which writes all 64 columns of every row.  New memory is cleared once, so that
+// what lies behind the last row is finite.  (The buffer was also cleared before every product whose rank is no multiple of 16:
+// up to five more links of 1.5 to 3 us in each layer's chain of launches.)
+static __half* lowrank_buf(DevBuf& b, int M) {
   const size_t want = (size_t)M * 64 * sizeof(__half);
-  bool clear = false;
-  if (want > b.bytes) {
-    if (!b.reserve(want + want / 2)) return nullptr;
-    clear = true;
-  }
-  if (cur_rank < 0 || rank % 16 != 0) clear = true;
-  if (clear) cudaMemsetAsync(b.p, 0, want, c->stream);
-  cur_rank = rank;
-  return b.as<__half>();
+  return b.reserve(want <= b.bytes ? want : want + want / 2, true) ? b.as<__half>() : nullptr;
 }
 
 rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out) {
@@ -105,7 +95,7 @@ rt_status linear_forward_dev(rt_linear* l, LinearScratch& sc, const __half* x16,
   if (l->lora_active()) {
     lora_refresh(l);
     const int r = l->lora.rank;
-    __half* hs = hs_keep ? hs_keep : lowrank_buf(c, sc.hs, sc.hs_rank, M, r);
+    __half* hs = hs_keep ? hs_keep : lowrank_buf(sc.hs, M);
     if (!hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     if (!(hs_keep && hs_ready)) {
       RT_TRY(linear_lora_h(l, x16, M, hs));
@@ -157,8 +147,8 @@ rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16
   if (lora) {
     lora_refresh(l);
     const int r = l->lora.rank;
-    __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(c, sc.hs, sc.hs_rank, M, r);
-    __half* gs = lowrank_buf(c, sc.gs[sc.n_jobs], sc.gs_rank[sc.n_jobs], M, r);
+    __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(sc.hs, M);
+    __half* gs = lowrank_buf(sc.gs[sc.n_jobs], M);
     if (!hs || !gs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     // Hs = X . (sA)^T: recomputed as src/linear.rs:105 does, unless the caller kept it
     if (!hs_saved) RT_TRY(linear_lora_h(l, x16, M, hs));
@@ -304,7 +294,7 @@ rt_status group_forward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, i
   group_lora_on(g, &any);
   if (any) {
     group_refresh(g, c->stream);
-    __half* hs = hs_keep ? hs_keep : lowrank_buf(c, sc.hs, sc.hs_rank, M, g.rank_total);
+    __half* hs = hs_keep ? hs_keep : lowrank_buf(sc.hs, M);
     if (!hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     if (!(hs_keep && hs_ready)) {
       if (launch_lowrank_tc(c, x16, g.a_s, M, g.w.cols, g.rank_total, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
@@ -341,8 +331,8 @@ rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, 
   if (any) {
     group_refresh(g, c->stream);
     const int R = g.rank_total;
-    __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(c, sc.hs, sc.hs_rank, M, R);
-    __half* gs = lowrank_buf(c, sc.gs[sc.n_jobs], sc.gs_rank[sc.n_jobs], M, R);
+    __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(sc.hs, M);
+    __half* gs = lowrank_buf(sc.gs[sc.n_jobs], M);
     if (!hs || !gs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     if (!hs_saved && launch_lowrank_tc(c, x16, g.a_s, M, K, R, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
     if (launch_lowrank_tc(c, dy16, g.bt_s, M, NT, R, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");

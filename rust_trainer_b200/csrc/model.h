@@ -56,7 +56,6 @@ struct rt_linear {
 // Scratch of the Linear calls of a model, or of those on a ctx outside any model (one call at a time per ctx).
 struct LinearScratch {
   DevBuf hs, gs[rt::LORA_GRAD_JOBS], grad_ws;
-  int hs_rank = -1, gs_rank[rt::LORA_GRAD_JOBS] = {-1, -1, -1, -1};
   // Adapter gradients wait here for the other linears of their block (`defer`), to be computed by one
   // launch: what they read has to stay in place until lora_grads_flush.
   bool defer = false;
