@@ -1,5 +1,6 @@
 // C ABI, level 1: the FrozenMatmul trait (reference src/frozen.rs:14-25) over host buffers.
 #include "ctx.h"
+#include "pdl.cuh"
 #include "../../include/rt_b200.h"
 #include <stdio.h>
 #include <stdlib.h>
@@ -425,6 +426,7 @@ static rt_status frozen_matmul_host(rt_frozen* f, int dir, const float* in_host,
   a.out_dtype = rt::OUT_F32;
   a.accumulate = accumulate ? 1 : 0;
   a.row_scale = row_scale;
+  const rt::PdlScope pdl_scope(t);
   int rc = rt::frozen_matmul_launch(c, f->w, a);
   if (rc) return c->fail(rc, "qgemm launch failed");
   RT_CUDA(c, cudaMemcpyAsync(out_host, out_f32, t * out_dim * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
@@ -457,6 +459,7 @@ static rt_status frozen_matmul_dev(rt_frozen* f, int dir, const void* in_dev, in
   a.out = out_dev;
   a.out_dtype = out_dtype;
   a.accumulate = accumulate ? 1 : 0;
+  const rt::PdlScope pdl_scope(t);
   int rc = rt::frozen_matmul_launch(c, f->w, a);
   if (rc) return c->fail(rc, "qgemm launch failed");
   return RT_OK;
