@@ -73,7 +73,6 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   uint64_t* done = bars + 2 * LG_NS;         // [2] a split's products have completed
   uint64_t* drained = bars + 2 * LG_NS + 2;  // [2] ... and been read
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * LG_NS + 4);
-  pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   int jx = 0;
   while (jx + 1 < ga.n_jobs && (int)blockIdx.x >= ga.job[jx + 1].first) ++jx;
@@ -110,6 +109,7 @@ lora_grads_tc_kernel(const __grid_constant__ LgArgs ga, int* status) {
   tc_fence_after();
   const uint32_t tmem_base = *(volatile uint32_t*)tmem_slot;
   pdl_wait();
+  pdl_launch_dependents();  // only now: a matmul behind this kernel takes everything older as complete (QGemmArgs::end_wait)
 
   if (warp == 4) {
     if (elect_one()) {

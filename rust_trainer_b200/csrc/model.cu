@@ -312,7 +312,7 @@ rt_status group_forward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, i
 // dx[M x K] (+)= dY[M x rows_total] . [W_0; W_1; ..] (+ Gs . A), dY row-normalised with ONE factor per token
 // for the whole row; each member's dA, dB from its slices.
 rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, const __half* dy16, const float* dscale,
-                             int M, float* dx, int accumulate, const __half* hs_saved) {
+                             int M, float* dx, int accumulate, const __half* hs_saved, bool last) {
   rt_ctx* c = g.lin[0]->ctx;
   if (M <= 0) return RT_OK;
   const int K = g.w.cols, NT = g.rows_total;
@@ -347,9 +347,15 @@ rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, 
     a.lora.rank = R;
     a.late_wait = 1;
   }
+  if (any && last) {  // the block's gradients run first: the matmul needs nothing of theirs and starts beside them
+    RT_TRY(lora_grads_add(c, sc, job, M));
+    RT_TRY(lora_grads_flush(c, sc, M));
+    a.late_wait = 0;
+    a.end_wait = 1;
+  }
   int rc = qgemm_launch(c, g.w, a);
   if (rc) return c->fail(rc, "frozen backward matmul launch failed");
-  return any ? lora_grads_add(c, sc, job, M) : RT_OK;
+  return any && !last ? lora_grads_add(c, sc, job, M) : RT_OK;
 }
 
 // tensor.rs:155-199 Rng, host side, for Lora::new's A ~ U(-1/sqrt(in), 1/sqrt(in))
@@ -1146,7 +1152,7 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   launch_swiglu_bwd(m->dhm.p, 1, sc_y, A.g16, A.u16, A.gu_pitch, M, g.ff, dg16, du16, A.gu_pitch, m->sc_g.as<float>(),
                     m->sc_u.as<float>(), st);
   if (A.gu_group) {
-    RT_TRY(group_backward_dev(b.gu, m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4)));
+    RT_TRY(group_backward_dev(b.gu, m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4), false));
   } else {
     RT_TRY(linear_backward_dev(b.lin[4], m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4)));
     RT_TRY(linear_backward_dev(b.lin[5], m->lsc, A.n2, du16, m->sc_u.as<float>(), M, m->dn.as<float>(), 1, HS(5)));
@@ -1170,7 +1176,7 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
                      m->rope_sin.as<float>(), M, g.n_heads, g.n_kv_heads, g.head_dim, g.rot_dim, g.rope_neox, g.rms_eps,
                      dq16, dk16, dv16, A.qkv_pitch, m->sc_q.as<float>(), m->sc_k.as<float>(), m->sc_v.as<float>(), st);
   if (A.qkv_group) {
-    RT_TRY(group_backward_dev(b.qkv, m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0)));
+    RT_TRY(group_backward_dev(b.qkv, m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0), true));
   } else {
     RT_TRY(linear_backward_dev(b.lin[0], m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0)));
     RT_TRY(linear_backward_dev(b.lin[1], m->lsc, A.n1, dk16, m->sc_k.as<float>(), M, m->dn.as<float>(), 1, HS(1)));

@@ -8,7 +8,7 @@
 //     brings along and no kernel writes (tile lists, where sequences start) may be read before it;
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
 //     every CTA of this one has started.
-// Two pairs of kernels depart from both.  (1) A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
+// Three pairs of kernels depart from both.  (1) A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
 // weights, activations and residual without waiting and waits only where it loads the stream's result.  That
 // is sound because of what lowrank_tc_kernel and the matmul keep between them:
 //   - lowrank_tc_kernel triggers only after its own wait, so that everything older than it is complete and
@@ -19,6 +19,9 @@
 // (2) The attention's dQ kernel behind its dK/dV kernel, which it needs nothing from (attention_tc.cu): dK/dV triggers only
 // after its own wait, so that what both read is complete and visible; neither writes what the other reads or writes;
 // and every CTA of dQ waits before it ends, so that whoever waits for dQ has waited for both.
+// (3) A matmul behind the adapter gradients of its block (QGemmArgs::end_wait), under the same conditions: the gradients read
+// what the matmul reads and write what nothing in the block reads; they trigger after their wait; every CTA of the matmul
+// waits before it ends.
 // Inside stream capture these launches become programmatic edges of the graph.
 // Used for passes of up to PDL_MAX_TOKENS tokens, whose kernels leave SMs free for the next one's CTAs to
 // start on: the 28-layer 0.6B step 10.67 -> 10.14 ms at 1024 tokens, scoring 157 tokens 3.01 -> 2.84 ms.  At

@@ -138,7 +138,7 @@ struct KParams {
   const float* bias;
   uint32_t idesc;
   int* status;
-  int late_wait;  // see QGemmArgs
+  int late_wait, end_wait;  // see QGemmArgs
 };
 
 // ------------------------------------------------------------------ unpackers
@@ -385,7 +385,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   // barriers, TMEM and descriptors are set up; from here on the kernel reads what its predecessor wrote.  Packed weights
   // no kernel of a pass writes: their bricks are fetched and unpacked under the predecessor's end.
   const bool weights_only = PACKED && (role == R_RAW || role == R_UNPACK);
-  if (!p.late_wait && !weights_only) pdl_wait();
+  if (!p.late_wait && !p.end_wait && !weights_only) pdl_wait();
 
   // Where the 32 accumulator lanes of quarter wq belong.  A slim pair's accumulator has 64 rows in each CTA: lanes 0..63 hold
   // them for the tile's first half of the tokens, lanes 64..127 for the second, in half as many columns.
@@ -594,7 +594,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   const int q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
   auto tail_helper = [&](int turn, int hslot) {
     if (n_my == 0 || (!SLIM && q_res * 32 >= C::ROWS)) return;
-    if (!p.late_wait && weights_only) pdl_wait();
+    if (!p.late_wait && !p.end_wait && weights_only) pdl_wait();
     const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
     QG_ITEM_DECODE(item);
     (void)s_begin; (void)n_steps; (void)s_main;
@@ -927,6 +927,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   }
 
   // ---------------------------------------------------------------- teardown
+  if (p.end_wait) pdl_wait();
   if (*(volatile int*)p.status != 0) {
     // A wait gave up somewhere: give copies already in flight time to land before smem goes away.
     for (int i = 0; i < 1000; ++i) __nanosleep(1000);
@@ -1208,6 +1209,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   p.row_scale = a.row_scale;
   p.residual = a.residual;
   p.late_wait = a.late_wait && a.lora.rank > 0 ? 1 : 0;
+  p.end_wait = a.end_wait;
   p.dir = a.dir;
   p.out_rows = out_rows;
   p.M = a.M;
@@ -1310,7 +1312,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() || a.end_wait ? 1 : 0;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = 2;
     at[1].val.clusterDim.y = 1;

@@ -66,6 +66,9 @@ struct QGemmArgs {
   // only after its own wait: a programmatic launch may start at once and waits only where it reads that result
   // (pdl.cuh has the conditions).
   int late_wait = 0;
+  // The launch right before this one shares nothing with it, and let it start only after its own wait, so that all that this
+  // one reads is complete: it waits before it ends, and nowhere else (pdl.cuh).
+  int end_wait = 0;
 };
 
 int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a);
