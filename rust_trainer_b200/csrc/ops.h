@@ -54,9 +54,10 @@ struct LoraRefreshJob {
   float s;
   unsigned first_block;  // of this job in the grid; jobs are in increasing order
 };
+constexpr unsigned LORA_REFRESH_PER_BLOCK = 2048;  // elements
 inline unsigned lora_refresh_job_blocks(const LoraRefreshJob& j) {
   const size_t na = (size_t)j.r * j.K, nb = (size_t)j.N * (j.pad64 ? 64 : j.r);
-  return (unsigned)(((na > nb ? na : nb) + 255) / 256);
+  return (unsigned)(((na > nb ? na : nb) + LORA_REFRESH_PER_BLOCK - 1) / LORA_REFRESH_PER_BLOCK);
 }
 void launch_lora_refresh_table(const LoraRefreshJob* jobs_dev, int n_jobs, unsigned total_blocks, cudaStream_t st);
 void launch_sumsq(const float* g, size_t n, double* part, double* out, cudaStream_t st);
