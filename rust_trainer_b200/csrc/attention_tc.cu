@@ -1048,7 +1048,7 @@ int bwd_tc_impl(rt_ctx* c, const __half* q, const __half* k, const __half* v, co
     return 3;
   // dQ reads nothing of dK/dV's: it starts as soon as that kernel's last CTAs have, in passes of every size.
   PdlLaunch dq_launch = pdl(attn_bwd_dq_tc_kernel<HD>, (unsigned)nh * n_tiles, DQ_THREADS, LQ::TOTAL, st);
-  dq_launch.programmatic = true;
+  dq_launch.programmatic = pdl_any_size();
   if (dq_launch(tq128, tdo128, tk64, tv64, row_scale, lse, query_vecs, b.seq_start, gap, b.tiles_q, M, nh, nkv, scale, dq, c->status_dev) != cudaSuccess)
     return 3;
   RT_COUNT_LAUNCH(3);

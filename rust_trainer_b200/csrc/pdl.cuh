@@ -50,13 +50,17 @@ struct PdlScope {
   explicit PdlScope(size_t tokens) : before(g_pdl_tokens) { g_pdl_tokens = tokens > (1u << 30) ? 1 << 30 : (int)tokens; }
   ~PdlScope() { g_pdl_tokens = before; }
 };
-inline bool pdl_enabled() {
+inline int pdl_forced() {  // 1 always, 0 never, -1 by the pass's size
   static const int forced = [] {
     const char* e = getenv("RT_B200_PDL");
     return e ? (atoi(e) ? 1 : 0) : -1;
   }();
-  return forced >= 0 ? forced != 0 : g_pdl_tokens > 0 && g_pdl_tokens <= PDL_MAX_TOKENS;
+  return forced;
 }
+inline bool pdl_enabled() {
+  return pdl_forced() >= 0 ? pdl_forced() != 0 : g_pdl_tokens > 0 && g_pdl_tokens <= PDL_MAX_TOKENS;
+}
+inline bool pdl_any_size() { return pdl_forced() != 0; }  // for a kernel that runs beside the one in front of it
 
 template <typename... KArgs>
 struct PdlLaunch {

@@ -1312,7 +1312,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() || a.end_wait ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() || (a.end_wait && pdl_any_size()) ? 1 : 0;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = 2;
     at[1].val.clusterDim.y = 1;
