@@ -153,6 +153,28 @@ def test_reruns_are_bit_identical_and_batching_is_neutral(ctx):
     om.close()
 
 
+@pytest.mark.parametrize("n_layers", [36, 37, 40])
+def test_adapter_copies_of_deep_models(ctx, n_layers):
+    """The copies of all stale adapters are rebuilt by one launch whose blocks count through the table 256 rows at a time: 252,
+    259 and 280 adapters, ranks that end inside a block's share of elements."""
+    spec = synth.preset("tiny-qwen3", quant="Q8_0", seed=3, w_std=0.02, n_layers=n_layers)
+    tensors = synth.build_tensors(spec)
+    ads = synth.lora_adapters(spec, 5, 10.0, seed=7, b_std=0.02)
+    om = O.OracleModel(spec.config(), tensors)
+    om.attach_lora(ads)
+    gm = rt.Model(ctx, spec.config(), tensors)
+    gm.attach_lora(5, 10.0, None, 1)
+    gm.load_adapters(ads)
+    seqs, tp, tt, per_seq = _batch(spec, [33], 5)
+    w = np.full(tp.size, 1.0 / tp.size, np.float32)
+    lp, _ = gm.forward_backward(seqs, tp, tt, w)
+    om.zero_grad()
+    want = om.forward_backward(seqs[0], *per_seq[0], w)[0]
+    assert np.max(np.abs(lp - want) / np.abs(want)) < LOSS_TOL
+    assert rel_l2(_gpu_flat(gm, "ga", "gb"), _flat(om.lora, "ga", "gb")) < GRAD_TOL
+    gm.close()
+
+
 def test_grouped_and_separate_projections_agree(ctx, monkeypatch):
     """q|k|v and gate|up run as one stacked matmul each (one scale per token for the whole
     gradient row); RT_B200_NO_GROUPS=1 keeps one matmul per projection.  Both meet the oracle, and
