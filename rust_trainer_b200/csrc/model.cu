@@ -62,13 +62,11 @@ rt_status lora_refresh(rt_linear* l) {
   return RT_OK;
 }
 
-// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16 columns, and the zeros it needs
-// from the rank on come from lowrank_tc_kernel, which writes all 64 columns of every row.  New memory is cleared once, so that
-// what lies behind the last row is finite.  (The buffer was also cleared before every product whose rank is no multiple of 16:
-// up to five more links of 1.5 to 3 us in each layer's chain of launches.)
+// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16 columns; lowrank_tc_kernel writes all
+// 64 columns of every row, zeros from the rank on, and every reader's tensor map ends at row M: new memory needs no clear.
 static __half* lowrank_buf(DevBuf& b, int M) {
   const size_t want = (size_t)M * 64 * sizeof(__half);
-  return b.reserve(want <= b.bytes ? want : want + want / 2, true) ? b.as<__half>() : nullptr;
+  return b.reserve(want <= b.bytes ? want : want + want / 2) ? b.as<__half>() : nullptr;
 }
 
 rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out) {

@@ -161,3 +161,44 @@ def test_a_contexts_scratch_goes_with_it():
     before = free_bytes()
     assert use() < before - (100 << 20)
     assert abs(free_bytes() - before) < 32 << 20
+
+
+def test_a_first_call_does_not_wait_for_other_streams(ctx):
+    """The scratch of a context's first calls with an adapter comes without stopping the device: a host whose other stream is
+    busy gets both calls back while it still is."""
+    import torch
+
+    from rust_trainer_b200._lib import DT_F32, lib
+
+    L = lib()
+    n, k, m, r = 256, 128, 50, 12
+    x, dy = (torch.randn(m, c, device="cuda").half() for c in (k, n))
+
+    def calls(c, between=lambda: None):
+        packed, _, _, _, f, lin = _make(c, np.random.default_rng(3), Q.Q8_0, n, k, r)
+        y, dx = (torch.full((m, cols), float("nan"), device="cuda") for cols in (n, k))
+        torch.cuda.synchronize()
+        state = between()
+        c.check(L.rt_linear_forward_dev(lin._h, x.data_ptr(), m, y.data_ptr(), DT_F32, 0))
+        c.check(L.rt_linear_backward_dev(lin._h, x.data_ptr(), dy.data_ptr(), None, m, dx.data_ptr(), 0))
+        waited = state is not None and state.query()
+        c.synchronize()
+        torch.cuda.synchronize()
+        g = lin.lora()
+        lin.close()
+        f.close()
+        return waited, [y.cpu().numpy(), dx.cpu().numpy(), g["ga"], g["gb"]]
+
+    def busy():
+        side, done = torch.cuda.Stream(), torch.cuda.Event()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1_000_000_000)  # half a second
+            done.record(side)
+        return done
+
+    _, want = calls(ctx)  # (also loads the kernels)
+    c2 = rt.Context(0)
+    waited, got = calls(c2, busy)
+    assert not waited
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    c2.close()
