@@ -768,6 +768,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tmem_alloc(tmem_slot, L::TMEM_COLS);
     tmem_relinquish();
   }
+  if (warp == 0) pdl_unwaited();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

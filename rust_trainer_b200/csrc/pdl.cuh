@@ -22,6 +22,9 @@
 // (3) A matmul behind the adapter gradients of its block (QGemmArgs::end_wait), under the same conditions: the gradients read
 // what the matmul reads and write what nothing in the block reads; they trigger after their wait; every CTA of the matmul
 // waits before it ends.
+// Complete means that the writes are in L2.  A line that the SM's L1 holds from before them is only sure to be gone after the wait,
+// so a CTA of the three that reads by ordinary loads what the pass computes executes pdl_unwaited() first, in one warp in front of
+// the barrier at the end of its set-up.  (TMA and cp.async.cg read L2.)
 // Inside stream capture these launches become programmatic edges of the graph.
 // Used for passes of up to PDL_MAX_TOKENS tokens, whose kernels leave SMs free for the next one's CTAs to
 // start on: the 28-layer 0.6B step 10.67 -> 10.14 ms at 1024 tokens, scoring 157 tokens 3.01 -> 2.84 ms.  At
@@ -37,6 +40,9 @@ namespace rt {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// In place of the wait, where a kernel reads what was complete before it could start: an acquire fence, so that its loads do not
+// take from L1 what an earlier kernel left there.  (Loads past L1 instead, in the epilogues: scoring 157 tokens 1.98 -> 2.04 ms.)
+__device__ __forceinline__ void pdl_unwaited() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 // the usual entry sequence of a kernel that has no prologue worth overlapping
 __device__ __forceinline__ void pdl_entry() {
   pdl_launch_dependents();

@@ -1,0 +1,36 @@
+"""Rules of kernels that are launched while the one in front of them still runs (csrc/pdl.cuh), read from the source."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "rust_trainer_b200" / "csrc"
+
+
+def kernels():
+    """{name: text of the kernel, from its parameters to the end of its body}, comments taken out."""
+    out = {}
+    for path in CSRC.glob("*.cu"):
+        src = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\((?:[^()]|\([^()]*\))*\))*\)\s+)?(\w+)\(", src):
+            at = end = src.index("{", m.end())
+            depth = 0
+            while True:
+                depth += {"{": 1, "}": -1}.get(src[end], 0)
+                if depth == 0:
+                    break
+                end += 1
+            out[m[1]] = src[m.end():end]
+    return out
+
+
+@pytest.mark.parametrize("name,when", [("qgemm_kernel", "warp == 2 && (p.late_wait || p.end_wait)"), ("attn_bwd_dq_tc_kernel", "warp == 0")])
+def test_what_is_read_without_a_wait_comes_after_an_acquire_fence(name, when):
+    """Only the wait is defined to make earlier kernels' writes visible: without it an ordinary load may find an L1 line from
+    before them.  One warp's fence in front of the CTA's barrier orders every warp's loads behind it."""
+    body = kernels()[name]
+    fence = body.index(f"if ({when}) pdl_unwaited();")
+    assert body.index("tmem_alloc") < fence < body.index("__syncthreads();", fence) < body.index("tmem_base =")
+    for read in ("row_scale[", "lse[", "query_vecs["):
+        assert body.find(read) == -1 or body.find(read) > fence
+    assert "fence.acq_rel.gpu;" in (CSRC / "pdl.cuh").read_text()
