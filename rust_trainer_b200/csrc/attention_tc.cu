@@ -53,7 +53,9 @@ struct FwdLayout {
   // rounding the base up to a 1 KB boundary is 768 bytes: enough for any base that is 256-byte
   // aligned (the kernel checks, and reports a status instead of running, if it ever is not).
   static constexpr uint32_t USED = OFF_BAR + 256;
-  static constexpr uint32_t TOTAL = USED + 768;
+  // No less than what keeps a low-rank block away from two of these (64-wide heads): the kernel lets the next one start before
+  // its blocks hold their TMEM (pdl.cuh).
+  static constexpr uint32_t TOTAL = USED + 768 > TWO_BLOCKS_SMEM ? USED + 768 : TWO_BLOCKS_SMEM;
   static constexpr uint32_t TMEM_COLS = 256;               // S[2] (64 each) + O (hd <= 128)
   static constexpr uint32_t COL_S = 0, COL_O = 2 * BN;
 };
@@ -392,6 +394,7 @@ struct DkvLayout {
   static constexpr uint32_t AUX_BYTES = 2 * BQ * 4;  // exponent offset and scaled -delta per query row
   static constexpr uint32_t OFF_BAR = OFF_AUX + NS * AUX_BYTES;
   static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 1024;
+  static_assert(TOTAL >= TMEM_KERNEL_SMEM, "a matmul's block could share its SM (pdl.cuh)");
   static constexpr uint32_t COL_ST = 0, COL_DPT = 2 * BQ, COL_DV = 4 * BQ, COL_DK = 4 * BQ + HD;
   static constexpr uint32_t TMEM_COLS = 512;
   // the CTA's sums for its cluster, [2][128 keys][hd + 4] f32, over the operands once those are used up
@@ -702,7 +705,8 @@ struct DqLayout {
   static constexpr int NK = 2;  // K slots (a slot is released by its tile's dQ product; V's one slot by the dP product)
   static constexpr uint32_t OFF_Q = 0, OFF_DO = Q_BYTES, OFF_K = 2 * Q_BYTES, OFF_V = OFF_K + NK * KV_BYTES;
   static constexpr uint32_t OFF_BAR = OFF_V + KV_BYTES;
-  static constexpr uint32_t USED = OFF_BAR + 256, TOTAL = USED + 768;  // slack as in the forward's layout
+  static constexpr uint32_t USED = OFF_BAR + 256;
+  static constexpr uint32_t TOTAL = USED + 768 > TWO_BLOCKS_SMEM ? USED + 768 : TWO_BLOCKS_SMEM;  // slack and least as in the forward's layout
   static constexpr uint32_t COL_S = 0, COL_DP = BN, COL_DQ = 2 * BN, TMEM_COLS = 256;
   static constexpr int PITCH = HD + 4;  // dQ as f32 over the operands once those are used up
   static_assert(BM * PITCH * 4 <= (int)OFF_BAR, "dQ fits over the operands");

@@ -42,6 +42,7 @@ constexpr int LG_NS = 3, LG_THREADS = 192, LG_CTAS_PER_SM = 3;
 constexpr uint32_t LG_Q_BYTES = 2 * 64 * 128, LG_P_BYTES = 64 * 128, LG_STAGE = LG_Q_BYTES + LG_P_BYTES;
 constexpr uint32_t LG_OFF_BAR = LG_NS * LG_STAGE;
 constexpr uint32_t LG_TOTAL = LG_OFF_BAR + 256 + 1024;
+static_assert(LG_TOTAL >= TMEM_KERNEL_SMEM, "a matmul's block could share its SM (pdl.cuh)");
 enum { SITE_LG_FREE = 495, SITE_LG_FULL, SITE_LG_DONE, SITE_LG_DRAINED };
 
 struct LgMaps {

@@ -42,6 +42,7 @@ struct LrCfg {
   // the CTA's sums, [TN tokens][64 + 4] f32 (a cluster) or [TN][64] f16 (a CTA alone), take the place of the
   // operand stages once those are used up
   static constexpr int PITCH = 68;
+  static_assert(TOTAL >= LOWRANK_KERNEL_SMEM, "blocks of kernels with TMEM in front of it could share its SM (pdl.cuh)");
   static_assert(STAGE % 1024 == 0, "stages start on a swizzle atom");
   static_assert(TN * PITCH * 4 <= NS * STAGE, "the sums fit over the stages");
 };

@@ -7,7 +7,12 @@
 //     early return (a grid that is complete has then waited, so ordering stays transitive).  What a batch
 //     brings along and no kernel writes (tile lists, where sequences start) may be read before it;
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
-//     every CTA of this one has started.
+//     every CTA of this one has started.  A CTA that has not got its TMEM yet must then find it: a CTA of a later kernel that took the
+//     columns on the same SM waits for this kernel, which would wait for them.  So a kernel with TMEM lets the next one start once it
+//     holds its columns; or no block of a kernel that could take them fits beside its blocks: none at all beside a
+//     matmul's, no low-rank one beside two of the attention's forward or dQ (256 columns each; behind them the low-rank
+//     kernel is the first with TMEM, and it lets nothing start before they are complete).  The constants below say so.  (Later, once
+//     it holds its columns, in the matmul too: scoring 157 tokens 2.00 -> 2.02 ms.)
 // Three pairs of kernels depart from both.  (1) A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
 // weights, activations and residual without waiting and waits only where it loads the stream's result.  That
 // is sound because of what lowrank_tc_kernel and the matmul keep between them:
@@ -48,6 +53,14 @@ __device__ __forceinline__ void pdl_entry() {
   pdl_launch_dependents();
   pdl_wait();
 }
+
+// Shared memory of an SM, 1 KB of each block's being the system's; the least a block of the low-rank kernel takes, and of any kernel
+// with TMEM but the matmul; what a block takes so that two of it and one of the first do not fit, and so that it and one of the
+// second do not.
+constexpr int SMEM_PER_SM = 228 * 1024, LOWRANK_KERNEL_SMEM = 97 * 1024, TMEM_KERNEL_SMEM = 64 * 1024;
+constexpr int TWO_BLOCKS_SMEM = 65 * 1024, ALONE_SMEM = 163 * 1024;
+static_assert(2 * (TWO_BLOCKS_SMEM + 1024) + LOWRANK_KERNEL_SMEM + 1024 > SMEM_PER_SM && TWO_BLOCKS_SMEM >= TMEM_KERNEL_SMEM &&
+              ALONE_SMEM + TMEM_KERNEL_SMEM + 2 * 1024 > SMEM_PER_SM);
 
 constexpr int PDL_MAX_TOKENS = 4096;
 inline thread_local int g_pdl_tokens = 0;  // tokens of the pass this thread is launching, see PdlScope

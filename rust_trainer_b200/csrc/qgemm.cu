@@ -114,7 +114,9 @@ struct QCfg {
   static constexpr int OFF_OUT = (OFF_RAW + NR * RAW_STAGE + 1023) / 1024 * 1024;  // (a swizzled store's source starts on its pattern)
   static constexpr int OFF_BAR = OFF_OUT + 4 * OUT_WARP;
   static constexpr int N_BARS = 3 * NS + 2 * NR + 5;
-  static constexpr int SMEM_BYTES = OFF_BAR + N_BARS * 8 + 16 + 1024;
+  // At least so much that no other kernel with TMEM fits beside it: it lets the next one start before it holds its columns (pdl.cuh).
+  static constexpr int SMEM_USED = OFF_BAR + N_BARS * 8 + 16 + 1024;
+  static constexpr int SMEM_BYTES = SMEM_USED > ALONE_SMEM ? SMEM_USED : ALONE_SMEM;
   static_assert(SMEM_BYTES <= SMEM_MAX && N_BARS * 8 + 16 <= 512, "shared memory plan exceeds one SM");
   static_assert(OFF_RAW >= 11 * 8192, "the last tile's helpers stage in the operand stages");
 };

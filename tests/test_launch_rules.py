@@ -34,3 +34,24 @@ def test_what_is_read_without_a_wait_comes_after_an_acquire_fence(name, when):
     for read in ("row_scale[", "lse[", "query_vecs["):
         assert body.find(read) == -1 or body.find(read) > fence
     assert "fence.acq_rel.gpu;" in (CSRC / "pdl.cuh").read_text()
+
+
+#: kernels that let the next one start before they hold their TMEM, and the layouts of shared memory that keep it free for them
+EARLY = {"qgemm_kernel": ("qgemm.cu", r"SMEM_BYTES = SMEM_USED > ALONE_SMEM \? SMEM_USED : ALONE_SMEM;", 1),
+         "attn_fwd_tc_kernel": ("attention_tc.cu", r"TOTAL = USED \+ 768 > TWO_BLOCKS_SMEM \? USED \+ 768 : TWO_BLOCKS_SMEM;", 2),
+         "attn_bwd_dq_tc_kernel": ("attention_tc.cu", r"TOTAL = USED \+ 768 > TWO_BLOCKS_SMEM \? USED \+ 768 : TWO_BLOCKS_SMEM;", 2)}
+
+
+@pytest.mark.parametrize("name", sorted(n for n, body in kernels().items() if "tmem_alloc" in body))
+def test_no_later_kernel_takes_the_tmem_a_started_one_still_needs(name):
+    """Otherwise a CTA of a later kernel on the same SM could take the columns first and wait for this kernel, which waits for
+    them."""
+    body = kernels()[name]
+    assert "pdl_entry" not in body and body.count("pdl_launch_dependents();") == 1
+    if body.rindex("tmem_alloc") < body.index("tmem_base =") < body.index("pdl_launch_dependents();"):
+        return
+    file, layout, times = EARLY[name]
+    assert len(re.findall(layout, (CSRC / file).read_text())) == times
+    for file, least in (("lowrank_tc.cu", "TOTAL >= LOWRANK_KERNEL_SMEM"), ("lora_grads_tc.cu", "LG_TOTAL >= TMEM_KERNEL_SMEM"),
+                        ("attention_tc.cu", "TOTAL >= TMEM_KERNEL_SMEM")):
+        assert f"static_assert({least}" in (CSRC / file).read_text()
