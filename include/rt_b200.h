@@ -133,6 +133,11 @@ rt_status rt_frozen_forward_dev(rt_frozen* w, const void* x_dev, int in_dtype, s
                                 int out_dtype, int accumulate);
 rt_status rt_frozen_backward_input_dev(rt_frozen* w, const void* dy_dev, int in_dtype, size_t t, void* dx_dev,
                                        int out_dtype, int accumulate);
+/* Which kind of tile the two calls above run on for `t` rows, and how many tokens wide it is (0 in `backward`: the
+ * forward).  Nothing runs; the choice changes no result.  For tests, and for whoever reads a profile; no counterpart in
+ * the reference.  (Frozen matmuls of every level choose alike; f32 weights run twice on the same tiles.) */
+enum { RT_TILE_PAIR = 0, RT_TILE_WIDE = 1, RT_TILE_NARROW = 2, RT_TILE_HALF = 3, RT_TILE_NARROW_TMEM = 4, RT_TILE_SLIM = 5 };
+rt_status rt_frozen_tile(const rt_frozen* w, int backward, size_t t, int in_dtype, int out_dtype, int* kind, int* tokens);
 /* The same operation as rt_frozen_backward_input_dev for callers that must not allocate device
  * memory while they run: a host inside a memory-budgeted serving or training process that has
  * handed every byte of HBM to its own pool, a real-time loop that cannot take the driver's

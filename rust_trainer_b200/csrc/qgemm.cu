@@ -1187,44 +1187,18 @@ static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, in
   return best;
 }
 
-int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
-  const int num_sms = ctx->num_sms;
-  cudaStream_t st = ctx->stream;
-  if (!g_encode) {
-    int rc = qgemm_init();
-    if (rc) return rc;
-  }
-  if (a.M <= 0) return RT_OK;
-  const bool is16 = fmt_is_16bit(w.fmt);
-  const int contract = a.dir == QG_FWD ? w.cols : w.rows;
-  const int out_rows = a.dir == QG_FWD ? w.rows : w.cols;
-  if (contract % 8 != 0 || (is16 && w.cols % 8 != 0)) return RT_ERR_BAD_SHAPE;
-  if ((a.accumulate || a.residual) && a.out_dtype != OUT_F32) return RT_ERR_BAD_ARG;
-  if (a.lora.rank > 64 || (a.lora.rank > 0 && (!a.lora.act || !a.lora.w))) return RT_ERR_BAD_ARG;
-
-  KParams p;
-  p.bricks = w.bricks;
-  p.nb = a.dir == QG_FWD ? w.nbr : w.nbk;
-  p.nbk = w.nbk;
-  p.act_f16 = a.act_f16 ? 1 : 0;
-  p.conv16 = (w.fmt == GGML_F16 && !a.act_f16) ? 1 : (w.fmt == GGML_BF16 && a.act_f16) ? 2 : 0;
-  const int kfmt = !is16 ? w.fmt : p.conv16 ? QF_16CONV : QF_16;
-  p.row_scale = a.row_scale;
-  p.residual = a.residual;
-  p.late_wait = a.late_wait && a.lora.rank > 0 ? 1 : 0;
-  p.end_wait = a.end_wait;
-  p.dir = a.dir;
-  p.out_rows = out_rows;
-  p.M = a.M;
-  p.n_main = (contract + 63) / 64;
-  p.lora_mmas = a.lora.rank > 0 ? (a.lora.rank + 15) / 16 : 0;
-  p.out = a.out;
-  p.out_dtype = a.out_dtype;
-  p.accumulate = a.accumulate;
-  p.ld_out = a.ld_out > 0 ? a.ld_out : out_rows;
-  p.bias = a.dir == QG_FWD ? a.bias : nullptr;
-  p.status = ctx->status_dev;
-
+// How a product runs: the weight as the kernel sees it, where the contraction is cut, and the tiles.
+struct QSetup {
+  int kfmt, conv16, contract, out_rows, n_main, steps_per_split, n_splits;
+  QPlan plan;
+};
+static QSetup qgemm_setup(const rt_ctx* ctx, const QWeight& w, int dir, bool act_f16, int M, int out_dtype) {
+  QSetup q;
+  q.conv16 = (w.fmt == GGML_F16 && !act_f16) ? 1 : (w.fmt == GGML_BF16 && act_f16) ? 2 : 0;
+  q.kfmt = !fmt_is_16bit(w.fmt) ? w.fmt : q.conv16 ? QF_16CONV : QF_16;
+  q.contract = dir == QG_FWD ? w.cols : w.rows;
+  q.out_rows = dir == QG_FWD ? w.rows : w.cols;
+  q.n_main = (q.contract + 63) / 64;
   // How the contraction is cut into accumulation chains depends on the weight's shape ONLY, never
   // on the number of tokens: the tensor core's accumulator does not round to nearest, so two
   // partitions of one sum differ by a few 1e-6 relative, which the next 16-bit rounding of the
@@ -1234,12 +1208,52 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   // A very long contraction (the head's backward runs over the whole vocabulary) is accumulated
   // in pieces of a FIXED 8192 elements whose f32 partial sums are added afterwards: the error of
   // one chain grows with its length (about 3e-4 relative over 150 000 elements).
-  p.steps_per_split = p.n_main;
-  if (a.out_dtype == OUT_F32 && p.n_main > 256) p.steps_per_split = 128;
-  p.n_splits = (p.n_main + p.steps_per_split - 1) / p.steps_per_split;
+  q.steps_per_split = q.n_main;
+  if (out_dtype == OUT_F32 && q.n_main > 256) q.steps_per_split = 128;
+  q.n_splits = (q.n_main + q.steps_per_split - 1) / q.steps_per_split;
+  q.plan = qgemm_plan(q.kfmt, dir, M, q.out_rows, q.n_splits, q.steps_per_split, ctx->num_sms, out_dtype != OUT_F32);
+  return q;
+}
 
-  const QPlan plan = qgemm_plan(kfmt, a.dir, a.M, out_rows, p.n_splits, p.steps_per_split, num_sms,
-                                a.out_dtype != OUT_F32);
+int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
+  const int num_sms = ctx->num_sms;
+  cudaStream_t st = ctx->stream;
+  if (!g_encode) {
+    int rc = qgemm_init();
+    if (rc) return rc;
+  }
+  if (a.M <= 0) return RT_OK;
+  const bool is16 = fmt_is_16bit(w.fmt);
+  const QSetup setup = qgemm_setup(ctx, w, a.dir, a.act_f16 != 0, a.M, a.out_dtype);
+  const QPlan plan = setup.plan;
+  const int kfmt = setup.kfmt, contract = setup.contract, out_rows = setup.out_rows;
+  if (contract % 8 != 0 || (is16 && w.cols % 8 != 0)) return RT_ERR_BAD_SHAPE;
+  if ((a.accumulate || a.residual) && a.out_dtype != OUT_F32) return RT_ERR_BAD_ARG;
+  if (a.lora.rank > 64 || (a.lora.rank > 0 && (!a.lora.act || !a.lora.w))) return RT_ERR_BAD_ARG;
+
+  KParams p;
+  p.bricks = w.bricks;
+  p.nb = a.dir == QG_FWD ? w.nbr : w.nbk;
+  p.nbk = w.nbk;
+  p.act_f16 = a.act_f16 ? 1 : 0;
+  p.conv16 = setup.conv16;
+  p.row_scale = a.row_scale;
+  p.residual = a.residual;
+  p.late_wait = a.late_wait && a.lora.rank > 0 ? 1 : 0;
+  p.end_wait = a.end_wait;
+  p.dir = a.dir;
+  p.out_rows = out_rows;
+  p.M = a.M;
+  p.n_main = setup.n_main;
+  p.lora_mmas = a.lora.rank > 0 ? (a.lora.rank + 15) / 16 : 0;
+  p.out = a.out;
+  p.out_dtype = a.out_dtype;
+  p.accumulate = a.accumulate;
+  p.ld_out = a.ld_out > 0 ? a.ld_out : out_rows;
+  p.bias = a.dir == QG_FWD ? a.bias : nullptr;
+  p.status = ctx->status_dev;
+  p.steps_per_split = setup.steps_per_split;
+  p.n_splits = setup.n_splits;
   const bool pair = plan.kind == QK_PAIR || plan.kind == QK_SLIM;
   p.TN = plan.TN;
   const int tile_rows = plan.kind == QK_PAIR ? 256 : plan.kind == QK_HALF ? 64 : 128;
@@ -1392,6 +1406,19 @@ extern "C" rt_status rt_ctx_selftest_wait_timeout(rt_ctx* c, uint64_t limit_cycl
   rt::wait_selftest_kernel<<<1, 32, 0, c->stream>>>(c->status_dev, (long long)limit_cycles);
   if (cudaGetLastError() != cudaSuccess) return c->fail(RT_ERR_CUDA, "self-test launch failed");
   return c->check_device_status("rt_ctx_selftest_wait_timeout");  // expected: RT_ERR_DEVICE_WAIT_TIMEOUT, site 999
+}
+
+extern "C" rt_status rt_frozen_tile(const rt_frozen* f, int backward, size_t t, int in_dtype, int out_dtype, int* kind, int* tokens) {
+  static_assert(RT_TILE_PAIR == rt::QK_PAIR && RT_TILE_WIDE == rt::QK_WIDE && RT_TILE_NARROW == rt::QK_NARROW && RT_TILE_HALF == rt::QK_HALF &&
+                    RT_TILE_NARROW_TMEM == rt::QK_NARROW_T && RT_TILE_SLIM == rt::QK_SLIM,
+                "the header's kinds are the kernel's");
+  if (!f || !kind || !tokens || t == 0 || t > (1u << 24)) return RT_ERR_BAD_ARG;
+  if ((in_dtype != RT_DT_F16 && in_dtype != RT_DT_BF16) || out_dtype < 0 || out_dtype > 2) return RT_ERR_BAD_ARG;
+  const rt::QPlan plan =
+      rt::qgemm_setup(f->ctx, f->w, backward ? rt::QG_BWD : rt::QG_FWD, in_dtype == RT_DT_F16, (int)t, out_dtype).plan;
+  *kind = plan.kind;
+  *tokens = plan.TN;
+  return RT_OK;
 }
 
 extern "C" rt_status rt_frozen_backward_input_dev_noalloc(rt_frozen* f, const void* dy_dev, int in_dtype, size_t t,

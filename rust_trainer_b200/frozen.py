@@ -11,7 +11,7 @@ import ctypes as C
 import numpy as np
 
 from . import quants
-from ._lib import OK, RtError, lib
+from ._lib import DT_F16, DT_F32, OK, RtError, lib
 
 _F32P = C.POINTER(C.c_float)
 
@@ -183,6 +183,15 @@ class Frozen:
             raise RtError(6, "row index out of range")
         self.ctx.check(lib().rt_frozen_row(self._h, r, _fp(out)))
         return out
+
+    #: kinds of matmul tiles, in the order of RT_TILE_*
+    TILES = ("pair", "wide", "narrow", "half", "narrow_tmem", "slim")
+
+    def tile(self, t: int, backward: bool = False, in_dtype: int = DT_F16, out_dtype: int = DT_F32) -> tuple[str, int]:
+        """The kind of tile that `t` rows run on, and its width in tokens.  Nothing runs."""
+        kind, tokens = C.c_int(), C.c_int()
+        self.ctx.check(lib().rt_frozen_tile(self._h, int(backward), t, in_dtype, out_dtype, C.byref(kind), C.byref(tokens)))
+        return self.TILES[kind.value], tokens.value
 
     def close(self) -> None:
         if self._h:

@@ -74,7 +74,7 @@ def test_adjoint_identity_on_device(ctx, t):
     f.close()
 
 
-@pytest.mark.parametrize("n,k,tokens", [(512, 256, 300), (384, 256, 1000), (1024, 128, 4133)])
+@pytest.mark.parametrize("n,k,tokens", [(512, 256, 300), (384, 256, 1000), (1024, 128, 4133), (1024, 512, 4133)])
 def test_16_bit_outputs_are_the_rounded_f32_outputs(ctx, n, k, tokens):
     """The device entry points write f32, f16 or bf16.  The 16-bit epilogue (fragment-layout TMEM
     loads, paired rounding, transposing matrix stores, swizzled TMA store) must give exactly the
@@ -92,6 +92,7 @@ def test_16_bit_outputs_are_the_rounded_f32_outputs(ctx, n, k, tokens):
     torch.cuda.synchronize()
     ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, tokens, y32.data_ptr(), DT_F32, 0))
     for dt, tdt in ((DT_F16, torch.float16), (DT_BF16, torch.bfloat16)):
+        assert (f.tile(tokens, False, DT_F16, dt)[0] == "pair") == (k == 512)
         y16 = torch.full((tokens + 1, n), 7.0, device="cuda", dtype=tdt)  # one guard row behind the output
         torch.cuda.synchronize()
         ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, tokens, y16.data_ptr(), dt, 0))
@@ -201,7 +202,8 @@ def test_builtin_f32_and_q8_0_weights(ctx):
 
 
 @pytest.mark.parametrize("t,n,k,big", [(Q.Q4_0, 320, 704, 2600), (Q.Q8_0, 320, 704, 2600), (Q.Q4_K, 192, 768, 2600), (Q.Q6_K, 1088, 768, 1300),
-                                       (Q.F16, 320, 704, 2600), (Q.BF16, 320, 704, 2600), (Q.F16, 128, 64, 40000)],
+                                       (Q.F16, 320, 704, 2600), (Q.BF16, 320, 704, 2600), (Q.F16, 128, 64, 40000), (Q.Q4_0, 1088, 704, 2600),
+                                       (Q.Q8_0, 1088, 704, 2600), (Q.Q4_K, 1088, 768, 2600), (Q.Q6_K, 1088, 768, 2600), (Q.F16, 1088, 704, 2600)],
                          ids=lambda v: Q.NAMES.get(v, v) if isinstance(v, int) and v < 64 else str(v))
 def test_a_row_gets_the_same_bits_in_any_batch(ctx, t, n, k, big):
     """An output element is one accumulation chain whatever tile it falls into, so every tile kind, unpacking into shared memory
@@ -217,7 +219,11 @@ def test_a_row_gets_the_same_bits_in_any_batch(ctx, t, n, k, big):
     f.backward_input(dy, big, dx)
     rows = rng.integers(0, big, 64)
     assert rel_l2(y[rows], O.frozen_forward(t, n, k, packed, x[rows], 64)) < MATMUL_TOL
-    for m in (1, 31, 33, 64, 65, 157, 640, 1100):
+    sizes = (1, 31, 33, 64, 65, 157, 640, 1100)
+    if (n, big) == (1088, 2600):
+        kinds = {f.tile(m, backward)[0] for m in sizes + (big,) for backward in (False, True)}
+        assert f.tile(big)[0] == f.tile(big, True)[0] == "pair" and {"half", "narrow" if t == Q.F16 else "narrow_tmem"} <= kinds, kinds
+    for m in sizes:
         at = big - m
         assert np.array_equal(f.forward(x[at:], m), y[at:]), m
         part = np.zeros((m, k), np.float32)
@@ -226,33 +232,58 @@ def test_a_row_gets_the_same_bits_in_any_batch(ctx, t, n, k, big):
     f.close()
 
 
-@pytest.mark.parametrize("t", [Q.Q4_0, Q.Q8_0, Q.Q6_K], ids=lambda t: Q.NAMES[t])
-@pytest.mark.parametrize("m", [1, 32, 33, 64, 65, 127, 128, 129, 250])
-def test_slim_pair_tiles_at_their_edges(ctx, t, m):
+SLIM_ROWS = (1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 250)
+SLIM = [(t, 712, 6400, False, SLIM_ROWS) for t in (Q.Q4_0, Q.Q4_K, Q.Q6_K, Q.F16)]
+SLIM += [(Q.Q4_0, 6400, 672, True, SLIM_ROWS), (Q.Q4_K, 6400, 768, True, SLIM_ROWS), (Q.Q6_K, 6400, 768, True, SLIM_ROWS), (Q.F16, 6400, 712, True, SLIM_ROWS)]
+
+
+@pytest.mark.parametrize("t,n,k,backward,rows", SLIM, ids=[f"{Q.NAMES[c[0]]}-{c[1]}x{c[2]}" for c in SLIM])
+def test_slim_pair_tiles_at_their_edges(ctx, t, n, k, backward, rows):
     """Tiles of 128 weight rows over a CTA pair whose accumulator holds the two halves of the tokens in the two halves of its
-    lanes: tokens that end inside a tile, at its half and inside a block, rows that end inside a tile and inside a CTA's half,
-    an odd number of contraction steps; f32, 16-bit and accumulated results."""
+    lanes: tokens that end inside a tile, at its half and inside a block, rows that end inside a tile and inside a CTA's half;
+    f32, 16-bit (by TMA, and at an address it does not take) and accumulated results have the bits of 256-row pair tiles."""
     import torch
 
     from rust_trainer_b200._lib import DT_BF16, DT_F16, DT_F32, lib
 
-    L, n, k = lib(), 2 * 128 + 72, 1280 if t == Q.Q6_K else 19 * 64  # long enough for slim pairs to be the choice
-    g = torch.Generator(device="cuda").manual_seed(m)
-    packed = Q.quantize((np.random.default_rng(m).standard_normal((n, k)) * 0.05).astype(np.float32), t)
+    L, big = lib(), 2600
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    packed = Q.quantize((np.random.default_rng(n + k).standard_normal((n, k)) * 0.05).astype(np.float32), t)
     f = rt.Frozen(ctx, t, n, k, packed)
-    x, dy = (torch.randn(m, c, generator=g, device="cuda").half() for c in (k, n))
-    y, dx0 = (torch.randn(m + 1, c, generator=g, device="cuda") for c in (n, k))  # one guard row behind the results
-    y16, dx, guard = torch.full((m + 1, n), 7.0, device="cuda").bfloat16(), dx0.clone(), y[m].clone()
+    call = L.rt_frozen_backward_input_dev if backward else L.rt_frozen_forward_dev
+    ci, co = (n, k) if backward else (k, n)
+    x, want = torch.randn(big, ci, generator=g, device="cuda").half(), torch.empty(big, co, device="cuda")
     torch.cuda.synchronize()
-    ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, m, y.data_ptr(), DT_F32, 0))
-    ctx.check(L.rt_frozen_forward_dev(f._h, x.data_ptr(), DT_F16, m, y16.data_ptr(), DT_BF16, 0))
-    ctx.check(L.rt_frozen_backward_input_dev(f._h, dy.data_ptr(), DT_F16, m, dx.data_ptr(), DT_F32, 1))
+    ctx.check(call(f._h, x.data_ptr(), DT_F16, big, want.data_ptr(), DT_F32, 0))
     ctx.synchronize()
+    assert f.tile(big, backward)[0] == "pair"
     w = torch.from_numpy(O.dequant_rows(t, packed, n, k)).cuda().double()
-    assert rel_l2(y[:m].cpu().numpy(), (x.double() @ w.T).cpu().numpy()) < MATMUL_TOL
-    assert rel_l2((dx - dx0)[:m].cpu().numpy(), (dy.double() @ w).cpu().numpy()) < MATMUL_TOL
-    assert torch.equal(y16[:m], y[:m].bfloat16())
-    assert torch.equal(y[m], guard) and torch.equal(dx[m], dx0[m]) and bool((y16[m] == 7.0).all())
+    assert rel_l2(want[-250:].cpu().numpy(), (x[-250:].double() @ (w if backward else w.T)).cpu().numpy()) < MATMUL_TOL
+    widths = set()
+    for m in rows:
+        part, exp = x[big - m:], want[big - m:]
+
+        def run(out_dtype, out, accumulate=0):
+            kind, width = f.tile(m, backward, DT_F16, out_dtype)
+            assert kind == "slim", (m, kind)
+            widths.add(width)
+            torch.cuda.synchronize()
+            ctx.check(call(f._h, part.data_ptr(), DT_F16, m, out.data_ptr(), out_dtype, accumulate))
+            ctx.synchronize()
+
+        for dt, tdt in ((DT_F32, torch.float32), (DT_F16, torch.float16), (DT_BF16, torch.bfloat16)):
+            y = torch.full((m + 1, co), 7.0, device="cuda", dtype=tdt)  # one guard row behind the results
+            run(dt, y)
+            assert torch.equal(y[:m], exp.to(tdt)) and bool((y[m] == 7.0).all()), (m, dt)
+        odd = torch.full(((m + 1) * co + 1,), 7.0, device="cuda", dtype=torch.float16)[1:].view(m + 1, co)
+        run(DT_F16, odd)
+        assert torch.equal(odd[:m], exp.half()) and bool((odd[m] == 7.0).all()), m
+        base = torch.randn(m + 1, co, generator=g, device="cuda")
+        acc = base.clone()
+        run(DT_F32, acc, 1)
+        assert torch.equal(acc[:m], base[:m] + exp) and torch.equal(acc[m], base[m]), m
+    if rows is SLIM_ROWS:
+        assert widths == {32, 64, 128}
     f.close()
 
 

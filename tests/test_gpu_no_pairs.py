@@ -11,11 +11,15 @@ from rust_trainer_b200 import quants as Q
 
 pytestmark = pytest.mark.gpu
 CASES = [(Q.Q4_0, 320, 704, 2600), (Q.Q8_0, 1088, 704, 300), (Q.Q4_K, 192, 768, 2600), (Q.Q6_K, 1088, 768, 1300), (Q.F16, 320, 704, 2600), (Q.BF16, 256, 704, 97)]
+# pairs in both directions, and slim pairs in one, where there are pairs
+PAIRED = [(Q.Q4_0, 1088, 704, 2600), (Q.Q8_0, 1088, 704, 2600), (Q.Q4_K, 1280, 768, 2500), (Q.Q6_K, 1088, 1280, 2600), (Q.F16, 1088, 1024, 2600)]
+SLIM = [(Q.Q6_K, 6400, 256, 130)]
 
 
 def products(ctx):
-    out = []
-    for t, n, k, m in CASES:
+    """Results of every case, and the kind of tile of its products: forward and backward."""
+    out, kinds = [], []
+    for t, n, k, m in CASES + PAIRED + SLIM:
         rng = np.random.default_rng(n + k)
         f = rt.Frozen(ctx, t, n, k, Q.quantize((rng.standard_normal((n, k)) * 0.02).astype(np.float32), t))
         lin = rt.Linear("l", f, rng.standard_normal(n).astype(np.float32))
@@ -24,9 +28,10 @@ def products(ctx):
         dx = np.zeros((m, k), np.float32)
         f.backward_input(dy, m, dx)
         out += [f.forward(x, m), dx, lin.forward(x, m), lin.backward(x, dy, m)]
+        kinds.append([f.tile(m)[0], f.tile(m, True)[0]])
         lin.close()
         f.close()
-    return out
+    return out + [np.array(kinds)]
 
 
 def test_wide_tiles_give_the_bits_of_pairs(ctx, tmp_path):
@@ -35,5 +40,8 @@ def test_wide_tiles_give_the_bits_of_pairs(ctx, tmp_path):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=root, env=dict(os.environ, RT_B200_NO_PAIR="1"))
     got = np.load(tmp_path / "o.npz")
-    for i, w in enumerate(want):
-        assert np.array_equal(got[f"arr_{i}"], w), (CASES[i // 4], i % 4)
+    kinds, without, n = want[-1], got[f"arr_{len(want) - 1}"], len(PAIRED) + len(SLIM)
+    assert (kinds[-n:-len(SLIM)] == "pair").all() and (kinds[-len(SLIM):, 1] == "slim").all()
+    assert (without[-n:-len(SLIM)] == "wide").all() and not np.isin(without, ["pair", "slim"]).any()
+    for i, w in enumerate(want[:-1]):
+        assert np.array_equal(got[f"arr_{i}"], w), ((CASES + PAIRED + SLIM)[i // 4], i % 4)
