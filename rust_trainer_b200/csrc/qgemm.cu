@@ -1141,15 +1141,21 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 }
 
 // Which kernel and token-tile width a product gets: the one whose persistent grid is estimated to finish
-// first: the launch + rounds of tiles x (contraction steps x the step's time + a tile's own time).  The constants (us, 64
-// contraction elements a step) are fitted to times of every kind and width for 576 products (9 shapes of 128..8192 rows and
-// columns, both directions, 3..2048 tokens, four formats, weights from memory, launches that follow each other
-// programmatically); the launches of the pair kinds are given 1 to 2 us more than the fit, which they lose behind other
-// kernels than themselves.  What a step's time stands for: a pair's for its MMAs from about 200 tokens of width on and
-// for the hand-offs between the roles below; a slim pair's for shared memory; the narrow kinds' for one round of unpacking.
-// Slim pairs came in where narrow tiles ran before, at 1024 tokens (Q4_0 | Q6_K, the same unpack loop on both
-// sides): 6144x1024 backward 26.0 -> 18.8 | 30.3 -> 20.5 us, 4096x1024 backward 19.0 -> 14.7 | 21.7 -> 15.8,
-// 1024x3072 forward 14.0 -> 12.3 | 15.7 -> 13.3; 8192x3072 Q6_K backward at 24 tokens 24.5 -> 22.1 (half tiles before).
+// first: the launch + rounds of tiles x (contraction steps x the step's time + a tile's own time), in us, 64 contraction
+// elements a step.  The constants are fitted so that the choice is right, not each time: to every kind and width of 2880 products
+// (21 shapes of 128..16384 rows and columns, both directions, 1..8192 tokens, five formats, weights from memory), each
+// behind itself, where launches overlap, and behind a kernel that lets nothing start under it.  Against the best kind and
+// width of each, the choice is 0.9 % off on average (0.84 and 0.92 on the two halves of the products); 3 % of the products are off by
+// more than 10 % in one of the two, nearly all of them launches below 10 us, the worst by 26 % (4096x1024 Q8_0 at 100 tokens, 8.0
+// us on half tiles, 6.4 on narrow ones).  (Before, with 0.5 to 1 us more for the launch of pairs and slim pairs and a fourth more
+// for their steps, 3.0 % off, a tenth of the times by more than 10 %: 3072x1024 Q4_0 at 400 tokens on narrow tiles 10.4 us, and 14.7
+// behind a kernel that lets nothing start, on pairs 9.3 and 12.9.)
+// What a step's time stands for: a pair's for its MMAs from about 96 tokens of width on and for the hand-offs between the
+// roles below; a slim pair's for shared memory; half and narrow tiles' for one round of unpacking, which is
+// shortest for Q8_0's codes.
+// Slim pairs against narrow tiles at 1024 tokens, Q4_0 | Q6_K: 6144x1024 backward 25.6 -> 18.4 | 30.1 -> 20.5 us, 4096x1024 backward
+// 18.6 -> 14.1 | 21.4 -> 15.3, 1024x3072 forward 13.4 -> 11.9 | 15.2 -> 12.8; against half tiles, 8192x3072 Q6_K backward at 24
+// tokens 26.7 -> 24.2.
 // The choice changes no result: an output element's contraction is one chain in any tile.
 struct QPlan {
   int kind, TN;
@@ -1173,14 +1179,15 @@ static QPlan qgemm_plan(int kfmt, int dir, int M, int out_rows, int n_splits, in
     for (int tn = 256; tn >= 128; tn -= 32) consider(QK_WIDE, tn, 0.25 + 0.0012 * tn, 0.5, 0);
     return best;
   }
+  const bool q8 = kfmt == GGML_Q8_0;
   for (int tn = M > 32 ? 64 : 32; tn >= 32; tn -= 32) {
-    if (packed && dir == QG_FWD) consider(QK_NARROW_T, tn, 0.2, 0.4, 2.5);
-    else consider(QK_NARROW, tn, 0.23, 0.7, 2.3);
-    consider(QK_HALF, tn, 0.19, 0.6, 2.1);
+    if (packed && dir == QG_FWD) consider(QK_NARROW_T, tn, q8 ? 0.17 : 0.195, 0.4, 2.5);
+    else consider(QK_NARROW, tn, 0.23, 0.45, 2.7);
+    consider(QK_HALF, tn, (q8 ? 0.14 : packed ? 0.215 : 0.23) - (tn == 32 ? 0.01 : 0.0), 0.6, 2.1);
   }
   if (g_pair_workers > 0) {
-    for (int tn = M > 64 ? 128 : M > 32 || out16 ? 64 : 32; tn >= (out16 ? 64 : 32); tn /= 2) consider(QK_SLIM, tn, 0.16, 0.9, 4.6);
-    for (int tn = 256; tn >= 64 && M > 64; tn -= 32) consider(QK_PAIR, tn, 0.165 + 0.0008 * tn > 0.3 ? 0.165 + 0.0008 * tn : 0.3, 0.4, 5.5);
+    for (int tn = M > 64 ? 128 : M > 32 || out16 ? 64 : 32; tn >= (out16 ? 64 : 32); tn /= 2) consider(QK_SLIM, tn, packed ? 0.14 : 0.128, 0.87, packed ? 3.6 : 4.2);
+    for (int tn = 256; tn >= 64 && M > 64; tn -= 32) consider(QK_PAIR, tn, 0.146 + 0.0008 * tn > 0.218 ? 0.146 + 0.0008 * tn : 0.218, 0.4, 5.0);
   } else if (M > 64) {  // without pairs: 8192x3072 Q8_0 at 4096 tokens 171-181 us, 279-341 on 64-token tiles
     for (int tn = 256; tn >= 96; tn -= 32) consider(QK_WIDE, tn, 0.15 + 0.0012 * tn > 0.35 ? 0.15 + 0.0012 * tn : 0.35, 0.5, 2.4);
   }
