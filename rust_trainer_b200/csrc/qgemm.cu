@@ -5,8 +5,8 @@
 //
 // both read the SAME packed weight bytes (64x64 bricks of ggml codes, see qformat.cuh); no
 // dequantised copy of W exists in global memory.  The weight is the UMMA "A" operand (128
-// weight rows or columns per tile), the activations are the "B" operand (up to 256 tokens per
-// tile), so the TMEM accumulator is the transposed output tile [128 x tokens].
+// weight rows or columns per CTA, 64 in half tiles and slim pairs), the activations are the "B" operand (up
+// to 256 tokens per tile), so the TMEM accumulator is the transposed output tile [rows x tokens].
 //
 // One persistent CTA per SM, warp-specialised (23 warps, 15 without unpacking; roles by warp id, see the kernel):
 //   producer : one thread issues the TMA tiles of activations (and of 16-bit weights), 128B swizzle
@@ -36,14 +36,15 @@ enum QKind : int {
   QK_HALF = 3,    // one CTA per tile of 64 weight rows x up to 64 tokens
   // Narrow tiles of packed weights in the forward direction, with the unpacked weights in TMEM: a thread that owns a
   // weight row is the TMEM lane the MMA reads it from, and the weight tile no longer passes through shared
-  // memory twice.  1024x4096 in Q8_0 at 157 tokens 7.0 us, on slim pairs 8.2; at 64 tokens 5.8 and 6.5.  (Backward reads the
+  // memory twice.  4096x1024 in Q8_0 at 157 tokens 7.0 us, on slim pairs 8.3.  (Backward reads the
   // bricks down their columns: only the shared-memory operand can be read transposed.  Half tiles leave half of the
   // lanes, and so of the unpack warps, without a row.)
   QK_NARROW_T = 4,
   // A CTA pair per tile of 128 weight rows x up to 128 tokens: 64 rows of weights and half of the tokens in each CTA, so that a CTA
   // unpacks, writes and hands to the tensor core half the weights of a narrow tile for the same number of results.
-  // What bounds a narrow tile is shared memory: 128 rows written and read, 64 tokens written and read, the codes in and out,
-  // about 460 cycles of its 128 bytes a cycle for each 64 contraction elements, against 290 here.
+  // What bounds a narrow tile is shared memory: 128 rows written and read, 64 tokens written and read, the codes in and out, by
+  // its 128 bytes a cycle 420 cycles for each 64 contraction elements (Q4_0) against 290 here.  6144x1024 Q4_0 backward at 1024
+  // tokens, one round of 96 such steps: 25.6 us on narrow tiles, 18.4 on slim pairs.
   QK_SLIM = 5,
 };
 // How the results leave: a kernel holds the code of one way only (all of them in one kernel cost the small
@@ -77,7 +78,7 @@ struct QCfg {
   static constexpr int NUW = PACKED ? 16 : 8;
   // + activation / brick producers, MMA, 4 epilogue warps, and one idle where four unpack warps of each residue are needed
   static constexpr int THREADS = 32 * (7 + NUW + (TM ? 1 : 0));
-  // 64-element contraction steps per stage.  Two for narrow and half tiles: their MMAs are short, and one
+  // 64-element contraction steps per stage.  Two for narrow and half tiles and slim pairs: their MMAs are short, and one
   // hand-off between the roles costs about 500 cycles whatever it hands over.
   static constexpr int KS = NARROW || HALF || SLIM ? 2 : 1;
   // Activation / unpacked-weight stages, and packed-brick stages in the room that is left beside them and
@@ -130,7 +131,7 @@ struct KParams {
   int n_main, lora_mmas;
   int n_splits, steps_per_split;  // work item = (tile, piece of the contraction); partial results go to `part`
   float* part;                    // [n_splits][M][out_rows] f32 partials when n_splits > 1
-  int n_row_tiles, n_tok_tiles;   // a row tile is 128 weight rows, 256 for a CTA pair
+  int n_row_tiles, n_tok_tiles;   // a row tile is 128 weight rows, 256 for a pair, 64 for a half tile
   int tok_first;                  // a row tile's token tiles are neighbours, instead of a token tile's row tiles
   int inner;                      // tiles of a run of neighbours
   void* out;
@@ -273,6 +274,9 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
 //   bytes that TMA writes and the tensor core reads.  Barriers that gate the MMA (full, acc_empty)
 //   live in the leader and are arrived on from both CTAs; barriers the MMA releases (stage_empty,
 //   acc_full) exist in both CTAs and are signalled by one multicast commit.
+// SLIM: a pair that shares a tile of 128 weight rows: each CTA holds 64 of them and half of the tokens, and the MMA (M = 128
+//   over the pair) writes, in each CTA's TMEM, its 64 rows to lanes 0..63 for the first half of the tokens and to lanes 64..127
+//   for the second, in half as many columns.  All the rest is as for PAIR, which is set for both.
 template <int KIND, int FMT, int OUT>
 __global__ void __launch_bounds__((QCfg<KIND, FMT>::THREADS), 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w16,
