@@ -382,7 +382,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     if (PAIR) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
     else { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   }
-  if (warp == 2 && (p.late_wait || p.end_wait)) pdl_unwaited();
+  if (warp == 2 && (p.late_wait || p.end_wait) && (p.row_scale || (p.residual && OUT != QO_RES))) pdl_unwaited();
   tc_fence_before();
   __syncwarp();
   if (PAIR) cluster_sync_all();  // both CTAs' barriers are initialised and both hold their TMEM columns

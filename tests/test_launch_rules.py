@@ -24,7 +24,9 @@ def kernels():
     return out
 
 
-@pytest.mark.parametrize("name,when", [("qgemm_kernel", "warp == 2 && (p.late_wait || p.end_wait)"), ("attn_bwd_dq_tc_kernel", "warp == 0")])
+@pytest.mark.parametrize("name,when", [
+    ("qgemm_kernel", "warp == 2 && (p.late_wait || p.end_wait) && (p.row_scale || (p.residual && OUT != QO_RES))"),
+    ("attn_bwd_dq_tc_kernel", "warp == 0")])
 def test_what_is_read_without_a_wait_comes_after_an_acquire_fence(name, when):
     """Only the wait is defined to make earlier kernels' writes visible: without it an ordinary load may find an L1 line from
     before them.  One warp's fence in front of the CTA's barrier orders every warp's loads behind it."""
