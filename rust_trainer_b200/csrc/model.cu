@@ -69,9 +69,17 @@ static __half* lowrank_buf(DevBuf& b, int M) {
   return b.reserve(want <= b.bytes ? want : want + want / 2) ? b.as<__half>() : nullptr;
 }
 
+// out [M x 64] = X [M x K] . W^T, W [r x K]; 0 or not.  A matmul may start under it (QGemmArgs::late_wait).
+static int launch_lowrank(rt_ctx* c, const __half* x, const __half* w, int M, int K, int r, __half* out) {
+  // (what is not aligned the other launch refuses)
+  if (!lowrank_rows_takes(K, r) || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15)) return launch_lowrank_tc(c, x, w, M, K, r, out);
+  launch_lowrank_rows(x, M, K, LowRank{w, r, out}, c->stream);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
 rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out) {
   lora_refresh(l);
-  if (launch_lowrank_tc(l->ctx, x16, l->lora.a_s, M, l->in_dim(), l->lora.rank, hs_out))
+  if (launch_lowrank(l->ctx, x16, l->lora.a_s, M, l->in_dim(), l->lora.rank, hs_out))
     return l->ctx->fail(RT_ERR_CUDA, "lora H kernel launch failed");
   return RT_OK;
 }
@@ -126,7 +134,7 @@ rt_status lora_grads_flush(rt_ctx* c, LinearScratch& sc, int M) {
 
 rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16, const __half* dy16,
                               const float* dscale, int M, void* dx, int accumulate, const __half* hs_saved,
-                              bool unscaled_f16_out) {
+                              bool unscaled_f16_out, bool gs_ready) {
   rt_ctx* c = l->ctx;
   if (M <= 0) return RT_OK;
   if (unscaled_f16_out && accumulate) return c->fail(RT_ERR_BAD_ARG, "an unscaled f16 gradient cannot accumulate");
@@ -151,11 +159,11 @@ rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16
     // Hs = X . (sA)^T: recomputed as src/linear.rs:105 does, unless the caller kept it
     if (!hs_saved) RT_TRY(linear_lora_h(l, x16, M, hs));
     // Gs = dY~ . (sB)   (unit rows: the row scale is applied where Gs is consumed)
-    if (launch_lowrank_tc(c, dy16, l->lora.bt_s, M, N, r, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
+    if (!gs_ready && launch_lowrank(c, dy16, l->lora.bt_s, M, N, r, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
     a.lora.act = gs;
     a.lora.w = l->lora.a_h;
     a.lora.rank = r;
-    a.late_wait = 1;
+    a.late_wait = !gs_ready;
     // gb[N x r] += dY^T . Hs ; ga[r x K] += Gs^T . X   on the tensor cores, contraction over tokens
     job = LoraGradJob{hs, dy16, gs, x16, dscale, N, N, K, r, {{{l->lora.gb, l->lora.ga, 0, N, 0, r}}, 1}};
   }
@@ -202,6 +210,20 @@ static void group_refresh(LinGroup& g, cudaStream_t st) {
                               g.bt_s + (size_t)g.rank_off[i] * g.rows_total + g.row_off[i], (size_t)g.rows_total, st);
     g.seen[i] = lo.version;
   }
+}
+
+// The low-rank products of adapters that a row kernel makes beside their input: Hs of a linear (group) from its x, Gs from
+// its dy, into `out`; none without adapters.
+static LowRank lowrank_h(LinGroup& g, __half* out) {
+  bool any;
+  if (!group_lora_on(g, &any) || !any) return {};
+  group_refresh(g, g.lin[0]->ctx->stream);
+  return {g.a_s, g.rank_total, out};
+}
+static LowRank lowrank_g(rt_linear* l, __half* out) {
+  if (!l->lora_active()) return {};
+  lora_refresh(l);
+  return {l->lora.bt_s, l->lora.rank, out};
 }
 
 // Rebuilds, in one launch, every 16-bit adapter copy the next pass over the model will read and
@@ -295,7 +317,7 @@ rt_status group_forward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, i
     __half* hs = hs_keep ? hs_keep : lowrank_buf(sc.hs, M);
     if (!hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
     if (!(hs_keep && hs_ready)) {
-      if (launch_lowrank_tc(c, x16, g.a_s, M, g.w.cols, g.rank_total, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
+      if (launch_lowrank(c, x16, g.a_s, M, g.w.cols, g.rank_total, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
       a.late_wait = 1;
     }
     a.lora.act = hs;
@@ -310,7 +332,7 @@ rt_status group_forward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, i
 // dx[M x K] (+)= dY[M x rows_total] . [W_0; W_1; ..] (+ Gs . A), dY row-normalised with ONE factor per token
 // for the whole row; each member's dA, dB from its slices.
 rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, const __half* dy16, const float* dscale,
-                             int M, float* dx, int accumulate, const __half* hs_saved, bool last) {
+                             int M, float* dx, int accumulate, const __half* hs_saved, bool last, bool gs_ready) {
   rt_ctx* c = g.lin[0]->ctx;
   if (M <= 0) return RT_OK;
   const int K = g.w.cols, NT = g.rows_total;
@@ -332,8 +354,8 @@ rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, 
     __half* hs = hs_saved ? const_cast<__half*>(hs_saved) : lowrank_buf(sc.hs, M);
     __half* gs = lowrank_buf(sc.gs[sc.n_jobs], M);
     if (!hs || !gs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-    if (!hs_saved && launch_lowrank_tc(c, x16, g.a_s, M, K, R, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
-    if (launch_lowrank_tc(c, dy16, g.bt_s, M, NT, R, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
+    if (!hs_saved && launch_lowrank(c, x16, g.a_s, M, K, R, hs)) return c->fail(RT_ERR_CUDA, "lora H kernel launch failed");
+    if (!gs_ready && launch_lowrank(c, dy16, g.bt_s, M, NT, R, gs)) return c->fail(RT_ERR_CUDA, "lora G kernel launch failed");
     job = LoraGradJob{hs, dy16, gs, x16, dscale, NT, NT, K, R, {}};
     job.t.n = 0;
     for (int i = 0; i < g.n; ++i) {
@@ -343,7 +365,7 @@ rt_status group_backward_dev(LinGroup& g, LinearScratch& sc, const __half* x16, 
     a.lora.act = gs;
     a.lora.w = g.a_h;
     a.lora.rank = R;
-    a.late_wait = 1;
+    a.late_wait = !gs_ready;
   }
   if (any && last) {  // the block's gradients run first: the matmul needs nothing of theirs and starts beside them
     RT_TRY(lora_grads_add(c, sc, job, M));
@@ -1083,6 +1105,21 @@ static rt_status ensure_rope(rt_model* m, int max_pos) {
 
 
 
+// RMSNorm, and the low-rank product of what it writes where `lr` asks for it.
+static rt_status norm_forward(rt_model* m, const float* x, const float* w, int M, __half* y16, const LowRank& lr) {
+  const rt_model_config& g = m->cfg;
+  if (!lr.w) launch_rmsnorm_fwd(x, w, M, g.hidden, g.rms_eps, y16, m->ctx->stream);
+  else if (launch_rmsnorm_fwd_lr(m->ctx, x, w, M, g.hidden, g.rms_eps, y16, lr)) return m->ctx->fail(RT_ERR_CUDA, "RMSNorm launch failed");
+  return RT_OK;
+}
+static rt_status norm_backward(rt_model* m, const float* x, const float* w, int M, __half* dy16, float* sc, const LowRank& lr) {
+  const rt_model_config& g = m->cfg;
+  float *dx = m->dx.as<float>(), *dn = m->dn.as<float>();
+  if (!lr.w) launch_rmsnorm_bwd(x, w, dn, dx, M, g.hidden, g.rms_eps, dx, dy16, sc, m->ctx->stream);
+  else if (launch_rmsnorm_bwd_lr(m->ctx, x, w, dn, dx, M, g.hidden, g.rms_eps, dx, dy16, sc, lr)) return m->ctx->fail(RT_ERR_CUDA, "RMSNorm backward launch failed");
+  return RT_OK;
+}
+
 // Block::forward (src/model.rs:165-183).  x_in is read only; h receives x_in + attention;
 // when x_out is non-null it receives the block output (h + mlp), and may alias h.  With `keep`
 // the adapters' Hs = X.(sA)^T are left in A.hs for the block's backward.
@@ -1096,9 +1133,14 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   BlockDev& b = m->blocks[li];
   cudaStream_t st = c->stream;
   const int d = g.hidden;
-  launch_rmsnorm_fwd(x_in, b.input_norm, M, d, g.rms_eps, A.n1, st);
+  __half* scratch_hs = keep ? nullptr : lowrank_buf(m->lsc.hs, M);
+  if (!keep && !scratch_hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
+  auto hs_at = [&](int i) { return keep ? A.hs[i] : scratch_hs; };
+  LowRank lr;  // made where the linear's input is made, and not a second time
+  if (A.qkv_group && !hs_ready && rmsnorm_takes_lowrank(d, b.qkv.rank_total)) lr = lowrank_h(b.qkv, hs_at(0));
+  RT_TRY(norm_forward(m, x_in, b.input_norm, M, A.n1, lr));
   if (A.qkv_group) {
-    RT_TRY(group_forward_dev(b.qkv, m->lsc, A.n1, M, A.q_raw, RT_DT_F32, keep ? A.hs[0] : nullptr, hs_ready));
+    RT_TRY(group_forward_dev(b.qkv, m->lsc, A.n1, M, A.q_raw, RT_DT_F32, hs_at(0), hs_ready || lr.w));
   } else {
     RT_TRY(linear_forward_dev(b.lin[0], m->lsc, A.n1, M, A.q_raw, RT_DT_F32, 0, keep ? A.hs[0] : nullptr, hs_ready));
     RT_TRY(linear_forward_dev(b.lin[1], m->lsc, A.n1, M, A.k_raw, RT_DT_F32, 0, keep ? A.hs[1] : nullptr, hs_ready));
@@ -1111,9 +1153,11 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
     return c->fail(RT_ERR_CUDA, "attention forward launch failed");
   // the residual comes in where the product goes out: in place, or from the buffer that keeps it
   RT_TRY(linear_forward_dev(b.lin[3], m->lsc, A.o16, M, h, RT_DT_F32, h == x_in, keep ? A.hs[3] : nullptr, hs_ready, h == x_in ? nullptr : x_in));
-  launch_rmsnorm_fwd(h, b.post_norm, M, d, g.rms_eps, A.n2, st);
+  lr = {};
+  if (A.gu_group && !hs_ready && rmsnorm_takes_lowrank(d, b.gu.rank_total)) lr = lowrank_h(b.gu, hs_at(4));
+  RT_TRY(norm_forward(m, h, b.post_norm, M, A.n2, lr));
   if (A.gu_group) {
-    RT_TRY(group_forward_dev(b.gu, m->lsc, A.n2, M, A.g16, RT_DT_F16, keep ? A.hs[4] : nullptr, hs_ready));
+    RT_TRY(group_forward_dev(b.gu, m->lsc, A.n2, M, A.g16, RT_DT_F16, hs_at(4), hs_ready || lr.w));
   } else {
     RT_TRY(linear_forward_dev(b.lin[4], m->lsc, A.n2, M, A.g16, RT_DT_F16, 0, keep ? A.hs[4] : nullptr, hs_ready));
     RT_TRY(linear_forward_dev(b.lin[5], m->lsc, A.n2, M, A.u16, RT_DT_F16, 0, keep ? A.hs[5] : nullptr, hs_ready));
@@ -1127,9 +1171,20 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   return RT_OK;
 }
 
+// Gs of the linear whose backward comes next, to be made where RMSNorm's backward makes its dy; none where that kernel does
+// not take it.
+static rt_status lowrank_from_gradient(rt_model* m, rt_linear* l, int M, LowRank* lr) {
+  if (!l->lora_active() || !rmsnorm_takes_lowrank(m->cfg.hidden, l->lora.rank)) return RT_OK;
+  __half* gs = lowrank_buf(m->lsc.gs[m->lsc.n_jobs], M);
+  if (!gs) return m->ctx->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
+  *lr = lowrank_g(l, gs);
+  return RT_OK;
+}
+
 // Block::backward (src/model.rs:185-197).  On entry dx holds the gradient of the block output
-// and (dy16, sc_y) its row-normalised f16 copy; on exit both describe the block input's.
-static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, const BlockActs& A) {
+// and (dy16, sc_y) its row-normalised f16 copy; on exit both describe the block input's.  gs_ready: Gs of the block's last
+// linear has been made beside dy16; next_gs_ready: the block below's has.
+static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, const BlockActs& A, bool gs_ready, bool* next_gs_ready) {
   rt_ctx* c = m->ctx;
   const rt_model_config& g = m->cfg;
   BlockDev& b = m->blocks[li];
@@ -1143,14 +1198,14 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   m->lsc.n_jobs = 0;
   // Mlp::backward (src/model.rs:120-134)
   // d(hm) leaves the matmul as f16 rows still lacking sc_y: SwiGLU's backward folds the factor into its own scales
-  RT_TRY(linear_backward_dev(b.lin[6], m->lsc, A.hm16, dy16, sc_y, M, m->dhm.p, 0, HS(6), true));
+  RT_TRY(linear_backward_dev(b.lin[6], m->lsc, A.hm16, dy16, sc_y, M, m->dhm.p, 0, HS(6), true, gs_ready));
   const size_t T = (size_t)M, ff = g.ff;
   __half* dg16 = m->dg16.as<__half>();
   __half* du16 = A.gu_group ? dg16 + ff : dg16 + T * ff;
   launch_swiglu_bwd(m->dhm.p, 1, sc_y, A.g16, A.u16, A.gu_pitch, M, g.ff, dg16, du16, A.gu_pitch, m->sc_g.as<float>(),
                     m->sc_u.as<float>(), st);
   if (A.gu_group) {
-    RT_TRY(group_backward_dev(b.gu, m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4), false));
+    RT_TRY(group_backward_dev(b.gu, m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4), false, false));
   } else {
     RT_TRY(linear_backward_dev(b.lin[4], m->lsc, A.n2, dg16, m->sc_g.as<float>(), M, m->dn.as<float>(), 0, HS(4)));
     RT_TRY(linear_backward_dev(b.lin[5], m->lsc, A.n2, du16, m->sc_u.as<float>(), M, m->dn.as<float>(), 1, HS(5)));
@@ -1158,10 +1213,12 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   // dh = dy + rmsnorm_backward(h, post_norm, dn2)
   __half* dy16o = m->dy16o.as<__half>();
   float* sc_yo = m->sc_yo.as<float>();
-  launch_rmsnorm_bwd(A.h, b.post_norm, m->dn.as<float>(), dx, M, d, g.rms_eps, dx, dy16o, sc_yo, st);
+  LowRank lr;
+  RT_TRY(lowrank_from_gradient(m, b.lin[3], M, &lr));
+  RT_TRY(norm_backward(m, A.h, b.post_norm, M, dy16o, sc_yo, lr));
   // Attention::backward (src/attention.rs:246-367)
   // d(attention output) leaves the matmul as f16 rows still lacking sc_yo; the attention backward takes the factors per query row
-  RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16o, sc_yo, M, m->dO16.p, 0, HS(3), true));
+  RT_TRY(linear_backward_dev(b.lin[3], m->lsc, A.o16, dy16o, sc_yo, M, m->dO16.p, 0, HS(3), true, lr.w));
   if (launch_attn_bwd_tc(c, A.q16, A.k16, A.v16, A.o16, m->dO16.as<__half>(), sc_yo, A.lse, m->attn_batch(M), g.n_heads, g.n_kv_heads,
                          g.head_dim, m->delta.as<float>(), m->dq.as<float>(), m->dk.as<float>(), m->dv.as<float>()))
     return c->fail(RT_ERR_CUDA, "attention backward launch failed");
@@ -1174,7 +1231,7 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
                      m->rope_sin.as<float>(), M, g.n_heads, g.n_kv_heads, g.head_dim, g.rot_dim, g.rope_neox, g.rms_eps,
                      dq16, dk16, dv16, A.qkv_pitch, m->sc_q.as<float>(), m->sc_k.as<float>(), m->sc_v.as<float>(), st);
   if (A.qkv_group) {
-    RT_TRY(group_backward_dev(b.qkv, m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0), true));
+    RT_TRY(group_backward_dev(b.qkv, m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0), true, false));
   } else {
     RT_TRY(linear_backward_dev(b.lin[0], m->lsc, A.n1, dq16, m->sc_q.as<float>(), M, m->dn.as<float>(), 0, HS(0)));
     RT_TRY(linear_backward_dev(b.lin[1], m->lsc, A.n1, dk16, m->sc_k.as<float>(), M, m->dn.as<float>(), 1, HS(1)));
@@ -1183,7 +1240,10 @@ static rt_status block_backward(rt_model* m, int li, int M, const float* x_in, c
   m->lsc.defer = false;
   RT_TRY(lora_grads_flush(c, m->lsc, M));  // before dy16, the first of the gradients it reads, is overwritten
   // dx = dh + rmsnorm_backward(x, input_norm, dn1)
-  launch_rmsnorm_bwd(x_in, b.input_norm, m->dn.as<float>(), dx, M, d, g.rms_eps, dx, dy16, sc_y, st);
+  lr = {};
+  if (li > 0) RT_TRY(lowrank_from_gradient(m, m->blocks[li - 1].lin[6], M, &lr));
+  RT_TRY(norm_backward(m, x_in, b.input_norm, M, dy16, sc_y, lr));
+  *next_gs_ready = lr.w;
 #undef HS
   return RT_OK;
 }
@@ -1333,11 +1393,12 @@ static rt_status run_staged_body(rt_model* m, bool backward, float* logits_out_h
   else RT_CUDA(c, cudaMemsetAsync(m->hits(), 0, 4, st));
   if (!backward) return RT_OK;
   launch_normalize_rows(m->dx.as<float>(), M, g.hidden, m->dy16.as<__half>(), m->sc_y.as<float>(), st);
+  bool gs_ready = false;
   for (int li = g.n_layers - 1; li >= 0; --li) {
     const float* x_in = m->ckpt.as<float>() + (size_t)li * xd;
     const BlockActs A = block_acts(m, li, M, store);
     if (!store) RT_TRY(block_forward(m, li, M, x_in, A.h, nullptr, A, 2));  // rebuild the block's caches (Hs is still there)
-    RT_TRY(block_backward(m, li, M, x_in, A));
+    RT_TRY(block_backward(m, li, M, x_in, A, gs_ready, &gs_ready));
   }
   return RT_OK;
 }

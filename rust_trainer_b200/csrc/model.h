@@ -77,10 +77,10 @@ rt_status linear_forward_dev(rt_linear* l, LinearScratch& sc, const __half* x16,
 rt_status linear_lora_h(rt_linear* l, const __half* x16, int M, __half* hs_out);
 // dy16 is row-normalised f16 with per-row scales `dscale` (null = all ones).  With
 // unscaled_f16_out, dx receives f16 rows WITHOUT their factor dscale[row] (the consumer applies
-// it): half the output bytes, no accumulate.
+// it): half the output bytes, no accumulate.  gs_ready: Gs lies in sc.gs[sc.n_jobs] already.
 rt_status linear_backward_dev(rt_linear* l, LinearScratch& sc, const __half* x16, const __half* dy16,
                               const float* dscale, int M, void* dx, int accumulate,
-                              const __half* hs_saved = nullptr, bool unscaled_f16_out = false);
+                              const __half* hs_saved = nullptr, bool unscaled_f16_out = false, bool gs_ready = false);
 // computes the adapter gradients that are waiting in `sc`
 rt_status lora_grads_flush(rt_ctx* c, LinearScratch& sc, int M);
 rt_status lora_refresh(rt_linear* l);

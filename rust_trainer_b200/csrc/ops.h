@@ -1,5 +1,6 @@
 // Launchers of the memory-bound device ops (ops.cu) and attention (attention.cu).
 #pragma once
+#include "lowrank_rows.cuh"
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -15,6 +16,12 @@ void launch_normalize_rows(const float* x, int rows, int d, __half* y16, float* 
 void launch_rmsnorm_fwd(const float* x, const float* w, int rows, int d, float eps, __half* y16, cudaStream_t st);
 void launch_rmsnorm_bwd(const float* x, const float* w, const float* dn, const float* dres, int rows, int d, float eps,
                         float* out, __half* out16, float* scale, cudaStream_t st);
+// ..._lr: with the low-rank product of the 16-bit rows, in the same launch, for the shapes that takes_lowrank says (16-byte aligned
+// operands); what a row gets is the same in any batch; 0 or 3 (launch failure).
+bool rmsnorm_takes_lowrank(int d, int r);
+int launch_rmsnorm_fwd_lr(rt_ctx* c, const float* x, const float* w, int rows, int d, float eps, __half* y16, const LowRank& lr);
+int launch_rmsnorm_bwd_lr(rt_ctx* c, const float* x, const float* w, const float* dn, const float* dres, int rows, int d, float eps,
+                          float* out, __half* out16, float* scale, const LowRank& lr);
 void launch_rope_table(const float* inv_freq, int half, int max_pos, float* cs, float* sn, cudaStream_t st);
 // raw_pitch / out_pitch = 0: q, k, v are separate row-major matrices.  Otherwise they are column
 // slices of ONE matrix with that row pitch (elements); with out_pitch the three f16 outputs also
@@ -65,6 +72,9 @@ void launch_adamw(float* p, float* g, float* m, float* v, size_t n, const double
                   float beta1, float beta2, float eps, float wd, float bc1, float bc2, float* norm_out,
                   cudaStream_t st);
 
+// lr.out = the low-rank product of X [rows x K]; a matmul may start under it (QGemmArgs::late_wait)
+bool lowrank_rows_takes(int K, int r);
+void launch_lowrank_rows(const __half* x, int rows, int K, const LowRank& lr, cudaStream_t st);
 // ---- lowrank_tc.cu: out64[M x 64] (f16, zero from column r up) = X[M x K] . Wt[r x K]^T on tcgen05; 1 = shape not taken
 int launch_lowrank_tc(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64);
 // A linear's (or a stacked group's) adapters as the token contractions see them: member j owns rows

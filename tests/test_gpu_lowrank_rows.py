@@ -1,0 +1,70 @@
+"""The adapters' low-rank products inside the RMSNorm kernels and over rows in memory (csrc/lowrank_rows.cuh): every group count of
+rank indices, row lengths with full and ragged shares of K, batches that end inside a group of eight tokens, and both forms of each
+kernel (up to 2048 tokens and beyond) against each other."""
+import numpy as np
+import pytest
+
+import rust_trainer_b200 as rt
+from conftest import cosine, rel_l2
+from oracle import oracle as O
+from rust_trainer_b200 import synth
+from test_gpu_model import GRAD_COS, GRAD_TOL, LOSS_TOL, _batch, _flat, _gpu_flat, _oracle_step
+
+pytestmark = pytest.mark.gpu
+
+
+def _spec(hidden, seed=5):
+    return synth.preset("tiny-qwen3", quant="Q8_0", seed=seed, w_std=0.05, hidden=hidden)
+
+
+def _model(ctx, spec, rank):
+    tensors = synth.build_tensors(spec)
+    synth.perturb_norms(tensors, 7)
+    ads = synth.lora_adapters(spec, rank, 2.0 * rank, seed=9, b_std=0.02)
+    gm = rt.Model(ctx, spec.config(), tensors)
+    gm.attach_lora(rank, 2.0 * rank, None, 1)
+    gm.load_adapters(ads)
+    return tensors, ads, gm
+
+
+# hidden sizes: one block of K per warp and fewer, 28 blocks on eight warps, the widest; ranks: 1 to 64 of a linear, 24 to 64 of a stack
+@pytest.mark.parametrize("hidden,rank,lens", [(128, 8, [1 + 8]), (384, 1, [7, 2]), (640, 24, [17]), (896, 16, [70, 3]), (1024, 32, [33, 8]),
+                                              (1024, 64, [5, 60]), (256, 40, [41])])
+def test_gradients_match_the_oracle(ctx, hidden, rank, lens):
+    spec = _spec(hidden)
+    tensors, ads, gm = _model(ctx, spec, rank)
+    om = O.OracleModel(spec.config(), tensors)
+    om.attach_lora(ads)
+    seqs, tp, tt, per_seq = _batch(spec, lens, seed=11)
+    w = np.full(tp.size, 1.0 / tp.size, np.float32)
+    lp_o = _oracle_step(om, seqs, per_seq, w)
+    gm.zero_grad()
+    lp_g, _ = gm.forward_backward(seqs, tp, tt, w)
+    assert np.max(np.abs(lp_g - lp_o) / np.abs(lp_o)) < LOSS_TOL
+    go, gg = _flat(om.lora, "ga", "gb"), _gpu_flat(gm, "ga", "gb")
+    assert rel_l2(gg, go) < GRAD_TOL and cosine(gg, go) > GRAD_COS
+    for lin, e in zip(gm.lora_linears(), om.lora):
+        g = lin.lora()
+        assert cosine(np.concatenate([g["ga"].ravel(), g["gb"].ravel()]), np.concatenate([e["ga"].ravel(), e["gb"].ravel()])) > GRAD_COS
+    gm.close()
+    om.close()
+
+
+@pytest.mark.parametrize("hidden,rank,more", [(1024, 16, 17), (896, 8, 20), (128, 64, 63), (1024, 32, 17)])
+def test_a_sequence_gets_the_same_products_in_a_small_and_a_large_batch(ctx, hidden, rank, more):
+    """One sequence of 128 tokens alone, and as the first of a batch of more than 2048 whose other targets have no weight."""
+    spec = _spec(hidden)
+    _, _, gm = _model(ctx, spec, rank)
+    toks = synth.token_batch(spec, more + 1, 128, 3)
+    tp, tt = synth.answer_targets(toks[0], 64)
+    w = np.full(tp.size, 1.0 / tp.size, np.float32)
+    gm.zero_grad()
+    alone, _ = gm.forward_backward([toks[0]], tp, tt, w)
+    g_alone = _gpu_flat(gm, "ga", "gb")
+    gm.zero_grad()
+    many, _ = gm.forward_backward(list(toks), np.concatenate([tp, tp + 128]), np.concatenate([tt, tt]), np.concatenate([w, 0 * w]))
+    assert np.array_equal(alone, many[:tp.size])
+    # the gradients' last f32 sums (over key tiles, over splits of tokens) fall differently, a few 2^-24; another rounding of a
+    # 16-bit product anywhere would show as 2^-12 of its value
+    assert rel_l2(_gpu_flat(gm, "ga", "gb"), g_alone) < 1e-6 and np.abs(g_alone).max() > 0
+    gm.close()
