@@ -46,8 +46,8 @@ struct LrWeights {
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
       const __half* p = w + (size_t)(16 * m + g) * K + k + 8 * q;
-      lo[m] = 16 * m + g < r ? __ldg((const uint4*)p) : make_uint4(0, 0, 0, 0);
-      hi[m] = 16 * m + g + 8 < r ? __ldg((const uint4*)(p + (size_t)8 * K)) : make_uint4(0, 0, 0, 0);
+      lo[m] = 16 * m + g < r ? *(const uint4*)p : make_uint4(0, 0, 0, 0);
+      hi[m] = 16 * m + g + 8 < r ? *(const uint4*)(p + (size_t)8 * K) : make_uint4(0, 0, 0, 0);
     }
   }
 };

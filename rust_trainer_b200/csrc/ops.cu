@@ -309,7 +309,7 @@ struct RmsLr {
 };
 template <int NV, int MT, int NT>
 __global__ void __launch_bounds__(256 * NT, (RmsLr<NV, MT, NT>::FWD_CTAS))
-rmsnorm_fwd_lr_kernel(const float* __restrict__ x, const float* __restrict__ w, int rows, float eps, __half* __restrict__ y16,
+rmsnorm_fwd_lr_kernel(const float* x, const float* __restrict__ w, int rows, float eps, __half* __restrict__ y16,
                       const LowRank lr) {
   using C = RmsLr<NV, MT, NT>;
   extern __shared__ __align__(16) uint8_t lr_smem[];
@@ -340,7 +340,7 @@ rmsnorm_fwd_lr_kernel(const float* __restrict__ x, const float* __restrict__ w, 
 }
 template <int NV, int MT, bool SHARED>
 __global__ void __launch_bounds__(256, (SHARED ? RmsLr<NV, MT, 1>::BWD_CTAS : 1))
-rmsnorm_bwd_lr_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ dn, const float* dres, int rows,
+rmsnorm_bwd_lr_kernel(const float* x, const float* __restrict__ w, const float* dn, const float* dres, int rows,
                       float eps, float* out, __half* __restrict__ out16, float* __restrict__ scale, const LowRank lr) {
   using C = RmsLr<NV, MT, 1>;
   extern __shared__ __align__(16) uint8_t lr_smem[];
@@ -1353,7 +1353,7 @@ void launch_swiglu_fwd(const __half* g, const __half* u, size_t in_pitch, int ro
 // 16.3).  2048 columns, 16 indices, in a step of 1024 tokens 5.8 -> 3.6 us, of 8192 as fast.
 constexpr int LR_WARPS = 16;
 template <int NT>
-__global__ void __launch_bounds__(32 * LR_WARPS) lowrank_rows_kernel(const __half* __restrict__ x, int K, int rows, const LowRank lr) {
+__global__ void __launch_bounds__(32 * LR_WARPS) lowrank_rows_kernel(const __half* x, int K, int rows, const LowRank lr) {
   __shared__ __align__(16) float sums[lr_sum_floats(LR_WARPS, 1)];
   lr_prefetch(lr.w, lr.r, K);
   pdl_wait();
