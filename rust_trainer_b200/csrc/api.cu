@@ -24,11 +24,11 @@ void* rt_ctx::get_scratch(int slot, size_t bytes) {
 }
 
 rt_status rt_ctx::check_device_status(const char* where) {
-  cudaError_t e = cudaMemcpyAsync(status_host, status_dev, sizeof(int), cudaMemcpyDeviceToHost, stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  const cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, where);
-  int s = *status_host;
+  const int s = *(volatile int*)status_host;  // written by the kernel that reported it (StatusBlock)
   if (s == 0) return RT_OK;
+  *(volatile int*)status_host = 0;
   cudaMemsetAsync(status_dev, 0, sizeof(int), stream);
   char buf[160];
   if (s == RT_ERR_BAD_INDEX) {
@@ -167,10 +167,14 @@ rt_status rt_ctx_create(int device, rt_ctx** out) {
   }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   c->stream = c->own_stream;
-  if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->status_dev, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the clear ran on the legacy stream; own_stream does not wait for it
+  if (e == cudaSuccess) e = cudaMalloc(&c->status_dev, sizeof(rt::StatusBlock));
   if (e == cudaSuccess) e = cudaMallocHost(&c->status_host, 2 * sizeof(int));
+  if (e == cudaSuccess) {
+    c->status_host[0] = c->status_host[1] = 0;
+    const rt::StatusBlock block = {0, 0, c->status_host};
+    e = cudaMemcpy(c->status_dev, &block, sizeof block, cudaMemcpyHostToDevice);
+  }
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();  // the copy ran on the legacy stream; own_stream does not wait for it
   if (e != cudaSuccess || rt::qgemm_init() != RT_OK) {
     fprintf(stderr, "rt_b200: context creation failed: %s\n", cudaGetErrorString(e));
     delete c;

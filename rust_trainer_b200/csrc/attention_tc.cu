@@ -78,7 +78,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   pdl_launch_dependents();
   if (pad + L::USED > L::TOTAL) {
     pdl_wait();
-    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_CUDA);
+    if (threadIdx.x == 0) report_status(status, RT_ERR_CUDA);
     return;
   }
   uint8_t* sm = smem_raw + pad;
@@ -728,7 +728,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   pdl_launch_dependents();
   if (pad + L::USED > L::TOTAL) {
     pdl_wait();
-    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_CUDA);
+    if (threadIdx.x == 0) report_status(status, RT_ERR_CUDA);
     return;
   }
   uint8_t* sm = smem_raw + pad;

@@ -13,8 +13,8 @@ struct rt_ctx {
   int num_sms = 0;
   cudaStream_t stream = nullptr;       // the stream in use (own_stream unless the host set one)
   cudaStream_t own_stream = nullptr;
-  int* status_dev = nullptr;   // device word the kernels report bounded-wait failures into
-  int* status_host = nullptr;  // pinned: the mirror of that word, then one word for a scalar result
+  int* status_dev = nullptr;   // the StatusBlock (ptx.cuh) that kernels report into
+  int* status_host = nullptr;  // page-locked, written by kernels: the reported code, then one word for a scalar result
   std::string err;
   uint64_t launches = 0;       // kernels launched through this ctx
   bool profiling = false;

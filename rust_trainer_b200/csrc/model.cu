@@ -837,8 +837,8 @@ rt_status rt_model_finalize(rt_model* m) {
     for (int i = 0; i < 7; ++i)
       if (!b.lin[i]) { snprintf(buf, sizeof buf, "blk.%d.%s.weight missing", li, LIN_NAMES[i]); return c->fail(RT_ERR_BAD_ARG, buf); }
   }
-  // opt_scalars: [0,1024) f64 partials, [1024] f64 sum, then one f32 norm
-  if (!m->opt_scalars.reserve(1025 * sizeof(double) + 16)) return c->fail(RT_ERR_CUDA, "out of device memory");
+  // opt_scalars: [0,1024) f64 partials, [1024] f64 sum
+  if (!m->opt_scalars.reserve(1025 * sizeof(double))) return c->fail(RT_ERR_CUDA, "out of device memory");
   if (!m->finalized) {
     const char* e = getenv("RT_B200_NO_GROUPS");  // measurement aid: one matmul per projection
     if (!(e && e[0] == '1'))
@@ -1598,16 +1598,15 @@ rt_status rt_optim_step(rt_model* m, float lr, float max_norm, float beta1, floa
   cudaStream_t st = c->stream;
   double* part = m->opt_scalars.as<double>();
   double* sum = part + 1024;
-  float* normd = (float*)(sum + 1);
+  float* norm = (float*)(c->status_host + 1);  // page-locked: the kernel writes it where it is read
   launch_sumsq(m->G.as<float>(), m->n_params, part, sum, st);
   m->opt_t += 1;
   const float bc1 = 1.0f - powf(beta1, (float)m->opt_t), bc2 = 1.0f - powf(beta2, (float)m->opt_t);
   launch_adamw(m->P.as<float>(), m->G.as<float>(), m->Mo.as<float>(), m->Vo.as<float>(), m->n_params, sum, max_norm, lr,
-               beta1, beta2, eps, wd, bc1, bc2, normd, st);
+               beta1, beta2, eps, wd, bc1, bc2, norm, st);
   for (rt_linear* l : m->lora_order) { l->lora.stale = true; ++l->lora.version; }
-  RT_CUDA(c, cudaMemcpyAsync(c->status_host + 1, normd, 4, cudaMemcpyDeviceToHost, st));
   rt_status s = c->check_device_status("rt_optim_step");
-  if (norm_out) memcpy(norm_out, c->status_host + 1, 4);
+  if (norm_out) *norm_out = *(volatile float*)norm;
   return s;
 }
 

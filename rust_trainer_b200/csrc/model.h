@@ -127,7 +127,7 @@ struct rt_model {
 
   // flat LoRA state: [A_0 | B_0 | A_1 | B_1 ...] in parameter order
   size_t n_params = 0;
-  DevBuf P, G, Mo, Vo, opt_scalars;  // opt_scalars: 1024 f64 partials + 1 f64 sum + 1 f32 norm
+  DevBuf P, G, Mo, Vo, opt_scalars;  // opt_scalars: 1024 f64 partials + 1 f64 sum
   uint64_t opt_t = 0;
 
   // RoPE tables

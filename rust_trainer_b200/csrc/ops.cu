@@ -1316,12 +1316,12 @@ __global__ void swiglu_fwd_kernel(const __half* __restrict__ g, const __half* __
   if (i + 7 < n) {
     const uint4 o = swiglu8(*(const uint4*)(g + i), *(const uint4*)(u + i));
     *(uint4*)(h + i) = o;
-    if (status && any_nonfinite_f16x8(o)) atomicCAS(status, 0, RT_ERR_NONFINITE);
+    if (status && any_nonfinite_f16x8(o)) report_status(status, RT_ERR_NONFINITE);
   } else {
     for (; i < n; ++i) {
       const __half v = __float2half_rn(silu_f(__half2float(g[i])) * __half2float(u[i]));
       h[i] = v;
-      if (status && (__hisinf(v) || __hisnan(v))) atomicCAS(status, 0, RT_ERR_NONFINITE);
+      if (status && (__hisinf(v) || __hisnan(v))) report_status(status, RT_ERR_NONFINITE);
     }
   }
 }
@@ -1334,7 +1334,7 @@ __global__ void swiglu_fwd_pitched_kernel(const __half* __restrict__ g, const __
   const size_t r = i / ff, c = i % ff;
   const uint4 o = swiglu8(*(const uint4*)(g + r * pitch + c), *(const uint4*)(u + r * pitch + c));
   *(uint4*)(h + i) = o;
-  if (status && any_nonfinite_f16x8(o)) atomicCAS(status, 0, RT_ERR_NONFINITE);
+  if (status && any_nonfinite_f16x8(o)) report_status(status, RT_ERR_NONFINITE);
 }
 void launch_swiglu_fwd(const __half* g, const __half* u, size_t in_pitch, int rows, int ff, __half* h, int* status,
                        cudaStream_t st) {
@@ -1602,7 +1602,7 @@ __global__ void ce_row_kernel(const float* __restrict__ logits, int v, const int
   const float* row = logits + r * v;
   const int tgt = target[r];
   if (tgt < 0 || tgt >= v) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_BAD_INDEX);
+    if (threadIdx.x == 0) report_status(status, RT_ERR_BAD_INDEX);
     return;
   }
   float m = -INFINITY;
@@ -1649,7 +1649,7 @@ ce_row_vec_kernel(const float* __restrict__ logits, int v, const int* __restrict
   const int n4 = v >> 2, tid = threadIdx.x;
   const int tgt = target[r];
   if (tgt < 0 || tgt >= v) {
-    if (tid == 0) atomicCAS(status, 0, RT_ERR_BAD_INDEX);
+    if (tid == 0) report_status(status, RT_ERR_BAD_INDEX);
     return;
   }
   const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);

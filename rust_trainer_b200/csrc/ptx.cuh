@@ -53,6 +53,18 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity
       : "memory");
   return ok;
 }
+// A context's status block on the device: the first code that a kernel reported, and where the host reads it (page-locked memory).
+// Without the second a call that only waits for its stream would copy the word too, 6 us of a chain of short calls.
+struct StatusBlock {
+  int code, unused;
+  int* host;
+};
+__device__ __forceinline__ void report_status(int* status, int code) {
+  if (atomicCAS(status, 0, code) != 0) return;
+  *(volatile int*)((const StatusBlock*)status)->host = code;
+  __threadfence_system();
+}
+
 // Bounded wait. Returns false (and records `code` in *status) after ~4e9 SM cycles (about two
 // seconds).  The bound counts this SM's own cycle counter, which nothing outside the kernel can
 // step or re-synchronise.
@@ -67,7 +79,7 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parit
     for (int i = 0; i < 256; ++i)
       if (mbar_try_wait(bar, parity)) return true;
     if (clock64() - t0 > limit_cycles) {
-      atomicCAS(status, 0, code);
+      report_status(status, code);
       return false;
     }
     if (*(volatile int*)status != 0) return false;  // another role already gave up

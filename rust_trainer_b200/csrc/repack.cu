@@ -2,6 +2,7 @@
 // dequantisation (FrozenMatmul::row, reference src/rie.rs:122-124) and the embedding gather
 // built on it (Model::embed_tokens, reference src/model.rs:446-454).
 #include "qformat.cuh"
+#include "ptx.cuh"
 #include "rt_internal.h"
 
 namespace rt {
@@ -140,7 +141,7 @@ __global__ void gather_rows_kernel(QWeight w, const int* __restrict__ ids, int n
   if (i >= n) return;
   int r = ids ? ids[i] : i;
   if (r < 0 || r >= w.rows) {
-    if (threadIdx.x == 0) atomicCAS(status, 0, RT_ERR_BAD_INDEX);
+    if (threadIdx.x == 0) report_status(status, RT_ERR_BAD_INDEX);
     return;
   }
   for (int k = threadIdx.x; k < w.cols; k += blockDim.x) out[(size_t)i * w.cols + k] = brick_value(w, r, k);
