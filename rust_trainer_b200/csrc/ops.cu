@@ -1808,17 +1808,20 @@ __global__ void lora_refresh_group_kernel(const float* __restrict__ a, const flo
   }
 }
 // Every stale adapter of a model in one launch: a block finds its row of the table by counting the rows that start no later, then
-// does what the two kernels above do for one adapter, eight elements a thread with their loads in flight together.  (One element a
-// thread behind a bisection of the table: 81 us for the 196 adapters of the 0.6B shape at rank 16, 115 MB; now 55, what is left being
-// the two-byte stores down bt_s.)
+// does what the two kernels above do for one adapter, eight elements a thread with their loads in flight together.  What goes down
+// bt_s is turned round in shared memory, so that a warp writes neighbours of a row of it.  (Two bytes into each of 16 rows at a
+// time: 55 us for the 196 adapters of the 0.6B shape at rank 16, 115 MB; now 46.)
 __global__ void __launch_bounds__(256) lora_refresh_table_kernel(const LoraRefreshJob* __restrict__ jobs, int n_jobs) {
+  // [rank index][rows of b], rows an odd number of words apart where a block's rows are a power of two
+  __shared__ __half turned[LORA_REFRESH_PER_BLOCK + 5 * 64];
   int row = -1;
   for (int t = 0; t < n_jobs; t += 256)
     row += __syncthreads_count(t + (int)threadIdx.x < n_jobs && jobs[t + threadIdx.x].first_block <= blockIdx.x);
   const LoraRefreshJob j = jobs[row];
   constexpr int PT = LORA_REFRESH_PER_BLOCK / 256;
-  const size_t i0 = (size_t)(blockIdx.x - j.first_block) * LORA_REFRESH_PER_BLOCK + threadIdx.x;
-  const size_t na = (size_t)j.r * j.K, nb = (size_t)j.N * (j.pad64 ? 64 : j.r);
+  const size_t first = (size_t)(blockIdx.x - j.first_block) * LORA_REFRESH_PER_BLOCK, i0 = first + threadIdx.x;
+  const unsigned width = j.pad64 ? 64u : (unsigned)j.r;  // elements of a row of b as they are counted
+  const size_t na = (size_t)j.r * j.K, nb = (size_t)j.N * width;
   float va[PT], vb[PT];
   unsigned n[PT], c[PT];
 #pragma unroll
@@ -1826,9 +1829,10 @@ __global__ void __launch_bounds__(256) lora_refresh_table_kernel(const LoraRefre
     const size_t i = i0 + k * 256;
     va[k] = i < na ? j.a[i] : 0.f;
     n[k] = j.pad64 ? (unsigned)(i >> 6) : (unsigned)i / (unsigned)j.r;
-    c[k] = j.pad64 ? (unsigned)i & 63u : (unsigned)i - n[k] * (unsigned)j.r;
+    c[k] = (unsigned)i - n[k] * width;
     vb[k] = i < nb && c[k] < (unsigned)j.r ? j.b[(size_t)n[k] * j.r + c[k]] : 0.f;
   }
+  const unsigned n0 = (unsigned)first / width, rows = ((unsigned)first + LORA_REFRESH_PER_BLOCK - 1) / width - n0 + 1, pitch = (rows + 1) / 2 * 2 + 2;
 #pragma unroll
   for (int k = 0; k < PT; ++k) {
     const size_t i = i0 + k * 256;
@@ -1838,8 +1842,14 @@ __global__ void __launch_bounds__(256) lora_refresh_table_kernel(const LoraRefre
     }
     if (i < nb) {
       j.bp[(size_t)n[k] * 64 + c[k]] = __float2half_rn(vb[k]);
-      if (c[k] < (unsigned)j.r) j.bt_s[(size_t)c[k] * j.ldb + n[k]] = __float2half_rn(vb[k] * j.s);
+      if (c[k] < (unsigned)j.r) turned[c[k] * pitch + (n[k] - n0)] = __float2half_rn(vb[k] * j.s);
     }
+  }
+  __syncthreads();
+  for (unsigned e = threadIdx.x; e < (unsigned)j.r * rows; e += 256) {
+    const unsigned cc = e / rows, m = e - cc * rows;
+    const size_t i = (size_t)(n0 + m) * width + cc;  // (a row that two blocks share: each writes its own part)
+    if (i >= first && i < first + LORA_REFRESH_PER_BLOCK && i < nb) j.bt_s[(size_t)cc * j.ldb + n0 + m] = turned[cc * pitch + m];
   }
 }
 void launch_lora_refresh_table(const LoraRefreshJob* jobs_dev, int n_jobs, unsigned total_blocks, cudaStream_t st) {
@@ -1859,12 +1869,20 @@ void launch_lora_refresh(const float* a, const float* b, int r, int K, int N, fl
 
 // ------------------------------------------------------------------ optimiser (reference src/optim.rs:48-90)
 // Sum of squares in f64: fixed-size blocks write partials, one block adds them in order.
-__global__ void sumsq_partial_kernel(const float* __restrict__ g, size_t n, double* __restrict__ part) {
+__global__ void __launch_bounds__(256) sumsq_partial_kernel(const float* __restrict__ g, size_t n, double* __restrict__ part) {
+  const size_t at = (size_t)blockIdx.x * blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x, n4 = n / 4;
   double s = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    double v = (double)g[i];
-    s += v * v;
+  for (size_t i = at; i < n4; i += 4 * step) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = i + k * step < n4 ? ((const float4*)g)[i + k * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double x = v[k].x, y = v[k].y, z = v[k].z, w = v[k].w;
+      s += x * x + y * y + (z * z + w * w);
+    }
   }
+  if (at < n % 4) s += (double)g[4 * n4 + at] * (double)g[4 * n4 + at];
   s = block_sum_d(s);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
@@ -1875,37 +1893,53 @@ __global__ void sumsq_final_kernel(const double* __restrict__ part, int n, doubl
   if (threadIdx.x == 0) out[0] = s;
 }
 void launch_sumsq(const float* g, size_t n, double* part /* >= 1024 */, double* out, cudaStream_t st) {
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 1024) blocks = 1024;
-  if (blocks < 1) blocks = 1;
+  // sixteen values a thread, at most what is on the GPU at a time and `part` has room for
+  const int blocks = (int)std::min<size_t>(1024, std::max<size_t>(1, (n + 4095) / 4096));
   { sumsq_partial_kernel<<<blocks, 256, 0, st>>>(g, n, part); RT_COUNT_LAUNCH(1); }
   { sumsq_final_kernel<<<1, 256, 0, st>>>(part, blocks, out); RT_COUNT_LAUNCH(1); }
 }
-// clip (scale read from the device-side norm) fused with the AdamW update.
-__global__ void adamw_kernel(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                             size_t n, const double* __restrict__ sumsq, float max_norm, float lr, float beta1,
-                             float beta2, float eps, float wd, float bc1, float bc2, float* __restrict__ norm_out) {
+// clip (scale read from the device-side norm) fused with the AdamW update.  Bound: DRAM, four arrays read and three or, where the norm
+// clips, four written; four parameters a thread (10 million: one a thread 81 us, now 41; the copy rate would take 49 with the gradients' write).
+__device__ __forceinline__ void adamw_one(float& p, float& g, float& m, float& v, float clip, float lr, float beta1, float beta2, float eps, float wd,
+                                          float bc1, float bc2) {
+  if (clip != 1.0f) g *= clip;
+  m = beta1 * m + (1.0f - beta1) * g;
+  v = beta2 * v + (1.0f - beta2) * g * g;
+  const float mh = m / bc1, vh = v / bc2;
+  p -= lr * (mh / (sqrtf(vh) + eps) + wd * p);
+}
+__global__ void __launch_bounds__(256) adamw_kernel(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+                                                    size_t n, const double* __restrict__ sumsq, float max_norm, float lr, float beta1,
+                                                    float beta2, float eps, float wd, float bc1, float bc2, float* __restrict__ norm_out) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, i = 4 * t;
+  const bool whole = i + 3 < n;
+  float4 pv, gv, mv, vv;
+  if (whole) {  // before the norm, a load that these do not depend on
+    pv = *(const float4*)(p + i); gv = *(const float4*)(g + i); mv = *(const float4*)(m + i); vv = *(const float4*)(v + i);
+  }
   const float norm = (float)sqrt(sumsq[0]);
   float clip = 1.0f;
   if (max_norm > 0.f && norm > max_norm) clip = max_norm / (norm + 1e-6f);
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0 && norm_out) norm_out[0] = norm;
-  if (i >= n) return;
-  const float gi = clip != 1.0f ? g[i] * clip : g[i];
-  g[i] = gi;
-  const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-  const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float mh = mi / bc1, vh = vi / bc2;
-  p[i] -= lr * (mh / (sqrtf(vh) + eps) + wd * p[i]);
+  if (t == 0 && norm_out) norm_out[0] = norm;
+  if (whole) {
+    adamw_one(pv.x, gv.x, mv.x, vv.x, clip, lr, beta1, beta2, eps, wd, bc1, bc2);
+    adamw_one(pv.y, gv.y, mv.y, vv.y, clip, lr, beta1, beta2, eps, wd, bc1, bc2);
+    adamw_one(pv.z, gv.z, mv.z, vv.z, clip, lr, beta1, beta2, eps, wd, bc1, bc2);
+    adamw_one(pv.w, gv.w, mv.w, vv.w, clip, lr, beta1, beta2, eps, wd, bc1, bc2);
+    *(float4*)(p + i) = pv;
+    if (clip != 1.0f) *(float4*)(g + i) = gv;
+    *(float4*)(m + i) = mv;
+    *(float4*)(v + i) = vv;
+  } else {
+    for (size_t k = i; k < n; ++k) adamw_one(p[k], g[k], m[k], v[k], clip, lr, beta1, beta2, eps, wd, bc1, bc2);
+  }
 }
 void launch_adamw(float* p, float* g, float* m, float* v, size_t n, const double* sumsq, float max_norm, float lr,
                   float beta1, float beta2, float eps, float wd, float bc1, float bc2, float* norm_out,
                   cudaStream_t st) {
   if (n == 0) return;
-  { adamw_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, g, m, v, n, sumsq, max_norm, lr, beta1, beta2, eps, wd,
-                                                             bc1, bc2, norm_out); RT_COUNT_LAUNCH(1); }
+  { adamw_kernel<<<(unsigned)((n + 1023) / 1024), 256, 0, st>>>(p, g, m, v, n, sumsq, max_norm, lr, beta1, beta2, eps, wd,
+                                                               bc1, bc2, norm_out); RT_COUNT_LAUNCH(1); }
 }
 
 }  // namespace rt
