@@ -61,12 +61,15 @@ constexpr int QF_16 = 0;       // 16-bit weights of the activations' type, strai
 constexpr int QF_16CONV = 1;   // 16-bit weights of the other 16-bit type, converted in place
 
 // Shared-memory plan of one CTA.
-template <int KIND, int FMT>
+template <int KIND, int FMT, int OUT>
 struct QCfg {
   static constexpr bool SLIM = KIND == QK_SLIM, PAIR = KIND == QK_PAIR || SLIM, HALF = KIND == QK_HALF, NARROW = KIND == QK_NARROW || KIND == QK_NARROW_T;
   static constexpr bool TM = KIND == QK_NARROW_T;  // unpacked weights in TMEM
-  // Weight rows of the CTA's tile.  The MMA always takes 128: a half tile's upper 64 are whatever follows it in
-  // shared memory, and their accumulator lanes are not read.
+  // Weight rows of the CTA's tile, as many as its MMA takes (a slim pair's takes both CTAs').  A half tile whose results are staged
+  // takes 128 all the same, because a quarter of the accumulator then has the 32 rows of a staged block: the upper 64 are
+  // whatever follows the tile in shared memory, and their lanes are not read.  (Without staging 6144x1024 Q4_0 at 157 tokens to f16 13.8 us, 9.6
+  // so; f32 results of 3072x8192 at 157 tokens 25.6 us with 128 rows, 24.5 with 64.)
+  static constexpr bool M64 = HALF && OUT == QO_DIRECT;
   static constexpr int ROWS = HALF || SLIM ? 64 : 128, BRICKS = ROWS / 64;
   static constexpr int W_SUB = ROWS * 128;  // bytes of a [ROWS x 64] 16-bit weight tile
   static constexpr bool PACKED = FMT > QF_16CONV;
@@ -91,8 +94,10 @@ struct QCfg {
   // TMEM columns of a stage's unpacked weights, beside the two accumulators of up to 64 columns at 0 and 256
   __device__ static constexpr uint32_t a_col(int st) { return 128u + (uint32_t)(st & 1) * 64u + (uint32_t)(st >> 1) * 256u; }
   static_assert(!TM || (PACKED && NS <= 4), "four stages fit TMEM");
-  // Epilogue staging of 16-bit outputs per warp: three blocks of [32 tokens x 32 features], 2 KB each.
-  static constexpr int OUT_BUFS = 3, OUT_WARP = OUT_BUFS * 2048;
+  // Epilogue staging per warp of 16-bit outputs and of residuals: three blocks of [32 tokens x 32 features], 2 KB each.  What leaves
+  // straight from registers has none, and its room goes to the brick ring: Q8_0 on pairs and slim pairs has seven slots so, four with
+  // it (8192x3072 at 24 tokens backward on slim pairs 29.5 -> 25.5 us, at 157 forward on pairs 21.1 -> 18.4, 3072x8192 at 1024 forward 53.2 -> 49.1).
+  static constexpr int OUT_BUFS = 3, OUT_WARP = OUT == QO_DIRECT ? 0 : OUT_BUFS * 2048;
   static constexpr int SMEM_MAX = 232448, SMEM_REST = 4 * OUT_WARP + 512 + 2 * 1024;  // staging, barriers, alignment
   static constexpr int NR_FIT = PACKED ? (SMEM_MAX - SMEM_REST - NS * (ACT_STAGE + W_BYTES)) / (RAW_STAGE ? RAW_STAGE : 1) : 0;
   static constexpr int NR = NR_FIT > 8 ? 8 : NR_FIT;
@@ -119,7 +124,7 @@ struct QCfg {
   static constexpr int SMEM_USED = OFF_BAR + N_BARS * 8 + 16 + 1024;
   static constexpr int SMEM_BYTES = SMEM_USED > ALONE_SMEM ? SMEM_USED : ALONE_SMEM;
   static_assert(SMEM_BYTES <= SMEM_MAX && N_BARS * 8 + 16 <= 512, "shared memory plan exceeds one SM");
-  static_assert(OFF_RAW >= 11 * 8192, "the last tile's helpers stage in the operand stages");
+  static_assert(OUT == QO_DIRECT || OFF_RAW >= 11 * 8192, "the last tile's helpers stage in the operand stages");
 };
 
 struct KParams {
@@ -278,11 +283,11 @@ __device__ __forceinline__ void unpack_unit(const uint8_t* brick, int t, uint32_
 //   over the pair) writes, in each CTA's TMEM, its 64 rows to lanes 0..63 for the first half of the tokens and to lanes 64..127
 //   for the second, in half as many columns.  All the rest is as for PAIR, which is set for both.
 template <int KIND, int FMT, int OUT>
-__global__ void __launch_bounds__((QCfg<KIND, FMT>::THREADS), 1)
+__global__ void __launch_bounds__((QCfg<KIND, FMT, OUT>::THREADS), 1)
 qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__ CUtensorMap tm_w16,
              const __grid_constant__ CUtensorMap tm_lact, const __grid_constant__ CUtensorMap tm_lw,
              const __grid_constant__ CUtensorMap tm_out, const KParams p) {
-  using C = QCfg<KIND, FMT>;
+  using C = QCfg<KIND, FMT, OUT>;
   constexpr bool PAIR = C::PAIR, SLIM = C::SLIM, TM = C::TM, PACKED = C::PACKED, CONV = FMT == QF_16CONV, IS16 = !PACKED;
   constexpr int NS = C::NS, NR = C::NR, UG = C::UG, UTG = C::UTG, KS = C::KS;
   extern __shared__ uint8_t smem_raw[];
@@ -397,7 +402,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   // Where the 32 accumulator lanes of quarter wq belong.  A slim pair's accumulator has 64 rows in each CTA: lanes 0..63 hold
   // them for the tile's first half of the tokens, lanes 64..127 for the second, in half as many columns.
   const int tn_q = SLIM ? p.TN >> 1 : p.TN;  // tokens (columns) of a quarter
-  auto q_row = [&](int wq) { return SLIM ? (wq & 1) * 32 : wq * 32; };
+  // An accumulator of 64 rows in one CTA has them in the first sixteen lanes of each quarter.
+  auto q_row = [&](int wq) { return SLIM ? (wq & 1) * 32 : C::M64 ? wq * 16 : wq * 32; };
   auto q_tok = [&](int wq) { return SLIM ? (wq >> 1) * tn_q : 0; };
 
   // One [32 tokens x 32 features] block of a 16-bit output -> staging -> TMA store.  `stage_base` is
@@ -475,7 +481,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     if (tok0 >= p.M) return;
     uint32_t v[32];
     tmem_ld32(tmem_base + acc * 256 + ((uint32_t)(wq * 32) << 16) + c * 32, v);
-    const bool row_ok = row < p.out_rows;
+    const bool row_ok = row < p.out_rows && (!C::M64 || lane < 16);
     const int nvalid = min(min(32, tn_q - c * 32), p.M - tok0);
     const bool fin_out = p.part == nullptr;  // partial sums are scaled, biased and added up by the reduce kernel
     float rs_lane = 1.0f;
@@ -600,7 +606,7 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   const int q_res = warp & 3;
   const int q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
   auto tail_helper = [&](int turn, int hslot) {
-    if (n_my == 0 || (!SLIM && q_res * 32 >= C::ROWS)) return;
+    if (n_my == 0 || (!SLIM && !C::M64 && q_res * 32 >= C::ROWS)) return;
     if (!p.late_wait && !p.end_wait && weights_only) pdl_wait();
     const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
     QG_ITEM_DECODE(item);
@@ -911,8 +917,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
       const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
-      const bool mine = SLIM || wq * 32 < C::ROWS;
       const uint32_t stage = smem_u32(sOut + wq * C::OUT_WARP);
+      const bool mine = SLIM || C::M64 || wq * 32 < C::ROWS;
       if (OUT == QO_RES && mine) residual_start(wq, 0, stride, r0, m0, stage);
       if (!mbar_wait(&acc_full[acc], aph, p.status, 401)) break;
       tc_fence_after();
@@ -984,7 +990,7 @@ struct QKernel {
 };
 template <int KIND, int FMT, int OUT>
 static QKernel qkernel() {
-  return {(const void*)qgemm_kernel<KIND, FMT, OUT>, QCfg<KIND, FMT>::THREADS, QCfg<KIND, FMT>::SMEM_BYTES};
+  return {(const void*)qgemm_kernel<KIND, FMT, OUT>, QCfg<KIND, FMT, OUT>::THREADS, QCfg<KIND, FMT, OUT>::SMEM_BYTES};
 }
 // fmt: a packed ggml format, QF_16 or QF_16CONV
 template <int KIND, int OUT>
@@ -1154,6 +1160,8 @@ static int make_out_map(rt_ctx* ctx, CUtensorMap* m, const void* base, uint64_t 
 // us on half tiles, 6.4 on narrow ones).  (Before, with 0.5 to 1 us more for the launch of pairs and slim pairs and a fourth more
 // for their steps, 3.0 % off, a tenth of the times by more than 10 %: 3072x1024 Q4_0 at 400 tokens on narrow tiles 10.4 us, and 14.7
 // behind a kernel that lets nothing start, on pairs 9.3 and 12.9.)
+// (On 1400 products of twelve shapes, in graphs, since f32 results gave their staging's room to the brick ring: 2.4 % off behind itself,
+// 1.0 % behind such a kernel; the constants fitted anew would be 2.2 and 0.9 % off, and stand.)
 // What a step's time stands for: a pair's for its MMAs from about 96 tokens of width on and for the hand-offs between the
 // roles below; a slim pair's for shared memory; half and narrow tiles' for one round of unpacking, which is
 // shortest for Q8_0's codes.
@@ -1279,7 +1287,6 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
   const int tn_cta = pair ? p.TN / 2 : p.TN;  // each CTA of a pair fetches its half of the token tile
   // tcgen05.mma kind::f16 needs A and B of ONE 16-bit type (f16 x bf16 is an illegal instruction).
   const int ab_fmt = a.act_f16 ? 0 : 1;
-  p.idesc = umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, plan.kind == QK_PAIR ? 256 : 128, p.TN);
 
   CUtensorMap tm_act, tm_w16, tm_lact, tm_lw;
   int rc = make_map(&tm_act, a.act, (uint64_t)a.M, (uint64_t)contract, 64, (uint32_t)tn_cta, !a.act_f16);
@@ -1319,6 +1326,7 @@ int qgemm_launch(rt_ctx* ctx, const QWeight& w, const QGemmArgs& a) {
     if (rc) return rc;
     out_kind = QO_TMA16;
   }
+  p.idesc = umma_idesc(ab_fmt, ab_fmt, a.dir == QG_BWD ? 1 : 0, 0, plan.kind == QK_PAIR ? 256 : plan.kind == QK_HALF && out_kind == QO_DIRECT ? 64 : 128, p.TN);
   const int n_items = p.n_row_tiles * p.n_tok_tiles * p.n_splits;
   const int workers = pair ? g_pair_workers : num_sms;
   const int grid = (n_items < workers ? n_items : workers) * (pair ? 2 : 1);
