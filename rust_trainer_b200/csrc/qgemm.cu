@@ -596,38 +596,8 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
     }
     cp_async_wait<0>();
   };
-  // The epilogue of a CTA's LAST tile has nothing to hide behind, so the warps whose own work
-  // is over by then help: every warp with residue q (mod 4) may read TMEM lane quarter q.
-  // Quarter q's blocks go round-robin over its epilogue warp (turn 0) and its helpers (turns
-  // 1..) among warps 0..14: residues 0 and 2 have three unpack warps each, residue 3 two, residue
-  // 1 the two producer warps.  Helpers stage in the operand stages, which are idle once the last
-  // accumulator is complete.
   const int n_my = worker < n_items ? (n_items - worker + n_workers - 1) / n_workers : 0;
-  const int q_res = warp & 3;
-  const int q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
-  auto tail_helper = [&](int turn, int hslot) {
-    if (n_my == 0 || (!SLIM && !C::M64 && q_res * 32 >= C::ROWS)) return;
-    if (!p.late_wait && !p.end_wait && weights_only) pdl_wait();
-    const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
-    QG_ITEM_DECODE(item);
-    (void)s_begin; (void)n_steps; (void)s_main;
-    QG_TILE_ORIGIN();
-    const int acc = tc_last & 1;
-    if (!mbar_wait(last_full, 0, p.status, 402)) return;
-    tc_fence_after();
-    uint32_t cnt = 0;
-    if (OUT == QO_RES) {
-      const uint32_t stage = smem_u32(smem + hslot * 8192);
-      residual_start(q_res, turn, q_turns, r0, m0, stage);
-      residual_tile(acc, q_res, turn, q_turns, r0, m0, stage);
-      return;
-    }
-    for (int c = turn; c * 32 < tn_q; c += q_turns) {
-      if (OUT == QO_TMA16) tma_chunk(acc, q_res, c, r0, m0, smem + hslot * 8192, cnt);
-      else direct_chunk(acc, q_res, c, r0, m0, split);
-    }
-    if (lane == 0) bulk_wait_group_read<0>();  // staging may go once read; the writes land by the end of the grid
-  };
+  uint32_t out_chunk = 0;  // of an epilogue warp, staged so far
 
   if (role == R_PROD) {
     // ------------------------------------------------------------ producer
@@ -681,8 +651,6 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         }
       }
     }
-    __syncwarp();
-    if (warp < 15) tail_helper(warp >> 2, warp - 4);
   } else if (role == R_MMA) {
     // ------------------------------------------------------------ MMA issue (the leader's thread only)
     if (rank == 0 && elect_one()) {
@@ -867,7 +835,6 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         if (PACKED && n_steps > n_main_st && --rs < 0) { rs += NR; rph ^= 1; }  // a low-rank step takes a stage but no bricks
       }
     }
-    if (warp < 15) tail_helper(warp >> 2, warp - 4);
   } else if (role == R_RAW) {
     // ------------------------------------------------------------ packed-brick producer
     // Runs ahead of the stage ring: a brick pair is fetched as soon as its slot in the raw ring
@@ -904,27 +871,24 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
         }
       }
     }
-    __syncwarp();
-    if (warp < 15) tail_helper(warp >> 2, warp - 4);
   } else if (role == R_EPI) {
-    // ------------------------------------------------------------ epilogue
+    // ------------------------------------------------------------ epilogue of all tiles but the last
     const int wq = warp & 3;  // TMEM lane quarter this warp may read
-    uint32_t tcount = 0, out_chunk = 0;
-    for (int item = worker; item < n_items; item += n_workers, ++tcount) {
+    uint32_t tcount = 0;
+    for (int item = worker; item + n_workers < n_items; item += n_workers, ++tcount) {
       QG_ITEM_DECODE(item);
       (void)s_begin; (void)n_steps; (void)s_main;
       QG_TILE_ORIGIN();
       const int acc = tcount & 1;
       const uint32_t aph = (tcount >> 1) & 1;
-      const int stride = (int)tcount == n_my - 1 ? q_turns : 1;  // the last tile's other blocks are the helpers'
-      const uint32_t stage = smem_u32(sOut + wq * C::OUT_WARP);
       const bool mine = SLIM || C::M64 || wq * 32 < C::ROWS;
-      if (OUT == QO_RES && mine) residual_start(wq, 0, stride, r0, m0, stage);
+      const uint32_t stage = smem_u32(sOut + wq * C::OUT_WARP);
+      if (OUT == QO_RES && mine) residual_start(wq, 0, 1, r0, m0, stage);
       if (!mbar_wait(&acc_full[acc], aph, p.status, 401)) break;
       tc_fence_after();
       if (OUT == QO_RES) {
-        if (mine) residual_tile(acc, wq, 0, stride, r0, m0, stage);
-      } else for (int c = mine ? 0 : p.TN; c * 32 < tn_q; c += stride) {
+        if (mine) residual_tile(acc, wq, 0, 1, r0, m0, stage);
+      } else for (int c = mine ? 0 : p.TN; c * 32 < tn_q; ++c) {
         if (OUT == QO_TMA16) tma_chunk(acc, wq, c, r0, m0, sOut + wq * C::OUT_WARP, out_chunk);
         else direct_chunk(acc, wq, c, r0, m0, split);
       }
@@ -934,6 +898,37 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
       if (lane == 0) {
         if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[acc]), 0));
         else mbar_arrive(&acc_empty[acc]);
+      }
+    }
+  }
+  // The epilogue of a CTA's LAST tile has nothing to hide behind, so the warps whose own work
+  // is over by then help: every warp with residue q (mod 4) may read TMEM lane quarter q.
+  // Quarter q's blocks go round-robin over its epilogue warp (turn 0) and its helpers (turns
+  // 1..) among warps 0..14: residues 0 and 2 have three unpack warps each, residue 3 two, residue
+  // 1 the two producer warps.  Helpers stage in the operand stages, which are idle once the last
+  // accumulator is complete.  All of them run the same instructions: in a launch of one tile they are cold, and a copy of them in
+  // each role was fetched by each role (from the complete accumulator to the end of the launch 2.3 us of 10.2, 1024x2048 Q4_0 at 1024 tokens).
+  __syncwarp();
+  const int q_res = warp & 3;
+  const bool epi = role == R_EPI;
+  if (n_my > 0 && (epi || (warp < 15 && role != R_MMA)) && (SLIM || C::M64 || q_res * 32 < C::ROWS)) {
+    if (!p.late_wait && !p.end_wait && weights_only) pdl_wait();
+    const int turn = epi ? 0 : warp >> 2, q_turns = (q_res == 0 || q_res == 2) ? 4 : 3;  // epilogue warp + helpers of this residue
+    uint8_t* stage = epi ? sOut + q_res * C::OUT_WARP : smem + (warp - 4) * 8192;
+    const int tc_last = n_my - 1, item = worker + tc_last * n_workers;
+    QG_ITEM_DECODE(item);
+    (void)s_begin; (void)n_steps; (void)s_main;
+    QG_TILE_ORIGIN();
+    const int acc = tc_last & 1;
+    if (OUT == QO_RES && epi) residual_start(q_res, turn, q_turns, r0, m0, smem_u32(stage));
+    if (mbar_wait(last_full, 0, p.status, 402)) {
+      tc_fence_after();
+      if (OUT == QO_RES) {
+        if (!epi) residual_start(q_res, turn, q_turns, r0, m0, smem_u32(stage));  // (only now: over the operand stages)
+        residual_tile(acc, q_res, turn, q_turns, r0, m0, smem_u32(stage));
+      } else for (int c = turn; c * 32 < tn_q; c += q_turns) {
+        if (OUT == QO_TMA16) tma_chunk(acc, q_res, c, r0, m0, stage, out_chunk);
+        else direct_chunk(acc, q_res, c, r0, m0, split);
       }
     }
     if (lane == 0) bulk_wait_group_read<0>();  // staging may go once read; the writes land by the end of the grid
