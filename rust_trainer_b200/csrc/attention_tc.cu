@@ -1017,7 +1017,8 @@ attn_delta_tc_kernel(const __half* o, const __half* dO, const float* lse,
     const float top = mx > 0 ? __int_as_float((mx + 0x007FFFFF) & 0x7F800000) : 1.f;
     const float w = fmaxf(my_scale, 0.f) / top;
     if (h == 0) tops[m] = top;
-    if (w > 0.f) off = log2f(w) + P_BOOST_LOG2 - my_lse * LOG2E;
+    // (fused by name: whether the compiler fuses it depends on where the load stands)
+    if (w > 0.f) off = fmaf(-my_lse, LOG2E, log2f(w) + P_BOOST_LOG2);
     delta = s_delta[threadIdx.x];
   }
   query_vecs[(size_t)h * pitch + m] = off;

@@ -57,3 +57,9 @@ def test_no_later_kernel_takes_the_tmem_a_started_one_still_needs(name):
     for file, least in (("lowrank_tc.cu", "TOTAL >= LOWRANK_KERNEL_SMEM"), ("lora_grads_tc.cu", "LG_TOTAL >= TMEM_KERNEL_SMEM"),
                         ("attention_tc.cu", "TOTAL >= TMEM_KERNEL_SMEM")):
         assert f"static_assert({least}" in (CSRC / file).read_text()
+
+
+def test_the_exponents_offset_of_attention_is_fused_by_name():
+    """Left to the compiler, a load moved from beside the multiplication to the kernel's front took the fused multiply-add apart: the
+    gradients of a 3B step moved by 1e-3."""
+    assert re.search(r"off = fmaf\(-my_lse, LOG2E, log2f\(w\) \+ P_BOOST_LOG2\);", kernels()["attn_delta_tc_kernel"])
