@@ -205,12 +205,16 @@ __device__ __forceinline__ uint2 half4(float4 v) {
   __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
   return make_uint2(*(uint32_t*)&a, *(uint32_t*)&b);
 }
+// The four products of a lane's float4, and a x - b y: fused by name, so that a row gets the same bits in every kernel it may run
+// through (a block's second forward takes the one without a product, and the backward's form goes by the number of rows).
+__device__ __forceinline__ float dot4(const float4& a, const float4& b) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.x, b.x, a.y * b.y))); }
+__device__ __forceinline__ float ax_by(float a, float x, float b, float y) { return fmaf(a, x, -(b * y)); }
 // put(k, four f16): what lane + 32 k of the result is
 template <int NV, class Put>
 __device__ __forceinline__ void rms_fwd_row(const float4* v, const float* __restrict__ w, float eps, int lane, Put put) {
   float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < NV; ++k) ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+  for (int k = 0; k < NV; ++k) ss += dot4(v[k], v[k]);
   ss = warp_sum(ss);
   const float ir = 1.0f / sqrtf(ss / (float)(128 * NV) + eps);
   const float4* w4 = (const float4*)w;
@@ -242,8 +246,8 @@ __device__ __forceinline__ float rms_bwd_row(const float4* xv, float4* gv, const
   for (int k = 0; k < NV; ++k) {
     const float4 wv = w4[lane + 32 * k];
     gv[k] = make_float4(gv[k].x * wv.x, gv[k].y * wv.y, gv[k].z * wv.z, gv[k].w * wv.w);
-    ss += xv[k].x * xv[k].x + xv[k].y * xv[k].y + xv[k].z * xv[k].z + xv[k].w * xv[k].w;
-    gx += gv[k].x * xv[k].x + gv[k].y * xv[k].y + gv[k].z * xv[k].z + gv[k].w * xv[k].w;
+    ss += dot4(xv[k], xv[k]);
+    gx += dot4(gv[k], xv[k]);
   }
   ss = warp_sum(ss);
   gx = warp_sum(gx);
@@ -252,8 +256,8 @@ __device__ __forceinline__ float rms_bwd_row(const float4* xv, float4* gv, const
   float m = 0.f;
 #pragma unroll
   for (int k = 0; k < NV; ++k) {
-    float4 v = make_float4(gv[k].x * ir - xv[k].x * c, gv[k].y * ir - xv[k].y * c, gv[k].z * ir - xv[k].z * c,
-                           gv[k].w * ir - xv[k].w * c);
+    float4 v = make_float4(ax_by(gv[k].x, ir, xv[k].x, c), ax_by(gv[k].y, ir, xv[k].y, c), ax_by(gv[k].z, ir, xv[k].z, c),
+                           ax_by(gv[k].w, ir, xv[k].w, c));
     v.x += rv[k].x; v.y += rv[k].y; v.z += rv[k].z; v.w += rv[k].w;
     gv[k] = v;
     m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));

@@ -68,3 +68,20 @@ def test_a_sequence_gets_the_same_products_in_a_small_and_a_large_batch(ctx, hid
     # 16-bit product anywhere would show as 2^-12 of its value
     assert rel_l2(_gpu_flat(gm, "ga", "gb"), g_alone) < 1e-6 and np.abs(g_alone).max() > 0
     gm.close()
+
+
+@pytest.mark.parametrize("hidden,rank,lens", [(128, 16, [128, 77]), (128, 8, [900] * 4), (384, 20, [205]), (896, 8, [70, 3]), (1024, 32, [300])])
+def test_recomputed_blocks_get_the_bits_of_kept_ones(ctx, hidden, rank, lens):
+    """A block's second forward keeps Hs and takes RMSNorm without the product: the same rows all the same."""
+    spec = synth.preset("tiny-qwen3", quant="Q8_0", seed=5, w_std=0.05, hidden=hidden, n_layers=4)
+    _, _, gm = _model(ctx, spec, rank)
+    seqs, tp, tt, _ = _batch(spec, lens, seed=11)
+    w = np.full(tp.size, 1.0 / tp.size, np.float32)
+    got = []
+    for mode in (0, 1):
+        gm.set_checkpointing(mode)
+        gm.zero_grad()
+        gm.forward_backward(seqs, tp, tt, w)
+        got.append(_gpu_flat(gm, "ga", "gb"))
+    assert np.array_equal(*got) and np.abs(got[0]).max() > 0
+    gm.close()
