@@ -212,20 +212,6 @@ static void group_refresh(LinGroup& g, cudaStream_t st) {
   }
 }
 
-// The low-rank products of adapters that a row kernel makes beside their input: Hs of a linear (group) from its x, Gs from
-// its dy, into `out`; none without adapters.
-static LowRank lowrank_h(LinGroup& g, __half* out) {
-  bool any;
-  if (!group_lora_on(g, &any) || !any) return {};
-  group_refresh(g, g.lin[0]->ctx->stream);
-  return {g.a_s, g.rank_total, out};
-}
-static LowRank lowrank_g(rt_linear* l, __half* out) {
-  if (!l->lora_active()) return {};
-  lora_refresh(l);
-  return {l->lora.bt_s, l->lora.rank, out};
-}
-
 // Rebuilds, in one launch, every 16-bit adapter copy the next pass over the model will read and
 // that is older than its adapter: the stacked copies of usable groups, the own copies of the
 // linears outside them.  Runs before a pass (never inside a captured one: a copy that happened
@@ -1120,6 +1106,18 @@ static rt_status norm_backward(rt_model* m, const float* x, const float* w, int 
   return RT_OK;
 }
 
+// Hs of a group, to be made where RMSNorm makes its x, kept or in scratch; none without an active adapter (whose scratch is not
+// asked for then) or where that kernel does not take it.
+static rt_status lowrank_from_norm(rt_model* m, LinGroup& g, int M, __half* kept, LowRank* lr) {
+  bool any;
+  if (!rmsnorm_takes_lowrank(m->cfg.hidden, g.rank_total) || !group_lora_on(g, &any) || !any) return RT_OK;
+  __half* hs = kept ? kept : lowrank_buf(m->lsc.hs, M);
+  if (!hs) return m->ctx->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
+  group_refresh(g, m->ctx->stream);
+  *lr = {g.a_s, g.rank_total, hs};
+  return RT_OK;
+}
+
 // Block::forward (src/model.rs:165-183).  x_in is read only; h receives x_in + attention;
 // when x_out is non-null it receives the block output (h + mlp), and may alias h.  With `keep`
 // the adapters' Hs = X.(sA)^T are left in A.hs for the block's backward.
@@ -1133,14 +1131,11 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   BlockDev& b = m->blocks[li];
   cudaStream_t st = c->stream;
   const int d = g.hidden;
-  __half* scratch_hs = keep ? nullptr : lowrank_buf(m->lsc.hs, M);
-  if (!keep && !scratch_hs) return c->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-  auto hs_at = [&](int i) { return keep ? A.hs[i] : scratch_hs; };
   LowRank lr;  // made where the linear's input is made, and not a second time
-  if (A.qkv_group && !hs_ready && rmsnorm_takes_lowrank(d, b.qkv.rank_total)) lr = lowrank_h(b.qkv, hs_at(0));
+  if (A.qkv_group && !hs_ready) RT_TRY(lowrank_from_norm(m, b.qkv, M, keep ? A.hs[0] : nullptr, &lr));
   RT_TRY(norm_forward(m, x_in, b.input_norm, M, A.n1, lr));
   if (A.qkv_group) {
-    RT_TRY(group_forward_dev(b.qkv, m->lsc, A.n1, M, A.q_raw, RT_DT_F32, hs_at(0), hs_ready || lr.w));
+    RT_TRY(group_forward_dev(b.qkv, m->lsc, A.n1, M, A.q_raw, RT_DT_F32, keep ? A.hs[0] : lr.out, hs_ready || lr.w));
   } else {
     RT_TRY(linear_forward_dev(b.lin[0], m->lsc, A.n1, M, A.q_raw, RT_DT_F32, 0, keep ? A.hs[0] : nullptr, hs_ready));
     RT_TRY(linear_forward_dev(b.lin[1], m->lsc, A.n1, M, A.k_raw, RT_DT_F32, 0, keep ? A.hs[1] : nullptr, hs_ready));
@@ -1154,10 +1149,10 @@ static rt_status block_forward(rt_model* m, int li, int M, const float* x_in, fl
   // the residual comes in where the product goes out: in place, or from the buffer that keeps it
   RT_TRY(linear_forward_dev(b.lin[3], m->lsc, A.o16, M, h, RT_DT_F32, h == x_in, keep ? A.hs[3] : nullptr, hs_ready, h == x_in ? nullptr : x_in));
   lr = {};
-  if (A.gu_group && !hs_ready && rmsnorm_takes_lowrank(d, b.gu.rank_total)) lr = lowrank_h(b.gu, hs_at(4));
+  if (A.gu_group && !hs_ready) RT_TRY(lowrank_from_norm(m, b.gu, M, keep ? A.hs[4] : nullptr, &lr));
   RT_TRY(norm_forward(m, h, b.post_norm, M, A.n2, lr));
   if (A.gu_group) {
-    RT_TRY(group_forward_dev(b.gu, m->lsc, A.n2, M, A.g16, RT_DT_F16, hs_at(4), hs_ready || lr.w));
+    RT_TRY(group_forward_dev(b.gu, m->lsc, A.n2, M, A.g16, RT_DT_F16, keep ? A.hs[4] : lr.out, hs_ready || lr.w));
   } else {
     RT_TRY(linear_forward_dev(b.lin[4], m->lsc, A.n2, M, A.g16, RT_DT_F16, 0, keep ? A.hs[4] : nullptr, hs_ready));
     RT_TRY(linear_forward_dev(b.lin[5], m->lsc, A.n2, M, A.u16, RT_DT_F16, 0, keep ? A.hs[5] : nullptr, hs_ready));
@@ -1177,7 +1172,8 @@ static rt_status lowrank_from_gradient(rt_model* m, rt_linear* l, int M, LowRank
   if (!l->lora_active() || !rmsnorm_takes_lowrank(m->cfg.hidden, l->lora.rank)) return RT_OK;
   __half* gs = lowrank_buf(m->lsc.gs[m->lsc.n_jobs], M);
   if (!gs) return m->ctx->fail(RT_ERR_CUDA, "out of device memory (lora scratch)");
-  *lr = lowrank_g(l, gs);
+  lora_refresh(l);
+  *lr = {l->lora.bt_s, l->lora.rank, gs};
   return RT_OK;
 }
 

@@ -85,3 +85,26 @@ def test_recomputed_blocks_get_the_bits_of_kept_ones(ctx, hidden, rank, lens):
         got.append(_gpu_flat(gm, "ga", "gb"))
     assert np.array_equal(*got) and np.abs(got[0]).max() > 0
     gm.close()
+
+
+def test_only_a_pass_with_active_adapters_asks_for_their_scratch():
+    """Scoring with the base model (no adapter enabled) leaves Hs' memory, 128 bytes a token, unasked for."""
+    import torch
+
+    c = rt.Context(0)
+    spec = _spec(256)
+    _, _, gm = _model(c, spec, 8)
+    toks = synth.token_batch(spec, 64, 1024, 3)
+    tp, tt = synth.answer_targets(toks[0], 64)
+
+    def free_after_a_pass():
+        gm.score(list(toks), tp, tt)
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    gm.set_lora_enabled(False)
+    base = free_after_a_pass()
+    gm.set_lora_enabled(True)
+    assert base - free_after_a_pass() >= 64 * 1024 * 64 * 2
+    gm.close()
+    c.close()
