@@ -412,7 +412,7 @@ template <int HD>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                         const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                        const float* __restrict__ tops, const float* __restrict__ query_vecs, const int* __restrict__ seq_start,
+                        const float* tops, const float* query_vecs, const int* __restrict__ seq_start,
                         const int2* __restrict__ gap, const int2* __restrict__ tiles, int M, int nh, int nkv, int heads_per_cta,
                         int n_ctas, float scale, float* __restrict__ dk, float* __restrict__ dv, int* status) {
   using L = DkvLayout<HD>;
@@ -718,8 +718,8 @@ template <int HD>
 __global__ void __launch_bounds__(DQ_THREADS, 2)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                      const float* __restrict__ row_scale, const float* __restrict__ lse,
-                      const float* __restrict__ query_vecs, const int* __restrict__ seq_start, const int2* __restrict__ gap,
+                      const float* row_scale, const float* lse,
+                      const float* query_vecs, const int* __restrict__ seq_start, const int2* __restrict__ gap,
                       const int* __restrict__ tiles, int M, int nh, int nkv, float scale, float* __restrict__ dq, int* status) {
   using L = DqLayout<HD>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];

@@ -120,7 +120,7 @@ void launch_split_f32_hi_lo(const float* w, size_t n, __half* hi, __half* lo, cu
 }
 
 // Row-normalised f16 copy: y16[r,:] = x[r,:] / amax_r, scale[r] = amax_r (1 if the row is zero).
-__global__ void normalize_rows_kernel(const float* __restrict__ x, int d, __half* __restrict__ y16,
+__global__ void normalize_rows_kernel(const float* x, int d, __half* __restrict__ y16,
                                       float* __restrict__ scale) {
   pdl_entry();
   const size_t r = blockIdx.x;
@@ -167,7 +167,7 @@ __device__ __forceinline__ void block_sum2(float& a, float& b) {
   a = b = 0.f;
   for (int k = 0; k < nw; ++k) { a += sa[k]; b += sb[k]; }
 }
-__global__ void __launch_bounds__(1024) rmsnorm_fwd_row_kernel(const float* __restrict__ x, const float* __restrict__ w, int d, float eps,
+__global__ void __launch_bounds__(1024) rmsnorm_fwd_row_kernel(const float* x, const float* __restrict__ w, int d, float eps,
                                                                __half* __restrict__ y16) {
   pdl_entry();
   const size_t r = blockIdx.x;
@@ -226,7 +226,7 @@ __device__ __forceinline__ void rms_fwd_row(const float4* v, const float* __rest
 }
 template <int NV>
 __global__ void __launch_bounds__(256)
-rmsnorm_fwd_warp_kernel(const float* __restrict__ x, const float* __restrict__ w, int rows, float eps,
+rmsnorm_fwd_warp_kernel(const float* x, const float* __restrict__ w, int rows, float eps,
                         __half* __restrict__ y16) {
   pdl_entry();
   constexpr int D = 128 * NV;
@@ -266,7 +266,7 @@ __device__ __forceinline__ float rms_bwd_row(const float4* xv, float4* gv, const
 }
 template <int NV>
 __global__ void __launch_bounds__(256)
-rmsnorm_bwd_warp_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ dn,
+rmsnorm_bwd_warp_kernel(const float* x, const float* __restrict__ w, const float* dn,
                         const float* dres, int rows, float eps, float* out, __half* __restrict__ out16,
                         float* __restrict__ scale) {
   pdl_entry();
@@ -443,8 +443,8 @@ __global__ void rmsnorm_bwd_kernel(const float* __restrict__ x, const float* __r
     if (threadIdx.x == 0) scale[r] = m;
   }
 }
-__global__ void __launch_bounds__(1024) rmsnorm_bwd_row_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                               const float* __restrict__ dn, const float* dres, int d, float eps,
+__global__ void __launch_bounds__(1024) rmsnorm_bwd_row_kernel(const float* x, const float* __restrict__ w,
+                                                               const float* dn, const float* dres, int d, float eps,
                                                                float* out, __half* __restrict__ out16, float* __restrict__ scale) {
   pdl_entry();
   const size_t r = blockIdx.x;
@@ -735,7 +735,7 @@ __device__ __forceinline__ void store_epl_h(__half* p, const float* v) {
 
 template <int EPL, int HPW>
 __global__ void __launch_bounds__(256)
-qk_rope_fwd_reg_kernel(const float* __restrict__ q_raw, const float* __restrict__ k_raw, const float* __restrict__ v_raw,
+qk_rope_fwd_reg_kernel(const float* q_raw, const float* k_raw, const float* v_raw,
                        size_t pq, size_t pk, size_t pv,  // row pitches of the three inputs, in elements
                        const float* __restrict__ qw, const float* __restrict__ kw, const int* __restrict__ pos,
                        const float* __restrict__ cs, const float* __restrict__ sn, int nh, int nkv, int rot, int neox,
@@ -793,7 +793,7 @@ qk_rope_fwd_reg_kernel(const float* __restrict__ q_raw, const float* __restrict_
 // arithmetic; it is bound by instruction issue, not by bytes.
 template <int EPL, int QPW, int KPW, bool NEOX, bool NORM>
 __global__ void __launch_bounds__(256)
-qk_rope_fwd_fast_kernel(const float* __restrict__ q_raw, const float* __restrict__ k_raw, const float* __restrict__ v_raw,
+qk_rope_fwd_fast_kernel(const float* q_raw, const float* k_raw, const float* v_raw,
                         size_t pq, size_t pk, size_t pv, const float* __restrict__ qw, const float* __restrict__ kw,
                         const int* __restrict__ pos, const float* __restrict__ cs, const float* __restrict__ sn, float eps,
                         __half* __restrict__ q16, __half* __restrict__ k16, __half* __restrict__ v16) {
@@ -865,8 +865,8 @@ qk_rope_fwd_fast_kernel(const float* __restrict__ q_raw, const float* __restrict
 
 template <int EPL, int HPW>
 __global__ void __launch_bounds__(256, 4)
-qk_rope_bwd_reg_kernel(const float* __restrict__ dq, const float* __restrict__ dk, const float* __restrict__ dv,
-                       const float* __restrict__ q_raw, const float* __restrict__ k_raw, size_t pq, size_t pk,
+qk_rope_bwd_reg_kernel(const float* dq, const float* dk, const float* dv,
+                       const float* q_raw, const float* k_raw, size_t pq, size_t pk,
                        size_t oq, size_t ok, size_t ov, int common,  // output row pitches; one scale for all three
                        const float* __restrict__ qw,
                        const float* __restrict__ kw, const int* __restrict__ pos, const float* __restrict__ cs,
@@ -963,8 +963,8 @@ qk_rope_bwd_reg_kernel(const float* __restrict__ dq, const float* __restrict__ d
 // that are multiples of eight, both norms or none): no per-head decisions left.
 template <int EPL, int QPW, int KPW, bool NEOX, bool NORM>
 __global__ void __launch_bounds__(256, (QPW + 2 * KPW <= 4) ? 4 : ((QPW + 2 * KPW <= 6) ? 3 : 2))
-qk_rope_bwd_fast_kernel(const float* __restrict__ dq, const float* __restrict__ dk, const float* __restrict__ dv,
-                        const float* __restrict__ q_raw, const float* __restrict__ k_raw, size_t pq, size_t pk, size_t oq,
+qk_rope_bwd_fast_kernel(const float* dq, const float* dk, const float* dv,
+                        const float* q_raw, const float* k_raw, size_t pq, size_t pk, size_t oq,
                         size_t ok, size_t ov, int common, const float* __restrict__ qw, const float* __restrict__ kw,
                         const int* __restrict__ pos, const float* __restrict__ cs, const float* __restrict__ sn, float eps,
                         __half* __restrict__ dq16, __half* __restrict__ dk16, __half* __restrict__ dv16,
@@ -1313,7 +1313,7 @@ __device__ __forceinline__ uint4 swiglu8(const uint4& gv, const uint4& uv) {
   }
   return o;
 }
-__global__ void swiglu_fwd_kernel(const __half* __restrict__ g, const __half* __restrict__ u, __half* __restrict__ h,
+__global__ void swiglu_fwd_kernel(const __half* g, const __half* u, __half* __restrict__ h,
                                   size_t n, int* status) {
   pdl_entry();
   size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -1330,7 +1330,7 @@ __global__ void swiglu_fwd_kernel(const __half* __restrict__ g, const __half* __
   }
 }
 // gate and up as column slices of one [rows x pitch] matrix (ff a multiple of 8)
-__global__ void swiglu_fwd_pitched_kernel(const __half* __restrict__ g, const __half* __restrict__ u, size_t pitch, int ff,
+__global__ void swiglu_fwd_pitched_kernel(const __half* g, const __half* u, size_t pitch, int ff,
                                           size_t n, __half* __restrict__ h, int* status) {
   pdl_entry();
   const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
@@ -1429,9 +1429,9 @@ __device__ __forceinline__ void swiglu_grad8(const Raw8<DT>& dh, const Raw8<__ha
 // dh is f32, or f16 rows that still lack their per-row factor in_scale[r] (which then only
 // multiplies the two output scales).
 template <typename DT>  // NCH 8-element chunks per thread, kept in registers: ff <= NCH * 8 * blockDim.x, ff % 8 == 0
-__global__ void __launch_bounds__(512) swiglu_bwd_cached_kernel(const DT* __restrict__ dh, const float* __restrict__ in_scale,
-                                         const __half* __restrict__ g,
-                                         const __half* __restrict__ u, size_t gp, int ff, __half* __restrict__ dg16,
+__global__ void __launch_bounds__(512) swiglu_bwd_cached_kernel(const DT* dh, const float* in_scale,
+                                         const __half* g,
+                                         const __half* u, size_t gp, int ff, __half* __restrict__ dg16,
                                          __half* __restrict__ du16, size_t op, int common, float* __restrict__ sg,
                                          float* __restrict__ su) {
   pdl_entry();
@@ -1552,7 +1552,7 @@ void launch_swiglu_bwd(const void* dh, int dh_f16, const float* in_scale, const 
 }
 
 // ------------------------------------------------------------------ row gather / scatter
-__global__ void gather_f32_rows_kernel(const float* __restrict__ x, const int* __restrict__ idx, int d,
+__global__ void gather_f32_rows_kernel(const float* x, const int* __restrict__ idx, int d,
                                        float* __restrict__ out) {
   pdl_entry();
   const size_t r = blockIdx.x;
@@ -1563,8 +1563,8 @@ void launch_gather_f32_rows(const float* x, const int* idx, int rows, int d, flo
   if (rows > 0) { pdl(gather_f32_rows_kernel, rows, 256, 0, st)(x, idx, d, out); RT_COUNT_LAUNCH(1); }
 }
 // dx[idx[r], :] += src[r, :]   (atomic: two targets may name the same position)
-__global__ void scatter_add_rows_kernel(const float* __restrict__ src, const int* __restrict__ idx, int d,
-                                        float* __restrict__ dx) {
+__global__ void scatter_add_rows_kernel(const float* src, const int* __restrict__ idx, int d,
+                                        float* dx) {
   pdl_entry();
   const size_t r = blockIdx.x;
   float* dst = dx + (size_t)idx[r] * d;
@@ -1580,7 +1580,7 @@ void launch_scatter_add_rows(const float* src, const int* idx, int rows, int d, 
 // w (so dlogits = w*(p - onehot) exactly as the reference forms it).
 // The greedy token of a row: the LAST index holding the maximum, which is what the reference's
 // Iterator::max_by(total_cmp) returns on ties (src/eval.rs:167).  One more read of the row.
-__device__ void ce_row_argmax(const float* __restrict__ row, int v, float m, int* __restrict__ out) {
+__device__ void ce_row_argmax(const float* row, int v, float m, int* __restrict__ out) {
   __shared__ int s_arg[32];
   int best = -1;
   for (int i = threadIdx.x; i < v; i += blockDim.x)
@@ -1598,8 +1598,8 @@ __device__ void ce_row_argmax(const float* __restrict__ row, int v, float m, int
   }
 }
 
-__global__ void ce_row_kernel(const float* __restrict__ logits, int v, const int* __restrict__ target,
-                              const float* __restrict__ weight, float* __restrict__ logp, int* __restrict__ hits,
+__global__ void ce_row_kernel(const float* logits, int v, const int* __restrict__ target,
+                              const float* __restrict__ weight, float* __restrict__ logp, int* hits,
                               __half* __restrict__ d16, float* __restrict__ scale, int* __restrict__ argmax, int* status) {
   pdl_entry();
   const size_t r = blockIdx.x;
@@ -1643,8 +1643,8 @@ __global__ void ce_row_kernel(const float* __restrict__ logits, int v, const int
 // blocks that reads each logit once into registers (nothing runs under its reductions).
 constexpr int CE_THREADS = 1024, CE_REG4 = 5, CE_CHUNK_BYTES = 4 * CE_THREADS * 16;
 __global__ void __launch_bounds__(CE_THREADS, 1)
-ce_row_vec_kernel(const float* __restrict__ logits, int v, const int* __restrict__ target,
-                  const float* __restrict__ weight, float* __restrict__ logp, int* __restrict__ hits,
+ce_row_vec_kernel(const float* logits, int v, const int* __restrict__ target,
+                  const float* __restrict__ weight, float* __restrict__ logp, int* hits,
                   __half* __restrict__ d16, float* __restrict__ scale, int* __restrict__ argmax, int* status, int n_chunks) {
   extern __shared__ float4 s_row[];  // [n_chunks <= 3][4][CE_THREADS]
   pdl_entry();

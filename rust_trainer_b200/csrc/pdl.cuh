@@ -6,8 +6,9 @@
 //   - every CTA executes pdl_wait() before its first access to anything the pass computes and before any
 //     early return (a grid that is complete has then waited, so ordering stays transitive).  What a batch
 //     brings along and no kernel writes (tile lists, where sequences start) may be read before it;
-//   - new kernels read what the pass computes through plain pointers.  const __restrict__ tells the compiler that it does not change while
-//     the kernel runs, and then a conditional load may move in front of the wait (a kernel that was not kept read its input too early);
+//   - what the pass computes is read through plain pointers.  __restrict__ promises the compiler that nobody else writes there while the
+//     kernel runs, which the kernel in front of it still does: a conditional load may then move in front of the wait (a kernel that
+//     was not kept read its input too early), or go through a cache that neither the wait nor pdl_unwaited's fence refreshes;
 //   - pdl_launch_dependents() is called at entry: the next kernel may be scheduled as soon as
 //     every CTA of this one has started.  A CTA that has not got its TMEM yet must then find it: a CTA of a later kernel that took the
 //     columns on the same SM waits for this kernel, which would wait for them.  So a kernel with TMEM lets the next one start once it

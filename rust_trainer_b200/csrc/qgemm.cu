@@ -960,9 +960,9 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
 
 // Sums the pieces' partials in order (deterministic) and applies the epilogue the fused path would have
 // applied: per-token scale, bias, accumulate or residual.  Output is f32 with row pitch ld.
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, int M, int R, float* __restrict__ out, size_t ld,
-                                     const float* __restrict__ row_scale, const float* __restrict__ bias, int accumulate,
-                                     const float* __restrict__ residual) {
+__global__ void splitk_reduce_kernel(const float* part, int splits, int M, int R, float* out, size_t ld,
+                                     const float* row_scale, const float* __restrict__ bias, int accumulate,
+                                     const float* residual) {
   pdl_entry();
   const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n = (size_t)M * R;

@@ -63,3 +63,25 @@ def test_the_exponents_offset_of_attention_is_fused_by_name():
     """Left to the compiler, a load moved from beside the multiplication to the kernel's front took the fused multiply-add apart: the
     gradients of a 3B step moved by 1e-3."""
     assert re.search(r"off = fmaf\(-my_lse, LOG2E, log2f\(w\) \+ P_BOOST_LOG2\);", kernels()["attn_delta_tc_kernel"])
+
+
+#: what may be declared __restrict__ in a kernel that starts under the one in front of it: what no kernel of a pass writes (norm
+#: weights, biases, tables, what a batch brings along), and results that the kernel only writes
+UNWRITTEN = {"w", "qw", "kw", "bias", "cs", "sn", "pos", "idx", "target", "weight", "seq_start", "gap", "tiles"}
+ONLY_WRITTEN = {"y16", "out16", "scale", "q16", "k16", "v16", "dq16", "dk16", "dv16", "sq", "sk", "sv", "h", "dg16", "du16", "sg", "su", "d16",
+                "logp", "argmax", "lse", "dk", "dv", "dq", "query_vecs", "tops"}
+WAITS = sorted(n for n, body in kernels().items() if "pdl_wait();" in body or "pdl_entry();" in body)
+
+
+@pytest.mark.parametrize("name", WAITS)
+def test_what_a_pass_computes_is_read_through_plain_pointers(name):
+    """__restrict__ promises that nobody else writes behind the pointer while the kernel runs, which the kernel in front of it still
+    does: the compiler may then load before the wait, or through a cache that neither wait nor fence refreshes."""
+    body = kernels()[name]
+    params = body[:body.index("{")]
+    read = {m[1] for m in re.finditer(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params)}
+    declared = {m[1] for m in re.finditer(r"__restrict__\s+(\w+)", params)}
+    assert read <= UNWRITTEN, read - UNWRITTEN
+    # (others also read their `out`: a product may be accumulated, a gradient be added where it lies)
+    written = ONLY_WRITTEN | ({"out"} if name in ("lowrank_tc_kernel", "gather_f32_rows_kernel") else set())
+    assert declared - read <= written, declared - read - written
