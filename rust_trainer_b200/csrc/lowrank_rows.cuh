@@ -68,23 +68,24 @@ struct LrAcc {
 __host__ __device__ constexpr int lr_pitch(int mt) { return 16 * mt + 4; }  // keeps a warp's stores in different banks
 __host__ __device__ constexpr int lr_sum_floats(int warps, int mt) { return warps * LR_TOKENS * lr_pitch(mt); }
 
-// Adds the warps' sums up and writes tokens m0.. (those below M) of NT groups.  Called by the whole CTA, WARPS warps for each
-// group; nobody reads `sums` any more.
-template <int MT, int NT, int WARPS>
-__device__ __forceinline__ void lr_finish(const LrAcc<MT>& acc, float* sums, int group, int slice, int lane, int m0, int M, __half* __restrict__ out) {
+// A warp's sum of a group, where lr_sum finds it.
+template <int MT, int WARPS>
+__device__ __forceinline__ void lr_put(const LrAcc<MT>& acc, float* sums, int group, int slice, int lane) {
   constexpr int P = lr_pitch(MT);
-  {
-    float* s = sums + (group * WARPS + slice) * (LR_TOKENS * P) + 2 * (lane & 3) * P + (lane >> 2);
+  float* s = sums + (group * WARPS + slice) * (LR_TOKENS * P) + 2 * (lane & 3) * P + (lane >> 2);
 #pragma unroll
-    for (int m = 0; m < MT; ++m) {
-      s[16 * m] = acc.d[m][0];
-      s[16 * m + P] = acc.d[m][1];
-      s[16 * m + 8] = acc.d[m][2];
-      s[16 * m + 8 + P] = acc.d[m][3];
-    }
+  for (int m = 0; m < MT; ++m) {
+    s[16 * m] = acc.d[m][0];
+    s[16 * m + P] = acc.d[m][1];
+    s[16 * m + 8] = acc.d[m][2];
+    s[16 * m + 8 + P] = acc.d[m][3];
   }
-  __syncthreads();
-  const int t = ((group * WARPS + slice) * 32 + lane) >> 4, c = (lane & 15) * 4;
+}
+// Adds the warps' sums up and writes tokens m0.. (those below M) of NT groups; thread: of the CTA.
+template <int MT, int NT, int WARPS>
+__device__ __forceinline__ void lr_sum(const float* sums, int thread, int m0, int M, __half* __restrict__ out) {
+  constexpr int P = lr_pitch(MT);
+  const int t = thread >> 4, c = (thread & 15) * 4;
   if (t < NT * LR_TOKENS && m0 + t < M) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < 16 * MT) {
@@ -98,6 +99,13 @@ __device__ __forceinline__ void lr_finish(const LrAcc<MT>& acc, float* sums, int
     const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
     *(uint2*)(out + (size_t)(m0 + t) * 64 + c) = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
   }
+}
+// Both, called by the whole CTA, WARPS warps for each group; nobody reads `sums` any more.
+template <int MT, int NT, int WARPS>
+__device__ __forceinline__ void lr_finish(const LrAcc<MT>& acc, float* sums, int group, int slice, int lane, int m0, int M, __half* __restrict__ out) {
+  lr_put<MT, WARPS>(acc, sums, group, slice, lane);
+  __syncthreads();
+  lr_sum<MT, NT, WARPS>(sums, (group * WARPS + slice) * 32 + lane, m0, M, out);
 }
 
 // The CTAs' shares of the weights on their way to L2 while the kernel in front still runs (nothing is read).

@@ -73,7 +73,7 @@ static __half* lowrank_buf(DevBuf& b, int M) {
 static int launch_lowrank(rt_ctx* c, const __half* x, const __half* w, int M, int K, int r, __half* out) {
   // (what is not aligned the other launch refuses)
   if (!lowrank_rows_takes(K, r) || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15)) return launch_lowrank_tc(c, x, w, M, K, r, out);
-  launch_lowrank_rows(x, M, K, LowRank{w, r, out}, c->stream);
+  launch_lowrank_rows(c, x, M, K, LowRank{w, r, out});
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
 

@@ -1355,7 +1355,7 @@ void launch_swiglu_fwd(const __half* g, const __half* u, size_t in_pitch, int ro
 // every CTA reads all the weights, so that the tcgen05 stream, which reads them once for 64 or 128 tokens, is the better one where they
 // are larger (4096 columns with 48 indices in a step of 1024 tokens 14 us against 5.8, 3072 with 16 at 8192 tokens 17.8 against
 // 16.3).  2048 columns, 16 indices, in a step of 1024 tokens 5.8 -> 3.6 us, of 8192 as fast.
-constexpr int LR_WARPS = 16;
+constexpr int LR_WARPS = 16, LR_MANY_K = 1024, LR_MANY_GROUPS = 2;
 template <int NT>
 __global__ void __launch_bounds__(32 * LR_WARPS) lowrank_rows_kernel(const __half* x, int K, int rows, const LowRank lr) {
   __shared__ __align__(16) float sums[lr_sum_floats(LR_WARPS, 1)];
@@ -1384,11 +1384,61 @@ __global__ void __launch_bounds__(32 * LR_WARPS) lowrank_rows_kernel(const __hal
     lr_finish<1, 1, LR_WARPS>(acc[n], sums, 0, warp, lane, m0 + n * LR_TOKENS, rows, lr.out);
   }
 }
+// The same sums for rows of up to 1024 columns and more tokens than the GPU holds at a time: two CTAs an SM that keep their warps' two
+// blocks of the weights in registers and fetch the next tokens under the sums of these.  Bound: DRAM (1024 columns, 16 indices, 16384 tokens
+// before a product of 1024 features: 43.3 us with a CTA for every 16 tokens, which all wait for their weights; 40.9 behind the
+// tcgen05 stream; 39.4 so).
+__global__ void __launch_bounds__(32 * LR_WARPS, 2) lowrank_rows_many_kernel(const __half* x, int K, int rows, const LowRank lr) {
+  constexpr int NT = LR_MANY_GROUPS, NB = LR_MANY_K / 32 / LR_WARPS;
+  __shared__ __align__(16) float sums[2][NT * lr_sum_floats(LR_WARPS, 1)];  // in turn: one barrier for each group
+  lr_prefetch(lr.w, lr.r, K);
+  pdl_wait();
+  pdl_launch_dependents();  // only now: QGemmArgs::late_wait
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, step = (int)gridDim.x * (LR_TOKENS * NT);
+  const __half* xr = x + (size_t)(lane >> 2) * K + warp * 32 + (lane & 3) * 8;
+  int m0 = (int)blockIdx.x * (LR_TOKENS * NT);
+  uint4 v[NB][NT];
+  auto fetch = [&](int m) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        const int k = b * (LR_WARPS * 32), t = m + n * LR_TOKENS;
+        v[b][n] = warp * 32 + k < K && t + (lane >> 2) < rows ? *(const uint4*)(xr + (size_t)t * K + k) : make_uint4(0, 0, 0, 0);
+      }
+  };
+  fetch(m0);
+  LrWeights<1> w[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int k = warp * 32 + b * (LR_WARPS * 32);
+    w[b] = {};
+    if (k < K) w[b].load(lr.w, lr.r, K, k, lane);
+  }
+  for (int buf = 0; m0 < rows; m0 += step, buf ^= 1) {
+    LrAcc<1> acc[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      acc[n].clear();
+#pragma unroll
+      for (int b = 0; b < NB; ++b) acc[n].add(w[b], v[b][n]);
+    }
+    fetch(m0 + step);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) lr_put<1, LR_WARPS>(acc[n], sums[buf], n, warp, lane);
+    __syncthreads();
+    lr_sum<1, NT, LR_WARPS>(sums[buf], (int)threadIdx.x, m0, rows, lr.out);
+  }
+}
 bool lowrank_rows_takes(int K, int r) { return K % 32 == 0 && K <= 2048 && r >= 1 && r <= 16; }
-void launch_lowrank_rows(const __half* x, int rows, int K, const LowRank& lr, cudaStream_t st) {
+void launch_lowrank_rows(rt_ctx* c, const __half* x, int rows, int K, const LowRank& lr) {
   if (rows <= 0) return;
-  if (rows <= 2048) pdl(lowrank_rows_kernel<1>, (rows + LR_TOKENS - 1) / LR_TOKENS, 32 * LR_WARPS, 0, st)(x, K, rows, lr);
-  else pdl(lowrank_rows_kernel<2>, (rows + 2 * LR_TOKENS - 1) / (2 * LR_TOKENS), 32 * LR_WARPS, 0, st)(x, K, rows, lr);
+  constexpr int CTA = 2 * LR_TOKENS;  // tokens of a CTA beyond 2048 of them
+  static_assert(CTA == LR_MANY_GROUPS * LR_TOKENS);
+  const int at_a_time = 2 * c->num_sms;  // CTAs; from 6000 tokens on the persistent ones are faster (9000 of 1024: 25.7 -> 23.9 us), at 4096 as fast
+  if (rows <= 2048) pdl(lowrank_rows_kernel<1>, (rows + LR_TOKENS - 1) / LR_TOKENS, 32 * LR_WARPS, 0, c->stream)(x, K, rows, lr);
+  else if (K > LR_MANY_K || rows <= at_a_time * CTA) pdl(lowrank_rows_kernel<2>, (rows + CTA - 1) / CTA, 32 * LR_WARPS, 0, c->stream)(x, K, rows, lr);
+  else pdl(lowrank_rows_many_kernel, at_a_time, 32 * LR_WARPS, 0, c->stream)(x, K, rows, lr);
   RT_COUNT_LAUNCH(1);
 }
 // dg = dh*u*silu'(g), du = dh*silu(g); both written row-normalised in f16 with per-row scales.

@@ -74,7 +74,7 @@ void launch_adamw(float* p, float* g, float* m, float* v, size_t n, const double
 
 // lr.out = the low-rank product of X [rows x K]; a matmul may start under it (QGemmArgs::late_wait)
 bool lowrank_rows_takes(int K, int r);
-void launch_lowrank_rows(const __half* x, int rows, int K, const LowRank& lr, cudaStream_t st);
+void launch_lowrank_rows(rt_ctx* c, const __half* x, int rows, int K, const LowRank& lr);
 // ---- lowrank_tc.cu: out64[M x 64] (f16, zero from column r up) = X[M x K] . Wt[r x K]^T on tcgen05; 1 = shape not taken
 int launch_lowrank_tc(rt_ctx* c, const __half* X, const __half* Wt, int M, int K, int r, __half* out64);
 // A linear's (or a stacked group's) adapters as the token contractions see them: member j owns rows

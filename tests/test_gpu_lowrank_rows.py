@@ -7,6 +7,7 @@ import pytest
 import rust_trainer_b200 as rt
 from conftest import cosine, rel_l2
 from oracle import oracle as O
+from rust_trainer_b200 import quants as Q
 from rust_trainer_b200 import synth
 from test_gpu_model import GRAD_COS, GRAD_TOL, LOSS_TOL, _batch, _flat, _gpu_flat, _oracle_step
 
@@ -108,3 +109,26 @@ def test_only_a_pass_with_active_adapters_asks_for_their_scratch():
     assert base - free_after_a_pass() >= 64 * 1024 * 64 * 2
     gm.close()
     c.close()
+
+
+# columns: one block of K for one warp, a ragged share of the second block, all of it; tokens: just beyond what the GPU holds at a
+# time, ragged last groups, several rounds
+@pytest.mark.parametrize("k,r,m", [(32, 1, 4737), (544, 3, 9475), (896, 16, 16391), (1024, 8, 30001)])
+def test_products_of_many_tokens(ctx, k, r, m):
+    """A linear whose weights are zero gives the adapter alone: the reference's value, and the bits of the same tokens in batches
+    small enough for the other kernel."""
+    rng = np.random.default_rng(m)
+    n = 64
+    f = rt.Frozen.from_f32(ctx, np.zeros((n, k), np.float32), Q.Q8_0)
+    lin = rt.Linear("l", f)
+    a, b = rng.standard_normal((r, k)).astype(np.float32), rng.standard_normal((n, r)).astype(np.float32)
+    lin.attach_lora(r, 2.0 * r, a, b)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    y = lin.forward(x, m)
+    # x, s A, the product and B are rounded to f16, 2^-12 of each value on average at most, and the sums are f32
+    want = 2.0 * (x.astype(np.float64) @ a.T.astype(np.float64)) @ b.T.astype(np.float64)
+    assert rel_l2(y, want) < 4 * 2.0 ** -12
+    parts = [lin.forward(x[i:i + 4096], min(4096, m - i)) for i in range(0, m, 4096)]
+    assert np.array_equal(y, np.concatenate(parts))
+    lin.close()
+    f.close()
