@@ -29,7 +29,10 @@ rt_status rt_ctx::check_device_status(const char* where) {
   const int s = *(volatile int*)status_host;  // written by the kernel that reported it (StatusBlock)
   if (s == 0) return RT_OK;
   *(volatile int*)status_host = 0;
+  // complete before the host goes on, which may launch on another stream: a kernel that still found the old code would give up its
+  // waits and, not being the first, report nothing
   cudaMemsetAsync(status_dev, 0, sizeof(int), stream);
+  cudaStreamSynchronize(stream);
   char buf[160];
   if (s == RT_ERR_BAD_INDEX) {
     snprintf(buf, sizeof buf, "%s: index out of range on device", where);

@@ -85,3 +85,13 @@ def test_what_a_pass_computes_is_read_through_plain_pointers(name):
     # (others also read their `out`: a product may be accumulated, a gradient be added where it lies)
     written = ONLY_WRITTEN | ({"out"} if name in ("lowrank_tc_kernel", "gather_f32_rows_kernel") else set())
     assert declared - read <= written, declared - read - written
+
+
+def test_the_device_word_is_clear_before_a_call_that_reports_an_error_returns():
+    """A host that goes on on another stream would otherwise launch kernels that find the old code, give up their waits and, not being
+    the first to report, leave the page-locked word at "no error"."""
+    src = (CSRC / "api.cu").read_text()
+    body = src[src.index("rt_status rt_ctx::check_device_status"):]
+    body = body[:body.index("\n}")]
+    clear = body.index("cudaMemsetAsync(status_dev, 0")
+    assert clear < body.index("cudaStreamSynchronize(stream)", clear) < body.index("return RT_ERR_BAD_INDEX")
