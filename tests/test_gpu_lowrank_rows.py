@@ -51,23 +51,37 @@ def test_gradients_match_the_oracle(ctx, hidden, rank, lens):
     om.close()
 
 
-@pytest.mark.parametrize("hidden,rank,more", [(1024, 16, 17), (896, 8, 20), (128, 64, 63), (1024, 32, 17)])
-def test_a_sequence_gets_the_same_products_in_a_small_and_a_large_batch(ctx, hidden, rank, more):
-    """One sequence of 128 tokens alone, and as the first of a batch of more than 2048 whose other targets have no weight."""
+# widths and ranks of every form beyond 2048 tokens: forward products of one to four groups of rank indices (stacks of two and three
+# adapters of up to 20), backward ones of one to four
+@pytest.mark.parametrize("hidden,rank", [(256, 4), (1024, 16), (896, 20), (640, 12), (384, 40), (128, 64)])
+def test_a_sequence_gets_the_same_products_in_a_small_and_a_large_batch(ctx, hidden, rank):
+    """Two sequences alone, and as the first and the last of a batch of 9347 tokens: persistent CTAs take two to eight groups of rows
+    in turn (at most two of an SM, with eight or sixteen rows each: 4736 tokens at a time), and the last group is not full."""
     spec = _spec(hidden)
     _, _, gm = _model(ctx, spec, rank)
-    toks = synth.token_batch(spec, more + 1, 128, 3)
-    tp, tt = synth.answer_targets(toks[0], 64)
-    w = np.full(tp.size, 1.0 / tp.size, np.float32)
-    gm.zero_grad()
-    alone, _ = gm.forward_backward([toks[0]], tp, tt, w)
-    g_alone = _gpu_flat(gm, "ga", "gb")
-    gm.zero_grad()
-    many, _ = gm.forward_backward(list(toks), np.concatenate([tp, tp + 128]), np.concatenate([tt, tt]), np.concatenate([w, 0 * w]))
-    assert np.array_equal(alone, many[:tp.size])
-    # the gradients' last f32 sums (over key tiles, over splits of tokens) fall differently, a few 2^-24; another rounding of a
-    # 16-bit product anywhere would show as 2^-12 of its value
-    assert rel_l2(_gpu_flat(gm, "ga", "gb"), g_alone) < 1e-6 and np.abs(g_alone).max() > 0
+    fill = list(synth.token_batch(spec, 71, 128, 3))
+    ends = [synth.token_batch(spec, 1, n, 5 + n)[0] for n in (128, 131)]
+    parts = [synth.answer_targets(q, 64) for q in ends]
+
+    def run(seqs, tp, tt, w):
+        gm.zero_grad()
+        lp, _ = gm.forward_backward(seqs, tp, tt, w)
+        return lp, _gpu_flat(gm, "ga", "gb")
+
+    def weights(n):
+        return np.full(n, 1.0 / 64, np.float32)
+
+    alone = [run([q], p, t, weights(p.size)) for q, (p, t) in zip(ends, parts)]
+    lead = 128 * (1 + len(fill))  # (sequences that start on a tile boundary)
+    idle = np.arange(128, lead - 1, 97)
+    tp = np.concatenate([parts[0][0], idle, parts[1][0] + lead])
+    tt = np.concatenate([parts[0][1], 0 * idle, parts[1][1]])
+    w = np.concatenate([weights(parts[0][0].size), np.zeros(idle.size, np.float32), weights(parts[1][0].size)])
+    lp, grads = run([ends[0], *fill, ends[1]], tp, tt, w)
+    assert np.array_equal(alone[0][0], lp[:parts[0][0].size]) and np.array_equal(alone[1][0], lp[-parts[1][0].size:])
+    # the gradients' last f32 sums (over key tiles, over splits of tokens, over the two sequences) fall differently, a few 2^-24; another
+    # rounding of a 16-bit product anywhere would show as 2^-12 of its value
+    assert rel_l2(grads, alone[0][1] + alone[1][1]) < 1e-6 and all(np.abs(g).max() > 0 for _, g in alone)
     gm.close()
 
 

@@ -95,3 +95,22 @@ def test_the_device_word_is_clear_before_a_call_that_reports_an_error_returns():
     body = body[:body.index("\n}")]
     clear = body.index("cudaMemsetAsync(status_dev, 0")
     assert clear < body.index("cudaStreamSynchronize(stream)", clear) < body.index("return RT_ERR_BAD_INDEX")
+
+
+@pytest.mark.parametrize("name", ["lowrank_tc_kernel", "lowrank_rows_kernel", "lowrank_rows_many_kernel", "attn_bwd_dkdv_tc_kernel", "lora_grads_tc_kernel"])
+def test_a_kernel_with_a_successor_that_reads_unwaited_lets_it_start_after_its_own_wait(name):
+    """What is older than such a kernel is then complete when its successor, which reads that without waiting, starts."""
+    body = kernels()[name]
+    assert "pdl_entry" not in body and body.count("pdl_launch_dependents();") == 1
+    assert 0 <= body.index("pdl_wait();") < body.index("pdl_launch_dependents();")
+
+
+@pytest.mark.parametrize("name", ["lowrank_rows_kernel", "lowrank_rows_many_kernel", "rmsnorm_fwd_lr_kernel", "rmsnorm_bwd_lr_kernel"])
+def test_only_prefetches_come_before_the_wait(name):
+    body = kernels()[name]
+    before = body[body.index("{") + 1:body.index("pdl_wait();")]
+    allowed = (r"using C = [^;]*;|constexpr [^;]*;|extern __shared__ [^;]*;|__shared__ [^;]*;|\w+\*? ?\*?\w+ = \(?[\w*]*\)?\(?lr_smem[^;]*;|pdl_launch_dependents\(\);"
+               r"|lr_prefetch\([^;]*\);")
+    assert re.sub(allowed, "", before).strip() == ""
+    prefetch = re.search(r"void lr_prefetch\([^{]*\{(.*?)\n\}", (CSRC / "lowrank_rows.cuh").read_text(), re.S)[1]
+    assert "prefetch.global.L2" in prefetch and "ld." not in prefetch and "*(" not in prefetch
