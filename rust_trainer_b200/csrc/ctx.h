@@ -53,7 +53,7 @@ struct rt_ctx {
     smem_raised.insert(fn);
     return true;
   }
-  // Reads the device status word (after synchronising); maps non-zero to an error.
+  // Waits for the stream and reads the page-locked status word; maps non-zero to an error and clears it and the device's.
   rt_status check_device_status(const char* where);
 };
 

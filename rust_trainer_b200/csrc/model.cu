@@ -62,8 +62,9 @@ rt_status lora_refresh(rt_linear* l) {
   return RT_OK;
 }
 
-// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16 columns; lowrank_tc_kernel writes all
-// 64 columns of every row, zeros from the rank on, and every reader's tensor map ends at row M: new memory needs no clear.
+// Hs / Gs are [M x 64] f16.  The low-rank chunk of the big matmul reads whole groups of 16 columns; whatever makes them (lowrank_tc_kernel,
+// the two lowrank_rows kernels, RMSNorm's forward and backward with a product) writes all 64 columns of every row, zeros from the
+// rank on, and every reader's tensor map ends at row M: new memory needs no clear.
 static __half* lowrank_buf(DevBuf& b, int M) {
   const size_t want = (size_t)M * 64 * sizeof(__half);
   return b.reserve(want <= b.bytes ? want : want + want / 2) ? b.as<__half>() : nullptr;
@@ -1420,7 +1421,7 @@ static uint64_t buffer_signature(rt_model* m) {
 }
 
 // The staged step replays as ONE CUDA graph once the same shape has run eagerly (the eager run
-// sizes every buffer and encodes every TMA descriptor; capture then records the step's launches, 1100
+// sizes every buffer and encodes every TMA descriptor; capture then records the step's launches, 983
 // for 28 layers, with no host work between them).  Which shapes are captured: graph_cache.h.
 static rt_status run_staged(rt_model* m, bool backward, float* logits_out_host) {
   rt_ctx* c = m->ctx;

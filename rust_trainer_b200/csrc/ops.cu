@@ -521,11 +521,15 @@ void launch_rmsnorm_bwd(const float* x, const float* w, const float* dn, const f
   RT_COUNT_LAUNCH(1);
 }
 
-// Up to so many rows: forward eight rows per CTA, beyond sixteen, which read the weights half as often; backward a CTA for every
-// eight rows with the weights from L2 (1024 rows of 1024, 16 rank indices, in a step 5.1 us; persistent 7.6, its row's registers
+// Up to so many rows: forward eight rows of a CTA at a time, beyond sixteen, which read the weights half as often (as many CTAs as
+// fit in either case, which loop where there are more groups: 1024 columns with 48 rank indices from 1185 rows on); backward a CTA
+// for every eight rows with the weights from L2 (1024 rows of 1024, 16 rank indices, in a step 5.1 us; persistent 7.6, its row's registers
 // no longer fit), beyond persistent ones (8192 rows 28 us, 33 the other way).
 constexpr int RMS_LR_WIDE = 2048;
-// The two with the product, for rows of 128..1024 floats.
+// The two with the product, for rows of 128..1024 floats and all that its 64 columns hold.  A 0.6B layer's forward and backward against
+// products of their own: 32 rank indices (stacks of 64) 349 us at 1024 tokens (351 with the forward's apart, 359 with the backward's), 459
+// (463, 466) at 2048, 644 (644, 651) at 4096, 1087 (1086, 1089) at 8192; 64 indices, which only the backward takes, 392 (403), 514 (520),
+// 700 (705), 1136 (1135); at 16384 tokens and with 256 or 512 columns the same picture.
 bool rmsnorm_takes_lowrank(int d, int r) { return d % 128 == 0 && d <= 1024 && r >= 1 && r <= 64; }
 template <class Kernel, class... A>
 static int launch_rms_lr(rt_ctx* c, Kernel* kernel, int rows, int nt, int ctas, int most_smem, int smem, A... a) {

@@ -19,7 +19,7 @@
 // Three pairs of kernels depart from both.  (1) A matmul behind a low-rank stream (QGemmArgs::late_wait) reads
 // weights, activations and residual without waiting and waits only where it loads the stream's result.  That
 // is sound because of what lowrank_tc_kernel and the matmul keep between them:
-//   - lowrank_tc_kernel (and lowrank_rows_kernel in its place) triggers only after its own wait, so that everything older than it is complete and
+//   - lowrank_tc_kernel (and the lowrank_rows kernels in its place) triggers only after its own wait, so that everything older than it is complete and
 //     visible once the matmul runs.  Moved to the kernel's entry, the trigger would make a race of this;
 //   - it writes nothing the matmul reads but that result, and the matmul writes nothing it reads;
 //   - at least one CTA of the matmul waits (the last piece of a contraction always ends in the low-rank

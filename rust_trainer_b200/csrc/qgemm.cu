@@ -470,18 +470,17 @@ qgemm_kernel(const __grid_constant__ CUtensorMap tm_act, const __grid_constant__
   };
   // The same block straight from registers to memory (lane = output feature, register j = token): f32
   // results, partial sums, and 16-bit outputs TMA cannot address.  A warp writes 128 contiguous
-  // bytes per token.  (f32 blocks used to go through two 4 KB staging buffers and TMA: the store of
+  // bytes per token, of a half tile's 64 rows 64.  (f32 blocks used to go through two 4 KB staging buffers and TMA: the store of
   // the block before last had to be read out first, and the 4096x1024 product at 8192 tokens
   // waited for its epilogue, 73 us; its stores knocked out it ran in 61.)
   // The epilogue warps share their schedulers with the unpack warps, so what counts is the number of
   // instructions per value: whole blocks take straight-line code without a test per value (with one,
   // the same product took 135 us).
-  // A residual is added before anything is stored, eight loads in flight.  In the ragged last block of a
-  // batch it used to be read value by value, each load behind the store before it, which it might have
-  // aliased: for 1 to 31 tokens a chain of as many round trips to L2.  Scoring 157 tokens 1780 -> 1724 us,
-  // accumulating over ragged batches 32.7 -> 31.4 ms; without a residual the test for one per value is
-  // gone, 24 tokens through a frozen [8192 x 3072] 47.4 -> 45.9 us.  Whole blocks are as fast as with a loop of their own (4 x 256 tokens 7.07-7.16 against 7.11 ms).
-  // Eight at a time: with four, or all 32 left to the compiler, 4 x 256 takes 7.20 and 7.16 ms.
+  // A residual is added before anything is stored, eight loads in flight, in whole and ragged blocks alike: a load behind a store
+  // that it might alias waits for it, in a last block of 1 to 31 tokens a chain of as many round trips to L2.  Value by value there
+  // scoring 157 tokens took 1780 us instead of 1724, accumulating over ragged batches 32.7 ms instead of 31.4, and, with a test per value
+  // for whether there is a residual, 24 tokens through a frozen [8192 x 3072] 47.4 us instead of 45.9 (one call after the other, with their host work).
+  // A loop of their own for whole blocks: 4 x 256 tokens 7.11 ms against 7.07-7.16; four values at a time, or all 32 left to the compiler, 7.20 and 7.16.
   auto direct_chunk = [&](int acc, int wq, int c, int r0, int m0, int split) {
     const int tok0 = m0 + q_tok(wq) + c * 32, row = r0 + q_row(wq) + lane;
     if (tok0 >= p.M) return;
