@@ -8,21 +8,12 @@
 #include "lowrank_rows.cuh"
 #include "ops.h"
 #include "pdl.cuh"
+#include "rmsnorm_row.cuh"
 #include <algorithm>
 
 namespace rt {
 
 // ------------------------------------------------------------------ reductions
-__device__ __forceinline__ float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -192,38 +183,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_fwd_row_kernel(const float* x, c
     *(uint2*)(y16 + r * d + 4 * i) = make_uint2(*(uint32_t*)&a, *(uint32_t*)&b);
   }
 }
-// Warp-per-row versions for rows of up to 1024 floats (a multiple of 128): the row lives in
-// registers, the reductions are warp shuffles, and eight rows per CTA keep far more bytes in
+// Warp-per-row versions for rows of up to 1024 floats (rmsnorm_row.cuh): eight rows per CTA keep far more bytes in
 // flight per SM than one small CTA per row.
-// A warp's row: lane l holds float4 l, l + 32, ..
-template <int NV>  // float4s per lane: d = 128 * NV
-__device__ __forceinline__ void rms_load_row(const float* row, int lane, float4* v) {
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = ((const float4*)row)[lane + 32 * k];
-}
-__device__ __forceinline__ uint2 half4(float4 v) {
-  __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
-  return make_uint2(*(uint32_t*)&a, *(uint32_t*)&b);
-}
-// The four products of a lane's float4, and a x - b y: fused by name, so that a row gets the same bits in every kernel it may run
-// through (a block's second forward takes the one without a product, and the backward's form goes by the number of rows).
-__device__ __forceinline__ float dot4(const float4& a, const float4& b) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.x, b.x, a.y * b.y))); }
-__device__ __forceinline__ float ax_by(float a, float x, float b, float y) { return fmaf(a, x, -(b * y)); }
-// put(k, four f16): what lane + 32 k of the result is
-template <int NV, class Put>
-__device__ __forceinline__ void rms_fwd_row(const float4* v, const float* __restrict__ w, float eps, int lane, Put put) {
-  float ss = 0.f;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) ss += dot4(v[k], v[k]);
-  ss = warp_sum(ss);
-  const float ir = 1.0f / sqrtf(ss / (float)(128 * NV) + eps);
-  const float4* w4 = (const float4*)w;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const float4 g = w4[lane + 32 * k];
-    put(k, half4(make_float4(v[k].x * ir * g.x, v[k].y * ir * g.y, v[k].z * ir * g.z, v[k].w * ir * g.w)));
-  }
-}
 template <int NV>
 __global__ void __launch_bounds__(256)
 rmsnorm_fwd_warp_kernel(const float* x, const float* __restrict__ w, int rows, float eps,
@@ -236,33 +197,6 @@ rmsnorm_fwd_warp_kernel(const float* x, const float* __restrict__ w, int rows, f
   float4 v[NV];
   rms_load_row<NV>(x + r * D, lane, v);
   rms_fwd_row<NV>(v, w, eps, lane, [&](int k, uint2 o) { *(uint2*)(y16 + r * D + 4 * (lane + 32 * k)) = o; });
-}
-// v becomes the row of `out`, its largest magnitude is returned (of the warp's row); g: the row of dn, r: of dres or zeros
-template <int NV>
-__device__ __forceinline__ float rms_bwd_row(const float4* xv, float4* gv, const float4* rv, const float* __restrict__ w, float eps, int lane) {
-  float ss = 0.f, gx = 0.f;
-  const float4* w4 = (const float4*)w;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const float4 wv = w4[lane + 32 * k];
-    gv[k] = make_float4(gv[k].x * wv.x, gv[k].y * wv.y, gv[k].z * wv.z, gv[k].w * wv.w);
-    ss += dot4(xv[k], xv[k]);
-    gx += dot4(gv[k], xv[k]);
-  }
-  ss = warp_sum(ss);
-  gx = warp_sum(gx);
-  const float ir = 1.0f / sqrtf(ss / (float)(128 * NV) + eps);
-  const float c = gx * ir * ir * ir / (float)(128 * NV);
-  float m = 0.f;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    float4 v = make_float4(ax_by(gv[k].x, ir, xv[k].x, c), ax_by(gv[k].y, ir, xv[k].y, c), ax_by(gv[k].z, ir, xv[k].z, c),
-                           ax_by(gv[k].w, ir, xv[k].w, c));
-    v.x += rv[k].x; v.y += rv[k].y; v.z += rv[k].z; v.w += rv[k].w;
-    gv[k] = v;
-    m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-  }
-  return m;
 }
 template <int NV>
 __global__ void __launch_bounds__(256)
@@ -295,100 +229,6 @@ rmsnorm_bwd_warp_kernel(const float* x, const float* __restrict__ w, const float
   }
 }
 
-// Both with the low-rank product of their 16-bit rows (lowrank_rows.cuh): persistent CTAs of NT groups of eight warps that
-// keep the product's weights in shared memory, a warp per row; the rows' f16 copies go into shared memory as well as to where they belong.
-// Bound: the chain of launches at 1024 rows (forward 3.8 us + 5 for a low-rank launch of its own -> 4.3; backward 6.2 + 4.8 ->
-// 5.1, and the matmul behind it finds all SMs free), DRAM at 8192 (forward with 48 rank indices 17.2 -> 15.3 us, backward 29.1 -> 28.1;
-// with the weights read from L2 by every eight rows 21.5 and 33).
-template <int NV, int MT, int NT>
-struct RmsLr {
-  static constexpr int D = 128 * NV, PITCH = lr_row_pitch(D);  // of weights and rows
-  static constexpr int TILE = NT * LR_TOKENS * PITCH, SUMS = NT * lr_sum_floats(LR_SLICES, MT) * 4;
-  static constexpr int bytes(int r) { return TILE + SUMS + r * PITCH; }
-  static constexpr int ctas(int most) {  // of an SM
-    const int fit = SMEM_PER_SM / (bytes(16 * MT) + 1024);
-    return fit < most ? fit : most;
-  }
-  static constexpr int FWD_CTAS = ctas(4 / NT), BWD_CTAS = ctas(2);
-};
-template <int NV, int MT, int NT>
-__global__ void __launch_bounds__(256 * NT, (RmsLr<NV, MT, NT>::FWD_CTAS))
-rmsnorm_fwd_lr_kernel(const float* x, const float* __restrict__ w, int rows, float eps, __half* __restrict__ y16,
-                      const LowRank lr) {
-  using C = RmsLr<NV, MT, NT>;
-  extern __shared__ __align__(16) uint8_t lr_smem[];
-  uint8_t* tile = lr_smem;
-  float* sums = (float*)(lr_smem + C::TILE);
-  uint8_t* weights = lr_smem + C::TILE + C::SUMS;
-  pdl_launch_dependents();
-  lr_prefetch(lr.w, lr.r, C::D);
-  pdl_wait();
-  lr_fetch_weights(lr.w, lr.r, C::D, weights, C::PITCH);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int step = (int)gridDim.x * 8 * NT;
-  float4 v[NV];
-  int r = (int)blockIdx.x * 8 * NT + warp;
-  if (r < rows) rms_load_row<NV>(x + (size_t)r * C::D, lane, v);
-  for (; r - warp < rows; r += step) {
-    uint8_t* t = tile + warp * C::PITCH + 8 * lane;
-    if (r < rows)
-      rms_fwd_row<NV>(v, w, eps, lane, [&](int k, uint2 o) {
-        *(uint2*)(y16 + (size_t)r * C::D + 4 * (lane + 32 * k)) = o;
-        *(uint2*)(t + 256 * k) = o;
-      });
-    if (r + step < rows) rms_load_row<NV>(x + (size_t)(r + step) * C::D, lane, v);  // the next rows, under this one's product
-    cp_async_wait<0>();
-    __syncthreads();
-    lr_of_rows<MT, NT, C::D, true>(lr, tile, weights, {}, C::PITCH, sums, warp, lane, r - warp, rows);
-  }
-}
-template <int NV, int MT, bool SHARED>
-__global__ void __launch_bounds__(256, (SHARED ? RmsLr<NV, MT, 1>::BWD_CTAS : 1))
-rmsnorm_bwd_lr_kernel(const float* x, const float* __restrict__ w, const float* dn, const float* dres, int rows,
-                      float eps, float* out, __half* __restrict__ out16, float* __restrict__ scale, const LowRank lr) {
-  using C = RmsLr<NV, MT, 1>;
-  extern __shared__ __align__(16) uint8_t lr_smem[];
-  uint8_t* tile = lr_smem;
-  float* sums = (float*)(lr_smem + C::TILE);
-  uint8_t* weights = lr_smem + C::TILE + C::SUMS;
-  pdl_launch_dependents();
-  lr_prefetch(lr.w, lr.r, C::D);
-  pdl_wait();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  LrWeights<MT> first = {};
-  if (SHARED) lr_fetch_weights(lr.w, lr.r, C::D, weights, C::PITCH);
-  else if (warp * 32 < C::D) first.load(lr.w, lr.r, C::D, warp * 32, lane);
-  const int step = (int)gridDim.x * 8;
-  for (int r = (int)blockIdx.x * 8 + warp; r - warp < rows; r += step) {
-    uint8_t* t = tile + warp * C::PITCH + 8 * lane;
-    if (r < rows) {
-      const size_t at = (size_t)r * C::D;
-      float4 xv[NV], gv[NV], rv[NV];
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        xv[k] = ((const float4*)(x + at))[lane + 32 * k];
-        gv[k] = ((const float4*)(dn + at))[lane + 32 * k];
-        rv[k] = dres ? ((const float4*)(dres + at))[lane + 32 * k] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      float m = rms_bwd_row<NV>(xv, gv, rv, w, eps, lane);
-#pragma unroll
-      for (int k = 0; k < NV; ++k) ((float4*)(out + at))[lane + 32 * k] = gv[k];
-      m = warp_max(m);
-      const float sc = m > 0.f ? m : 1.f, inv = 1.f / sc;
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        const uint2 o = half4(make_float4(gv[k].x * inv, gv[k].y * inv, gv[k].z * inv, gv[k].w * inv));
-        *(uint2*)(out16 + at + 4 * (lane + 32 * k)) = o;
-        *(uint2*)(t + 256 * k) = o;
-      }
-      if (lane == 0) scale[r] = m;
-    }
-    if (SHARED) cp_async_wait<0>();
-    __syncthreads();
-    lr_of_rows<MT, 1, C::D, SHARED>(lr, tile, weights, first, C::PITCH, sums, warp, lane, r - warp, rows);
-    if (!SHARED) break;  // a CTA for every eight rows
-  }
-}
 void launch_rmsnorm_fwd(const float* x, const float* w, int rows, int d, float eps, __half* y16, cudaStream_t st) {
   if (rows <= 0) return;
   const int nv = d / 128, grid = (rows + 7) / 8;
@@ -519,68 +359,6 @@ void launch_rmsnorm_bwd(const float* x, const float* w, const float* dn, const f
     rmsnorm_bwd_kernel<<<rows, 256, 0, st>>>(x, w, dn, dres, d, eps, out, out16, scale);
   }
   RT_COUNT_LAUNCH(1);
-}
-
-// Up to so many rows: forward eight rows of a CTA at a time, beyond sixteen, which read the weights half as often (as many CTAs as
-// fit in either case, which loop where there are more groups: 1024 columns with 48 rank indices from 1185 rows on); backward a CTA
-// for every eight rows with the weights from L2 (1024 rows of 1024, 16 rank indices, in a step 5.1 us; persistent 7.6, its row's registers
-// no longer fit), beyond persistent ones (8192 rows 28 us, 33 the other way).
-constexpr int RMS_LR_WIDE = 2048;
-// The two with the product, for rows of 128..1024 floats and all that its 64 columns hold.  A 0.6B layer's forward and backward against
-// products of their own: 32 rank indices (stacks of 64) 349 us at 1024 tokens (351 with the forward's apart, 359 with the backward's), 459
-// (463, 466) at 2048, 644 (644, 651) at 4096, 1087 (1086, 1089) at 8192; 64 indices, which only the backward takes, 392 (403), 514 (520),
-// 700 (705), 1136 (1135); at 16384 tokens and with 256 or 512 columns the same picture.
-bool rmsnorm_takes_lowrank(int d, int r) { return d % 128 == 0 && d <= 1024 && r >= 1 && r <= 64; }
-template <class Kernel, class... A>
-static int launch_rms_lr(rt_ctx* c, Kernel* kernel, int rows, int nt, int ctas, int most_smem, int smem, A... a) {
-  if (!c->raise_smem(kernel, most_smem)) return 3;
-  const int groups = (rows + 8 * nt - 1) / (8 * nt);
-  if (pdl(kernel, ctas ? std::min(groups, ctas * c->num_sms) : groups, 256 * nt, smem, c->stream)(a...) != cudaSuccess) return 3;
-  RT_COUNT_LAUNCH(1);
-  return 0;
-}
-template <int NV, int MT>
-static int rmsnorm_fwd_lr(rt_ctx* c, const float* x, const float* w, int rows, float eps, __half* y16, const LowRank& lr) {
-  using A = RmsLr<NV, MT, 1>;
-  using B = RmsLr<NV, MT, 2>;
-  if (rows <= RMS_LR_WIDE) return launch_rms_lr(c, rmsnorm_fwd_lr_kernel<NV, MT, 1>, rows, 1, A::FWD_CTAS, A::bytes(16 * MT), A::bytes(lr.r), x, w, rows, eps, y16, lr);
-  return launch_rms_lr(c, rmsnorm_fwd_lr_kernel<NV, MT, 2>, rows, 2, B::FWD_CTAS, B::bytes(16 * MT), B::bytes(lr.r), x, w, rows, eps, y16, lr);
-}
-#define RT_LR_MT(F, NV, ...)                          \
-  switch ((lr.r + 15) / 16) {                         \
-    case 1: return F<NV, 1>(__VA_ARGS__);             \
-    case 2: return F<NV, 2>(__VA_ARGS__);             \
-    case 3: return F<NV, 3>(__VA_ARGS__);             \
-    default: return F<NV, 4>(__VA_ARGS__);            \
-  }
-#define RT_LR_NV(F, ...)                              \
-  switch (d / 128) {                                  \
-    case 1: RT_LR_MT(F, 1, __VA_ARGS__)               \
-    case 2: RT_LR_MT(F, 2, __VA_ARGS__)               \
-    case 3: RT_LR_MT(F, 3, __VA_ARGS__)               \
-    case 4: RT_LR_MT(F, 4, __VA_ARGS__)               \
-    case 5: RT_LR_MT(F, 5, __VA_ARGS__)               \
-    case 6: RT_LR_MT(F, 6, __VA_ARGS__)               \
-    case 7: RT_LR_MT(F, 7, __VA_ARGS__)               \
-    default: RT_LR_MT(F, 8, __VA_ARGS__)              \
-  }
-int launch_rmsnorm_fwd_lr(rt_ctx* c, const float* x, const float* w, int rows, int d, float eps, __half* y16, const LowRank& lr) {
-  if (rows <= 0) return 0;
-  if (!rmsnorm_takes_lowrank(d, lr.r)) return 3;
-  RT_LR_NV(rmsnorm_fwd_lr, c, x, w, rows, eps, y16, lr)
-}
-template <int NV, int MT>
-static int rmsnorm_bwd_lr(rt_ctx* c, const float* x, const float* w, const float* dn, const float* dres, int rows, float eps, float* out,
-                          __half* out16, float* scale, const LowRank& lr) {
-  using C = RmsLr<NV, MT, 1>;
-  if (rows <= RMS_LR_WIDE) return launch_rms_lr(c, rmsnorm_bwd_lr_kernel<NV, MT, false>, rows, 1, 0, C::bytes(0), C::bytes(0), x, w, dn, dres, rows, eps, out, out16, scale, lr);
-  return launch_rms_lr(c, rmsnorm_bwd_lr_kernel<NV, MT, true>, rows, 1, C::BWD_CTAS, C::bytes(16 * MT), C::bytes(lr.r), x, w, dn, dres, rows, eps, out, out16, scale, lr);
-}
-int launch_rmsnorm_bwd_lr(rt_ctx* c, const float* x, const float* w, const float* dn, const float* dres, int rows, int d, float eps,
-                          float* out, __half* out16, float* scale, const LowRank& lr) {
-  if (rows <= 0) return 0;
-  if (!rmsnorm_takes_lowrank(d, lr.r)) return 3;
-  RT_LR_NV(rmsnorm_bwd_lr, c, x, w, dn, dres, rows, eps, out, out16, scale, lr)
 }
 
 // ------------------------------------------------------------------ RoPE tables (reference src/ops.rs:118-154)

@@ -114,3 +114,8 @@ def test_only_prefetches_come_before_the_wait(name):
     assert re.sub(allowed, "", before).strip() == ""
     prefetch = re.search(r"void lr_prefetch\([^{]*\{(.*?)\n\}", (CSRC / "lowrank_rows.cuh").read_text(), re.S)[1]
     assert "prefetch.global.L2" in prefetch and "ld." not in prefetch and "*(" not in prefetch
+
+
+def test_row_kernels_with_a_product_are_not_loaded_with_the_others():
+    """CUDA loads a file's kernels with the first that is launched, and these are 128 instantiations."""
+    assert "_lr_kernel" not in (CSRC / "ops.cu").read_text() and "rmsnorm_fwd_lr_kernel" in kernels()
