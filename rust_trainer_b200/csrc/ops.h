@@ -1,4 +1,4 @@
-// Launchers of the memory-bound device ops (ops.cu) and attention (attention.cu).
+// Launchers of the memory-bound device ops (ops.cu, rmsnorm_lr.cu) and attention (attention_tc.cu).
 #pragma once
 #include "lowrank_rows.cuh"
 #include <cuda_fp16.h>
