@@ -505,6 +505,12 @@ __device__ __forceinline__ void load_epl(const float* p, float* v) {
   if (EPL == 4) { const float4 t = *(const float4*)p; v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
   else { const float2 t = *(const float2*)p; v[0] = t.x; v[1] = t.y; }
 }
+// What is read once and not again, past L1.  (Volatile: it stays behind a wait, through whatever pointer.)
+template <int EPL>
+__device__ __forceinline__ void load_epl_once(const float* p, float* v) {
+  if constexpr (EPL == 4) asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+  else asm volatile("ld.global.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v[0]), "=f"(v[1]) : "l"(p));
+}
 template <int EPL>
 __device__ __forceinline__ void store_epl_h(__half* p, const float* v) {
   if (EPL == 4) {
@@ -579,7 +585,9 @@ qk_rope_fwd_fast_kernel(const float* q_raw, const float* k_raw, const float* v_r
                         size_t pq, size_t pk, size_t pv, const float* __restrict__ qw, const float* __restrict__ kw,
                         const int* __restrict__ pos, const float* __restrict__ cs, const float* __restrict__ sn, float eps,
                         __half* __restrict__ q16, __half* __restrict__ k16, __half* __restrict__ v16) {
-  pdl_entry();
+  pdl_launch_dependents();
+  const int p = pos[blockIdx.x];  // the batch's: the tables' rows are read with the wait over, not behind this too
+  pdl_wait();
   constexpr int HD = 32 * EPL, HALF = HD / 2, NH = 8 * QPW, NKV = 8 * KPW;
   const size_t m = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -589,18 +597,16 @@ qk_rope_fwd_fast_kernel(const float* q_raw, const float* k_raw, const float* v_r
   const float* vs = v_raw + m * pv + warp * HD + e0;
   float xq[QPW][EPL], xk[KPW][EPL], xv[KPW][EPL];
 #pragma unroll
-  for (int t = 0; t < QPW; ++t) load_epl<EPL>(qs + t * 8 * HD, xq[t]);
+  for (int t = 0; t < QPW; ++t) load_epl_once<EPL>(qs + t * 8 * HD, xq[t]);
 #pragma unroll
-  for (int t = 0; t < KPW; ++t) load_epl<EPL>(ks + t * 8 * HD, xk[t]);
+  for (int t = 0; t < KPW; ++t) load_epl_once<EPL>(ks + t * 8 * HD, xk[t]);
 #pragma unroll
-  for (int t = 0; t < KPW; ++t) load_epl<EPL>(vs + t * 8 * HD, xv[t]);
+  for (int t = 0; t < KPW; ++t) load_epl_once<EPL>(vs + t * 8 * HD, xv[t]);
   float wq[EPL], wk[EPL];
   if (NORM) {
     load_epl<EPL>(qw + e0, wq);
     load_epl<EPL>(kw + e0, wk);
   }
-  // the position -> cos/sin chain (two dependent loads) runs under the row loads
-  const int p = pos[m];
   const float* csr = cs + (size_t)p * HALF;
   const float* snr = sn + (size_t)p * HALF;
   float c[EPL], sg[EPL];
@@ -751,7 +757,9 @@ qk_rope_bwd_fast_kernel(const float* dq, const float* dk, const float* dv,
                         const int* __restrict__ pos, const float* __restrict__ cs, const float* __restrict__ sn, float eps,
                         __half* __restrict__ dq16, __half* __restrict__ dk16, __half* __restrict__ dv16,
                         float* __restrict__ sq, float* __restrict__ sk, float* __restrict__ sv) {
-  pdl_entry();
+  pdl_launch_dependents();
+  const int p = pos[blockIdx.x];  // the batch's: the tables' rows are read with the wait over, not behind this too
+  pdl_wait();
   constexpr int HD = 32 * EPL, HALF = HD / 2, NH = 8 * QPW, NKV = 8 * KPW;
   __shared__ float wmax[3][8];
   const size_t m = blockIdx.x;
@@ -774,7 +782,6 @@ qk_rope_bwd_fast_kernel(const float* dq, const float* dk, const float* dv,
     load_epl<EPL>(qw + e0, wq);
     load_epl<EPL>(kw + e0, wk);
   }
-  const int p = pos[m];
   const float* csr = cs + (size_t)p * HALF;
   const float* snr = sn + (size_t)p * HALF;
   float c[EPL], sg[EPL];  // sin signed for the FORWARD rotation; the inverse subtracts
